@@ -137,6 +137,13 @@ struct PrecD
 		return make_double2(__longlong_as_double(__double_as_longlong(a.x) ^ m), __longlong_as_double(__double_as_longlong(a.y) ^ m));
 	}
 	__device__ static T mul(T a, T x) { return make_double2(fma(a.x, x.x, -a.y * x.y), fma(a.x, x.y, a.y * x.x)); }
+	// x + p y for a real p (the real part of p) and x + q y for a complex q
+	__device__ static T axpy(T x, T p, T y) { return make_double2(fma(p.x, y.x, x.x), fma(p.x, y.y, x.y)); }
+	__device__ static T axpyc(T x, T q, T y)
+	{
+		return make_double2(fma(q.x, y.x, fma(-q.y, y.y, x.x)), fma(q.x, y.y, fma(q.y, y.x, x.y)));
+	}
+	__device__ static void acc_norm(Acc&) {}
 	// a x + b y for entries that are real or imaginary: a = (c_re, c_im) with c_re, c_im the
 	// coefficients of the (possibly swapped) components of x; swap when the entry is imaginary
 	__device__ static T madd2_ri(T a, bool ra, T x, T b, bool rb, T y)
@@ -197,6 +204,18 @@ struct PrecF
 		return make_float2(__uint_as_float(__float_as_uint(a.x) ^ m), __uint_as_float(__float_as_uint(a.y) ^ m));
 	}
 	__device__ static T mul(T a, T x) { return make_float2(fmaf(a.x, x.x, -a.y * x.y), fmaf(a.x, x.y, a.y * x.x)); }
+	__device__ static T axpy(T x, T p, T y) { return make_float2(fmaf(p.x, y.x, x.x), fmaf(p.x, y.y, x.y)); }
+	__device__ static T axpyc(T x, T q, T y)
+	{
+		return make_float2(fmaf(q.x, y.x, fmaf(-q.y, y.y, x.x)), fmaf(q.x, y.y, fmaf(q.y, y.x, x.y)));
+	}
+	// (hi, lo) renormalised
+	__device__ static void acc_norm(Acc& s)
+	{
+		float a, b;
+		fast_two_sum(s.rh, s.rl, a, b); s.rh = a; s.rl = b;
+		fast_two_sum(s.ih, s.il, a, b); s.ih = a; s.il = b;
+	}
 	__device__ static T madd2_ri(T a, bool ra, T x, T b, bool rb, T y)
 	{
 		const float xr = ra ? x.y : x.x, xi = ra ? x.x : x.y, yr = rb ? y.y : y.x, yi = rb ? y.x : y.y;
@@ -280,6 +299,22 @@ struct PrecX
 		return make_float4(__uint_as_float(__float_as_uint(a.x) ^ m), __uint_as_float(__float_as_uint(a.y) ^ m),
 			__uint_as_float(__float_as_uint(a.z) ^ m), __uint_as_float(__float_as_uint(a.w) ^ m));
 	}
+	// x + p y (p real) and x + q y: the products added to x by compensated sums
+	__device__ static T axpy(T x, T p, T y)
+	{
+		ff_acc_prod(x.x, x.z, p.x, p.z, y.x, y.z);
+		ff_acc_prod(x.y, x.w, p.x, p.z, y.y, y.w);
+		return x;
+	}
+	__device__ static T axpyc(T x, T q, T y)
+	{
+		ff_acc_prod(x.x, x.z, q.x, q.z, y.x, y.z);
+		ff_acc_prod(x.x, x.z, -q.y, -q.w, y.y, y.w);
+		ff_acc_prod(x.y, x.w, q.x, q.z, y.y, y.w);
+		ff_acc_prod(x.y, x.w, q.y, q.w, y.x, y.z);
+		return x;
+	}
+	__device__ static void acc_norm(Acc& s) { PrecF::acc_norm(s); }
 	// a x as two 2-term compensated dot products
 	__device__ static T mul(T a, T x)
 	{

@@ -1725,6 +1725,8 @@ __global__ void __launch_bounds__(256, 2) k_hessian(Args<P> a, long nitems)
 	}
 }
 
+#include "mgcu_fit.cuh"
+
 // ------------------------------------------------------------------------------------
 // small kernels: staging, reductions, symmetrisation
 // ------------------------------------------------------------------------------------
@@ -2365,6 +2367,8 @@ extern "C" int mgcu_target_apply(mgcu_target* t, const mgc* psi, mgc* out)
 // ======================================================================================
 // plans
 // ======================================================================================
+#include "mgcu_fit_build.cuh"
+
 struct mgcu_plan
 {
 	mgcu_plan_desc d;
@@ -2393,6 +2397,7 @@ struct mgcu_plan
 	DevBuf d_pass, d_gate, d_mats, d_pass_of, d_block, d_place, d_placew;
 	bool adj = false;              // gradient plan: checkpointed backward sweep (k_columns_adj)
 	bool hgroup = false;           // Hessian plan: one item per (column, block, entry), see k_hessian
+	FitProg fit;                   // the factored fitted circuit (k_fit)
 	bool adj_ok = false;           // the current gates are invertible (else the cached sweep)
 	DevBuf d_mats_inv, ck;
 	DevBuf su, sw, sh, cache, dcache, part_f, part_g, part_h, cols64, cols;
@@ -2534,6 +2539,32 @@ static int launch_columns(mgcu_plan* p, long b0, long b1, const typename P::T* d
 	if (!a.want_grad) a.cache = nullptr;
 	const long ncols = b1 - b0;
 	const int grid = (int)std::min<long>(p->grid_a, ncols);
+	if constexpr (P::kId != MG_PREC_FP32_ID)
+	if (p->fit.ok)
+	{
+		const FitProg& f = p->fit;
+		FitArgs<P> w;
+		w.L = p->L; w.nb = p->nb; w.kt = f.kt; w.npass = (int)f.sched.pass.size(); w.ngroups = (int)f.group.size(); w.nc = f.nc;
+		w.S = p->S;
+		w.pass = f.d_pass.as<PassRec>(); w.groups_of = f.d_pgroups.as<FitPass>(); w.groups = f.d_group.as<FitGroup>();
+		w.bases = f.d_bases.as<unsigned>();
+		w.gates = f.d_gates.as<FitGate<T>>(); w.tables = f.d_tab.as<T>(); w.final = w.tables + (size_t)2 * p->S * f.nflush;
+		w.dense = dense; w.dense_b0 = dense_b0; w.b0 = b0; w.b1 = b1;
+		w.su = p->su.as<T>(); w.sw = p->sw.as<T>(); w.cache = f.cache.as<T>();
+		w.part = p->d.want_grad ? p->part_g.as<double>() : p->part_f.as<double>();
+		w.nblocks = p->d.nblocks;
+		const int gf = (int)std::min<long>(f.grid, (ncols + f.nc - 1) / f.nc);
+		fit_kernel<P>(f.qc, p->d.want_grad != 0, f.threads)<<<gf, f.threads, f.smem, mgcu_stream()>>>(w);
+		MGCU_LAUNCHED();
+		return 0;
+	}
+	if (p->fit.built && !p->d.want_hess && p->d.want_grad)
+	{
+		// gates that do not factor: the cached sweep, its cache allocated on first need
+		const int e = p->cache.alloc((size_t)p->S * p->tsize * std::max(p->d.ngates, 1) * p->grid_a);
+		if (e) return e;
+		a.cache = p->cache.as<T>();
+	}
 	if (p->adj && p->adj_ok)
 	{
 		a.wmi = p->d_mats_inv.as<T>();
@@ -2575,6 +2606,9 @@ static int set_smem_attr()
 	for (auto k : tk) MGCU_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min<size_t>(c->smem_optin, 227 * 1024)));
 	void (*const wk[2])(Args<P>) = { k_target_w<P, 128, 2>, k_target_w<P, 256, 1> };
 	for (auto k : wk) MGCU_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min<size_t>(c->smem_optin, 227 * 1024)));
+	if constexpr (P::kId != MG_PREC_FP32_ID)
+	for (int q = 0; q < 12; q++)
+		MGCU_TRY(cudaFuncSetAttribute(fit_kernel<P>(q & 1, q & 2, 128 << (q >> 2)), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min<size_t>(c->smem_optin, 227 * 1024) - 4096));
 	MGCU_TRY(cudaFuncSetAttribute(k_hessian<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min<size_t>(c->smem_optin, 227 * 1024)));
 	return 0;
 }
@@ -2852,18 +2886,51 @@ extern "C" mgcu_plan* mgcu_plan_create(const mgcu_plan_desc* d)
 	if (opt_chunk > 0) chunk = std::min(chunk, opt_chunk);
 	p->chunk = chunk;
 
+	// the factored fitted circuit: gradients from L = 10 (whole evaluation, 5 layers: float-float
+	// 244 against 448 us, complex128 574 against 997 us; at L = 8 138 against 129 us and 263
+	// against 202 us, the tables and the few blocks cost more), f alone from L = 12 (L = 11: 318
+	// against 336 us), while the tables are small.  FP32 keeps the general kernels: there the
+	// factors' rounding is as large as the sweep's.  An explicit block size keeps them too
+	e = 0;
+	if (!d->want_hess && !p->adj && d->ngates > 0 && d->L <= 18 && opt_thr <= 0 && p->prec != MG_PREC_FP32_ID
+		&& d->L >= (d->want_grad ? 10 : 12))
+	{
+		p->fit.kt = p->kt;
+		// a sector of at most 128 KB is one tile (float-float L=14, 9 layers: 73 ms on 512 threads
+		// against 87 ms in two 64 KB tiles), a larger one tiles of 64 KB (L=16, 5 layers, 6001
+		// columns: 81 ms against 87 ms in tiles of 128 KB, one block per SM)
+		if (opt_kt <= 0 && p->nb <= 13) p->fit.kt = p->nb;
+		e = fit_build(p->L, p->fit.kt, p->wires.data(), d->ngates, p->block.data(), d->nblocks, (int)p->tsize, p->fit);
+		int per = 0;
+		if (!e)
+		{
+			auto occ = [&](auto k) { return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, p->fit.threads, p->fit.smem) != cudaSuccess; };
+			const bool g = d->want_grad != 0;
+			if (p->prec == MG_PREC_FP64_ID ? occ(fit_kernel<PrecD>(true, g, p->fit.threads)) : occ(fit_kernel<PrecX>(true, g, p->fit.threads)))
+				e = MG_ERR_DEVICE;
+		}
+		if (e) { delete p; return nullptr; }
+		if (opt_cps > 0) per = (int)std::min<long>(per, opt_cps);
+		const size_t slot = (size_t)p->fit.group.size() * p->fit.nc * col_bytes;
+		long gf = std::min((long)c->nsm * std::max(per, 1), (ncols_total + p->fit.nc - 1) / p->fit.nc);
+		if (d->want_grad) gf = std::max(1L, std::min(gf, (long)((32ull << 30) / slot)));
+		p->fit.grid = (int)gf;
+		if (d->want_grad) e = p->fit.cache.alloc(slot * gf);
+		if (e) { delete p; return nullptr; }
+	}
+	const long rows = std::max<long>(grid, p->fit.grid);
+
 	// device buffers
 	const int mdim = 8 * std::max(d->nblocks, 1);
-	e = 0;
 	if (!e) e = upload_sched(p->ws, p->d_pass, p->d_gate);
-	if (!e) e = p->su.alloc(col_bytes * grid);
-	if (!e) e = p->sw.alloc(col_bytes * grid);
-	if (!e && grad && !p->adj) e = p->cache.alloc(col_bytes * ng * (d->want_hess ? chunk : grid));
+	if (!e) e = p->su.alloc(col_bytes * rows);
+	if (!e) e = p->sw.alloc(col_bytes * rows);
+	if (!e && grad && !p->adj && !p->fit.built) e = p->cache.alloc(col_bytes * ng * (d->want_hess ? chunk : grid));
 	if (!e && p->adj) e = p->ck.alloc(col_bytes * p->ws.pass.size() * grid);
 	if (!e && d->want_hess) e = p->dcache.alloc(col_bytes * ng * chunk);
 	if (!e && d->want_hess) e = p->sh.alloc(col_bytes * p->grid_b);
-	if (!e) e = p->part_f.alloc(sizeof(double) * 2 * grid);
-	if (!e) e = p->part_g.alloc(sizeof(double) * 16 * ng * grid);
+	if (!e) e = p->part_f.alloc(sizeof(double) * 2 * rows);
+	if (!e) e = p->part_g.alloc(sizeof(double) * 16 * ng * rows);
 	if (!e && d->want_hess) e = p->part_h.alloc(sizeof(double) * 2 * (size_t)mdim * mdim * p->grid_b);
 	if (!e) e = p->out_f.alloc(sizeof(double) * 2);
 	if (!e) e = p->out_g.alloc(sizeof(double) * 16 * ng);
@@ -2899,6 +2966,12 @@ extern "C" int mgcu_plan_set_gates(mgcu_plan* p, const mgg* gates)
 	if (p->prec == MG_PREC_FP64_ID) e = upload_mats<PrecD>(gates, p->d.ngates, p->d_mats);
 	else if (p->prec == MG_PREC_FP32_ID) e = upload_mats<PrecF>(gates, p->d.ngates, p->d_mats);
 	else e = upload_mats<PrecX>(gates, p->d.ngates, p->d_mats);
+	if (!e && p->fit.built)
+	{
+		const mgcu_plan_desc& d = p->d;
+		if (p->prec == MG_PREC_FP64_ID) e = fit_set_gates<PrecD>(gates, d.ngates, d.block, d.nblocks, p->L, p->fit.kt, d.wires, p->fit);
+		else e = fit_set_gates<PrecX>(gates, d.ngates, d.block, d.nblocks, p->L, p->fit.kt, d.wires, p->fit);
+	}
 	if (e || !p->adj) return e;
 	if (p->prec == MG_PREC_FP32_ID) return upload_inverses<PrecF>(gates, p->d.ngates, p->d_mats_inv, p->adj_ok);
 	return upload_inverses<PrecX>(gates, p->d.ngates, p->d_mats_inv, p->adj_ok);
@@ -2978,7 +3051,14 @@ extern "C" int mgcu_plan_finish(mgcu_plan* p)
 	MgcuContext* c = mgcu_ctx();
 	cudaStream_t st = mgcu_stream();
 	const int ng = std::max(p->d.ngates, 1);
-	k_sum_parts<<<1, 32, 0, st>>>(p->part_f.as<double>(), p->grid_a, 2, p->out_f.as<double>());
+	if (p->fit.ok && p->d.want_grad)
+	{
+		k_fit_finish<<<p->d.nblocks, 128, 0, st>>>(p->part_g.as<double>(), p->fit.grid, p->d.nblocks, p->fit.d_blk.as<FitBlock>(),
+			p->out_f.as<double>(), p->out_blk.as<double>());
+		MGCU_LAUNCHED();
+		return 0;
+	}
+	k_sum_parts<<<1, 32, 0, st>>>(p->part_f.as<double>(), p->fit.ok ? p->fit.grid : p->grid_a, 2, p->out_f.as<double>());
 	MGCU_LAUNCHED();
 	if (p->d.want_grad || p->d.want_hess)
 	{

@@ -1,0 +1,602 @@
+// Fitted circuit in factored form (k_fit): f and block gradients of the columns whose
+// -conj(U e_b) are given.  Included by mgcu_engine.cu inside its anonymous namespace.
+//
+// Each 2x2 block is factored as diag(l0, l1) M diag(1, r1) with M = [[1, p], [q, 1]] or, when
+// the off-diagonal entries dominate, [[p, 1], [1, q]]: p is real, and q is real too for unitary
+// blocks (up to rounding, which q keeps in complex128).  M takes one real multiply-add per real
+// number instead of four, and the diagonal factors of all gates between two uses of a wire are
+// merged into one table with an entry per amplitude (a "flush": one complex multiply per
+// amplitude and brickwall layer).  Per gate and amplitude that is 24 FP32 operations in
+// float-float (80 unfactored) or 3 FP64 operations (8).
+//
+// Gates are applied in groups of up to two with disjoint wires: a thread owns the 16
+// amplitudes ("registers" 0..15) of the group's four tile bits, so there is one barrier and one
+// cached state per two gates, and the cache is stored in the order in which the threads own the
+// amplitudes.  A gate on the dropped qubit pairs along one tile bit, corner or center by the
+// parity of the rest; it takes a fourth, free bit by which each thread relabels its amplitudes
+// so that register 0 has even parity.
+//
+// Gradients: with Y the state and E the derivative after a gate's M, R[r][u] = sum E_r Y_u over
+// all columns determines the gradient of the gate: dG[r][t] = sum_u R[r][u] Minv[t][u] /
+// (l_r r_t), applied once at the end (k_fit_finish).  R of all gates of a parameter block are
+// summed, and f is the trace of R.
+//
+// Bound: issue (58 %) and the latency of the cached states in float-float, the FP64 pipe in
+// complex128.  Measured against k_columns (which stays for FP32, small sectors, Hessian caches
+// and gates that do not factor): float-float L=12, 7 layers 5.17 -> 2.88 ms; L=14, 9 layers
+// 122 -> 73 ms; L=16, 5 layers, 6001 columns 119 -> 81 ms; complex128 L=12, 5 layers
+// 12.2 -> 6.4 ms.
+
+constexpr int FIT_RENORM = 64;     // quartets per thread between renormalisations of the sums
+
+// register bits 0, 1: wires j, i of gate a; bits 2, 3: wires j, i of gate b (kind_b 1), or bit 2:
+// the compact wire of a gate on the dropped qubit and bit 3 free (kind_b 2)
+struct FitGroup
+{
+	unsigned m[4];        // byte offsets (swizzled) of the register bits
+	int cbit[14];         // compact bits: register bits 0..3, then the unit-index bits
+	int ga, gb, kind_b;   // gates (-1: none)
+	int rev;              // gate b is on the dropped qubit as wire i: its center pair is (z, y)
+	int blk_a, blk_b;
+	int blk_next;         // block of the first sum of the group before (gate b's, if it has one)
+	int flush;            // table multiplied in before the gates (-1: none)
+	int pass;
+	// per gate (a, b) and quartet: registers of |00>, |01>, |10>, |11> as byte offsets in the
+	// tile (swizzled, XOR) and in a unit's cached state
+	uint4 qs[2][4], qy[2][4];
+};
+
+template <class T> struct FitGate { T pc, qc, pk, qk; int swc, swk, pad[2]; };
+
+struct FitPass { int gbeg, gend; };
+
+// a group's record and gates in shared memory, copied asynchronously one group ahead
+template <class T> struct __align__(16) FitStage { FitGroup g; FitGate<T> gate[2]; };
+
+template <class T>
+__device__ __forceinline__ void fit_stage(FitStage<T>& d, const FitGroup* __restrict__ g, const FitGate<T>* __restrict__ gates)
+{
+	constexpr unsigned NG = sizeof(FitGroup) / 16, NT = 2 * sizeof(FitGate<T>) / 16;
+	const unsigned i = threadIdx.x;
+	if (i < NG + NT)
+	{
+		const char* src = i < NG ? reinterpret_cast<const char*>(g) + 16 * i : reinterpret_cast<const char*>(gates) + 16 * (i - NG);
+		const unsigned dst = smem_u32(&d) + 16 * i;
+		asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
+	}
+}
+__device__ __forceinline__ void fit_stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <class P>
+struct FitArgs
+{
+	typedef typename P::T T;
+	int L, nb, kt, npass, ngroups, nc;   // nc: columns per block
+	long S;
+	const PassRec* pass;        // tiles of the passes
+	const FitPass* groups_of;
+	const FitGroup* groups;
+	const unsigned* bases;      // [group][unit]: byte offset (swizzled) of register 0
+	const FitGate<T>* gates;    // [group][2]
+	const T* tables;            // [flush][parity][S], in thread order of the flush's group
+	const T* final;             // [parity][S]: the diagonal factors after the last gate
+	const T* dense;
+	long dense_b0, b0, b1;
+	T* su;
+	T* sw;
+	T* cache;                   // [block][group][column of the block][S]
+	double* part;               // [block][nblocks][16] (gradient) or [block][2]
+	int nblocks;
+};
+
+// swizzled slot of a tile index (16-byte amplitudes): its low bits XORed with the higher groups
+// of bits, so that the lanes of a wavefront hit distinct banks whenever their bits differ mod 3
+__host__ __device__ __forceinline__ unsigned fsw(unsigned e) { return e ^ ((e >> 3) & 7u) ^ ((e >> 6) & 7u) ^ ((e >> 9) & 7u); }
+
+// M (or its transpose) on the pair (f, s); sw: M = [[p, 1], [1, q]]
+template <class P, bool QC, bool TR>
+__device__ __forceinline__ void fit_pair(typename P::T& f, typename P::T& s, const typename P::T& p, const typename P::T& q, bool sw)
+{
+	typedef typename P::T T;
+	const T x = f, y = s;
+	if (sw)
+	{
+		f = P::axpy(y, p, x);
+		s = QC ? P::axpyc(x, q, y) : P::axpy(x, q, y);
+	}
+	else if (!TR)
+	{
+		f = P::axpy(x, p, y);
+		s = QC ? P::axpyc(y, q, x) : P::axpy(y, q, x);
+	}
+	else
+	{
+		f = QC ? P::axpyc(x, q, y) : P::axpy(x, q, y);
+		s = P::axpy(y, p, x);
+	}
+}
+
+// byte offset in the tile of register k of a unit whose register 0 is at `base`
+__device__ __forceinline__ unsigned fit_off(const FitGroup& G, unsigned base, int k)
+{
+	return base ^ ((k & 1) ? G.m[0] : 0u) ^ ((k & 2) ? G.m[1] : 0u) ^ ((k & 4) ? G.m[2] : 0u) ^ ((k & 8) ? G.m[3] : 0u);
+}
+
+// byte offset of register 0 of unit u; tpar: parity of the column and of the tile's nonlocal bits
+__device__ __forceinline__ unsigned fit_base(const FitGroup& G, const unsigned* __restrict__ bases, unsigned u, int tpar)
+{
+	const unsigned b = bases[u];
+	return (G.kind_b == 2 && ((__popc(u) + tpar) & 1)) ? b ^ G.m[3] : b;
+}
+
+// both gates of a group on the 16 registers
+template <class P, bool QC>
+__device__ __forceinline__ void fit_rotate(typename P::T (&v)[16], const FitGroup& G, const FitGate<typename P::T>* gates)
+{
+	typedef typename P::T T;
+	if (G.ga >= 0)
+	{
+		const FitGate<T>& g = gates[0];
+		{
+			const T p = g.pk, q = g.qk;
+			const bool sw = g.swk;
+#pragma unroll
+			for (int k = 0; k < 4; k++) fit_pair<P, QC, false>(v[4 * k], v[4 * k + 3], p, q, sw);
+		}
+		{
+			const T p = g.pc, q = g.qc;
+			const bool sw = g.swc;
+#pragma unroll
+			for (int k = 0; k < 4; k++) fit_pair<P, QC, false>(v[4 * k + 1], v[4 * k + 2], p, q, sw);
+		}
+	}
+	if (G.kind_b == 1)
+	{
+		const FitGate<T>& g = gates[1];
+		{
+			const T p = g.pk, q = g.qk;
+			const bool sw = g.swk;
+#pragma unroll
+			for (int k = 0; k < 4; k++) fit_pair<P, QC, false>(v[k], v[k + 12], p, q, sw);
+		}
+		{
+			const T p = g.pc, q = g.qc;
+			const bool sw = g.swc;
+#pragma unroll
+			for (int k = 0; k < 4; k++) fit_pair<P, QC, false>(v[k + 4], v[k + 8], p, q, sw);
+		}
+	}
+	else if (G.kind_b == 2)
+	{
+		// pairs along bit 2: corner where the other bits (0, 1, 3) have even parity
+		const FitGate<T>& g = gates[1];
+		{
+			const T p = g.pk, q = g.qk;
+			const bool sw = g.swk;
+			fit_pair<P, QC, false>(v[0], v[4], p, q, sw);
+			fit_pair<P, QC, false>(v[3], v[7], p, q, sw);
+			fit_pair<P, QC, false>(v[9], v[13], p, q, sw);
+			fit_pair<P, QC, false>(v[10], v[14], p, q, sw);
+		}
+		const T p = g.pc, q = g.qc;
+		const bool sw = g.swc;
+		if (!G.rev)
+		{
+			fit_pair<P, QC, false>(v[1], v[5], p, q, sw);
+			fit_pair<P, QC, false>(v[2], v[6], p, q, sw);
+			fit_pair<P, QC, false>(v[8], v[12], p, q, sw);
+			fit_pair<P, QC, false>(v[11], v[15], p, q, sw);
+		}
+		else
+		{
+			fit_pair<P, QC, false>(v[5], v[1], p, q, sw);
+			fit_pair<P, QC, false>(v[6], v[2], p, q, sw);
+			fit_pair<P, QC, false>(v[12], v[8], p, q, sw);
+			fit_pair<P, QC, false>(v[15], v[11], p, q, sw);
+		}
+	}
+}
+
+// one group on a unit, all 16 amplitudes in registers: one shared-memory round trip for both
+// gates.  For the forward sweep of f alone; beside the gradient sums' registers it spills
+// (float-float L=12, 42 gates: 3.8 ms against 3.3 ms quartet by quartet)
+template <class P, bool QC>
+__device__ __forceinline__ void fit_group16(const FitGroup& G, const FitGate<typename P::T>* gates, unsigned tc, unsigned base,
+	unsigned U, const typename P::T* __restrict__ tab)
+{
+	typedef typename P::T T;
+	T v[16];
+#pragma unroll
+	for (int k = 0; k < 16; k++) v[k] = lds<T>(tc + fit_off(G, base, k));
+	if (tab)
+	{
+#pragma unroll
+		for (int k = 0; k < 16; k++) v[k] = P::mul(tab[k * U], v[k]);
+	}
+	fit_rotate<P, QC>(v, G, gates);
+#pragma unroll
+	for (int k = 0; k < 16; k++) sts<T>(tc + fit_off(G, base, k), v[k]);
+}
+
+// both gates of a group on a unit, quartet by quartet in the tile.  Forward: flush (tab or null)
+// with the first gate, the state to the cache (out or null) with the last; transposed (TR):
+// flush with the last
+template <class P, bool QC, bool TR>
+__device__ __forceinline__ void fit_group(const FitGroup& G, const FitGate<typename P::T>* gates, unsigned tc, unsigned base,
+	const typename P::T* __restrict__ tab, typename P::T* __restrict__ out)
+{
+	typedef typename P::T T;
+	const int w0 = G.ga >= 0 ? 0 : 1, w1 = G.kind_b ? 1 : 0;
+#pragma unroll 1
+	for (int w = w0; w <= w1; w++)
+	{
+		const FitGate<T>& g = gates[w];
+		const T pk = g.pk, qk = g.qk, pc = g.pc, qc = g.qc;
+		const bool sk = g.swk, sc = g.swc;
+		const char* tb = (w == (TR ? w1 : w0)) ? reinterpret_cast<const char*>(tab) : nullptr;
+		char* ob = (!TR && w == w1) ? reinterpret_cast<char*>(out) : nullptr;
+#pragma unroll 1
+		for (int i = 0; i < 4; i++)
+		{
+			const uint4 o = G.qs[w][i], q = G.qy[w][i];
+			const unsigned ax = tc + (base ^ o.x), ay = tc + (base ^ o.y), az = tc + (base ^ o.z), aw = tc + (base ^ o.w);
+			T x = lds<T>(ax), y = lds<T>(ay), z = lds<T>(az), v = lds<T>(aw);
+			T tx, ty, tz, tv;
+			if (tb)
+			{
+				tx = *reinterpret_cast<const T*>(tb + q.x); ty = *reinterpret_cast<const T*>(tb + q.y);
+				tz = *reinterpret_cast<const T*>(tb + q.z); tv = *reinterpret_cast<const T*>(tb + q.w);
+			}
+			if (!TR && tb) { x = P::mul(tx, x); y = P::mul(ty, y); z = P::mul(tz, z); v = P::mul(tv, v); }
+			fit_pair<P, QC, TR>(x, v, pk, qk, sk);
+			fit_pair<P, QC, TR>(y, z, pc, qc, sc);
+			if (TR && tb) { x = P::mul(tx, x); y = P::mul(ty, y); z = P::mul(tz, z); v = P::mul(tv, v); }
+			sts<T>(ax, x); sts<T>(ay, y); sts<T>(az, z); sts<T>(aw, v);
+			if (ob)
+			{
+				*reinterpret_cast<T*>(ob + q.x) = x; *reinterpret_cast<T*>(ob + q.y) = y;
+				*reinterpret_cast<T*>(ob + q.z) = z; *reinterpret_cast<T*>(ob + q.w) = v;
+			}
+		}
+	}
+}
+
+// R sums of the gates first..last (1: b, 0: a) of a group over the quartets of a unit: the
+// derivative in the tile and the cached state ct, read one quartet ahead.  One loop for every
+// kind of gate, not unrolled: with each gate's quartets unrolled the kernel's code outgrew the
+// instruction caches (a third of its stalls).
+template <class P>
+__device__ __forceinline__ void fit_contract(const FitGroup& G, int first, int last, unsigned tc, unsigned base,
+	const typename P::T* __restrict__ ct, typename P::Acc (&acc)[8])
+{
+	typedef typename P::T T;
+	const char* cb = reinterpret_cast<const char*>(ct);
+	const uint4 *qs = &G.qs[0][0], *qy = &G.qy[0][0];
+	int i = 4 * first;
+	uint4 oy = qy[i];
+	T cx = *reinterpret_cast<const T*>(cb + oy.x), cy = *reinterpret_cast<const T*>(cb + oy.y);
+	T cz = *reinterpret_cast<const T*>(cb + oy.z), cw = *reinterpret_cast<const T*>(cb + oy.w);
+#pragma unroll 1
+	for (int k = 4 * (first - last + 1); k > 0; k--)
+	{
+		const uint4 o = qs[i];
+		const T x = lds<T>(tc + (base ^ o.x)), y = lds<T>(tc + (base ^ o.y)), z = lds<T>(tc + (base ^ o.z)), v = lds<T>(tc + (base ^ o.w));
+		const T sx = cx, sy = cy, sz = cz, sv = cw;
+		i = (i + 1) & 7;   // gate b's quartets 4..7, then gate a's 0..3
+		if (k > 1)
+		{
+			oy = qy[i];
+			cx = *reinterpret_cast<const T*>(cb + oy.x); cy = *reinterpret_cast<const T*>(cb + oy.y);
+			cz = *reinterpret_cast<const T*>(cb + oy.z); cw = *reinterpret_cast<const T*>(cb + oy.w);
+		}
+		contract_quartet<P>(acc, x, v, y, z, sx, sv, sy, sz);
+	}
+}
+
+// threads per block: 128, or 256 where a tile has that many units; four (two) blocks per SM
+// (registers), three of 128 in complex128, whose pipe is the bound
+template <class P, bool QC, bool GRAD, int FIT_NT>
+__global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 : P::kId == MG_PREC_FP64_ID ? 3 : 4) k_fit(FitArgs<P> a)
+{
+	typedef typename P::T T;
+	constexpr unsigned ES = sizeof(T);
+	extern __shared__ __align__(16) char smem_raw[];
+	__shared__ FitStage<T> stage[2];
+	const int kt = a.kt, nu = kt - 4;
+	const unsigned U = 1u << nu, n = 1u << kt;
+	const int nc = a.nc;
+	// units per thread (none for the threads beyond the block's units)
+	const unsigned its = U > FIT_NT ? U / FIT_NT : threadIdx.x < U * nc ? 1 : 0;
+	const unsigned tb = smem_u32(smem_raw);
+	Smem s;
+	s.dlo = reinterpret_cast<unsigned*>(smem_raw + (size_t)ES * n * nc);
+	s.dhi = s.dlo + 128;
+	s.red = reinterpret_cast<double*>(s.dhi + 128);
+	s.h = kt / 2;
+	const long S = a.S;
+	const unsigned mycol = min(threadIdx.x >> nu, (unsigned)nc - 1), u0 = nc > 1 ? (threadIdx.x & (U - 1)) : threadIdx.x;
+	const unsigned colb = mycol * n * ES;
+	T* su = a.su + (size_t)blockIdx.x * S;
+	T* sw = a.sw + (size_t)blockIdx.x * S;
+	T* cache = GRAD ? a.cache + (size_t)blockIdx.x * a.ngroups * nc * S + (size_t)mycol * S : nullptr;
+	const size_t cstride = (size_t)nc * S;
+	typename P::Acc acc[8];
+#pragma unroll
+	for (int e = 0; e < 8; e++) acc[e] = P::acc_zero();
+	typename P::Acc facc = P::acc_zero();
+	int nred = 0;
+
+	for (long cb = a.b0 + (long)blockIdx.x * nc; cb < a.b1; cb += (long)gridDim.x * nc)
+	{
+		// this thread's column (the last one again past the range: its derivative is zero)
+		const long b = min(cb + (long)mycol, a.b1 - 1);
+		const int par = __popcll(b) & 1;
+		for (int p = 0; p < a.npass; p++)
+		{
+			const PassRec& pr = a.pass[p];
+			const FitPass fp = a.groups_of[p];
+			__syncthreads();
+			setup_pass(pr, kt, s);
+			__syncthreads();
+			const bool last = p == a.npass - 1;
+			for (unsigned tau = 0; tau < (1u << pr.nnl); tau++)
+			{
+				const unsigned nlb = nl_base(pr, tau);
+				const int tpar = (__popc(nlb) + par) & 1;
+				fit_stage<T>(stage[fp.gbeg & 1], a.groups + fp.gbeg, a.gates + 2 * fp.gbeg);
+				for (unsigned e = threadIdx.x; e < n * nc; e += FIT_NT)
+				{
+					const unsigned c = gidx(s, nlb, e & (n - 1));
+					T v;
+					if (p == 0) v = c == (unsigned)(min(cb + (long)(e >> kt), a.b1 - 1) >> 1) ? P::make(1.0, 0.0) : P::zero();
+					else v = sw[c];
+					sts<T>(tb + ((e & ~(n - 1)) + fsw(e & (n - 1))) * ES, v);
+				}
+				fit_stage_wait();
+				__syncthreads();
+				for (int g = fp.gbeg; g < fp.gend; g++)
+				{
+					const FitGroup& G = stage[g & 1].g;
+					if (g + 1 < fp.gend) fit_stage<T>(stage[(g + 1) & 1], a.groups + g + 1, a.gates + 2 * (g + 1));
+					for (unsigned i = 0; i < its; i++)
+					{
+						const unsigned u = u0 + i * FIT_NT, base = fit_base(G, a.bases + (size_t)g * U, u, tpar);
+						const T* tab = G.flush >= 0 ? a.tables + ((size_t)(2 * G.flush + par) * S + ((size_t)tau << kt) + u) : nullptr;
+						T* out = GRAD ? cache + (size_t)g * cstride + ((size_t)tau << kt) + u : nullptr;
+						if (GRAD) fit_group<P, QC, false>(G, stage[g & 1].gate, tb + colb, base, tab, out);
+						else fit_group16<P, QC>(G, stage[g & 1].gate, tb + colb, base, U, tab);
+					}
+					fit_stage_wait();
+					__syncthreads();
+				}
+				if (!GRAD && last)
+				{
+					for (unsigned e = threadIdx.x; e < n * nc; e += FIT_NT)
+					{
+						const unsigned c = gidx(s, nlb, e & (n - 1));
+						const long be = cb + (long)(e >> kt);
+						if (be >= a.b1) continue;
+						const T d = P::mul(a.final[(size_t)(__popcll(be) & 1) * S + c], a.dense[(size_t)(be - a.dense_b0) * S + c]);
+						P::acc_mul_add(facc, d, lds<T>(tb + ((e & ~(n - 1)) + fsw(e & (n - 1))) * ES));
+					}
+				}
+				if (!last)
+					for (unsigned e = threadIdx.x; e < n; e += FIT_NT) sw[gidx(s, nlb, e)] = lds<T>(tb + fsw(e) * ES);
+				__syncthreads();
+			}
+		}
+		if (!GRAD) continue;
+		for (int p = a.npass - 1; p >= 0; p--)
+		{
+			const PassRec& pr = a.pass[p];
+			const FitPass fp = a.groups_of[p];
+			__syncthreads();
+			setup_pass(pr, kt, s);
+			__syncthreads();
+			const bool last = p == a.npass - 1;
+			for (unsigned tau = 0; tau < (1u << pr.nnl); tau++)
+			{
+				const unsigned nlb = nl_base(pr, tau);
+				const int tpar = (__popc(nlb) + par) & 1;
+				fit_stage<T>(stage[(fp.gend - 1) & 1], a.groups + fp.gend - 1, a.gates + 2 * (fp.gend - 1));
+				for (unsigned e = threadIdx.x; e < n * nc; e += FIT_NT)
+				{
+					const unsigned c = gidx(s, nlb, e & (n - 1));
+					T v;
+					if (last)
+					{
+						const long be = cb + (long)(e >> kt);
+						v = be < a.b1 ? P::mul(a.final[(size_t)(__popcll(be) & 1) * S + c], a.dense[(size_t)(be - a.dense_b0) * S + c])
+							: P::zero();
+					}
+					else v = su[c];
+					sts<T>(tb + ((e & ~(n - 1)) + fsw(e & (n - 1))) * ES, v);
+				}
+				fit_stage_wait();
+				__syncthreads();
+				int merged = 0;
+				for (int g = fp.gend - 1; g >= fp.gbeg; g--)
+				{
+					// the state is the one after both gates: both sums come before the
+					// transposed gates
+					const FitGroup& G = stage[g & 1].g;
+					if (g > fp.gbeg) fit_stage<T>(stage[(g - 1) & 1], a.groups + g - 1, a.gates + 2 * (g - 1));
+					const T* cg = cache + (size_t)g * cstride + ((size_t)tau << kt) + u0;
+					const T* tab = G.flush >= 0 ? a.tables + ((size_t)(2 * G.flush + par) * S + ((size_t)tau << kt) + u0) : nullptr;
+					const int blk = G.ga >= 0 ? G.blk_a : G.blk_b;
+					if (g > fp.gbeg)
+					{
+						// the next group's cached state to L2: two of the sixteen 128-byte lines that
+						// eight threads' registers take
+						const T* nx = cg - cstride - (threadIdx.x & 7);
+						for (unsigned i = 0; i < its; i++)
+							for (unsigned k = threadIdx.x & 7; k < 16; k += 8)
+								asm volatile("prefetch.global.L2 [%0];" :: "l"(nx + i * FIT_NT + k * U));
+					}
+					const bool split = G.ga >= 0 && G.kind_b && G.blk_b != blk;
+					if (split)
+					{
+						for (unsigned i = 0; i < its; i++)
+							fit_contract<P>(G, 1, 1, tb + colb, fit_base(G, a.bases + (size_t)g * U, u0 + i * FIT_NT, tpar), cg + i * FIT_NT, acc);
+						block_reduce8<P>(acc, s.red, a.part + ((size_t)blockIdx.x * a.nblocks + G.blk_b) * 16, 1.0, nred);
+#pragma unroll
+						for (int e = 0; e < 8; e++) acc[e] = P::acc_zero();
+					}
+					for (unsigned i = 0; i < its; i++)
+						fit_contract<P>(G, (G.kind_b && !split) ? 1 : 0, G.ga >= 0 ? 0 : 1, tb + colb,
+							fit_base(G, a.bases + (size_t)g * U, u0 + i * FIT_NT, tpar), cg + i * FIT_NT, acc);
+					if (g > 0)   // nothing uses the derivative before the first group
+						for (unsigned i = 0; i < its; i++)
+							fit_group<P, QC, true>(G, stage[g & 1].gate, tb + colb, fit_base(G, a.bases + (size_t)g * U, u0 + i * FIT_NT, tpar),
+								tab ? tab + i * FIT_NT : nullptr, nullptr);
+					merged += 8 * (int)max(its, 1u);
+					fit_stage_wait();
+					// the next group continues this sum when its gates are of the same block
+					bool more = false;
+					if (g > fp.gbeg)
+					{
+						more = G.blk_next == blk;
+					}
+					if (!more)
+					{
+						block_reduce8<P>(acc, s.red, a.part + ((size_t)blockIdx.x * a.nblocks + blk) * 16, 1.0, nred);
+#pragma unroll
+						for (int e = 0; e < 8; e++) acc[e] = P::acc_zero();
+						merged = 0;
+					}
+					else
+					{
+						if (merged >= FIT_RENORM)
+						{
+#pragma unroll
+							for (int e = 0; e < 8; e++) P::acc_norm(acc[e]);
+							merged = 0;
+						}
+						__syncthreads();
+					}
+				}
+				if (p > 0)
+					for (unsigned e = threadIdx.x; e < n; e += FIT_NT) su[gidx(s, nlb, e)] = lds<T>(tb + fsw(e) * ES);
+				__syncthreads();
+			}
+		}
+	}
+	if (!GRAD) block_reduce1<P>(facc, s.red, a.part + (size_t)blockIdx.x * 2);
+}
+
+// complex products in double-double, for the tables of complex128 (every entry correctly rounded
+// to a few 2^-100, so that the tables carry no common rounding error into all columns)
+struct Dd { double h, l; };
+__device__ __forceinline__ Dd dd_add(Dd a, Dd b)
+{
+	const double s = a.h + b.h, bb = s - a.h, e = (a.h - (s - bb)) + (b.h - bb) + (a.l + b.l);
+	Dd r;
+	r.h = s + e;
+	r.l = e - (r.h - s);
+	return r;
+}
+__device__ __forceinline__ Dd dd_mul(Dd a, Dd b)
+{
+	const double p = a.h * b.h, e = fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h);
+	Dd r;
+	r.h = p + e;
+	r.l = e - (r.h - p);
+	return r;
+}
+__device__ __forceinline__ Dd dd_neg(Dd a) { a.h = -a.h; a.l = -a.l; return a; }
+
+// one diagonal factor: entry 2 bit_i + bit_j (bits si, sj of the full index), (re, im) as
+// double-double
+struct FitDiag { double v[4][4]; int si, sj; };
+
+// entry (parity, position) of every flush's table and of the final one (flush == nflush)
+template <class P>
+__global__ void k_fit_tables(const FitDiag* __restrict__ diag, const int* __restrict__ beg, int nflush, const int* __restrict__ group_of,
+	const FitGroup* __restrict__ groups, const PassRec* __restrict__ pass, int kt, long S, typename P::T* __restrict__ tables)
+{
+	const int nu = kt - 4;
+	for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < 2 * S * (nflush + 1); q += (long)gridDim.x * blockDim.x)
+	{
+		const int f = (int)(q / (2 * S));
+		const long rest = q - f * 2 * S;
+		const int par = rest >= S;
+		unsigned c = (unsigned)(rest - par * S);
+		if (f < nflush)
+		{
+			// thread order of the flush's group: (tile, register, unit)
+			const FitGroup& G = groups[group_of[f]];
+			const PassRec& pr = pass[G.pass];
+			const unsigned tau = c >> kt, u = c & ((1u << nu) - 1u);
+			unsigned k = (c >> nu) & 15u;
+			c = nl_base(pr, tau);
+			if (G.kind_b == 2 && ((__popc(u) + __popc(c) + par) & 1)) k ^= 8u;
+			for (int j = 0; j < 4; j++) c |= ((k >> j) & 1u) << G.cbit[j];
+			for (int j = 0; j < nu; j++) c |= ((u >> j) & 1u) << G.cbit[4 + j];
+		}
+		const unsigned long full = ((unsigned long)c << 1) | ((__popc(c) + par) & 1);
+		Dd re = { 1, 0 }, im = { 0, 0 };
+		for (int d = beg[f]; d < beg[f + 1]; d++)
+		{
+			const FitDiag& D = diag[d];
+			const double* v = D.v[2 * ((full >> D.si) & 1) + ((full >> D.sj) & 1)];
+			if (P::kId == MG_PREC_FP64_ID)
+			{
+				const Dd a = { v[0], v[1] }, b = { v[2], v[3] };
+				const Dd r = dd_add(dd_mul(re, a), dd_neg(dd_mul(im, b)));
+				im = dd_add(dd_mul(re, b), dd_mul(im, a));
+				re = r;
+			}
+			else
+			{
+				const double r = re.h * v[0] - im.h * v[2];
+				im.h = re.h * v[2] + im.h * v[0];
+				re.h = r;
+			}
+		}
+		tables[q] = P::make(re.h, im.h);
+	}
+}
+
+// block gradients and f from the summed R: one block of threads per parameter block, the rows of
+// the parts summed by 8 threads each in a fixed order
+struct FitBlock { double minv[8][2]; double scale[8][2]; int ngates, pad; };   // see mgcu_fit_build.cuh
+
+__global__ void __launch_bounds__(128) k_fit_finish(const double* __restrict__ part, int nparts, int nblocks, const FitBlock* __restrict__ fb,
+	double* __restrict__ out_f, double* __restrict__ out_blk)
+{
+	__shared__ double sum[8][16];
+	const int blk = blockIdx.x, e = threadIdx.x & 15, w = threadIdx.x >> 4;
+	double s = 0;
+	for (int r = w; r < nparts; r += 8) s += part[((size_t)r * nblocks + blk) * 16 + e];
+	sum[w][e] = s;
+	__syncthreads();
+	if (threadIdx.x >= 16) return;
+	s = 0;
+	for (int r = 0; r < 8; r++) s += sum[r][threadIdx.x];
+	__syncwarp(0xffffu);
+	sum[0][threadIdx.x] = s;
+	__syncwarp(0xffffu);
+	const double* R = sum[0];
+	// entry q = 4 (corner) + 2 r + t
+	if (threadIdx.x < 8)
+	{
+		const int q = threadIdx.x, h = q & 4, r = (q >> 1) & 1, t = q & 1;
+		const FitBlock& B = fb[blk];
+		double gr = 0, gi = 0;
+		for (int k = 0; k < 2; k++)
+		{
+			const double* x = R + 2 * (h + 2 * r + k);
+			const double* m = B.minv[h + 2 * t + k];
+			gr += x[0] * m[0] - x[1] * m[1];
+			gi += x[0] * m[1] + x[1] * m[0];
+		}
+		const double* c = B.scale[q];
+		out_blk[blk * 16 + 2 * q] = gr * c[0] - gi * c[1];
+		out_blk[blk * 16 + 2 * q + 1] = gr * c[1] + gi * c[0];
+	}
+	if (blk == 0 && threadIdx.x >= 8 && threadIdx.x < 10)
+	{
+		const int c = threadIdx.x - 8;
+		out_f[c] = ((R[0 + c] + R[6 + c]) + (R[8 + c] + R[14 + c])) / fb[0].ngates;
+	}
+}

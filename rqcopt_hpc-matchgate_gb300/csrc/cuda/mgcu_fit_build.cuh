@@ -1,0 +1,369 @@
+// Host side of the factored fitted circuit (mgcu_fit.cuh): groups, flushes, factors.
+// Included by mgcu_engine.cu.
+
+struct FitProg
+{
+	bool built = false;            // the structure exists (groups, passes, flushes)
+	bool ok = false;               // the current gates factor (else the general kernels run)
+	bool qc = false;               // q needs its imaginary part
+	Sched sched;
+	std::vector<FitGroup> group;
+	std::vector<FitPass> pass_groups;
+	std::vector<std::array<int, 2>> diag;   // per table entry factor: gate, 0 left / 1 right
+	std::vector<int> beg, group_of;         // per flush (the last: the final table)
+	std::vector<int> block_gates;           // gates per block
+	int nflush = 0, grid = 0, nc = 1, threads = 128, kt = 0;
+	size_t smem = 0;
+	DevBuf d_pass, d_group, d_pgroups, d_gates, d_diag, d_beg, d_gof, d_tab, d_blk, d_bases, cache;
+};
+
+// wires of gate g as a mask
+static unsigned fit_wires(const int* w, int g) { return (1u << w[2 * g]) | (1u << w[2 * g + 1]); }
+
+// Passes as for the other sweeps (reordered: commuting gates only), then groups of up to two
+// gates within a pass, then flushes: before a group whose right factors are not merged yet, one
+// table of all pending left factors and of the right factors of every gate that comes next on
+// both of its wires (one flush per brickwall layer when the sector is one tile).
+static int fit_build(int L, int kt, const int* wires, int ng, const int* block, int nblocks, int es, FitProg& f)
+{
+	const int nb = L - 1;
+	schedule(L, kt, wires, ng, true, f.sched, 1);
+	std::vector<std::vector<int>> onq(L);
+	for (int g = 0; g < ng; g++) { onq[wires[2 * g]].push_back(g); onq[wires[2 * g + 1]].push_back(g); }
+	std::vector<size_t> next(L, 0);
+	std::vector<unsigned> bases;
+	std::vector<char> cdone(ng, 0);
+	std::vector<int> pending;
+	f.group.clear(); f.pass_groups.clear(); f.diag.clear(); f.beg.assign(1, 0); f.group_of.clear();
+	const unsigned pers = 3;   // swizzle period of the tile bits
+	for (size_t p = 0; p < f.sched.pass.size(); p++)
+	{
+		const PassRec& pr = f.sched.pass[p];
+		FitPass fp;
+		fp.gbeg = (int)f.group.size();
+		std::vector<int> rest;
+		std::vector<const GateRec*> rec(ng, nullptr);
+		for (int i = pr.gbeg; i < pr.gend; i++) { rest.push_back(f.sched.gate[i].g); rec[f.sched.gate[i].g] = &f.sched.gate[i]; }
+		while (!rest.empty())
+		{
+			int a = rest[0], b = -1;
+			unsigned used = fit_wires(wires, a);
+			size_t at = 0;
+			for (size_t i = 1; i < rest.size() && b < 0; i++)
+			{
+				if (!(fit_wires(wires, rest[i]) & used)) { b = rest[i]; at = i; }
+				used |= fit_wires(wires, rest[i]);
+			}
+			if (b >= 0) rest.erase(rest.begin() + at);
+			rest.erase(rest.begin());
+			// a gate on the dropped qubit is gate b
+			if (rec[a]->type != 0) std::swap(a, b);
+			FitGroup G;
+			memset(&G, 0, sizeof(G));
+			G.ga = a; G.gb = b;
+			G.blk_a = a >= 0 ? block[a] : -1;
+			G.blk_b = b >= 0 ? block[b] : -1;
+			G.kind_b = b < 0 ? 0 : (rec[b]->type == 0 ? 1 : 2);
+			G.rev = b >= 0 && rec[b]->type == 2;
+			G.pass = (int)p;
+			G.blk_next = f.group.empty() ? -1 : (f.group.back().kind_b ? f.group.back().blk_b : f.group.back().blk_a);
+			int bits[14], n = 0;
+			unsigned in = 0;
+			auto take = [&](int lb) { bits[n++] = lb; in |= 1u << lb; };
+			int rb[4] = { -1, -1, -1, -1 };
+			if (a >= 0) { rb[0] = rec[a]->lb; rb[1] = rec[a]->la; }
+			if (G.kind_b == 1) { rb[2] = rec[b]->lb; rb[3] = rec[b]->la; }
+			if (G.kind_b == 2) rb[2] = rec[b]->type == 1 ? rec[b]->la : rec[b]->lb;
+			for (int j = 0; j < 4; j++) if (rb[j] >= 0) in |= 1u << rb[j];
+			for (int j = 0; j < 4; j++)
+				if (rb[j] < 0)
+				{
+					// a free bit: the highest, which the lanes of a wavefront need least
+					int q = kt - 1;
+					while (in & (1u << q)) q--;
+					rb[j] = q;
+					in |= 1u << q;
+				}
+			for (int j = 0; j < 4; j++) bits[n++] = rb[j];
+			// unit bits: first the lowest ones of distinct swizzle classes, then the others
+			unsigned cls = 0;
+			for (int lb = 0; lb < kt; lb++)
+				if (!(in & (1u << lb)) && !(cls & (1u << (lb % pers)))) { cls |= 1u << (lb % pers); take(lb); }
+			for (int lb = 0; lb < kt; lb++) if (!(in & (1u << lb))) take(lb);
+			unsigned tm[10];
+			for (int j = 0; j < kt; j++)
+			{
+				G.cbit[j] = pr.lbits[bits[j]];
+				const unsigned off = fsw(1u << bits[j]) * (unsigned)es;
+				if (j < 4) G.m[j] = off; else tm[j - 4] = off;
+			}
+			for (unsigned u = 0; u < (1u << (kt - 4)); u++)
+			{
+				unsigned o = 0;
+				for (int j = 0; j < kt - 4; j++) if (u & (1u << j)) o ^= tm[j];
+				bases.push_back(o);
+			}
+			auto slot = [&](int k) {
+				unsigned o = 0;
+				for (int j = 0; j < 4; j++) if (k & (1 << j)) o ^= G.m[j];
+				return o;
+			};
+			for (int w = 0; w < 2; w++)
+				for (int i = 0; i < 4; i++)
+				{
+					int k[4];   // registers of |00>, |01>, |10>, |11>
+					if (w == 0) for (int j = 0; j < 4; j++) k[j] = 4 * i + j;
+					else if (G.kind_b != 2) for (int j = 0; j < 4; j++) k[j] = i + 4 * j;
+					else
+					{
+						// pairs along bit 2: corner where bits 0, 1, 3 have even parity
+						k[0] = (0xA930 >> (4 * i)) & 15;
+						k[3] = k[0] | 4;
+						k[1] = G.rev ? (k[0] ^ 5) : (k[0] ^ 1);
+						k[2] = G.rev ? (k[0] ^ 1) : (k[0] ^ 5);
+					}
+					const unsigned us = (1u << (kt - 4)) * (unsigned)es;
+					G.qs[w][i] = make_uint4(slot(k[0]), slot(k[1]), slot(k[2]), slot(k[3]));
+					G.qy[w][i] = make_uint4(k[0] * us, k[1] * us, k[2] * us, k[3] * us);
+				}
+			// flush
+			G.flush = -1;
+			bool need = false;
+			for (int s : { a, b })
+				if (s >= 0) need = need || !cdone[s];
+			if (need)
+			{
+				G.flush = f.nflush++;
+				f.group_of.push_back((int)f.group.size());
+				for (int s : pending) f.diag.push_back({ s, 0 });
+				pending.clear();
+				for (int q = 0; q < L; q++)
+				{
+					if (next[q] >= onq[q].size()) continue;
+					const int s = onq[q][next[q]], o = wires[2 * s] == q ? wires[2 * s + 1] : wires[2 * s];
+					if (cdone[s] || next[o] >= onq[o].size() || onq[o][next[o]] != s) continue;
+					cdone[s] = 1;
+					f.diag.push_back({ s, 1 });
+				}
+				f.beg.push_back((int)f.diag.size());
+			}
+			for (int s : { a, b })
+				if (s >= 0)
+				{
+					pending.push_back(s);
+					next[wires[2 * s]]++; next[wires[2 * s + 1]]++;
+				}
+			f.group.push_back(G);
+		}
+		fp.gend = (int)f.group.size();
+		f.pass_groups.push_back(fp);
+	}
+	for (int s : pending) f.diag.push_back({ s, 0 });
+	f.beg.push_back((int)f.diag.size());
+	f.block_gates.assign(nblocks, 0);
+	for (int g = 0; g < ng; g++) f.block_gates[block[g]]++;
+	const int U = 1 << (kt - 4);
+	f.threads = U >= 512 ? 512 : U >= 256 ? 256 : 128;
+	f.nc = (U < 128 && nb <= kt) ? 128 / U : 1;   // small sectors share a block
+	f.smem = (size_t)f.nc * ((size_t)1 << kt) * es + 2 * 128 * sizeof(unsigned) + red_bytes(f.threads);
+	int e = upload_sched(f.sched, f.d_pass, f.d_gates);
+	if (!e) e = f.d_group.alloc(sizeof(FitGroup) * f.group.size());
+	if (!e) e = f.d_pgroups.alloc(sizeof(FitPass) * f.pass_groups.size());
+	if (!e) e = f.d_gates.alloc(sizeof(FitGate<double2>) * 2 * f.group.size());
+	if (!e) e = f.d_diag.alloc(sizeof(FitDiag) * f.diag.size());
+	if (!e) e = f.d_beg.alloc(sizeof(int) * f.beg.size());
+	if (!e) e = f.d_gof.alloc(sizeof(int) * std::max(f.nflush, 1));
+	if (!e) e = f.d_tab.alloc((size_t)es * 2 * ((size_t)1 << nb) * (f.nflush + 1));
+	if (!e) e = f.d_blk.alloc(sizeof(FitBlock) * nblocks);
+	if (!e) e = f.d_bases.alloc(sizeof(unsigned) * bases.size());
+	if (e) return e;
+	cudaStream_t st = mgcu_stream();
+	MGCU_TRY(cudaMemcpyAsync(f.d_group.p, f.group.data(), sizeof(FitGroup) * f.group.size(), cudaMemcpyHostToDevice, st));
+	MGCU_TRY(cudaMemcpyAsync(f.d_pgroups.p, f.pass_groups.data(), sizeof(FitPass) * f.pass_groups.size(), cudaMemcpyHostToDevice, st));
+	MGCU_TRY(cudaMemcpyAsync(f.d_bases.p, bases.data(), sizeof(unsigned) * bases.size(), cudaMemcpyHostToDevice, st));
+	MGCU_TRY(cudaMemcpyAsync(f.d_beg.p, f.beg.data(), sizeof(int) * f.beg.size(), cudaMemcpyHostToDevice, st));
+	if (f.nflush) MGCU_TRY(cudaMemcpyAsync(f.d_gof.p, f.group_of.data(), sizeof(int) * f.nflush, cudaMemcpyHostToDevice, st));
+	MGCU_TRY(cudaStreamSynchronize(st));
+	f.built = true;
+	return 0;
+}
+
+// host double-double complex arithmetic for the factors
+struct Hdd { double h, l; };
+static Hdd hdd(double x) { return { x, 0 }; }
+static Hdd hadd(Hdd a, Hdd b)
+{
+	const double s = a.h + b.h, bb = s - a.h, e = (a.h - (s - bb)) + (b.h - bb) + (a.l + b.l);
+	const double r = s + e;
+	return { r, e - (r - s) };
+}
+static Hdd hneg(Hdd a) { return { -a.h, -a.l }; }
+static Hdd hmul(Hdd a, Hdd b)
+{
+	const double p = a.h * b.h, e = std::fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h);
+	const double r = p + e;
+	return { r, e - (r - p) };
+}
+static Hdd hdiv(Hdd a, Hdd b)
+{
+	const double q = a.h / b.h;
+	const Hdd r = hadd(a, hneg(hmul(hdd(q), b)));
+	const double q2 = r.h / b.h;
+	const double s = q + q2;
+	return { s, q2 - (s - q) };
+}
+struct Hcx { Hdd re, im; };
+static Hcx hcx(mgc z) { return { hdd(z.re), hdd(z.im) }; }
+static Hcx cmul(Hcx a, Hcx b)
+{
+	return { hadd(hmul(a.re, b.re), hneg(hmul(a.im, b.im))), hadd(hmul(a.re, b.im), hmul(a.im, b.re)) };
+}
+static Hcx cscale(Hcx a, double s) { return { hmul(a.re, hdd(s)), hmul(a.im, hdd(s)) }; }
+static Hcx cdiv(Hcx a, Hcx b)
+{
+	const Hdd d = hadd(hmul(b.re, b.re), hmul(b.im, b.im));
+	const Hcx n = cmul(a, { b.re, hneg(b.im) });
+	return { hdiv(n.re, d), hdiv(n.im, d) };
+}
+
+struct FitFactor { double p; mgc q; int sw; Hcx l[2], r[2]; };
+
+// diag(l) M diag(r) of a 2x2 block (entries a, b, c, d), r[0] = 1; false when an entry that M is
+// scaled by is too small (|entry| < 2^-8 of the largest) or M is near singular.  p has 64
+// candidates around |b / a| (|a / b| when swapped): p q = bc / (ad) is fixed, and the candidate
+// whose q rounds best leaves no rounding of the factors common to all amplitudes.
+static bool fit_factor(const mgc* e, FitFactor& F)
+{
+	double ab[4], mx = 0;
+	for (int k = 0; k < 4; k++) { ab[k] = std::hypot(e[k].re, e[k].im); mx = std::max(mx, ab[k]); }
+	if (!(mx > 1e-100 && mx < 1e100)) return false;
+	F.sw = ab[1] * ab[2] > ab[0] * ab[3];
+	// pivots (u, v) scaled to 1 and the others: unswapped M = [[1, p], [q, 1]], u = a, v = d
+	const int iu = F.sw ? 1 : 0, iv = F.sw ? 2 : 3, ip = F.sw ? 0 : 1, iq = F.sw ? 3 : 2;
+	if (ab[iu] < mx / 256 || ab[iv] < mx / 256) return false;
+	const Hcx u = hcx(e[iu]), v = hcx(e[iv]), ep = hcx(e[ip]), eq = hcx(e[iq]);
+	const Hcx one = { hdd(1), hdd(0) };
+	const Hcx k = cdiv(cmul(ep, eq), cmul(u, v));   // p q
+	F.p = 0;
+	if (ab[ip] > 1e-100)
+	{
+		const double p0 = ab[ip] / ab[iu];
+		double best = -1, p = p0;
+		for (int c = 0; c < 64; c++)
+		{
+			const double q = k.re.h / p, r = std::fabs(std::fma(-q, p, k.re.h) + k.re.l);
+			if (best < 0 || r < best) { best = r; F.p = p; }
+			p = std::nextafter(p, 2 * p0);
+		}
+	}
+	F.r[0] = one;
+	if (!F.sw)
+	{
+		// a = l0, b = l0 p r1, c = l1 q, d = l1 r1
+		F.l[0] = u;
+		F.r[1] = F.p > 0 ? cdiv(ep, cscale(u, F.p)) : one;
+		F.l[1] = cdiv(v, F.r[1]);
+	}
+	else
+	{
+		// a = l0 p, b = l0 r1, c = l1, d = l1 q r1
+		F.l[1] = v;
+		F.r[1] = F.p > 0 ? cdiv(cscale(u, F.p), ep) : one;
+		F.l[0] = cdiv(u, F.r[1]);
+	}
+	const Hcx q = cdiv(eq, F.sw ? cmul(F.l[1], F.r[1]) : F.l[1]);
+	F.q = mgc_make(q.re.h, q.im.h);
+	const double dr = 1 - F.p * F.q.re, di = -F.p * F.q.im;
+	return std::hypot(dr, di) > 1.0 / 256 && std::hypot(F.q.re, F.q.im) < 256 && F.p < 256;
+}
+
+// factors, tables and end transforms of the current gates; f.ok tells whether they factor
+template <class P>
+static int fit_set_gates(const mgg* gates, int ng, const int* block, int nblocks, int L, int kt, const int* wires, FitProg& f)
+{
+	typedef typename P::T T;
+	f.ok = false;
+	std::vector<int> first(nblocks, -1);
+	for (int g = 0; g < ng; g++)
+	{
+		if (first[block[g]] < 0) first[block[g]] = g;
+		else if (memcmp(&gates[g], &gates[first[block[g]]], sizeof(mgg))) return 0;   // a block's gates must be equal
+	}
+	std::vector<FitFactor> fac(2 * nblocks);
+	double qi = 0;
+	std::vector<FitBlock> fb(nblocks);
+	memset(fb.data(), 0, sizeof(FitBlock) * nblocks);
+	for (int b = 0; b < nblocks; b++)
+	{
+		if (first[b] < 0) continue;
+		fb[b].ngates = f.block_gates[b];
+		for (int h = 0; h < 2; h++)
+		{
+			FitFactor& F = fac[2 * b + h];
+			if (!fit_factor(h ? gates[first[b]].k : gates[first[b]].c, F)) return 0;
+			qi = std::max(qi, std::fabs(F.q.im));
+			// inverse of M and 1 / (l_r r_t)
+			const mgc det = mgc_make(1 - F.p * F.q.re, -F.p * F.q.im);
+			const double d2 = det.re * det.re + det.im * det.im;
+			const mgc id = mgc_make(det.re / d2, -det.im / d2), one = mgc_make(1, 0), p = mgc_make(F.p, 0);
+			auto neg = [](mgc z) { return mgc_make(-z.re, -z.im); };
+			const mgc mi[4] = { F.sw ? neg(F.q) : one, F.sw ? one : neg(p), F.sw ? one : neg(F.q), F.sw ? neg(p) : one };
+			for (int k = 0; k < 4; k++)
+			{
+				const mgc m = mgc_mul(mi[k], id);
+				fb[b].minv[4 * h + k][0] = m.re; fb[b].minv[4 * h + k][1] = m.im;
+				const Hcx s = cdiv({ hdd(1), hdd(0) }, cmul(F.l[k >> 1], F.r[k & 1]));
+				fb[b].scale[4 * h + k][0] = s.re.h; fb[b].scale[4 * h + k][1] = s.im.h;
+			}
+		}
+	}
+	// beyond the rounding of a unitary block q keeps its imaginary part (complex128: always)
+	f.qc = qi > (P::kId == MG_PREC_FP64_ID ? 0.0 : 1e-15);
+	std::vector<FitGate<T>> hg(2 * f.group.size());
+	memset(hg.data(), 0, sizeof(FitGate<T>) * hg.size());
+	for (size_t i = 0; i < hg.size(); i++)
+	{
+		const int g = i & 1 ? f.group[i / 2].gb : f.group[i / 2].ga;
+		if (g < 0) continue;
+		const FitFactor &c = fac[2 * block[g]], &k = fac[2 * block[g] + 1];
+		hg[i].pc = P::make(c.p, 0); hg[i].qc = P::make(c.q.re, c.q.im);
+		hg[i].pk = P::make(k.p, 0); hg[i].qk = P::make(k.q.re, k.q.im);
+		hg[i].swc = c.sw; hg[i].swk = k.sw;
+	}
+	std::vector<FitDiag> hd(f.diag.size());
+	for (size_t i = 0; i < hd.size(); i++)
+	{
+		const int g = f.diag[i][0];
+		const FitFactor &c = fac[2 * block[g]], &k = fac[2 * block[g] + 1];
+		const Hcx* fc = f.diag[i][1] ? c.r : c.l;
+		const Hcx* fk = f.diag[i][1] ? k.r : k.l;
+		const Hcx ent[4] = { fk[0], fc[0], fc[1], fk[1] };   // |00>, |01>, |10>, |11>
+		for (int q = 0; q < 4; q++)
+		{
+			hd[i].v[q][0] = ent[q].re.h; hd[i].v[q][1] = ent[q].re.l;
+			hd[i].v[q][2] = ent[q].im.h; hd[i].v[q][3] = ent[q].im.l;
+		}
+		hd[i].si = L - 1 - wires[2 * g]; hd[i].sj = L - 1 - wires[2 * g + 1];
+	}
+	cudaStream_t st = mgcu_stream();
+	MGCU_TRY(cudaMemcpyAsync(f.d_gates.p, hg.data(), sizeof(FitGate<T>) * hg.size(), cudaMemcpyHostToDevice, st));
+	MGCU_TRY(cudaMemcpyAsync(f.d_diag.p, hd.data(), sizeof(FitDiag) * hd.size(), cudaMemcpyHostToDevice, st));
+	MGCU_TRY(cudaMemcpyAsync(f.d_blk.p, fb.data(), sizeof(FitBlock) * nblocks, cudaMemcpyHostToDevice, st));
+	const long S = 1L << (L - 1);
+	k_fit_tables<P><<<grid_cap(2 * S * (f.nflush + 1), 128), 128, 0, st>>>(f.d_diag.as<FitDiag>(), f.d_beg.as<int>(), f.nflush, f.d_gof.as<int>(),
+		f.d_group.as<FitGroup>(), f.d_pass.as<PassRec>(), kt, S, f.d_tab.as<T>());
+	MGCU_LAUNCHED();
+	f.ok = true;
+	return 0;
+}
+
+template <class P, int NT>
+static void (*fit_kernel_nt(bool qc, bool grad))(FitArgs<P>)
+{
+	return qc ? (grad ? k_fit<P, true, true, NT> : k_fit<P, true, false, NT>) : (grad ? k_fit<P, false, true, NT> : k_fit<P, false, false, NT>);
+}
+template <class P>
+static void (*fit_kernel(bool qc, bool grad, int threads))(FitArgs<P>)
+{
+	return threads == 512 ? fit_kernel_nt<P, 512>(qc, grad) : threads == 256 ? fit_kernel_nt<P, 256>(qc, grad) : fit_kernel_nt<P, 128>(qc, grad);
+}

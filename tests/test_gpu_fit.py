@@ -1,0 +1,100 @@
+"""The factored fitted circuit (the default for gradients from 10 qubits, for f alone from 12)
+against the general kernels (kept by an explicit MG_OPT_THREADS), which apply the unfactored
+blocks: single tiles, several tiles per pass, odd qubit counts with an idle wire, gates whose
+off-diagonal entries dominate, gates on the dropped last qubit in both orders, diagonal and
+antidiagonal blocks, blocks of gates with equal matrices and one block per gate, non-unitary
+gates, ragged column ranges, and gates that do not factor (the general kernels run).
+
+Tolerances: both sides round each amplitude independently, so they agree within the precision of
+the sweep: 1e-12 in complex128, 1e-9 in float-float, 1e-4 in FP32, relative to the largest
+gradient entry, as elsewhere in these tests."""
+import numpy as np
+import pytest
+
+import mgcu
+import targets as T
+
+pytestmark = pytest.mark.gpu
+
+TOL = {mgcu.PREC_FP64: 1e-12, mgcu.PREC_MIXED: 1e-9, mgcu.PREC_FP32: 1e-4}
+
+
+def _both(lib, call, tile_bits):
+    """the factored result and the general kernels'"""
+    out = []
+    for threads in (0, 256):
+        lib.set_option(mgcu.OPT_THREADS, threads)
+        lib.set_option(mgcu.OPT_TILE_BITS, tile_bits)
+        try:
+            out.append(call())
+        finally:
+            lib.set_option(mgcu.OPT_THREADS, 0)
+            lib.set_option(mgcu.OPT_TILE_BITS, 0)
+    return out
+
+
+def _check(out, tol):
+    (rc0, f0, dv0), (rc1, f1, dv1) = out
+    assert rc0 == 0 and rc1 == 0
+    assert abs(f0 - f1) <= tol * max(abs(f1), np.max(np.abs(dv1)))
+    assert np.max(np.abs(dv0 - dv1)) <= tol * np.max(np.abs(dv1))
+
+
+def _layers(kind, n, rng):
+    if kind == "haar":
+        return T.haar_matchgates(n, rng)
+    if kind == "near":
+        return T.near_identity_brickwall(n, rng)
+    v = T.haar_matchgates(n, rng)
+    if kind == "special":   # diagonal, antidiagonal, identity and swapped blocks
+        for i in range(n):
+            c, k = [([1, 0, 0, 1j], [0, 1, 1j, 0]), ([0, 1, 1, 0], [1, 0, 0, 1]), ([1, 0, 0, 1], v[i, 4:]),
+                    (v[i, :4], [1, 0, 0, -1])][i % 4]
+            v[i] = np.concatenate([c, k])
+    if kind == "scaled":    # not unitary, well conditioned
+        v = v * (1 + 0.3 * rng.uniform(-1, 1, size=v.shape))
+    if kind == "singular":  # does not factor
+        v[n // 2, :4] = [1, 1, 1, 1]
+    return v
+
+
+@pytest.mark.parametrize("prec", [mgcu.PREC_FP64, mgcu.PREC_MIXED, mgcu.PREC_FP32])
+@pytest.mark.parametrize("L,nl,kind,tile_bits,cols", [
+    (10, 1, "haar", 0, None), (10, 5, "near", 0, None), (10, 4, "special", 0, (3, 1001)), (10, 3, "scaled", 6, None),
+    (10, 3, "singular", 0, None), (10, 4, "haar", 5, None), (12, 3, "special", 7, (100, 1900)), (12, 6, "haar", 0, (5, 6)),
+    (14, 2, "haar", 0, (4000, 4500)), (16, 2, "haar", 0, (30000, 30100))])
+def test_brickwall_gradient(mglib, L, nl, kind, tile_bits, cols, prec):
+    lib, rng = mglib, np.random.default_rng(L + nl)
+    v, perms = _layers(kind, nl, rng), T.brickwall_perms(L, nl)
+    t = lib.target_brickwall(T.haar_matchgates(4, rng), T.brickwall_perms(L, 4), L)
+    lib.set_precision(prec)
+    try:
+        _check(_both(lib, lambda: lib.brickwall_columns(lib.mg_target_apply, t, v, perms, L, *(cols or (0, 1 << L))), tile_bits), TOL[prec])
+    finally:
+        lib.set_precision(mgcu.PREC_FP64)
+        lib.target_free(t)
+
+
+@pytest.mark.parametrize("prec", [mgcu.PREC_FP64, mgcu.PREC_MIXED, mgcu.PREC_FP32])
+@pytest.mark.parametrize("L,ng,tile_bits,grad", [(11, 1, 0, True), (11, 23, 0, True), (12, 17, 6, True), (13, 31, 0, True),
+                                                 (12, 40, 0, False), (13, 29, 8, False)])
+def test_circuit(mglib, L, ng, tile_bits, grad, prec):
+    lib, rng = mglib, np.random.default_rng(L + ng)
+    w = np.array([rng.choice(L, 2, replace=False) for _ in range(ng)], np.int32)   # any pairs, both orders, some on wire L - 1
+    w[: ng // 3, 1] = L - 1
+    w[: ng // 3, 0] = rng.integers(0, L - 1, size=ng // 3)
+    w[::2] = w[::2, ::-1]
+    g = T.haar_matchgates(ng, rng)
+    u = T.haar_matchgates(20, rng)
+    uw = np.array([rng.choice(L, 2, replace=False) for _ in range(20)], np.int32)
+    t = lib.target_circuit(u, uw, L)
+    lib.set_precision(prec)
+    try:
+        if grad:
+            out = _both(lib, lambda: lib.circuit_target_and_gradient(lib.mg_target_apply, t, g, w, L), tile_bits)
+        else:
+            out = [(rc, f, np.ones(1) * np.sqrt(2.0 ** L)) for rc, f in _both(lib, lambda: lib.circuit_target(lib.mg_target_apply, t, g, w, L), tile_bits)]
+        _check(out, TOL[prec])
+    finally:
+        lib.set_precision(mgcu.PREC_FP64)
+        lib.target_free(t)
