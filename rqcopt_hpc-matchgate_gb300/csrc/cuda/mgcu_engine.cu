@@ -2550,15 +2550,30 @@ static int launch_columns(mgcu_plan* p, long b0, long b1, const typename P::T* d
 		w.bases = f.d_bases.as<unsigned>();
 		w.gates = f.d_gates.as<FitGate<T>>(); w.tables = f.d_tab.as<T>(); w.final = w.tables + (size_t)2 * p->S * f.nflush;
 		w.dense = dense; w.dense_b0 = dense_b0; w.b0 = b0; w.b1 = b1;
-		w.su = p->su.as<T>(); w.sw = p->sw.as<T>(); w.cache = f.cache.as<T>();
-		w.part = p->d.want_grad ? p->part_g.as<double>() : p->part_f.as<double>();
+		const bool wg = p->d.want_grad || p->d.want_hess;
+		w.su = p->su.as<T>(); w.sw = p->sw.as<T>();
+		w.cache = p->d.want_hess ? p->cache.as<T>() : f.cache.as<T>();
+		w.dcache = p->d.want_hess ? p->dcache.as<T>() : nullptr;
+		w.slot_per_column = p->d.want_hess ? 1 : 0;
+		w.part = wg ? p->part_g.as<double>() : p->part_f.as<double>();
 		w.nblocks = p->d.nblocks;
 		const int gf = (int)std::min<long>(f.grid, (ncols + f.nc - 1) / f.nc);
-		fit_kernel<P>(f.qc, p->d.want_grad != 0, f.threads)<<<gf, f.threads, f.smem, mgcu_stream()>>>(w);
+		fit_kernel<P>(f.qc, wg, f.threads)<<<gf, f.threads, f.smem, mgcu_stream()>>>(w);
 		MGCU_LAUNCHED();
+		if (p->d.want_hess)
+		{
+			FitHessArgs<P> h;
+			h.f = w;
+			h.place = p->d_place.as<int>(); h.place_group = f.d_pgroup.as<int>(); h.place_w = p->d_placew.as<double>();
+			h.block = p->d_block.as<int>(); h.nplace = p->d.nplace; h.ngates = p->d.ngates; h.mdim = 8 * p->d.nblocks;
+			h.hgroup = p->hgroup ? 1 : 0; h.part_h = p->part_h.as<double>();
+			const long nitems = (ncols + f.nc - 1) / f.nc * p->d.nplace * 8;
+			fit_hess_kernel<P>(f.qc, f.threads)<<<(int)std::min<long>(f.grid_h, nitems), f.threads, f.smem, mgcu_stream()>>>(h, nitems);
+			MGCU_LAUNCHED();
+		}
 		return 0;
 	}
-	if (p->fit.built && !p->d.want_hess && p->d.want_grad)
+	if (p->fit.built && p->d.want_grad && !p->d.want_hess)
 	{
 		// gates that do not factor: the cached sweep, its cache allocated on first need
 		const int e = p->cache.alloc((size_t)p->S * p->tsize * std::max(p->d.ngates, 1) * p->grid_a);
@@ -2607,8 +2622,12 @@ static int set_smem_attr()
 	void (*const wk[2])(Args<P>) = { k_target_w<P, 128, 2>, k_target_w<P, 256, 1> };
 	for (auto k : wk) MGCU_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min<size_t>(c->smem_optin, 227 * 1024)));
 	if constexpr (P::kId != MG_PREC_FP32_ID)
-	for (int q = 0; q < 12; q++)
-		MGCU_TRY(cudaFuncSetAttribute(fit_kernel<P>(q & 1, q & 2, 128 << (q >> 2)), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min<size_t>(c->smem_optin, 227 * 1024) - 4096));
+		for (int q = 0; q < 12; q++)
+		{
+			const int lim = (int)std::min<size_t>(c->smem_optin, 227 * 1024) - 4096;
+			MGCU_TRY(cudaFuncSetAttribute(fit_kernel<P>(q & 1, q & 2, 128 << (q >> 2)), cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+			if (!(q & 2)) MGCU_TRY(cudaFuncSetAttribute(fit_hess_kernel<P>(q & 1, 128 << (q >> 2)), cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+		}
 	MGCU_TRY(cudaFuncSetAttribute(k_hessian<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min<size_t>(c->smem_optin, 227 * 1024)));
 	return 0;
 }
@@ -2702,6 +2721,10 @@ static int tune_target_sweep(mgcu_plan* p)
 	p->threads_t = best[0]; p->nq_t = best[1]; p->smem_t = target_smem_bytes(p, best[0]);
 	return 0;
 }
+
+// Hessians take the factored items from L = 7 (whole evaluation: per-gate L = 7 float-float 550
+// against 1011 us, per-layer L = 8 533 against 1010 us; per-layer L = 6 414 against 385 us)
+constexpr int FIT_HESS_MIN_L = 7;
 
 extern "C" mgcu_plan* mgcu_plan_create(const mgcu_plan_desc* d)
 {
@@ -2892,30 +2915,50 @@ extern "C" mgcu_plan* mgcu_plan_create(const mgcu_plan_desc* d)
 	// against 336 us), while the tables are small.  FP32 keeps the general kernels: there the
 	// factors' rounding is as large as the sweep's.  An explicit block size keeps them too
 	e = 0;
-	if (!d->want_hess && !p->adj && d->ngates > 0 && d->L <= 18 && opt_thr <= 0 && p->prec != MG_PREC_FP32_ID
-		&& d->L >= (d->want_grad ? 10 : 12))
+	// (Hessians: one tile, L <= 14)
+	const bool fit_grad = d->want_grad || d->want_hess;
+	if (!p->adj && d->ngates > 0 && opt_thr <= 0 && p->prec != MG_PREC_FP32_ID
+		&& (d->want_hess ? (d->L >= FIT_HESS_MIN_L && d->L <= 14 && opt_kt <= 0) : (d->L >= (d->want_grad ? 10 : 12) && d->L <= 18)))
 	{
 		p->fit.kt = p->kt;
 		// a sector of at most 128 KB is one tile (float-float L=14, 9 layers: 73 ms on 512 threads
 		// against 87 ms in two 64 KB tiles), a larger one tiles of 64 KB (L=16, 5 layers, 6001
 		// columns: 81 ms against 87 ms in tiles of 128 KB, one block per SM)
 		if (opt_kt <= 0 && p->nb <= 13) p->fit.kt = p->nb;
-		e = fit_build(p->L, p->fit.kt, p->wires.data(), d->ngates, p->block.data(), d->nblocks, (int)p->tsize, p->fit);
+		e = fit_build(p->L, p->fit.kt, p->wires.data(), d->ngates, p->block.data(), d->nblocks, (int)p->tsize, d->want_hess != 0, p->fit);
 		int per = 0;
 		if (!e)
 		{
 			auto occ = [&](auto k) { return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, p->fit.threads, p->fit.smem) != cudaSuccess; };
-			const bool g = d->want_grad != 0;
+			const bool g = fit_grad;
 			if (p->prec == MG_PREC_FP64_ID ? occ(fit_kernel<PrecD>(true, g, p->fit.threads)) : occ(fit_kernel<PrecX>(true, g, p->fit.threads)))
 				e = MG_ERR_DEVICE;
 		}
 		if (e) { delete p; return nullptr; }
 		if (opt_cps > 0) per = (int)std::min<long>(per, opt_cps);
+		if (d->want_hess)
+		{
+			int ph = 0;
+			auto occ = [&](auto k) { return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ph, k, p->fit.threads, p->fit.smem) != cudaSuccess; };
+			if (p->prec == MG_PREC_FP64_ID ? occ(fit_hess_kernel<PrecD>(true, p->fit.threads)) : occ(fit_hess_kernel<PrecX>(true, p->fit.threads)))
+			{
+				mg_set_error("occupancy of the Hessian items kernel");
+				delete p;
+				return nullptr;
+			}
+			if (opt_cps > 0) ph = (int)std::min<long>(ph, opt_cps);
+			p->fit.grid_h = c->nsm * std::max(ph, 1);
+			std::vector<int> pg(std::max(p->d.nplace, 1), 0);
+			for (int q = 0; q < p->d.nplace; q++) pg[q] = p->fit.group_of_gate[p->place[q]];
+			e = p->fit.d_pgroup.alloc(sizeof(int) * pg.size());
+			if (!e && cudaMemcpy(p->fit.d_pgroup.p, pg.data(), sizeof(int) * pg.size(), cudaMemcpyHostToDevice) != cudaSuccess) e = MG_ERR_DEVICE;
+			if (e) { delete p; return nullptr; }
+		}
 		const size_t slot = (size_t)p->fit.group.size() * p->fit.nc * col_bytes;
 		long gf = std::min((long)c->nsm * std::max(per, 1), (ncols_total + p->fit.nc - 1) / p->fit.nc);
-		if (d->want_grad) gf = std::max(1L, std::min(gf, (long)((32ull << 30) / slot)));
+		if (fit_grad && !d->want_hess) gf = std::max(1L, std::min(gf, (long)((32ull << 30) / slot)));
 		p->fit.grid = (int)gf;
-		if (d->want_grad) e = p->fit.cache.alloc(slot * gf);
+		if (fit_grad && !d->want_hess) e = p->fit.cache.alloc(slot * gf);
 		if (e) { delete p; return nullptr; }
 	}
 	const long rows = std::max<long>(grid, p->fit.grid);
@@ -2925,17 +2968,19 @@ extern "C" mgcu_plan* mgcu_plan_create(const mgcu_plan_desc* d)
 	if (!e) e = upload_sched(p->ws, p->d_pass, p->d_gate);
 	if (!e) e = p->su.alloc(col_bytes * rows);
 	if (!e) e = p->sw.alloc(col_bytes * rows);
-	if (!e && grad && !p->adj && !p->fit.built) e = p->cache.alloc(col_bytes * ng * (d->want_hess ? chunk : grid));
+	const size_t ccols = d->want_hess ? (size_t)chunk + (p->fit.built ? p->fit.nc : 0) : (size_t)grid;   // whole blocks of columns
+	if (!e && grad && !p->adj && (d->want_hess || !p->fit.built)) e = p->cache.alloc(col_bytes * ng * ccols);
 	if (!e && p->adj) e = p->ck.alloc(col_bytes * p->ws.pass.size() * grid);
-	if (!e && d->want_hess) e = p->dcache.alloc(col_bytes * ng * chunk);
+	if (!e && d->want_hess) e = p->dcache.alloc(col_bytes * ng * ccols);
 	if (!e && d->want_hess) e = p->sh.alloc(col_bytes * p->grid_b);
 	if (!e) e = p->part_f.alloc(sizeof(double) * 2 * rows);
 	if (!e) e = p->part_g.alloc(sizeof(double) * 16 * ng * rows);
-	if (!e && d->want_hess) e = p->part_h.alloc(sizeof(double) * 2 * (size_t)mdim * mdim * p->grid_b);
+	if (!e && d->want_hess) e = p->part_h.alloc(sizeof(double) * 2 * (size_t)mdim * mdim * std::max(p->grid_b, p->fit.grid_h));
 	if (!e) e = p->out_f.alloc(sizeof(double) * 2);
 	if (!e) e = p->out_g.alloc(sizeof(double) * 16 * ng);
 	if (!e) e = p->out_blk.alloc(sizeof(double) * 16 * std::max(d->nblocks, 1));
 	if (!e && d->want_hess) e = p->out_h.alloc(sizeof(double) * 2 * (size_t)mdim * mdim);
+	if (!e && d->want_hess && p->fit.built) e = p->fit.cache.alloc(sizeof(double) * 2 * (size_t)mdim * mdim);   // the Hessian in moves
 	if (!e) e = p->d_block.alloc(sizeof(int) * ng);
 	if (!e) e = p->d_pass_of.alloc(sizeof(int) * ng);
 	if (!e) e = p->cols.alloc(col_bytes * chunk);
@@ -3051,10 +3096,21 @@ extern "C" int mgcu_plan_finish(mgcu_plan* p)
 	MgcuContext* c = mgcu_ctx();
 	cudaStream_t st = mgcu_stream();
 	const int ng = std::max(p->d.ngates, 1);
-	if (p->fit.ok && p->d.want_grad)
+	if (p->fit.ok && (p->d.want_grad || p->d.want_hess))
 	{
 		k_fit_finish<<<p->d.nblocks, 128, 0, st>>>(p->part_g.as<double>(), p->fit.grid, p->d.nblocks, p->fit.d_blk.as<FitBlock>(),
 			p->out_f.as<double>(), p->out_blk.as<double>());
+		MGCU_LAUNCHED();
+		if (!p->d.want_hess) return 0;
+		const long mdim = 8L * p->d.nblocks;
+		double2* A = p->fit.cache.as<double2>();
+		k_sum_parts<<<grid_cap(2 * mdim * mdim, 128), 128, 0, st>>>(p->part_h.as<double>(), p->fit.grid_h, 2 * mdim * mdim, p->fit.cache.as<double>());
+		MGCU_LAUNCHED();
+		k_fit_hess_finish<<<grid_cap(mdim * mdim, 128), 128, 0, st>>>(A, p->d.nblocks, p->fit.d_blk.as<FitBlock>(), p->out_h.as<double2>());
+		MGCU_LAUNCHED();
+		k_symm_diag<<<grid_cap(mdim * mdim, 256), 256, 0, st>>>(p->d.nblocks, p->out_h.as<double2>());
+		MGCU_LAUNCHED();
+		k_mirror<<<grid_cap(mdim * mdim, 256), 256, 0, st>>>(p->d.nblocks, p->out_h.as<double2>());
 		MGCU_LAUNCHED();
 		return 0;
 	}

@@ -37,6 +37,7 @@ struct FitGroup
 	int cbit[14];         // compact bits: register bits 0..3, then the unit-index bits
 	int ga, gb, kind_b;   // gates (-1: none)
 	int rev;              // gate b is on the dropped qubit as wire i: its center pair is (z, y)
+	int order;            // 1: gate b comes before gate a in the sequence
 	int blk_a, blk_b;
 	int blk_next;         // block of the first sum of the group before (gate b's, if it has one)
 	int flush;            // table multiplied in before the gates (-1: none)
@@ -84,7 +85,9 @@ struct FitArgs
 	long dense_b0, b0, b1;
 	T* su;
 	T* sw;
-	T* cache;                   // [block][group][column of the block][S]
+	T* cache;                   // [slot][group][column of the block][S]
+	T* dcache;                  // the derivatives, alike (Hessian plans; else null)
+	int slot_per_column;        // slot: the block's columns, counted from b0 (1), or the block (0)
 	double* part;               // [block][nblocks][16] (gradient) or [block][2]
 	int nblocks;
 };
@@ -265,9 +268,11 @@ __device__ __forceinline__ void fit_group(const FitGroup& G, const FitGate<typen
 // derivative in the tile and the cached state ct, read one quartet ahead.  One loop for every
 // kind of gate, not unrolled: with each gate's quartets unrolled the kernel's code outgrew the
 // instruction caches (a third of its stalls).
-template <class P>
+// eout (or null): the derivative also to its cache, with the last gate.  SW: the tile holds the
+// state and ct the derivative (Hessian items)
+template <class P, bool SW = false>
 __device__ __forceinline__ void fit_contract(const FitGroup& G, int first, int last, unsigned tc, unsigned base,
-	const typename P::T* __restrict__ ct, typename P::Acc (&acc)[8])
+	const typename P::T* __restrict__ ct, typename P::Acc (&acc)[8], typename P::T* __restrict__ eout = nullptr)
 {
 	typedef typename P::T T;
 	const char* cb = reinterpret_cast<const char*>(ct);
@@ -282,6 +287,13 @@ __device__ __forceinline__ void fit_contract(const FitGroup& G, int first, int l
 		const uint4 o = qs[i];
 		const T x = lds<T>(tc + (base ^ o.x)), y = lds<T>(tc + (base ^ o.y)), z = lds<T>(tc + (base ^ o.z)), v = lds<T>(tc + (base ^ o.w));
 		const T sx = cx, sy = cy, sz = cz, sv = cw;
+		if (!SW && eout && (i >> 2) == last)
+		{
+			const uint4 q = qy[i];
+			char* eb = reinterpret_cast<char*>(eout);
+			*reinterpret_cast<T*>(eb + q.x) = x; *reinterpret_cast<T*>(eb + q.y) = y;
+			*reinterpret_cast<T*>(eb + q.z) = z; *reinterpret_cast<T*>(eb + q.w) = v;
+		}
 		i = (i + 1) & 7;   // gate b's quartets 4..7, then gate a's 0..3
 		if (k > 1)
 		{
@@ -289,7 +301,8 @@ __device__ __forceinline__ void fit_contract(const FitGroup& G, int first, int l
 			cx = *reinterpret_cast<const T*>(cb + oy.x); cy = *reinterpret_cast<const T*>(cb + oy.y);
 			cz = *reinterpret_cast<const T*>(cb + oy.z); cw = *reinterpret_cast<const T*>(cb + oy.w);
 		}
-		contract_quartet<P>(acc, x, v, y, z, sx, sv, sy, sz);
+		if (SW) contract_quartet<P>(acc, sx, sv, sy, sz, x, v, y, z);
+		else contract_quartet<P>(acc, x, v, y, z, sx, sv, sy, sz);
 	}
 }
 
@@ -318,7 +331,6 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 	const unsigned colb = mycol * n * ES;
 	T* su = a.su + (size_t)blockIdx.x * S;
 	T* sw = a.sw + (size_t)blockIdx.x * S;
-	T* cache = GRAD ? a.cache + (size_t)blockIdx.x * a.ngroups * nc * S + (size_t)mycol * S : nullptr;
 	const size_t cstride = (size_t)nc * S;
 	typename P::Acc acc[8];
 #pragma unroll
@@ -331,6 +343,8 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 		// this thread's column (the last one again past the range: its derivative is zero)
 		const long b = min(cb + (long)mycol, a.b1 - 1);
 		const int par = __popcll(b) & 1;
+		const size_t coff = (size_t)(a.slot_per_column ? (cb - a.b0) / nc : blockIdx.x) * a.ngroups * cstride + (size_t)mycol * S;
+		T* cache = GRAD ? a.cache + coff : nullptr;
 		for (int p = 0; p < a.npass; p++)
 		{
 			const PassRec& pr = a.pass[p];
@@ -422,6 +436,7 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 					const FitGroup& G = stage[g & 1].g;
 					if (g > fp.gbeg) fit_stage<T>(stage[(g - 1) & 1], a.groups + g - 1, a.gates + 2 * (g - 1));
 					const T* cg = cache + (size_t)g * cstride + ((size_t)tau << kt) + u0;
+					T* eg = a.dcache ? a.dcache + coff + (size_t)g * cstride + ((size_t)tau << kt) + u0 : nullptr;
 					const T* tab = G.flush >= 0 ? a.tables + ((size_t)(2 * G.flush + par) * S + ((size_t)tau << kt) + u0) : nullptr;
 					const int blk = G.ga >= 0 ? G.blk_a : G.blk_b;
 					if (g > fp.gbeg)
@@ -444,7 +459,7 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 					}
 					for (unsigned i = 0; i < its; i++)
 						fit_contract<P>(G, (G.kind_b && !split) ? 1 : 0, G.ga >= 0 ? 0 : 1, tb + colb,
-							fit_base(G, a.bases + (size_t)g * U, u0 + i * FIT_NT, tpar), cg + i * FIT_NT, acc);
+							fit_base(G, a.bases + (size_t)g * U, u0 + i * FIT_NT, tpar), cg + i * FIT_NT, acc, eg ? eg + i * FIT_NT : nullptr);
 					if (g > 0)   // nothing uses the derivative before the first group
 						for (unsigned i = 0; i < its; i++)
 							fit_group<P, QC, true>(G, stage[g & 1].gate, tb + colb, fit_base(G, a.bases + (size_t)g * U, u0 + i * FIT_NT, tpar),
@@ -482,6 +497,158 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 		}
 	}
 	if (!GRAD) block_reduce1<P>(facc, s.red, a.part + (size_t)blockIdx.x * 2);
+}
+
+// ------------------------------------------------------------------------------------
+// Hessian items in factored form.  An item (placement, entry (r, u), a block's columns) carries
+// the tangent state B of moving amplitude u of the placement gate's pair onto r after its M:
+// B starts as that move of the cached state, passes through the later groups, and at each later
+// gate sum E_r' B_u' with the cached derivative gives the second derivative between the two
+// moves.  Grouped placements (see k_hessian): every gate of the placement's block adds its move,
+// after its own sum.  k_fit_hess_finish turns moves into gate entries.  Per gate and amplitude
+// 124 FP32 operations in float-float (176 unfactored) or 10.7 FP64 operations (16).  Measured
+// against k_hessian (which stays for FP32, several tiles and gates that do not factor):
+// translation-invariant L=12, 9 layers, float-float 152 -> 101 ms; per-layer L=12, 5 layers,
+// complex128 169 -> 128 ms (81 % of the FP64 rate); per-gate L=9, 19 gates, float-float
+// 3.97 -> 2.45 ms.
+// ------------------------------------------------------------------------------------
+template <class P>
+struct FitHessArgs
+{
+	FitArgs<P> f;
+	const int* place;          // placement gates
+	const int* place_group;    // their groups
+	const double* place_w;     // [nplace][ngates]
+	const int* block;          // [ngates]
+	int nplace, ngates, mdim, hgroup;
+	double* part_h;            // [grid][mdim][mdim][2]
+};
+
+// adds (init: sets, the rest of the unit zero) the move of entry x of gate w: one amplitude of
+// each quartet gains another of the cached state
+template <class P>
+__device__ __forceinline__ void fit_move(const FitGroup& G, int w, int x, unsigned tc, unsigned base, const typename P::T* __restrict__ ct, bool init)
+{
+	typedef typename P::T T;
+	const char* cb = reinterpret_cast<const char*>(ct);
+#pragma unroll 1
+	for (int i = 0; i < 4; i++)
+	{
+		const uint4 o = G.qs[w][i], q = G.qy[w][i];
+		const unsigned to = x < 4 ? ((x & 2) ? o.z : o.y) : ((x & 2) ? o.w : o.x);
+		const unsigned from = x < 4 ? ((x & 1) ? q.z : q.y) : ((x & 1) ? q.w : q.x);
+		const T v = *reinterpret_cast<const T*>(cb + from);
+		if (init)
+		{
+			const T zero = P::zero();
+			sts<T>(tc + (base ^ o.x), zero); sts<T>(tc + (base ^ o.y), zero);
+			sts<T>(tc + (base ^ o.z), zero); sts<T>(tc + (base ^ o.w), zero);
+			sts<T>(tc + (base ^ to), v);
+		}
+		else sts<T>(tc + (base ^ to), P::add(lds<T>(tc + (base ^ to)), v));
+	}
+}
+
+template <class P, bool QC, int FIT_NT>
+__global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 : P::kId == MG_PREC_FP64_ID ? 3 : 4) k_fit_hess(FitHessArgs<P> h, long nitems)
+{
+	typedef typename P::T T;
+	constexpr unsigned ES = sizeof(T);
+	extern __shared__ __align__(16) char smem_raw[];
+	__shared__ FitStage<T> stage[2];
+	const FitArgs<P>& a = h.f;
+	const int kt = a.kt, nu = kt - 4, nc = a.nc;
+	const unsigned U = 1u << nu, n = 1u << kt;
+	const unsigned its = U > FIT_NT ? U / FIT_NT : threadIdx.x < U * nc ? 1 : 0;
+	const unsigned tb = smem_u32(smem_raw);
+	double* red = reinterpret_cast<double*>(smem_raw + (size_t)ES * n * nc + 256 * sizeof(unsigned));
+	const unsigned mycol = min(threadIdx.x >> nu, (unsigned)nc - 1), u0 = nc > 1 ? (threadIdx.x & (U - 1)) : threadIdx.x;
+	const unsigned tc = tb + mycol * n * ES;
+	const size_t cstride = (size_t)nc * a.S;
+	double* parth = h.part_h + (size_t)blockIdx.x * h.mdim * h.mdim * 2;
+	typename P::Acc acc[8];
+#pragma unroll
+	for (int e = 0; e < 8; e++) acc[e] = P::acc_zero();
+	int nred = 0;
+
+	for (long it = blockIdx.x; it < nitems; it += gridDim.x)
+	{
+		const int x = (int)(it & 7);
+		const long rest = it >> 3;
+		const int p = (int)(rest % h.nplace);
+		const long cgi = rest / h.nplace;
+		const long b = min(a.b0 + cgi * nc + (long)mycol, a.b1 - 1);
+		const int par = __popcll(b) & 1;
+		const int k = h.place[p], g0 = h.place_group[p];
+		const int grp = h.hgroup ? h.block[k] : -1;
+		const double* wrow = h.place_w + (size_t)p * h.ngates;
+		double* hrow = parth + (size_t)(h.block[k] * 8 + x) * h.mdim * 2;
+		const size_t coff = (size_t)cgi * a.ngroups * cstride + (size_t)mycol * a.S + u0;
+		// the sums in acc: of gates of block cblk with weight cw (none: -1)
+		int cblk = -1, merged = 0;
+		double cw = 0;
+		auto flush = [&]() {
+			if (cblk < 0) return;
+			block_reduce8<P>(acc, red, hrow + (size_t)cblk * 16, cw, nred);
+#pragma unroll
+			for (int e = 0; e < 8; e++) acc[e] = P::acc_zero();
+			cblk = -1;
+			merged = 0;
+		};
+		__syncthreads();   // the previous item's last reads
+		fit_stage<T>(stage[g0 & 1], a.groups + g0, a.gates + 2 * g0);
+		fit_stage_wait();
+		__syncthreads();
+		for (int g = g0; g < a.ngroups; g++)
+		{
+			const FitGroup& G = stage[g & 1].g;
+			if (g + 1 < a.ngroups) fit_stage<T>(stage[(g + 1) & 1], a.groups + g + 1, a.gates + 2 * (g + 1));
+			const T* cg = a.cache + coff + (size_t)g * cstride;
+			const T* eg = a.dcache + coff + (size_t)g * cstride;
+			const unsigned* bs = a.bases + (size_t)g * U;
+			// the group's gates in sequence order; in the first group those after the placement
+			const int ngt = (G.ga >= 0 && G.kind_b) ? 2 : 1, w0 = ngt == 2 ? G.order : (G.ga >= 0 ? 0 : 1);
+			int st = 0;
+			if (g == g0)
+			{
+				const int w = G.ga == k ? 0 : 1;
+				for (unsigned i = 0; i < its; i++)
+					fit_move<P>(G, w, x, tc, fit_base(G, bs, u0 + i * FIT_NT, par), cg + i * FIT_NT, true);
+				st = w == w0 ? 1 : 2;
+			}
+			else
+			{
+				const T* tab = G.flush >= 0 ? a.tables + (size_t)(2 * G.flush + par) * a.S + u0 : nullptr;
+				for (unsigned i = 0; i < its; i++)
+					fit_group<P, QC, false>(G, stage[g & 1].gate, tc, fit_base(G, bs, u0 + i * FIT_NT, par), tab ? tab + i * FIT_NT : nullptr, nullptr);
+			}
+#pragma unroll 1
+			for (; st < ngt; st++)
+			{
+				const int w = w0 ^ st;
+				const int blk = w ? G.blk_b : G.blk_a;
+				const double wg = wrow[w ? G.gb : G.ga];
+				if (cblk != blk || cw != wg) flush();
+				if (merged >= FIT_RENORM)
+				{
+#pragma unroll
+					for (int e = 0; e < 8; e++) P::acc_norm(acc[e]);
+					merged = 0;
+				}
+				cblk = blk; cw = wg;
+				merged += 4 * (int)max(its, 1u);
+				for (unsigned i = 0; i < its; i++)
+				{
+					const unsigned base = fit_base(G, bs, u0 + i * FIT_NT, par);
+					fit_contract<P, true>(G, w, w, tc, base, eg + i * FIT_NT, acc);
+					if (blk == grp) fit_move<P>(G, w, x, tc, base, cg + i * FIT_NT, false);
+				}
+			}
+			fit_stage_wait();
+			__syncthreads();
+		}
+		flush();
+	}
 }
 
 // complex products in double-double, for the tables of complex128 (every entry correctly rounded
@@ -598,5 +765,31 @@ __global__ void __launch_bounds__(128) k_fit_finish(const double* __restrict__ p
 	{
 		const int c = threadIdx.x - 8;
 		out_f[c] = ((R[0 + c] + R[6 + c]) + (R[8 + c] + R[14 + c])) / fb[0].ngates;
+	}
+}
+
+// summed parts of the Hessian in moves -> gate entries: both indices transformed as the gradient
+__global__ void k_fit_hess_finish(const double2* __restrict__ A, int nb, const FitBlock* __restrict__ fb, double2* __restrict__ H)
+{
+	const int m = nb * 8;
+	for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < m * m; q += gridDim.x * blockDim.x)
+	{
+		const int r = q / m, c = q % m, bi = r >> 3, bj = c >> 3, x = r & 7, y = c & 7;
+		double sr = 0, si = 0;
+		for (int u = 0; u < 2; u++)
+		{
+			const double* mu = fb[bi].minv[(x & 4) + 2 * (x & 1) + u];
+			for (int v = 0; v < 2; v++)
+			{
+				const double* mv = fb[bj].minv[(y & 4) + 2 * (y & 1) + v];
+				const double2 e = A[(long)(bi * 8 + (x & 6) + u) * m + bj * 8 + (y & 6) + v];
+				const double wr = mu[0] * mv[0] - mu[1] * mv[1], wi = mu[0] * mv[1] + mu[1] * mv[0];
+				sr += e.x * wr - e.y * wi;
+				si += e.x * wi + e.y * wr;
+			}
+		}
+		const double *ci = fb[bi].scale[x], *cj = fb[bj].scale[y];
+		const double wr = ci[0] * cj[0] - ci[1] * cj[1], wi = ci[0] * cj[1] + ci[1] * cj[0];
+		H[q] = make_double2(sr * wr - si * wi, sr * wi + si * wr);
 	}
 }

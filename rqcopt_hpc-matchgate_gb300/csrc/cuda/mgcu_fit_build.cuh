@@ -12,9 +12,11 @@ struct FitProg
 	std::vector<std::array<int, 2>> diag;   // per table entry factor: gate, 0 left / 1 right
 	std::vector<int> beg, group_of;         // per flush (the last: the final table)
 	std::vector<int> block_gates;           // gates per block
+	std::vector<int> group_of_gate;
+	int grid_h = 0;                         // k_fit_hess blocks
 	int nflush = 0, grid = 0, nc = 1, threads = 128, kt = 0;
 	size_t smem = 0;
-	DevBuf d_pass, d_group, d_pgroups, d_gates, d_diag, d_beg, d_gof, d_tab, d_blk, d_bases, cache;
+	DevBuf d_pass, d_group, d_pgroups, d_gates, d_diag, d_beg, d_gof, d_tab, d_blk, d_bases, d_pgroup, cache;
 };
 
 // wires of gate g as a mask
@@ -23,11 +25,12 @@ static unsigned fit_wires(const int* w, int g) { return (1u << w[2 * g]) | (1u <
 // Passes as for the other sweeps (reordered: commuting gates only), then groups of up to two
 // gates within a pass, then flushes: before a group whose right factors are not merged yet, one
 // table of all pending left factors and of the right factors of every gate that comes next on
-// both of its wires (one flush per brickwall layer when the sector is one tile).
-static int fit_build(int L, int kt, const int* wires, int ng, const int* block, int nblocks, int es, FitProg& f)
+// both of its wires (one flush per brickwall layer when the sector is one tile).  ordered
+// (Hessians, one tile): the groups keep the sequence of the gates.
+static int fit_build(int L, int kt, const int* wires, int ng, const int* block, int nblocks, int es, bool ordered, FitProg& f)
 {
 	const int nb = L - 1;
-	schedule(L, kt, wires, ng, true, f.sched, 1);
+	schedule(L, kt, wires, ng, !ordered, f.sched, 1);
 	std::vector<std::vector<int>> onq(L);
 	for (int g = 0; g < ng; g++) { onq[wires[2 * g]].push_back(g); onq[wires[2 * g + 1]].push_back(g); }
 	std::vector<size_t> next(L, 0);
@@ -35,6 +38,7 @@ static int fit_build(int L, int kt, const int* wires, int ng, const int* block, 
 	std::vector<char> cdone(ng, 0);
 	std::vector<int> pending;
 	f.group.clear(); f.pass_groups.clear(); f.diag.clear(); f.beg.assign(1, 0); f.group_of.clear();
+	f.group_of_gate.assign(ng, 0);
 	const unsigned pers = 3;   // swizzle period of the tile bits
 	for (size_t p = 0; p < f.sched.pass.size(); p++)
 	{
@@ -53,6 +57,7 @@ static int fit_build(int L, int kt, const int* wires, int ng, const int* block, 
 			{
 				if (!(fit_wires(wires, rest[i]) & used)) { b = rest[i]; at = i; }
 				used |= fit_wires(wires, rest[i]);
+				if (ordered) break;
 			}
 			if (b >= 0) rest.erase(rest.begin() + at);
 			rest.erase(rest.begin());
@@ -66,6 +71,7 @@ static int fit_build(int L, int kt, const int* wires, int ng, const int* block, 
 			G.kind_b = b < 0 ? 0 : (rec[b]->type == 0 ? 1 : 2);
 			G.rev = b >= 0 && rec[b]->type == 2;
 			G.pass = (int)p;
+			G.order = a >= 0 && b >= 0 && b < a;
 			G.blk_next = f.group.empty() ? -1 : (f.group.back().kind_b ? f.group.back().blk_b : f.group.back().blk_a);
 			int bits[14], n = 0;
 			unsigned in = 0;
@@ -150,6 +156,7 @@ static int fit_build(int L, int kt, const int* wires, int ng, const int* block, 
 			for (int s : { a, b })
 				if (s >= 0)
 				{
+					f.group_of_gate[s] = (int)f.group.size();
 					pending.push_back(s);
 					next[wires[2 * s]]++; next[wires[2 * s + 1]]++;
 				}
@@ -366,4 +373,12 @@ template <class P>
 static void (*fit_kernel(bool qc, bool grad, int threads))(FitArgs<P>)
 {
 	return threads == 512 ? fit_kernel_nt<P, 512>(qc, grad) : threads == 256 ? fit_kernel_nt<P, 256>(qc, grad) : fit_kernel_nt<P, 128>(qc, grad);
+}
+
+template <class P>
+static void (*fit_hess_kernel(bool qc, int threads))(FitHessArgs<P>, long)
+{
+	return threads == 512 ? (qc ? k_fit_hess<P, true, 512> : k_fit_hess<P, false, 512>)
+		: threads == 256 ? (qc ? k_fit_hess<P, true, 256> : k_fit_hess<P, false, 256>)
+		: (qc ? k_fit_hess<P, true, 128> : k_fit_hess<P, false, 128>);
 }

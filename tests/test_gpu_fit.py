@@ -98,3 +98,40 @@ def test_circuit(mglib, L, ng, tile_bits, grad, prec):
     finally:
         lib.set_precision(mgcu.PREC_FP64)
         lib.target_free(t)
+
+
+@pytest.mark.parametrize("prec", [mgcu.PREC_FP64, mgcu.PREC_MIXED])
+@pytest.mark.parametrize("L,nl,kind,ti", [(8, 1, "haar", False), (8, 4, "special", False), (8, 4, "scaled", True), (10, 3, "haar", True),
+                                          (10, 5, "near", False), (8, 3, "singular", False), (12, 2, "haar", False)])
+def test_layer_hessian(mglib, L, nl, kind, ti, prec):
+    """factored Hessian items against k_hessian's; the same tolerances, relative to the largest entry"""
+    lib, rng = mglib, np.random.default_rng(L + nl)
+    v, perms = _layers(kind, nl, rng), T.brickwall_perms(L, nl)
+    t = lib.target_brickwall(T.haar_matchgates(4, rng), T.brickwall_perms(L, 4), L)
+    lib.set_precision(prec)
+    try:
+        out = _both(lib, lambda: lib.brickwall_target_gradient_hessian(lib.mg_target_apply, t, v, perms, L, ti=ti), 0)
+    finally:
+        lib.set_precision(mgcu.PREC_FP64)
+        lib.target_free(t)
+    _check([o[:3] for o in out], TOL[prec])
+    assert np.max(np.abs(out[0][3] - out[1][3])) <= TOL[prec] * np.max(np.abs(out[1][3]))
+
+
+@pytest.mark.parametrize("prec", [mgcu.PREC_FP64, mgcu.PREC_MIXED])
+@pytest.mark.parametrize("L,ng", [(7, 1), (7, 20), (9, 17), (11, 9)])
+def test_gate_hessian(mglib, L, ng, prec):
+    lib, rng = mglib, np.random.default_rng(L + ng)
+    w = np.array([rng.choice(L, 2, replace=False) for _ in range(ng)], np.int32)
+    w[: ng // 3, 1], w[: ng // 3, 0] = L - 1, rng.integers(0, L - 1, size=ng // 3)
+    w[::2] = w[::2, ::-1]
+    g, u = T.haar_matchgates(ng, rng), T.haar_matchgates(20, rng)
+    t = lib.target_circuit(u, np.array([rng.choice(L, 2, replace=False) for _ in range(20)], np.int32), L)
+    lib.set_precision(prec)
+    try:
+        out = _both(lib, lambda: lib.circuit_target_gradient_hessian(lib.mg_target_apply, t, g, w, L), 0)
+    finally:
+        lib.set_precision(mgcu.PREC_FP64)
+        lib.target_free(t)
+    _check([o[:3] for o in out], TOL[prec])
+    assert np.max(np.abs(out[0][3] - out[1][3])) <= TOL[prec] * max(np.max(np.abs(out[1][3])), np.max(np.abs(out[1][2])))
