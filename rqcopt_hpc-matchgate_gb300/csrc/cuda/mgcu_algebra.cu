@@ -24,25 +24,34 @@ __global__ void k_project_grad(const mgg* __restrict__ v, const double* __restri
 	mgg_tangent_to_real(&v[i], &d, &grad[i * 8]);
 }
 
-// one thread per (i, j >= i, k): column k of block (i, j)
+// eight threads per (i, j >= i, k): column k of block (i, j), one row of the block's product with
+// the direction each (one thread per column spent 40 us on 64 dependent complex products)
 __global__ void k_project_hess(const mgg* __restrict__ v, const mgg* __restrict__ dvc, const double2* __restrict__ hess, int nb, double* __restrict__ H)
 {
-	const int t = blockIdx.x * blockDim.x + threadIdx.x;
-	if (t >= nb * nb * 8) return;
-	const int k = t % 8, ij = t / 8;
+	const int t = blockIdx.x * blockDim.x + threadIdx.x, x = t & 7;
+	const int col = min(t >> 3, nb * nb * 8 - 1), k = col % 8, ij = col / 8;   // every lane takes part in the shuffles
 	const int i = ij / nb, j = ij % nb;
-	if (j < i) return;
 	const int m = 8 * nb;
-	mgc h[64];
-	for (int x = 0; x < 8; x++)
-		for (int y = 0; y < 8; y++)
-		{
-			const double2 e = hess[(long)(i * 8 + x) * m + j * 8 + y];
-			h[x * 8 + y] = mgc_make(e.x, e.y);
-		}
+	mgc h[8];
+	for (int y = 0; y < 8; y++)
+	{
+		const double2 e = hess[(long)(i * 8 + x) * m + j * 8 + y];
+		h[y] = mgc_make(e.x, e.y);
+	}
+	mgg Z, G;
+	mg_hessian_direction(&v[j], k, &Z);
+	const mgc g = mg_hessian_row(h, &Z);
+	for (int q = 0; q < 4; q++)
+	{
+		G.c[q] = mgc_make(__shfl_sync(0xffffffffu, g.re, q, 8), __shfl_sync(0xffffffffu, g.im, q, 8));
+		G.k[q] = mgc_make(__shfl_sync(0xffffffffu, g.re, q + 4, 8), __shfl_sync(0xffffffffu, g.im, q + 4, 8));
+	}
 	double r[8];
-	mg_project_hessian_column(&v[i], &v[j], &dvc[i], i == j, h, k, r);
-	for (int x = 0; x < 8; x++) H[(long)(i * 8 + x) * m + j * 8 + k] = r[x];
+	mg_project_hessian_column(&v[i], &dvc[i], i == j, &Z, &G, r);
+	if ((t >> 3) >= nb * nb * 8 || j < i) return;
+	double rx = r[0];
+	for (int q = 1; q < 8; q++) if (q == x) rx = r[q];
+	H[(long)(i * 8 + x) * m + j * 8 + k] = rx;
 }
 
 __global__ void k_mirror_real(int m, double* __restrict__ H)
@@ -55,10 +64,35 @@ __global__ void k_mirror_real(int m, double* __restrict__ H)
 }
 
 // ---- retraction (reference src/matchgate.c:548-562) ----
+// two threads per gate, one per 2x2 block: mgg_retract with its Newton iteration's inverses and
+// divisions, a serial chain of FP64 latencies (150 us with one thread per gate), side by side;
+// both blocks stop together, as there
 __global__ void k_retract(const mgg* __restrict__ u, const double* __restrict__ eta, int n, mgg* __restrict__ v)
 {
-	const int i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i < n) mgg_retract(&u[i], &eta[i * 8], &v[i]);
+	const int t = blockIdx.x * blockDim.x + threadIdx.x, i = min(t >> 1, n - 1), corner = t & 1;
+	mgg z, w;
+	mgg_real_to_antisymm(&eta[i * 8], &z);
+	z.k[0].re += 1; z.c[0].re += 1; z.c[3].re += 1; z.k[3].re += 1;
+	mgg_mul(&u[i], &z, &w);
+	mgc cur[4];
+	for (int q = 0; q < 4; q++) cur[q] = corner ? w.k[q] : w.c[q];
+	bool done = false;
+	for (int it = 0; it < 14; it++)
+	{
+		mgc inv[4], h[4];
+		mg2_inv(cur, inv);
+		for (int r = 0; r < 2; r++)
+			for (int c = 0; c < 2; c++) h[2 * r + c] = mgc_conj(inv[2 * c + r]);
+		if (!done)
+			for (int q = 0; q < 4; q++) cur[q] = mgc_scale(mgc_add(cur[q], h[q]), 0.5);
+		const double d = mg_unif_dist4(cur, h);
+		const double o = __shfl_xor_sync(0xffffffffu, d, 1);
+		done = done || (it >= 4 && d < 1e-14 && o < 1e-14);
+		if (__all_sync(0xffffffffu, done)) break;
+	}
+	if ((t >> 1) >= n) return;
+	mgc* out = corner ? v[i].k : v[i].c;
+	for (int q = 0; q < 4; q++) out[q] = cur[q];
 }
 
 // ---- truncated CG (reference src/trust_region.c:17-146), one block ----
@@ -166,7 +200,9 @@ int sync() { MGCU_TRY(cudaStreamSynchronize(mgcu_stream())); return 0; }
 
 }  // namespace
 
-int mgcu_project_dev(const mgg* vblocks, int nb, const double* dgrad_dev, const double* hess_dev, double* grad_vec, double* H)
+// the projection queued on the calling thread's stream; the results stay in *gv (8 nb) and, for a
+// Hessian, *Hp ((8 nb)^2) until the next call (callers hold the library lock)
+int mgcu_project_launch(const mgg* vblocks, int nb, const double* dgrad_dev, const double* hess_dev, double** gv, double** Hp)
 {
 	MgcuContext* c = mgcu_ctx();
 	if (!c) return MG_ERR_DEVICE;
@@ -176,17 +212,18 @@ int mgcu_project_dev(const mgg* vblocks, int nb, const double* dgrad_dev, const 
 	TRY(g_gv.alloc(sizeof(double) * m));
 	k_project_grad<<<(nb + 63) / 64, 64, 0, mgcu_stream()>>>(g_v.as<mgg>(), dgrad_dev, nb, g_gv.as<double>(), g_dv.as<mgg>());
 	MGCU_LAUNCHED();
-	if (grad_vec) TRY(down(grad_vec, g_gv, sizeof(double) * m));
-	if (hess_dev && H)
+	*gv = g_gv.as<double>();
+	*Hp = nullptr;
+	if (hess_dev)
 	{
 		TRY(g_H.alloc(sizeof(double) * m * m));
-		k_project_hess<<<(nb * nb * 8 + 63) / 64, 64, 0, mgcu_stream()>>>(g_v.as<mgg>(), g_dv.as<mgg>(), (const double2*)hess_dev, nb, g_H.as<double>());
+		k_project_hess<<<(nb * nb * 64 + 127) / 128, 128, 0, mgcu_stream()>>>(g_v.as<mgg>(), g_dv.as<mgg>(), (const double2*)hess_dev, nb, g_H.as<double>());
 		MGCU_LAUNCHED();
 		k_mirror_real<<<(m * m + 255) / 256, 256, 0, mgcu_stream()>>>(m, g_H.as<double>());
 		MGCU_LAUNCHED();
-		TRY(down(H, g_H, sizeof(double) * m * m));
+		*Hp = g_H.as<double>();
 	}
-	return sync();
+	return 0;
 }
 
 extern "C" int mgcu_retract(const mgg* u, const double* eta, int n, mgg* v)
@@ -196,7 +233,7 @@ extern "C" int mgcu_retract(const mgg* u, const double* eta, int n, mgg* v)
 	TRY(up(g_u, u, sizeof(mgg) * n));
 	TRY(up(g_eta, eta, sizeof(double) * 8 * n));
 	TRY(g_v.alloc(sizeof(mgg) * n));
-	k_retract<<<(n + 63) / 64, 64, 0, mgcu_stream()>>>(g_u.as<mgg>(), g_eta.as<double>(), n, g_v.as<mgg>());
+	k_retract<<<(2 * n + 63) / 64, 64, 0, mgcu_stream()>>>(g_u.as<mgg>(), g_eta.as<double>(), n, g_v.as<mgg>());
 	MGCU_LAUNCHED();
 	TRY(down(v, g_v, sizeof(mgg) * n));
 	return sync();

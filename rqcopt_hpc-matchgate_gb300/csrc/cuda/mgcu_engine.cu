@@ -1756,15 +1756,30 @@ __global__ void k_convert(const double2* __restrict__ in, long n, typename P::T*
 		out[u] = P::make(in[u].x, in[u].y);
 }
 
-// out[r] = sum over parts (fixed order) of part[c * len + r]
-__global__ void k_sum_parts(const double* __restrict__ part, int nparts, long len, double* __restrict__ out)
+// out[r] = sum over parts of part[c * len + r], in a fixed order: sixteen outputs per block, each
+// by sixteen threads over every sixteenth part (one thread per output spent 25 to 350 us on one
+// addition and one read per part)
+constexpr int SUM_OUT = 16, SUM_SPLIT = 16;
+__global__ void __launch_bounds__(SUM_OUT * SUM_SPLIT) k_sum_parts(const double* __restrict__ part, int nparts, long len, double* __restrict__ out)
 {
-	for (long r = blockIdx.x * (long)blockDim.x + threadIdx.x; r < len; r += (long)gridDim.x * blockDim.x)
-	{
-		double s = 0;
-		for (int c = 0; c < nparts; c++) s += part[(size_t)c * len + r];
-		out[r] = s;
-	}
+	__shared__ double sum[SUM_SPLIT][SUM_OUT];
+	const int e = threadIdx.x % SUM_OUT, w = threadIdx.x / SUM_OUT;
+	const long r = (long)blockIdx.x * SUM_OUT + e;
+	double s = 0;
+	if (r < len)
+#pragma unroll 8
+		for (int c = w; c < nparts; c += SUM_SPLIT) s += part[(size_t)c * len + r];
+	sum[w][e] = s;
+	__syncthreads();
+	if (w || r >= len) return;
+	s = 0;
+	for (int c = 0; c < SUM_SPLIT; c++) s += sum[c][e];
+	out[r] = s;
+}
+
+void sum_parts(const double* part, int nparts, long len, double* out, cudaStream_t st)
+{
+	k_sum_parts<<<(unsigned)((len + SUM_OUT - 1) / SUM_OUT), SUM_OUT * SUM_SPLIT, 0, st>>>(part, nparts, len, out);
 }
 
 // per-gate gradients [ngates][16] -> per-block sums [nblocks][16], gates in order
@@ -2019,8 +2034,8 @@ static int upload_mats(const mgg* gates, int ng, DevBuf& buf)
 		}
 	int e = buf.alloc(sizeof(T) * h.size());
 	if (e) return e;
+	// (from pageable memory: the copy has left h when the call returns)
 	MGCU_TRY(cudaMemcpyAsync(buf.p, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice, mgcu_stream()));
-	MGCU_TRY(cudaStreamSynchronize(mgcu_stream()));
 	return 0;
 }
 
@@ -2402,7 +2417,7 @@ struct mgcu_plan
 	DevBuf d_mats_inv, ck;
 	DevBuf su, sw, sh, cache, dcache, part_f, part_g, part_h, cols64, cols;
 	DevBuf out_f, out_g, out_blk, out_h, flush;
-	int nparts_h;
+	int rows_a = 0, rows_h = 0;    // partial rows (blocks) used in this evaluation
 };
 
 static size_t prec_tsize(int prec) { return prec == MG_PREC_FP32_ID ? 8 : 16; }
@@ -2558,6 +2573,7 @@ static int launch_columns(mgcu_plan* p, long b0, long b1, const typename P::T* d
 		w.part = wg ? p->part_g.as<double>() : p->part_f.as<double>();
 		w.nblocks = p->d.nblocks;
 		const int gf = (int)std::min<long>(f.grid, (ncols + f.nc - 1) / f.nc);
+		p->rows_a = std::max(p->rows_a, gf);
 		fit_kernel<P>(f.qc, wg, f.threads)<<<gf, f.threads, f.smem, mgcu_stream()>>>(w);
 		MGCU_LAUNCHED();
 		if (p->d.want_hess)
@@ -2568,7 +2584,9 @@ static int launch_columns(mgcu_plan* p, long b0, long b1, const typename P::T* d
 			h.block = p->d_block.as<int>(); h.nplace = p->d.nplace; h.ngates = p->d.ngates; h.mdim = 8 * p->d.nblocks;
 			h.hgroup = p->hgroup ? 1 : 0; h.part_h = p->part_h.as<double>();
 			const long nitems = (ncols + f.nc - 1) / f.nc * p->d.nplace * 8;
-			fit_hess_kernel<P>(f.qc, f.threads)<<<(int)std::min<long>(f.grid_h, nitems), f.threads, f.smem, mgcu_stream()>>>(h, nitems);
+			const int gh = (int)std::min<long>(f.grid_h, nitems);
+			p->rows_h = std::max(p->rows_h, gh);
+			fit_hess_kernel<P>(f.qc, f.threads)<<<gh, f.threads, f.smem, mgcu_stream()>>>(h, nitems);
 			MGCU_LAUNCHED();
 		}
 		return 0;
@@ -2580,6 +2598,7 @@ static int launch_columns(mgcu_plan* p, long b0, long b1, const typename P::T* d
 		if (e) return e;
 		a.cache = p->cache.as<T>();
 	}
+	p->rows_a = std::max(p->rows_a, grid);
 	if (p->adj && p->adj_ok)
 	{
 		a.wmi = p->d_mats_inv.as<T>();
@@ -2604,6 +2623,7 @@ static int launch_columns(mgcu_plan* p, long b0, long b1, const typename P::T* d
 		a.part_h = p->part_h.as<double>(); a.sh = p->sh.as<T>();
 		const long nitems = ncols * p->d.nplace * 8;
 		const int gb = (int)std::min<long>(p->grid_b, nitems);
+		p->rows_h = std::max(p->rows_h, gb);
 		k_hessian<P><<<gb, p->threads, p->smem, mgcu_stream()>>>(a, nitems);
 		MGCU_LAUNCHED();
 	}
@@ -3025,8 +3045,10 @@ extern "C" int mgcu_plan_set_gates(mgcu_plan* p, const mgg* gates)
 extern "C" int mgcu_plan_begin(mgcu_plan* p)
 {
 	cudaStream_t st = mgcu_stream();
-	MGCU_TRY(cudaMemsetAsync(p->part_f.p, 0, p->part_f.n, st));
-	MGCU_TRY(cudaMemsetAsync(p->part_g.p, 0, p->part_g.n, st));
+	p->rows_a = p->rows_h = 0;
+	const bool grad = p->d.want_grad || p->d.want_hess;
+	if (!(p->fit.ok && grad)) MGCU_TRY(cudaMemsetAsync(p->part_f.p, 0, p->part_f.n, st));   // there f is the trace of the gradient sums
+	if (grad) MGCU_TRY(cudaMemsetAsync(p->part_g.p, 0, p->part_g.n, st));
 	if (p->d.want_hess) MGCU_TRY(cudaMemsetAsync(p->part_h.p, 0, p->part_h.n, st));
 	return 0;
 }
@@ -3098,13 +3120,13 @@ extern "C" int mgcu_plan_finish(mgcu_plan* p)
 	const int ng = std::max(p->d.ngates, 1);
 	if (p->fit.ok && (p->d.want_grad || p->d.want_hess))
 	{
-		k_fit_finish<<<p->d.nblocks, 128, 0, st>>>(p->part_g.as<double>(), p->fit.grid, p->d.nblocks, p->fit.d_blk.as<FitBlock>(),
+		k_fit_finish<<<p->d.nblocks, FIT_FIN * 16, 0, st>>>(p->part_g.as<double>(), p->rows_a, p->d.nblocks, p->fit.d_blk.as<FitBlock>(),
 			p->out_f.as<double>(), p->out_blk.as<double>());
 		MGCU_LAUNCHED();
 		if (!p->d.want_hess) return 0;
 		const long mdim = 8L * p->d.nblocks;
 		double2* A = p->fit.cache.as<double2>();
-		k_sum_parts<<<grid_cap(2 * mdim * mdim, 128), 128, 0, st>>>(p->part_h.as<double>(), p->fit.grid_h, 2 * mdim * mdim, p->fit.cache.as<double>());
+		sum_parts(p->part_h.as<double>(), p->rows_h, 2 * mdim * mdim, p->fit.cache.as<double>(), st);
 		MGCU_LAUNCHED();
 		k_fit_hess_finish<<<grid_cap(mdim * mdim, 128), 128, 0, st>>>(A, p->d.nblocks, p->fit.d_blk.as<FitBlock>(), p->out_h.as<double2>());
 		MGCU_LAUNCHED();
@@ -3114,11 +3136,11 @@ extern "C" int mgcu_plan_finish(mgcu_plan* p)
 		MGCU_LAUNCHED();
 		return 0;
 	}
-	k_sum_parts<<<1, 32, 0, st>>>(p->part_f.as<double>(), p->fit.ok ? p->fit.grid : p->grid_a, 2, p->out_f.as<double>());
+	sum_parts(p->part_f.as<double>(), p->rows_a, 2, p->out_f.as<double>(), st);
 	MGCU_LAUNCHED();
 	if (p->d.want_grad || p->d.want_hess)
 	{
-		k_sum_parts<<<grid_cap(16L * ng, 128), 128, 0, st>>>(p->part_g.as<double>(), p->grid_a, 16L * ng, p->out_g.as<double>());
+		sum_parts(p->part_g.as<double>(), p->rows_a, 16L * ng, p->out_g.as<double>(), st);
 		MGCU_LAUNCHED();
 		k_block_sum<<<(16 * p->d.nblocks + 127) / 128, 128, 0, st>>>(p->out_g.as<double>(), p->d_block.as<int>(), p->d.ngates, p->d.nblocks, p->out_blk.as<double>());
 		MGCU_LAUNCHED();
@@ -3126,7 +3148,7 @@ extern "C" int mgcu_plan_finish(mgcu_plan* p)
 	if (p->d.want_hess)
 	{
 		const long mdim = 8L * p->d.nblocks;
-		k_sum_parts<<<grid_cap(2 * mdim * mdim, 128), 128, 0, st>>>(p->part_h.as<double>(), p->grid_b, 2 * mdim * mdim, p->out_h.as<double>());
+		sum_parts(p->part_h.as<double>(), p->rows_h, 2 * mdim * mdim, p->out_h.as<double>(), st);
 		MGCU_LAUNCHED();
 		k_symm_diag<<<grid_cap(mdim * mdim, 256), 256, 0, st>>>(p->d.nblocks, p->out_h.as<double2>());
 		MGCU_LAUNCHED();
@@ -3149,12 +3171,66 @@ extern "C" int mgcu_plan_fetch(mgcu_plan* p, mgc* f, mgg* dblocks, mgc* hess)
 }
 
 // projection of gradient and Hessian on the GPU (mgcu_algebra.cu)
-extern int mgcu_project_dev(const mgg* vblocks_host, int nblocks, const double* dgrad_dev, const double* hess_dev,
-	double* grad_vec, double* H);
+extern int mgcu_project_launch(const mgg* vblocks_host, int nblocks, const double* dgrad_dev, const double* hess_dev,
+	double** gv, double** Hp);
 
-extern "C" int mgcu_plan_project(mgcu_plan* p, const mgg* vblocks, double* grad_vec, double* H)
+// Device-to-host copies that end together: small ones go through this thread's pinned buffer
+// (asynchronous, one wait for all; a pageable copy waits by itself), larger ones directly.
+namespace {
+struct Pinned
 {
-	return mgcu_project_dev(vblocks, p->d.nblocks, p->out_blk.as<double>(), p->d.want_hess ? p->out_h.as<double>() : nullptr, grad_vec, H);
+	static constexpr size_t N = 64 << 10;
+	char* p = nullptr;
+	~Pinned() { if (p) cudaFreeHost(p); }
+};
+thread_local Pinned t_pinned;
+
+struct Fetch
+{
+	struct Item { void* dst; size_t off, n; };
+	Item item[8];
+	int n = 0;
+	size_t used = 0;
+	int get(void* dst, const void* src, size_t bytes)
+	{
+		if (!dst || !bytes) return 0;
+		if (!t_pinned.p && cudaHostAlloc(&t_pinned.p, Pinned::N, cudaHostAllocDefault) != cudaSuccess) { cudaGetLastError(); t_pinned.p = nullptr; }
+		const size_t room = (bytes + 15) & ~(size_t)15;
+		if (!t_pinned.p || used + room > Pinned::N || n == 8)
+		{
+			MGCU_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, mgcu_stream()));
+			return 0;
+		}
+		MGCU_TRY(cudaMemcpyAsync(t_pinned.p + used, src, bytes, cudaMemcpyDeviceToHost, mgcu_stream()));
+		item[n++] = { dst, used, bytes };
+		used += room;
+		return 0;
+	}
+	int finish()
+	{
+		MGCU_TRY(cudaStreamSynchronize(mgcu_stream()));
+		for (int i = 0; i < n; i++) memcpy(item[i].dst, t_pinned.p + item[i].off, item[i].n);
+		n = 0; used = 0;
+		return 0;
+	}
+};
+}  // namespace
+
+extern "C" int mgcu_plan_results(mgcu_plan* p, mgc* f, mgg* dblocks, mgc* hess, const mgg* vblocks, double* grad_vec, double* H)
+{
+	const bool grad = p->d.want_grad || p->d.want_hess;
+	const size_t m = 8 * (size_t)p->d.nblocks;
+	double *gv = nullptr, *Hp = nullptr;
+	int e = 0;
+	if (grad && (grad_vec || H))
+		e = mgcu_project_launch(vblocks, p->d.nblocks, p->out_blk.as<double>(), (p->d.want_hess && H) ? p->out_h.as<double>() : nullptr, &gv, &Hp);
+	Fetch ft;
+	if (!e) e = ft.get(f, p->out_f.p, sizeof(double) * 2);
+	if (!e && grad) e = ft.get(dblocks, p->out_blk.p, sizeof(double) * 2 * m);
+	if (!e && gv) e = ft.get(grad_vec, gv, sizeof(double) * m);
+	if (!e && Hp) e = ft.get(H, Hp, sizeof(double) * m * m);
+	if (!e && p->d.want_hess) e = ft.get(hess, p->out_h.p, sizeof(double) * 2 * m * m);
+	return e ? e : ft.finish();
 }
 
 extern "C" double mgcu_plan_time_ms(mgcu_plan* p, long b0, long b1, int steps, int flush_l2)
@@ -3229,26 +3305,44 @@ struct BatchRed
 	int nslots, ngates, nblocks;
 };
 
-__global__ void k_batch_reduce(const BatchRed* __restrict__ rd)
+// parameter block blockIdx.y of instance blockIdx.x (and, with y = 0, f): sixteen sums by
+// sixteen threads each over every sixteenth slot, in a fixed order (one thread per sum over all
+// slots and gates took 2.2 ms for twelve instances)
+__global__ void __launch_bounds__(256) k_batch_reduce(const BatchRed* __restrict__ rd)
 {
+	__shared__ double sum[16][16];
 	const BatchRed r = rd[blockIdx.x];
-	if (threadIdx.x < 2)
+	const int blk = blockIdx.y, e = threadIdx.x & 15, w = threadIdx.x >> 4;
+	if (blk >= r.nblocks) return;
+	if (blk == 0)
 	{
 		double s = 0;
-		for (int k = 0; k < r.nslots; k++) s += r.part_f[2 * k + threadIdx.x];
-		r.out_f[threadIdx.x] = s;
-	}
-	for (int q = threadIdx.x; q < r.nblocks * 16; q += blockDim.x)
-	{
-		const int blk = q >> 4, e = q & 15;
-		double s = 0;
-		for (int g = 0; g < r.ngates; g++)
+		if (e < 2)
+#pragma unroll 4
+			for (int k = w; k < r.nslots; k += 16) s += r.part_f[2 * k + e];
+		sum[w][e] = s;
+		__syncthreads();
+		if (threadIdx.x < 2)
 		{
-			if (r.block[g] != blk) continue;
-			for (int k = 0; k < r.nslots; k++) s += r.part_g[((size_t)k * r.ngates + g) * 16 + e];
+			s = 0;
+			for (int k = 0; k < 16; k++) s += sum[k][threadIdx.x];
+			r.out_f[threadIdx.x] = s;
 		}
-		r.out_blk[q] = s;
+		__syncthreads();
 	}
+	double s = 0;
+	for (int g = 0; g < r.ngates; g++)
+	{
+		if (r.block[g] != blk) continue;
+#pragma unroll 4
+		for (int k = w; k < r.nslots; k += 16) s += r.part_g[((size_t)k * r.ngates + g) * 16 + e];
+	}
+	sum[w][e] = s;
+	__syncthreads();
+	if (w) return;
+	s = 0;
+	for (int k = 0; k < 16; k++) s += sum[k][e];
+	r.out_blk[blk * 16 + e] = s;
 }
 
 struct BatchInst
@@ -3579,7 +3673,9 @@ static int batch_issue(mgcu_batch* B)
 			B->items.as<BatchItem>() + i0, ni, B->counters.as<int>() + k, B->scratch.as<T>(), B->slot_stride, B->cache_stride);
 		MGCU_LAUNCHED();
 	}
-	k_batch_reduce<<<B->n, 128, 0, st>>>(B->red.as<BatchRed>());
+	int nb = 1;
+	for (int i = 0; i < B->n; i++) nb = std::max(nb, B->inst[i].nblocks);
+	k_batch_reduce<<<dim3(B->n, nb), 256, 0, st>>>(B->red.as<BatchRed>());
 	MGCU_LAUNCHED();
 	return 0;
 }
@@ -3662,16 +3758,21 @@ extern "C" int mgcu_batch_fetch(mgcu_batch* B, int i, mgc* f, mgg* dblocks)
 {
 	if (i < 0 || i >= B->n) { mg_set_error("batch instance %d out of range", i); return MG_ERR_ARG; }
 	BatchInst& I = B->inst[i];
-	if (f) MGCU_TRY(cudaMemcpy(f, I.out_f.p, sizeof(double) * 2, cudaMemcpyDeviceToHost));
-	if (dblocks) MGCU_TRY(cudaMemcpy(dblocks, I.out_blk.p, sizeof(double) * 16 * I.nblocks, cudaMemcpyDeviceToHost));
-	return 0;
+	Fetch ft;
+	int e = ft.get(f, I.out_f.p, sizeof(double) * 2);
+	if (!e) e = ft.get(dblocks, I.out_blk.p, sizeof(double) * 16 * I.nblocks);
+	return e ? e : ft.finish();
 }
 
 extern "C" int mgcu_batch_project(mgcu_batch* B, int i, const mgg* vblocks, double* grad_vec)
 {
 	if (i < 0 || i >= B->n) { mg_set_error("batch instance %d out of range", i); return MG_ERR_ARG; }
 	BatchInst& I = B->inst[i];
-	return mgcu_project_dev(vblocks, I.nblocks, I.out_blk.as<double>(), nullptr, grad_vec, nullptr);
+	double *gv = nullptr, *Hp = nullptr;
+	int e = mgcu_project_launch(vblocks, I.nblocks, I.out_blk.as<double>(), nullptr, &gv, &Hp);
+	Fetch ft;
+	if (!e) e = ft.get(grad_vec, gv, sizeof(double) * 8 * I.nblocks);
+	return e ? e : ft.finish();
 }
 
 extern "C" int mgcu_batch_info(const mgcu_batch* B, int i, int* target_tile_bits, int* target_passes, int* items)
@@ -3884,9 +3985,9 @@ extern "C" int mg_noalloc_brickwall_target_and_gradient(const void* ugates, int 
 		k_columns<PrecD, true><<<grid, threads, smem, st>>>(a);
 		mgcu_count_launch();
 		NA_TRY(cudaGetLastError());
-		k_sum_parts<<<1, 32, 0, st>>>(a.part_f, grid, 2, reinterpret_cast<double*>(base + NA_OUT_F));
+		sum_parts(a.part_f, grid, 2, reinterpret_cast<double*>(base + NA_OUT_F), st);
 		mgcu_count_launch();
-		k_sum_parts<<<grid_cap(16L * ng, 128), 128, 0, st>>>(a.part_g, grid, 16L * ng, reinterpret_cast<double*>(base + NA_OUT_G));
+		sum_parts(a.part_g, grid, 16L * ng, reinterpret_cast<double*>(base + NA_OUT_G), st);
 		mgcu_count_launch();
 		k_block_sum<<<(16 * nlayers + 127) / 128, 128, 0, st>>>(reinterpret_cast<double*>(base + NA_OUT_G), reinterpret_cast<const int*>(base + NA_BLOCK),
 			ng, nlayers, reinterpret_cast<double*>(base + NA_OUT_BLK));

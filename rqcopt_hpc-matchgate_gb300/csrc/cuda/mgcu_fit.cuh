@@ -725,21 +725,23 @@ __global__ void k_fit_tables(const FitDiag* __restrict__ diag, const int* __rest
 }
 
 // block gradients and f from the summed R: one block of threads per parameter block, the rows of
-// the parts summed by 8 threads each in a fixed order
+// the parts summed by FIT_FIN threads each in a fixed order
+constexpr int FIT_FIN = 32;
 struct FitBlock { double minv[8][2]; double scale[8][2]; int ngates, pad; };   // see mgcu_fit_build.cuh
 
-__global__ void __launch_bounds__(128) k_fit_finish(const double* __restrict__ part, int nparts, int nblocks, const FitBlock* __restrict__ fb,
+__global__ void __launch_bounds__(FIT_FIN * 16) k_fit_finish(const double* __restrict__ part, int nparts, int nblocks, const FitBlock* __restrict__ fb,
 	double* __restrict__ out_f, double* __restrict__ out_blk)
 {
-	__shared__ double sum[8][16];
+	__shared__ double sum[FIT_FIN][16];
 	const int blk = blockIdx.x, e = threadIdx.x & 15, w = threadIdx.x >> 4;
 	double s = 0;
-	for (int r = w; r < nparts; r += 8) s += part[((size_t)r * nblocks + blk) * 16 + e];
+#pragma unroll 4
+	for (int r = w; r < nparts; r += FIT_FIN) s += part[((size_t)r * nblocks + blk) * 16 + e];
 	sum[w][e] = s;
 	__syncthreads();
 	if (threadIdx.x >= 16) return;
 	s = 0;
-	for (int r = 0; r < 8; r++) s += sum[r][threadIdx.x];
+	for (int r = 0; r < FIT_FIN; r++) s += sum[r][threadIdx.x];
 	__syncwarp(0xffffu);
 	sum[0][threadIdx.x] = s;
 	__syncwarp(0xffffu);

@@ -433,8 +433,7 @@ static int run_eval(linear_func ufunc, void* udata, const eval_req* q)
 	}
 	if (!rc) rc = mgcu_plan_finish(p);
 	mgc f;
-	if (!rc) rc = mgcu_plan_fetch(p, &f, (mgg*)q->dblocks, (mgc*)q->hess);
-	if (!rc && (q->grad_vec || q->H)) rc = mgcu_plan_project(p, (const mgg*)q->vblocks, q->grad_vec, q->H);
+	if (!rc) rc = mgcu_plan_results(p, &f, (mgg*)q->dblocks, (mgc*)q->hess, (const mgg*)q->vblocks, q->grad_vec, q->H);
 	mgcu_unlock();
 	if (rc)
 	{
@@ -734,8 +733,7 @@ int mg_plan_results(mg_plan* pl, numeric* fval, struct matchgate dvlist[], numer
 {
 	mgcu_lock();
 	mgc f;
-	int r = mgcu_plan_fetch(pl->p, &f, (mgg*)dvlist, (mgc*)hess);
-	if (!r && (grad_vec || H)) r = mgcu_plan_project(pl->p, (const mgg*)pl->vlist, grad_vec, H);
+	int r = mgcu_plan_results(pl->p, &f, (mgg*)dvlist, (mgc*)hess, (const mgg*)pl->vlist, grad_vec, H);
 	mgcu_unlock();
 	if (!r && fval) *fval = f.re + I * f.im;
 	return r;

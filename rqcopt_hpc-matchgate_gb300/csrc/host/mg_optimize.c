@@ -138,7 +138,10 @@ static int optimize(void* target, const struct matchgate vlist0[], const fit_t* 
 		f_iter[k] = fx;
 		if (prec_iter) prec_iter[k] = prec;
 		const bool on_boundary = truncated_cg_hmat(grad, H, n, radius, &params->tcg_params, eta);
-		for (int l = 0; l < nlayers; l++) retract_matchgate(&x[l], eta + 8 * l, &xn[l]);
+		mgcu_lock();
+		rc = mgcu_retract((const mgg*)x, eta, nlayers, (mgg*)xn);   /* all gates in one launch */
+		mgcu_unlock();
+		if (rc) break;
 		double fn;
 		rc = eval_f(&pl, xn, &fn);
 		if (rc) break;

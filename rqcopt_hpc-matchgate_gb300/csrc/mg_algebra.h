@@ -260,20 +260,26 @@ MG_HD void mgg_retract(const mgg* u, const double* eta, mgg* v)
  * for layer pair (i, j) and unit tangent direction k at gate j, given the complex
  * Hessian blocks hij (8x8 row-major, rows x of layer i, columns y of layer j),
  * returns the 8 reals of column k.  dvc_i is the conjugated gradient of gate i. */
-MG_HD void mg_project_hessian_column(const mgg* vi, const mgg* vj, const mgg* dvc_i, int same_layer,
-	const mgc* hij, int k, double* out8)
+/* the unit tangent direction k at vj */
+MG_HD void mg_hessian_direction(const mgg* vj, int k, mgg* Z)
 {
 	double r[8] = { 0, 0, 0, 0, 0, 0, 0, 0 };
 	r[k] = 1;
-	mgg Z, G;
-	mgg_real_to_tangent(r, vj, &Z);
-	mgg_zero(&G);
-	for (int x = 0; x < 4; x++)
-		for (int y = 0; y < 4; y++)
-		{
-			G.c[x] = mgc_add(G.c[x], mgc_add(mgc_mul(hij[x * 8 + y], Z.c[y]), mgc_mul(hij[x * 8 + y + 4], Z.k[y])));
-			G.k[x] = mgc_add(G.k[x], mgc_add(mgc_mul(hij[(x + 4) * 8 + y], Z.c[y]), mgc_mul(hij[(x + 4) * 8 + y + 4], Z.k[y])));
-		}
+	mgg_real_to_tangent(r, vj, Z);
+}
+
+/* row x of hij (8 entries) applied to the direction */
+MG_HD mgc mg_hessian_row(const mgc* hrow, const mgg* Z)
+{
+	mgc g = mgc_make(0, 0);
+	for (int y = 0; y < 4; y++) g = mgc_add(g, mgc_add(mgc_mul(hrow[y], Z->c[y]), mgc_mul(hrow[y + 4], Z->k[y])));
+	return g;
+}
+
+/* the 8 reals of the column from its rows G (G = hij Z) */
+MG_HD void mg_project_hessian_column(const mgg* vi, const mgg* dvc_i, int same_layer, const mgg* Zp, const mgg* Gp, double* out8)
+{
+	mgg Z = *Zp, G = *Gp;
 	mgg_conj(&G);
 	if (same_layer)
 	{
