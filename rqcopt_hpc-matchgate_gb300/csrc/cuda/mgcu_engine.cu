@@ -1846,6 +1846,27 @@ struct SectorProg
 	DevBuf steps, list, offs, drows;
 };
 
+// a fitted circuit's or target's program for k_fit (see mgcu_fit_build.cuh)
+struct FitProg
+{
+	bool factored = true;
+	bool built = false;            // the structure exists (groups, passes, flushes)
+	bool tried = false;            // a target's program: built or found not to apply
+	bool ok = false;               // the current gates factor (else the general kernels run)
+	int qc = 0;                    // 0 real q, 1 complex q, 2 unfactored
+	Sched sched;
+	std::vector<FitGroup> group;
+	std::vector<FitPass> pass_groups;
+	std::vector<std::array<int, 2>> diag;   // per table entry factor: gate, 0 left / 1 right
+	std::vector<int> beg, group_of;         // per flush (the last: the final table)
+	std::vector<int> block_gates;           // gates per block
+	std::vector<int> group_of_gate;
+	int grid_h = 0;                         // k_fit_hess blocks
+	int nflush = 0, grid = 0, nc = 1, threads = 128, kt = 0;
+	size_t smem = 0;
+	DevBuf d_pass, d_group, d_pgroups, d_gates, d_diag, d_beg, d_gof, d_tab, d_blk, d_bases, d_pgroup, cache;
+};
+
 struct TargetProg
 {
 	int kt = -1, prec = -1, threads = -1;
@@ -1857,6 +1878,7 @@ struct TargetProg
 	std::vector<int> first;        // first gate with the same matrix
 	DevBuf pass, gate, mats, kinds, tg, pm, pmats;
 	SectorProg sector;
+	FitProg fit;
 };
 
 // Exact classification of a 2x2 block (entries row-major); for BK_RI the entries are
@@ -2276,6 +2298,7 @@ static int build_target_prog(mgcu_target* t, int kt, int threads, TargetProg& tp
 		MGCU_TRY(cudaMemcpy(tp.pm.p, pmh.data(), sizeof(int2) * pmh.size(), cudaMemcpyHostToDevice));
 		tp.kw = kw;
 		tp.sector.state = -1;
+		tp.fit.built = tp.fit.tried = false;
 		tp.kt = kt;
 		tp.threads = threads;
 	}
@@ -2396,6 +2419,7 @@ struct mgcu_plan
 	bool w_t = false;              // the weight-restricted sweep (k_target_w)
 	int maxg_t = MAXPG;            // k_target_w: room for this many staged gate records
 	int nq_t = 2;                  // k_target_w: live quartets per thread and iteration
+	bool tfit = false;             // the target's columns by k_fit
 	bool sec = false;              // the sector sweep (k_sector)
 	DevBuf sec_items;              // its blocks per sector for the columns [sec_b0, sec_b1)
 	long sec_b0 = -1, sec_b1 = -1;
@@ -2432,6 +2456,17 @@ static size_t target_smem_bytes(const mgcu_plan* p, int tt)
 }
 
 static int plan_event(mgcu_plan* p, int which);
+
+// -conj(U e_b) for b in [b0, b1) by the target's k_fit program
+template <class P>
+static int launch_fit_columns(const FitProg& f, int L, long b0, long b1, typename P::T* out)
+{
+	FitArgs<P> w = fit_args<P>(f, L);
+	w.b0 = b0; w.b1 = b1; w.ucols = out;
+	fit_kernel<P>(f.qc, FIT_COLS, f.threads)<<<(int)std::min<long>(f.grid, (b1 - b0 + f.nc - 1) / f.nc), f.threads, f.smem, mgcu_stream()>>>(w);
+	MGCU_LAUNCHED();
+	return 0;
+}
 
 // the sector sweep of the columns [b0, b1): per sector, the rows (= columns) of the range in
 // blocks of 2^ln; the block list of a range is kept on the plan
@@ -2508,6 +2543,15 @@ static int launch_target(mgcu_plan* p, long b0, long b1, typename P::T* out)
 		if (!e && tp->sector.state != 1) { mg_set_error("the target's sector program is missing"); e = MG_ERR_ARG; }
 		return e ? e : launch_sector<P>(p, *tp, b0, b1, out);
 	}
+	if (p->tfit)
+	{
+		e = target_fit<P>(p->d.target, *tp, tp->fit);
+		if (!e && !tp->fit.built) { mg_set_error("the target's program is missing"); e = MG_ERR_ARG; }
+		if (!e) e = plan_event(p, 0);
+		if (e) return e;
+		e = launch_fit_columns<P>(tp->fit, p->L, b0, b1, out);
+		return e ? e : plan_event(p, 1);
+	}
 	a.U.pass = tp->pass.as<PassRec>(); a.U.gate = tp->gate.as<GateRec>(); a.U.npass = (int)tp->sched.pass.size();
 	a.um = tp->mats.as<T>();
 	a.utg = tp->tg.as<TGate>();
@@ -2554,28 +2598,22 @@ static int launch_columns(mgcu_plan* p, long b0, long b1, const typename P::T* d
 	if (!a.want_grad) a.cache = nullptr;
 	const long ncols = b1 - b0;
 	const int grid = (int)std::min<long>(p->grid_a, ncols);
-	if constexpr (P::kId != MG_PREC_FP32_ID)
 	if (p->fit.ok)
 	{
 		const FitProg& f = p->fit;
-		FitArgs<P> w;
-		w.L = p->L; w.nb = p->nb; w.kt = f.kt; w.npass = (int)f.sched.pass.size(); w.ngroups = (int)f.group.size(); w.nc = f.nc;
-		w.S = p->S;
-		w.pass = f.d_pass.as<PassRec>(); w.groups_of = f.d_pgroups.as<FitPass>(); w.groups = f.d_group.as<FitGroup>();
-		w.bases = f.d_bases.as<unsigned>();
-		w.gates = f.d_gates.as<FitGate<T>>(); w.tables = f.d_tab.as<T>(); w.final = w.tables + (size_t)2 * p->S * f.nflush;
+		FitArgs<P> w = fit_args<P>(f, p->L);
 		w.dense = dense; w.dense_b0 = dense_b0; w.b0 = b0; w.b1 = b1;
 		const bool wg = p->d.want_grad || p->d.want_hess;
 		w.su = p->su.as<T>(); w.sw = p->sw.as<T>();
 		w.cache = p->d.want_hess ? p->cache.as<T>() : f.cache.as<T>();
 		w.dcache = p->d.want_hess ? p->dcache.as<T>() : nullptr;
-		w.slot_per_column = p->d.want_hess ? 1 : 0;
 		w.part = wg ? p->part_g.as<double>() : p->part_f.as<double>();
 		w.nblocks = p->d.nblocks;
 		const int gf = (int)std::min<long>(f.grid, (ncols + f.nc - 1) / f.nc);
 		p->rows_a = std::max(p->rows_a, gf);
-		fit_kernel<P>(f.qc, wg, f.threads)<<<gf, f.threads, f.smem, mgcu_stream()>>>(w);
+		fit_kernel<P>(f.qc, p->d.want_hess ? FIT_HESS : wg ? FIT_GRAD : FIT_VALUE, f.threads)<<<gf, f.threads, f.smem, mgcu_stream()>>>(w);
 		MGCU_LAUNCHED();
+		if constexpr (P::kId != MG_PREC_FP32_ID)
 		if (p->d.want_hess)
 		{
 			FitHessArgs<P> h;
@@ -2641,13 +2679,13 @@ static int set_smem_attr()
 	for (auto k : tk) MGCU_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min<size_t>(c->smem_optin, 227 * 1024)));
 	void (*const wk[2])(Args<P>) = { k_target_w<P, 128, 2>, k_target_w<P, 256, 1> };
 	for (auto k : wk) MGCU_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min<size_t>(c->smem_optin, 227 * 1024)));
-	if constexpr (P::kId != MG_PREC_FP32_ID)
-		for (int q = 0; q < 12; q++)
-		{
-			const int lim = (int)std::min<size_t>(c->smem_optin, 227 * 1024) - 4096;
-			MGCU_TRY(cudaFuncSetAttribute(fit_kernel<P>(q & 1, q & 2, 128 << (q >> 2)), cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
-			if (!(q & 2)) MGCU_TRY(cudaFuncSetAttribute(fit_hess_kernel<P>(q & 1, 128 << (q >> 2)), cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
-		}
+	for (int q = 0; q < 24; q++)
+	{
+		const int lim = (int)std::min<size_t>(c->smem_optin, 227 * 1024) - 4096;
+		MGCU_TRY(cudaFuncSetAttribute(fit_kernel<P>(q & 1, (q >> 1) & 3, 128 << (q >> 3)), cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+		if constexpr (P::kId != MG_PREC_FP32_ID)
+			if (!(q & 6)) MGCU_TRY(cudaFuncSetAttribute(fit_hess_kernel<P>(q & 1, 128 << (q >> 3)), cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+	}
 	MGCU_TRY(cudaFuncSetAttribute(k_hessian<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::min<size_t>(c->smem_optin, 227 * 1024)));
 	return 0;
 }
@@ -2745,6 +2783,16 @@ static int tune_target_sweep(mgcu_plan* p)
 // Hessians take the factored items from L = 7 (whole evaluation: per-gate L = 7 float-float 550
 // against 1011 us, per-layer L = 8 533 against 1010 us; per-layer L = 6 414 against 385 us)
 constexpr int FIT_HESS_MIN_L = 7;
+
+template <class P>
+static int plan_target_fit(mgcu_target* t, int kt, int threads, bool& use)
+{
+	TargetProg* tp = nullptr;
+	int e = target_prog<P>(t, kt, threads, tp);
+	if (!e) e = target_fit<P>(t, *tp, tp->fit);
+	if (!e) use = tp->fit.built;
+	return e;
+}
 
 extern "C" mgcu_plan* mgcu_plan_create(const mgcu_plan_desc* d)
 {
@@ -2884,12 +2932,21 @@ extern "C" mgcu_plan* mgcu_plan_create(const mgcu_plan_desc* d)
 			else e = target_pm_cap<PrecX>(d->target, p->kt_t, tt, mp, wcons, mg);
 			if (e) { delete p; return nullptr; }
 			p->pm_cap = mp;
+			// from L = 10 the columns come from k_fit, unless an option asks for the full sweep or
+			// one of its shapes
+			if (opt_kt <= 0 && o <= 0 && ot <= 0 && p->nc_t == 1 && mgcu_option(MG_OPT_TARGET_DENSE_ID) == 0 && mgcu_option(MG_OPT_CTAS_PER_SM_ID) <= 0)
+			{
+				if (p->prec == MG_PREC_FP64_ID) e = plan_target_fit<PrecD>(d->target, p->kt_t, tt, p->tfit);
+				else if (p->prec == MG_PREC_FP32_ID) e = plan_target_fit<PrecF>(d->target, p->kt_t, tt, p->tfit);
+				else e = plan_target_fit<PrecX>(d->target, p->kt_t, tt, p->tfit);
+				if (e) { delete p; return nullptr; }
+			}
 		}
 		p->smem_t = target_smem_bytes(p, tt);
 		// the block size by timing (MG_OPT_TARGET_TUNE: 0 = when the trace has at least 2^14
 		// columns, 1 = never, 2 = always) unless TARGET_THREADS fixes it
 		const long tune = mgcu_option(MG_OPT_TARGET_TUNE_ID);
-		if (d->target && d->target->kind == 0 && !p->sec && ot <= 0 && p->nc_t == 1 && tune != 1 && (tune == 2 || d->L >= 14))
+		if (d->target && d->target->kind == 0 && !p->sec && !p->tfit && ot <= 0 && p->nc_t == 1 && tune != 1 && (tune == 2 || d->L >= 14))
 		{
 			int e = 0;
 			if (p->prec == MG_PREC_FP64_ID) e = tune_target_sweep<PrecD>(p);
@@ -2932,12 +2989,13 @@ extern "C" mgcu_plan* mgcu_plan_create(const mgcu_plan_desc* d)
 	// the factored fitted circuit: gradients from L = 10 (whole evaluation, 5 layers: float-float
 	// 244 against 448 us, complex128 574 against 997 us; at L = 8 138 against 129 us and 263
 	// against 202 us, the tables and the few blocks cost more), f alone from L = 12 (L = 11: 318
-	// against 336 us), while the tables are small.  FP32 keeps the general kernels: there the
-	// factors' rounding is as large as the sweep's.  An explicit block size keeps them too
+	// against 336 us), while the tables are small.  FP32 gradients keep the general kernels: there
+	// the factors' rounding is as large as the sweep's.  An explicit block size keeps them too
 	e = 0;
 	// (Hessians: one tile, L <= 14)
 	const bool fit_grad = d->want_grad || d->want_hess;
-	if (!p->adj && d->ngates > 0 && opt_thr <= 0 && p->prec != MG_PREC_FP32_ID
+	// FP32: f alone, with whole blocks
+	if (!p->adj && d->ngates > 0 && opt_thr <= 0 && (p->prec != MG_PREC_FP32_ID || !fit_grad)
 		&& (d->want_hess ? (d->L >= FIT_HESS_MIN_L && d->L <= 14 && opt_kt <= 0) : (d->L >= (d->want_grad ? 10 : 12) && d->L <= 18)))
 	{
 		p->fit.kt = p->kt;
@@ -2945,14 +3003,15 @@ extern "C" mgcu_plan* mgcu_plan_create(const mgcu_plan_desc* d)
 		// against 87 ms in two 64 KB tiles), a larger one tiles of 64 KB (L=16, 5 layers, 6001
 		// columns: 81 ms against 87 ms in tiles of 128 KB, one block per SM)
 		if (opt_kt <= 0 && p->nb <= 13) p->fit.kt = p->nb;
-		e = fit_build(p->L, p->fit.kt, p->wires.data(), d->ngates, p->block.data(), d->nblocks, (int)p->tsize, d->want_hess != 0, p->fit);
+		e = fit_build(p->L, p->fit.kt, p->wires.data(), d->ngates, p->block.data(), d->nblocks, (int)p->tsize, d->want_hess != 0 || p->prec == MG_PREC_FP32_ID, p->prec != MG_PREC_FP32_ID, p->fit);
 		int per = 0;
 		if (!e)
 		{
 			auto occ = [&](auto k) { return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, p->fit.threads, p->fit.smem) != cudaSuccess; };
 			const bool g = fit_grad;
-			if (p->prec == MG_PREC_FP64_ID ? occ(fit_kernel<PrecD>(true, g, p->fit.threads)) : occ(fit_kernel<PrecX>(true, g, p->fit.threads)))
-				e = MG_ERR_DEVICE;
+			const int mode = d->want_hess ? FIT_HESS : g ? FIT_GRAD : FIT_VALUE;
+			if (p->prec == MG_PREC_FP64_ID ? occ(fit_kernel<PrecD>(1, mode, p->fit.threads)) : p->prec == MG_PREC_FP32_ID
+				? occ(fit_kernel<PrecF>(2, mode, p->fit.threads)) : occ(fit_kernel<PrecX>(1, mode, p->fit.threads))) e = MG_ERR_DEVICE;
 		}
 		if (e) { delete p; return nullptr; }
 		if (opt_cps > 0) per = (int)std::min<long>(per, opt_cps);
@@ -3035,6 +3094,7 @@ extern "C" int mgcu_plan_set_gates(mgcu_plan* p, const mgg* gates)
 	{
 		const mgcu_plan_desc& d = p->d;
 		if (p->prec == MG_PREC_FP64_ID) e = fit_set_gates<PrecD>(gates, d.ngates, d.block, d.nblocks, p->L, p->fit.kt, d.wires, p->fit);
+		else if (p->prec == MG_PREC_FP32_ID) e = fit_set_gates<PrecF>(gates, d.ngates, d.block, d.nblocks, p->L, p->fit.kt, d.wires, p->fit);
 		else e = fit_set_gates<PrecX>(gates, d.ngates, d.block, d.nblocks, p->L, p->fit.kt, d.wires, p->fit);
 	}
 	if (e || !p->adj) return e;
@@ -3265,6 +3325,7 @@ extern "C" void mgcu_plan_target_config(const mgcu_plan* p, int* cfg)
 	cfg[1] = p->kt_t;
 	cfg[2] = p->threads_t;
 	cfg[3] = p->w_t ? p->nq_t : p->nc_t;
+	if (p->tfit) cfg[2] = p->d.target->progs[p->prec].fit.threads;
 	if (p->sec)
 	{
 		cfg[2] = p->d.target->progs[p->prec].sector.threads;
@@ -3527,6 +3588,10 @@ static int batch_build(mgcu_batch* B, const mgcu_batch_inst* d, int tune)
 		I.grid_c = c->nsm * std::max(pc, 1);
 		I.big = (1L << I.L) >= 4L * std::max(I.grid_t, I.grid_c);
 		if (!I.big) continue;
+		{
+			const int ef = target_fit<P>(I.target, I.tp, I.tp.fit);   // as for plans
+			if (ef) return ef;
+		}
 		I.chunk = std::max(1L, std::min(1L << I.L, (long)((8ull << 30) / ((size_t)I.S * sizeof(T)))));
 		stage_bytes = std::max(stage_bytes, sizeof(T) * (size_t)I.S * (size_t)I.chunk);
 		slot_max = std::max(slot_max, (size_t)I.S);
@@ -3652,10 +3717,18 @@ static int batch_issue(mgcu_batch* B)
 		for (long c0 = 0; c0 < N; c0 += I.chunk)
 		{
 			const long c1 = std::min(N, c0 + I.chunk);
-			Args<P> a = hat[i];
-			a.b0 = c0; a.b1 = c1; a.ucols = B->stage.as<T>();
-			kt_<<<(int)std::min<long>(I.grid_t, c1 - c0), B->threads, I.smem_t, st>>>(a);
-			MGCU_LAUNCHED();
+			if (I.tp.fit.built)
+			{
+				const int ef = launch_fit_columns<P>(I.tp.fit, I.L, c0, c1, B->stage.as<T>());
+				if (ef) return ef;
+			}
+			else
+			{
+				Args<P> a = hat[i];
+				a.b0 = c0; a.b1 = c1; a.ucols = B->stage.as<T>();
+				kt_<<<(int)std::min<long>(I.grid_t, c1 - c0), B->threads, I.smem_t, st>>>(a);
+				MGCU_LAUNCHED();
+			}
 			Args<P> w = hac[i];
 			w.b0 = c0; w.b1 = c1; w.dense = B->stage.as<T>(); w.dense_b0 = c0;
 			w.su = B->bsu.as<T>(); w.sw = B->bsw.as<T>();

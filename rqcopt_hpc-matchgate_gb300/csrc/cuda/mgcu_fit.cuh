@@ -47,17 +47,25 @@ struct FitGroup
 	uint4 qs[2][4], qy[2][4];
 };
 
+// QC: how a group's gates are applied -- 0: M with a real q, 1: with a complex q, 2: unfactored
+// (the whole blocks, in k_columns' and k_target's arithmetic)
 template <class T> struct FitGate { T pc, qc, pk, qk; int swc, swk, pad[2]; };
+template <class T> struct FitWhole { T c[4], k[4]; };
+template <class T, int QC> struct FitGateOf { typedef FitGate<T> type; };
+template <class T> struct FitGateOf<T, 2> { typedef FitWhole<T> type; };
+// what k_fit makes: f; f and gradients; -conj of the columns; f and gradients, with states and
+// derivatives cached per column (Hessian plans)
+enum { FIT_VALUE = 0, FIT_GRAD = 1, FIT_COLS = 2, FIT_HESS = 3 };
 
 struct FitPass { int gbeg, gend; };
 
 // a group's record and gates in shared memory, copied asynchronously one group ahead
-template <class T> struct __align__(16) FitStage { FitGroup g; FitGate<T> gate[2]; };
+template <class G> struct __align__(16) FitStage { FitGroup g; G gate[2]; };
 
-template <class T>
-__device__ __forceinline__ void fit_stage(FitStage<T>& d, const FitGroup* __restrict__ g, const FitGate<T>* __restrict__ gates)
+template <class G>
+__device__ __forceinline__ void fit_stage(FitStage<G>& d, const FitGroup* __restrict__ g, const G* __restrict__ gates)
 {
-	constexpr unsigned NG = sizeof(FitGroup) / 16, NT = 2 * sizeof(FitGate<T>) / 16;
+	constexpr unsigned NG = sizeof(FitGroup) / 16, NT = 2 * sizeof(G) / 16;
 	const unsigned i = threadIdx.x;
 	if (i < NG + NT)
 	{
@@ -78,23 +86,28 @@ struct FitArgs
 	const FitPass* groups_of;
 	const FitGroup* groups;
 	const unsigned* bases;      // [group][unit]: byte offset (swizzled) of register 0
-	const FitGate<T>* gates;    // [group][2]
+	const void* gates;          // [group][2], FitGate or FitWhole
 	const T* tables;            // [flush][parity][S], in thread order of the flush's group
 	const T* final;             // [parity][S]: the diagonal factors after the last gate
 	const T* dense;
 	long dense_b0, b0, b1;
+	T* ucols;                   // FIT_COLS: output columns [b - b0][S]
 	T* su;
 	T* sw;
-	T* cache;                   // [slot][group][column of the block][S]
-	T* dcache;                  // the derivatives, alike (Hessian plans; else null)
-	int slot_per_column;        // slot: the block's columns, counted from b0 (1), or the block (0)
+	T* cache;                   // [slot][group][column of the block][S]; slot: the block, or (FIT_HESS) its columns from b0
+	T* dcache;                  // the derivatives, alike (FIT_HESS)
 	double* part;               // [block][nblocks][16] (gradient) or [block][2]
 	int nblocks;
 };
 
-// swizzled slot of a tile index (16-byte amplitudes): its low bits XORed with the higher groups
-// of bits, so that the lanes of a wavefront hit distinct banks whenever their bits differ mod 3
-__host__ __device__ __forceinline__ unsigned fsw(unsigned e) { return e ^ ((e >> 3) & 7u) ^ ((e >> 6) & 7u) ^ ((e >> 9) & 7u); }
+// swizzled slot of a tile index: its low bits XORed with the higher groups of bits, so that the
+// lanes of a wavefront hit distinct banks whenever their bits differ mod 3 (mod 4 for 8 bytes)
+template <int ES>
+__host__ __device__ __forceinline__ unsigned fsw(unsigned e)
+{
+	return ES == 16 ? e ^ ((e >> 3) & 7u) ^ ((e >> 6) & 7u) ^ ((e >> 9) & 7u)
+	                : e ^ ((e >> 4) & 15u) ^ ((e >> 8) & 15u) ^ ((e >> 12) & 15u);
+}
 
 // M (or its transpose) on the pair (f, s); sw: M = [[p, 1], [1, q]]
 template <class P, bool QC, bool TR>
@@ -132,91 +145,83 @@ __device__ __forceinline__ unsigned fit_base(const FitGroup& G, const unsigned* 
 	return (G.kind_b == 2 && ((__popc(u) + tpar) & 1)) ? b ^ G.m[3] : b;
 }
 
-// both gates of a group on the 16 registers
-template <class P, bool QC>
-__device__ __forceinline__ void fit_rotate(typename P::T (&v)[16], const FitGroup& G, const FitGate<typename P::T>* gates)
+// the corner or center block of a gate on a pair, whole or as M
+template <class P, int QC>
+__device__ __forceinline__ void fit_apply(typename P::T& f, typename P::T& s, const typename FitGateOf<typename P::T, QC>::type& g, bool corner)
 {
 	typedef typename P::T T;
-	if (G.ga >= 0)
+	if constexpr (QC == 2)
 	{
-		const FitGate<T>& g = gates[0];
-		{
-			const T p = g.pk, q = g.qk;
-			const bool sw = g.swk;
-#pragma unroll
-			for (int k = 0; k < 4; k++) fit_pair<P, QC, false>(v[4 * k], v[4 * k + 3], p, q, sw);
-		}
-		{
-			const T p = g.pc, q = g.qc;
-			const bool sw = g.swc;
-#pragma unroll
-			for (int k = 0; k < 4; k++) fit_pair<P, QC, false>(v[4 * k + 1], v[4 * k + 2], p, q, sw);
-		}
+		const T* m = corner ? g.k : g.c;
+		const T x = f, y = s;
+		f = P::madd2(m[0], x, m[1], y);
+		s = P::madd2(m[2], x, m[3], y);
 	}
+	else if (corner) fit_pair<P, QC == 1, false>(f, s, g.pk, g.qk, g.swk);
+	else fit_pair<P, QC == 1, false>(f, s, g.pc, g.qc, g.swc);
+}
+
+template <class P, int QC>
+__device__ __forceinline__ void fit_gate_a(typename P::T (&v)[16], const typename FitGateOf<typename P::T, QC>::type& g)
+{
+#pragma unroll
+	for (int k = 0; k < 4; k++) fit_apply<P, QC>(v[4 * k], v[4 * k + 3], g, true);
+#pragma unroll
+	for (int k = 0; k < 4; k++) fit_apply<P, QC>(v[4 * k + 1], v[4 * k + 2], g, false);
+}
+
+template <class P, int QC>
+__device__ __forceinline__ void fit_gate_b(typename P::T (&v)[16], const FitGroup& G, const typename FitGateOf<typename P::T, QC>::type& g)
+{
 	if (G.kind_b == 1)
 	{
-		const FitGate<T>& g = gates[1];
-		{
-			const T p = g.pk, q = g.qk;
-			const bool sw = g.swk;
 #pragma unroll
-			for (int k = 0; k < 4; k++) fit_pair<P, QC, false>(v[k], v[k + 12], p, q, sw);
-		}
-		{
-			const T p = g.pc, q = g.qc;
-			const bool sw = g.swc;
+		for (int k = 0; k < 4; k++) fit_apply<P, QC>(v[k], v[k + 12], g, true);
 #pragma unroll
-			for (int k = 0; k < 4; k++) fit_pair<P, QC, false>(v[k + 4], v[k + 8], p, q, sw);
-		}
+		for (int k = 0; k < 4; k++) fit_apply<P, QC>(v[k + 4], v[k + 8], g, false);
+		return;
 	}
-	else if (G.kind_b == 2)
+	// pairs along bit 2: corner where the other bits (0, 1, 3) have even parity
+	fit_apply<P, QC>(v[0], v[4], g, true);
+	fit_apply<P, QC>(v[3], v[7], g, true);
+	fit_apply<P, QC>(v[9], v[13], g, true);
+	fit_apply<P, QC>(v[10], v[14], g, true);
+	if (!G.rev)
 	{
-		// pairs along bit 2: corner where the other bits (0, 1, 3) have even parity
-		const FitGate<T>& g = gates[1];
-		{
-			const T p = g.pk, q = g.qk;
-			const bool sw = g.swk;
-			fit_pair<P, QC, false>(v[0], v[4], p, q, sw);
-			fit_pair<P, QC, false>(v[3], v[7], p, q, sw);
-			fit_pair<P, QC, false>(v[9], v[13], p, q, sw);
-			fit_pair<P, QC, false>(v[10], v[14], p, q, sw);
-		}
-		const T p = g.pc, q = g.qc;
-		const bool sw = g.swc;
-		if (!G.rev)
-		{
-			fit_pair<P, QC, false>(v[1], v[5], p, q, sw);
-			fit_pair<P, QC, false>(v[2], v[6], p, q, sw);
-			fit_pair<P, QC, false>(v[8], v[12], p, q, sw);
-			fit_pair<P, QC, false>(v[11], v[15], p, q, sw);
-		}
-		else
-		{
-			fit_pair<P, QC, false>(v[5], v[1], p, q, sw);
-			fit_pair<P, QC, false>(v[6], v[2], p, q, sw);
-			fit_pair<P, QC, false>(v[12], v[8], p, q, sw);
-			fit_pair<P, QC, false>(v[15], v[11], p, q, sw);
-		}
+		fit_apply<P, QC>(v[1], v[5], g, false);
+		fit_apply<P, QC>(v[2], v[6], g, false);
+		fit_apply<P, QC>(v[8], v[12], g, false);
+		fit_apply<P, QC>(v[11], v[15], g, false);
+	}
+	else
+	{
+		fit_apply<P, QC>(v[5], v[1], g, false);
+		fit_apply<P, QC>(v[6], v[2], g, false);
+		fit_apply<P, QC>(v[12], v[8], g, false);
+		fit_apply<P, QC>(v[15], v[11], g, false);
 	}
 }
 
 // one group on a unit, all 16 amplitudes in registers: one shared-memory round trip for both
 // gates.  For the forward sweep of f alone; beside the gradient sums' registers it spills
 // (float-float L=12, 42 gates: 3.8 ms against 3.3 ms quartet by quartet)
-template <class P, bool QC>
-__device__ __forceinline__ void fit_group16(const FitGroup& G, const FitGate<typename P::T>* gates, unsigned tc, unsigned base,
+template <class P, int QC>
+__device__ __forceinline__ void fit_group16(const FitGroup& G, const typename FitGateOf<typename P::T, QC>::type* gates, unsigned tc, unsigned base,
 	unsigned U, const typename P::T* __restrict__ tab)
 {
 	typedef typename P::T T;
 	T v[16];
 #pragma unroll
 	for (int k = 0; k < 16; k++) v[k] = lds<T>(tc + fit_off(G, base, k));
-	if (tab)
+	if (QC != 2 && tab)
 	{
 #pragma unroll
 		for (int k = 0; k < 16; k++) v[k] = P::mul(tab[k * U], v[k]);
 	}
-	fit_rotate<P, QC>(v, G, gates);
+	// in sequence order (it matters to the rounding of whole blocks only)
+	if (QC == 2 && G.order) fit_gate_b<P, QC>(v, G, gates[1]);
+	if (G.ga >= 0) fit_gate_a<P, QC>(v, gates[0]);
+	if (G.kind_b && !(QC == 2 && G.order)) fit_gate_b<P, QC>(v, G, gates[1]);
 #pragma unroll
 	for (int k = 0; k < 16; k++) sts<T>(tc + fit_off(G, base, k), v[k]);
 }
@@ -224,7 +229,7 @@ __device__ __forceinline__ void fit_group16(const FitGroup& G, const FitGate<typ
 // both gates of a group on a unit, quartet by quartet in the tile.  Forward: flush (tab or null)
 // with the first gate, the state to the cache (out or null) with the last; transposed (TR):
 // flush with the last
-template <class P, bool QC, bool TR>
+template <class P, int QC, bool TR>
 __device__ __forceinline__ void fit_group(const FitGroup& G, const FitGate<typename P::T>* gates, unsigned tc, unsigned base,
 	const typename P::T* __restrict__ tab, typename P::T* __restrict__ out)
 {
@@ -251,8 +256,8 @@ __device__ __forceinline__ void fit_group(const FitGroup& G, const FitGate<typen
 				tz = *reinterpret_cast<const T*>(tb + q.z); tv = *reinterpret_cast<const T*>(tb + q.w);
 			}
 			if (!TR && tb) { x = P::mul(tx, x); y = P::mul(ty, y); z = P::mul(tz, z); v = P::mul(tv, v); }
-			fit_pair<P, QC, TR>(x, v, pk, qk, sk);
-			fit_pair<P, QC, TR>(y, z, pc, qc, sc);
+			fit_pair<P, QC == 1, TR>(x, v, pk, qk, sk);
+			fit_pair<P, QC == 1, TR>(y, z, pc, qc, sc);
 			if (TR && tb) { x = P::mul(tx, x); y = P::mul(ty, y); z = P::mul(tz, z); v = P::mul(tv, v); }
 			sts<T>(ax, x); sts<T>(ay, y); sts<T>(az, z); sts<T>(aw, v);
 			if (ob)
@@ -268,9 +273,9 @@ __device__ __forceinline__ void fit_group(const FitGroup& G, const FitGate<typen
 // derivative in the tile and the cached state ct, read one quartet ahead.  One loop for every
 // kind of gate, not unrolled: with each gate's quartets unrolled the kernel's code outgrew the
 // instruction caches (a third of its stalls).
-// eout (or null): the derivative also to its cache, with the last gate.  SW: the tile holds the
+// EOUT: the derivative also to its cache eout, with the last gate.  SW: the tile holds the
 // state and ct the derivative (Hessian items)
-template <class P, bool SW = false>
+template <class P, bool SW, bool EOUT>
 __device__ __forceinline__ void fit_contract(const FitGroup& G, int first, int last, unsigned tc, unsigned base,
 	const typename P::T* __restrict__ ct, typename P::Acc (&acc)[8], typename P::T* __restrict__ eout = nullptr)
 {
@@ -287,7 +292,7 @@ __device__ __forceinline__ void fit_contract(const FitGroup& G, int first, int l
 		const uint4 o = qs[i];
 		const T x = lds<T>(tc + (base ^ o.x)), y = lds<T>(tc + (base ^ o.y)), z = lds<T>(tc + (base ^ o.z)), v = lds<T>(tc + (base ^ o.w));
 		const T sx = cx, sy = cy, sz = cz, sv = cw;
-		if (!SW && eout && (i >> 2) == last)
+		if (EOUT && (i >> 2) == last)
 		{
 			const uint4 q = qy[i];
 			char* eb = reinterpret_cast<char*>(eout);
@@ -308,13 +313,15 @@ __device__ __forceinline__ void fit_contract(const FitGroup& G, int first, int l
 
 // threads per block: 128, or 256 where a tile has that many units; four (two) blocks per SM
 // (registers), three of 128 in complex128, whose pipe is the bound
-template <class P, bool QC, bool GRAD, int FIT_NT>
+template <class P, int QC, int MODE, int FIT_NT>
 __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 : P::kId == MG_PREC_FP64_ID ? 3 : 4) k_fit(FitArgs<P> a)
 {
 	typedef typename P::T T;
 	constexpr unsigned ES = sizeof(T);
 	extern __shared__ __align__(16) char smem_raw[];
-	__shared__ FitStage<T> stage[2];
+	typedef typename FitGateOf<T, QC>::type Gate;
+	constexpr bool GRAD = MODE == FIT_GRAD || MODE == FIT_HESS;
+	__shared__ FitStage<Gate> stage[2];
 	const int kt = a.kt, nu = kt - 4;
 	const unsigned U = 1u << nu, n = 1u << kt;
 	const int nc = a.nc;
@@ -329,8 +336,6 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 	const long S = a.S;
 	const unsigned mycol = min(threadIdx.x >> nu, (unsigned)nc - 1), u0 = nc > 1 ? (threadIdx.x & (U - 1)) : threadIdx.x;
 	const unsigned colb = mycol * n * ES;
-	T* su = a.su + (size_t)blockIdx.x * S;
-	T* sw = a.sw + (size_t)blockIdx.x * S;
 	const size_t cstride = (size_t)nc * S;
 	typename P::Acc acc[8];
 #pragma unroll
@@ -343,8 +348,10 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 		// this thread's column (the last one again past the range: its derivative is zero)
 		const long b = min(cb + (long)mycol, a.b1 - 1);
 		const int par = __popcll(b) & 1;
-		const size_t coff = (size_t)(a.slot_per_column ? (cb - a.b0) / nc : blockIdx.x) * a.ngroups * cstride + (size_t)mycol * S;
+		const size_t coff = (size_t)(MODE == FIT_HESS ? (cb - a.b0) / nc : blockIdx.x) * a.ngroups * cstride + (size_t)mycol * S;
 		T* cache = GRAD ? a.cache + coff : nullptr;
+		// the state between passes (one column per block then): the output column itself, or a slot
+		auto between = [&]() { return MODE == FIT_COLS ? a.ucols + (size_t)(cb - a.b0) * S : a.sw + (size_t)blockIdx.x * S; };
 		for (int p = 0; p < a.npass; p++)
 		{
 			const PassRec& pr = a.pass[p];
@@ -357,49 +364,63 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 			{
 				const unsigned nlb = nl_base(pr, tau);
 				const int tpar = (__popc(nlb) + par) & 1;
-				fit_stage<T>(stage[fp.gbeg & 1], a.groups + fp.gbeg, a.gates + 2 * fp.gbeg);
+				fit_stage<Gate>(stage[fp.gbeg & 1], a.groups + fp.gbeg, static_cast<const Gate*>(a.gates) + 2 * fp.gbeg);
 				for (unsigned e = threadIdx.x; e < n * nc; e += FIT_NT)
 				{
 					const unsigned c = gidx(s, nlb, e & (n - 1));
 					T v;
 					if (p == 0) v = c == (unsigned)(min(cb + (long)(e >> kt), a.b1 - 1) >> 1) ? P::make(1.0, 0.0) : P::zero();
-					else v = sw[c];
-					sts<T>(tb + ((e & ~(n - 1)) + fsw(e & (n - 1))) * ES, v);
+					else v = between()[c];
+					sts<T>(tb + ((e & ~(n - 1)) + fsw<ES>(e & (n - 1))) * ES, v);
 				}
 				fit_stage_wait();
 				__syncthreads();
 				for (int g = fp.gbeg; g < fp.gend; g++)
 				{
 					const FitGroup& G = stage[g & 1].g;
-					if (g + 1 < fp.gend) fit_stage<T>(stage[(g + 1) & 1], a.groups + g + 1, a.gates + 2 * (g + 1));
+					if (g + 1 < fp.gend) fit_stage<Gate>(stage[(g + 1) & 1], a.groups + g + 1, static_cast<const Gate*>(a.gates) + 2 * (g + 1));
 					for (unsigned i = 0; i < its; i++)
 					{
 						const unsigned u = u0 + i * FIT_NT, base = fit_base(G, a.bases + (size_t)g * U, u, tpar);
 						const T* tab = G.flush >= 0 ? a.tables + ((size_t)(2 * G.flush + par) * S + ((size_t)tau << kt) + u) : nullptr;
 						T* out = GRAD ? cache + (size_t)g * cstride + ((size_t)tau << kt) + u : nullptr;
-						if (GRAD) fit_group<P, QC, false>(G, stage[g & 1].gate, tb + colb, base, tab, out);
+						if constexpr (GRAD) fit_group<P, QC, false>(G, stage[g & 1].gate, tb + colb, base, tab, out);
 						else fit_group16<P, QC>(G, stage[g & 1].gate, tb + colb, base, U, tab);
 					}
 					fit_stage_wait();
 					__syncthreads();
 				}
-				if (!GRAD && last)
+				if (MODE == FIT_COLS && last)
 				{
 					for (unsigned e = threadIdx.x; e < n * nc; e += FIT_NT)
 					{
 						const unsigned c = gidx(s, nlb, e & (n - 1));
 						const long be = cb + (long)(e >> kt);
 						if (be >= a.b1) continue;
-						const T d = P::mul(a.final[(size_t)(__popcll(be) & 1) * S + c], a.dense[(size_t)(be - a.dense_b0) * S + c]);
-						P::acc_mul_add(facc, d, lds<T>(tb + ((e & ~(n - 1)) + fsw(e & (n - 1))) * ES));
+						T v = lds<T>(tb + ((e & ~(n - 1)) + fsw<ES>(e & (n - 1))) * ES);
+						if (QC != 2) v = P::mul(a.final[(size_t)(__popcll(be) & 1) * S + c], v);
+						a.ucols[(size_t)(be - a.b0) * S + c] = P::negconj(v);
+					}
+				}
+				if (MODE == FIT_VALUE && last)
+				{
+					for (unsigned e = threadIdx.x; e < n * nc; e += FIT_NT)
+					{
+						const unsigned c = gidx(s, nlb, e & (n - 1));
+						const long be = cb + (long)(e >> kt);
+						if (be >= a.b1) continue;
+						T d = a.dense[(size_t)(be - a.dense_b0) * S + c];
+						if (QC != 2) d = P::mul(a.final[(size_t)(__popcll(be) & 1) * S + c], d);
+						P::acc_mul_add(facc, d, lds<T>(tb + ((e & ~(n - 1)) + fsw<ES>(e & (n - 1))) * ES));
 					}
 				}
 				if (!last)
-					for (unsigned e = threadIdx.x; e < n; e += FIT_NT) sw[gidx(s, nlb, e)] = lds<T>(tb + fsw(e) * ES);
+					for (unsigned e = threadIdx.x; e < n; e += FIT_NT) between()[gidx(s, nlb, e)] = lds<T>(tb + fsw<ES>(e) * ES);
 				__syncthreads();
 			}
 		}
-		if (!GRAD) continue;
+		if constexpr (GRAD)
+		{
 		for (int p = a.npass - 1; p >= 0; p--)
 		{
 			const PassRec& pr = a.pass[p];
@@ -412,7 +433,7 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 			{
 				const unsigned nlb = nl_base(pr, tau);
 				const int tpar = (__popc(nlb) + par) & 1;
-				fit_stage<T>(stage[(fp.gend - 1) & 1], a.groups + fp.gend - 1, a.gates + 2 * (fp.gend - 1));
+				fit_stage<Gate>(stage[(fp.gend - 1) & 1], a.groups + fp.gend - 1, static_cast<const Gate*>(a.gates) + 2 * (fp.gend - 1));
 				for (unsigned e = threadIdx.x; e < n * nc; e += FIT_NT)
 				{
 					const unsigned c = gidx(s, nlb, e & (n - 1));
@@ -423,8 +444,8 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 						v = be < a.b1 ? P::mul(a.final[(size_t)(__popcll(be) & 1) * S + c], a.dense[(size_t)(be - a.dense_b0) * S + c])
 							: P::zero();
 					}
-					else v = su[c];
-					sts<T>(tb + ((e & ~(n - 1)) + fsw(e & (n - 1))) * ES, v);
+					else v = a.su[(size_t)blockIdx.x * S + c];
+					sts<T>(tb + ((e & ~(n - 1)) + fsw<ES>(e & (n - 1))) * ES, v);
 				}
 				fit_stage_wait();
 				__syncthreads();
@@ -434,9 +455,9 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 					// the state is the one after both gates: both sums come before the
 					// transposed gates
 					const FitGroup& G = stage[g & 1].g;
-					if (g > fp.gbeg) fit_stage<T>(stage[(g - 1) & 1], a.groups + g - 1, a.gates + 2 * (g - 1));
+					if (g > fp.gbeg) fit_stage<Gate>(stage[(g - 1) & 1], a.groups + g - 1, static_cast<const Gate*>(a.gates) + 2 * (g - 1));
 					const T* cg = cache + (size_t)g * cstride + ((size_t)tau << kt) + u0;
-					T* eg = a.dcache ? a.dcache + coff + (size_t)g * cstride + ((size_t)tau << kt) + u0 : nullptr;
+					T* eg = MODE == FIT_HESS ? a.dcache + coff + (size_t)g * cstride + ((size_t)tau << kt) + u0 : nullptr;
 					const T* tab = G.flush >= 0 ? a.tables + ((size_t)(2 * G.flush + par) * S + ((size_t)tau << kt) + u0) : nullptr;
 					const int blk = G.ga >= 0 ? G.blk_a : G.blk_b;
 					if (g > fp.gbeg)
@@ -452,14 +473,14 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 					if (split)
 					{
 						for (unsigned i = 0; i < its; i++)
-							fit_contract<P>(G, 1, 1, tb + colb, fit_base(G, a.bases + (size_t)g * U, u0 + i * FIT_NT, tpar), cg + i * FIT_NT, acc);
+							fit_contract<P, false, false>(G, 1, 1, tb + colb, fit_base(G, a.bases + (size_t)g * U, u0 + i * FIT_NT, tpar), cg + i * FIT_NT, acc);
 						block_reduce8<P>(acc, s.red, a.part + ((size_t)blockIdx.x * a.nblocks + G.blk_b) * 16, 1.0, nred);
 #pragma unroll
 						for (int e = 0; e < 8; e++) acc[e] = P::acc_zero();
 					}
 					for (unsigned i = 0; i < its; i++)
-						fit_contract<P>(G, (G.kind_b && !split) ? 1 : 0, G.ga >= 0 ? 0 : 1, tb + colb,
-							fit_base(G, a.bases + (size_t)g * U, u0 + i * FIT_NT, tpar), cg + i * FIT_NT, acc, eg ? eg + i * FIT_NT : nullptr);
+						fit_contract<P, false, MODE == FIT_HESS>(G, (G.kind_b && !split) ? 1 : 0, G.ga >= 0 ? 0 : 1, tb + colb,
+							fit_base(G, a.bases + (size_t)g * U, u0 + i * FIT_NT, tpar), cg + i * FIT_NT, acc, eg + i * FIT_NT);
 					if (g > 0)   // nothing uses the derivative before the first group
 						for (unsigned i = 0; i < its; i++)
 							fit_group<P, QC, true>(G, stage[g & 1].gate, tb + colb, fit_base(G, a.bases + (size_t)g * U, u0 + i * FIT_NT, tpar),
@@ -491,12 +512,13 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 					}
 				}
 				if (p > 0)
-					for (unsigned e = threadIdx.x; e < n; e += FIT_NT) su[gidx(s, nlb, e)] = lds<T>(tb + fsw(e) * ES);
+					for (unsigned e = threadIdx.x; e < n; e += FIT_NT) a.su[(size_t)blockIdx.x * S + gidx(s, nlb, e)] = lds<T>(tb + fsw<ES>(e) * ES);
 				__syncthreads();
 			}
 		}
+		}
 	}
-	if (!GRAD) block_reduce1<P>(facc, s.red, a.part + (size_t)blockIdx.x * 2);
+	if (MODE == FIT_VALUE) block_reduce1<P>(facc, s.red, a.part + (size_t)blockIdx.x * 2);
 }
 
 // ------------------------------------------------------------------------------------
@@ -549,13 +571,14 @@ __device__ __forceinline__ void fit_move(const FitGroup& G, int w, int x, unsign
 	}
 }
 
-template <class P, bool QC, int FIT_NT>
+template <class P, int QC, int FIT_NT>
 __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 : P::kId == MG_PREC_FP64_ID ? 3 : 4) k_fit_hess(FitHessArgs<P> h, long nitems)
 {
 	typedef typename P::T T;
 	constexpr unsigned ES = sizeof(T);
 	extern __shared__ __align__(16) char smem_raw[];
-	__shared__ FitStage<T> stage[2];
+	typedef FitGate<T> Gate;
+	__shared__ FitStage<Gate> stage[2];
 	const FitArgs<P>& a = h.f;
 	const int kt = a.kt, nu = kt - 4, nc = a.nc;
 	const unsigned U = 1u << nu, n = 1u << kt;
@@ -596,13 +619,13 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 			merged = 0;
 		};
 		__syncthreads();   // the previous item's last reads
-		fit_stage<T>(stage[g0 & 1], a.groups + g0, a.gates + 2 * g0);
+		fit_stage<Gate>(stage[g0 & 1], a.groups + g0, static_cast<const Gate*>(a.gates) + 2 * g0);
 		fit_stage_wait();
 		__syncthreads();
 		for (int g = g0; g < a.ngroups; g++)
 		{
 			const FitGroup& G = stage[g & 1].g;
-			if (g + 1 < a.ngroups) fit_stage<T>(stage[(g + 1) & 1], a.groups + g + 1, a.gates + 2 * (g + 1));
+			if (g + 1 < a.ngroups) fit_stage<Gate>(stage[(g + 1) & 1], a.groups + g + 1, static_cast<const Gate*>(a.gates) + 2 * (g + 1));
 			const T* cg = a.cache + coff + (size_t)g * cstride;
 			const T* eg = a.dcache + coff + (size_t)g * cstride;
 			const unsigned* bs = a.bases + (size_t)g * U;
@@ -640,7 +663,7 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 				for (unsigned i = 0; i < its; i++)
 				{
 					const unsigned base = fit_base(G, bs, u0 + i * FIT_NT, par);
-					fit_contract<P, true>(G, w, w, tc, base, eg + i * FIT_NT, acc);
+					fit_contract<P, true, false>(G, w, w, tc, base, eg + i * FIT_NT, acc);
 					if (blk == grp) fit_move<P>(G, w, x, tc, base, cg + i * FIT_NT, false);
 				}
 			}

@@ -1,24 +1,6 @@
 // Host side of the factored fitted circuit (mgcu_fit.cuh): groups, flushes, factors.
 // Included by mgcu_engine.cu.
 
-struct FitProg
-{
-	bool built = false;            // the structure exists (groups, passes, flushes)
-	bool ok = false;               // the current gates factor (else the general kernels run)
-	bool qc = false;               // q needs its imaginary part
-	Sched sched;
-	std::vector<FitGroup> group;
-	std::vector<FitPass> pass_groups;
-	std::vector<std::array<int, 2>> diag;   // per table entry factor: gate, 0 left / 1 right
-	std::vector<int> beg, group_of;         // per flush (the last: the final table)
-	std::vector<int> block_gates;           // gates per block
-	std::vector<int> group_of_gate;
-	int grid_h = 0;                         // k_fit_hess blocks
-	int nflush = 0, grid = 0, nc = 1, threads = 128, kt = 0;
-	size_t smem = 0;
-	DevBuf d_pass, d_group, d_pgroups, d_gates, d_diag, d_beg, d_gof, d_tab, d_blk, d_bases, d_pgroup, cache;
-};
-
 // wires of gate g as a mask
 static unsigned fit_wires(const int* w, int g) { return (1u << w[2 * g]) | (1u << w[2 * g + 1]); }
 
@@ -26,11 +8,12 @@ static unsigned fit_wires(const int* w, int g) { return (1u << w[2 * g]) | (1u <
 // gates within a pass, then flushes: before a group whose right factors are not merged yet, one
 // table of all pending left factors and of the right factors of every gate that comes next on
 // both of its wires (one flush per brickwall layer when the sector is one tile).  ordered
-// (Hessians, one tile): the groups keep the sequence of the gates.
-static int fit_build(int L, int kt, const int* wires, int ng, const int* block, int nblocks, int es, bool ordered, FitProg& f)
+// (Hessians, unfactored gates): the groups keep the sequence of the gates; unfactored: no flushes.
+static int fit_build(int L, int kt, const int* wires, int ng, const int* block, int nblocks, int es, bool ordered, bool factored, FitProg& f)
 {
 	const int nb = L - 1;
-	schedule(L, kt, wires, ng, !ordered, f.sched, 1);
+	schedule(L, kt, wires, ng, !ordered, f.sched, es >= 16 ? 1 : 2);
+	f.nflush = 0;
 	std::vector<std::vector<int>> onq(L);
 	for (int g = 0; g < ng; g++) { onq[wires[2 * g]].push_back(g); onq[wires[2 * g + 1]].push_back(g); }
 	std::vector<size_t> next(L, 0);
@@ -39,7 +22,7 @@ static int fit_build(int L, int kt, const int* wires, int ng, const int* block, 
 	std::vector<int> pending;
 	f.group.clear(); f.pass_groups.clear(); f.diag.clear(); f.beg.assign(1, 0); f.group_of.clear();
 	f.group_of_gate.assign(ng, 0);
-	const unsigned pers = 3;   // swizzle period of the tile bits
+	const unsigned pers = es == 16 ? 3 : 4;   // swizzle period of the tile bits
 	for (size_t p = 0; p < f.sched.pass.size(); p++)
 	{
 		const PassRec& pr = f.sched.pass[p];
@@ -100,7 +83,7 @@ static int fit_build(int L, int kt, const int* wires, int ng, const int* block, 
 			for (int j = 0; j < kt; j++)
 			{
 				G.cbit[j] = pr.lbits[bits[j]];
-				const unsigned off = fsw(1u << bits[j]) * (unsigned)es;
+				const unsigned off = (es == 16 ? fsw<16>(1u << bits[j]) : fsw<8>(1u << bits[j])) * (unsigned)es;
 				if (j < 4) G.m[j] = off; else tm[j - 4] = off;
 			}
 			for (unsigned u = 0; u < (1u << (kt - 4)); u++)
@@ -136,7 +119,7 @@ static int fit_build(int L, int kt, const int* wires, int ng, const int* block, 
 			G.flush = -1;
 			bool need = false;
 			for (int s : { a, b })
-				if (s >= 0) need = need || !cdone[s];
+				if (s >= 0) need = need || (factored && !cdone[s]);
 			if (need)
 			{
 				G.flush = f.nflush++;
@@ -170,13 +153,15 @@ static int fit_build(int L, int kt, const int* wires, int ng, const int* block, 
 	f.block_gates.assign(nblocks, 0);
 	for (int g = 0; g < ng; g++) f.block_gates[block[g]]++;
 	const int U = 1 << (kt - 4);
-	f.threads = U >= 512 ? 512 : U >= 256 ? 256 : 128;
+	f.threads = (U >= 512 && es == 16) ? 512 : U >= 256 ? 256 : 128;
+	f.kt = kt;
+	f.factored = factored;
 	f.nc = (U < 128 && nb <= kt) ? 128 / U : 1;   // small sectors share a block
 	f.smem = (size_t)f.nc * ((size_t)1 << kt) * es + 2 * 128 * sizeof(unsigned) + red_bytes(f.threads);
 	int e = upload_sched(f.sched, f.d_pass, f.d_gates);
 	if (!e) e = f.d_group.alloc(sizeof(FitGroup) * f.group.size());
 	if (!e) e = f.d_pgroups.alloc(sizeof(FitPass) * f.pass_groups.size());
-	if (!e) e = f.d_gates.alloc(sizeof(FitGate<double2>) * 2 * f.group.size());
+	if (!e) e = f.d_gates.alloc(std::max(sizeof(FitGate<double2>), sizeof(FitWhole<double2>)) * 2 * f.group.size());
 	if (!e) e = f.d_diag.alloc(sizeof(FitDiag) * f.diag.size());
 	if (!e) e = f.d_beg.alloc(sizeof(int) * f.beg.size());
 	if (!e) e = f.d_gof.alloc(sizeof(int) * std::max(f.nflush, 1));
@@ -290,6 +275,25 @@ static int fit_set_gates(const mgg* gates, int ng, const int* block, int nblocks
 {
 	typedef typename P::T T;
 	f.ok = false;
+	if (!f.factored)
+	{
+		std::vector<FitWhole<T>> hw(2 * f.group.size());
+		memset(hw.data(), 0, sizeof(FitWhole<T>) * hw.size());
+		for (size_t i = 0; i < hw.size(); i++)
+		{
+			const int g = i & 1 ? f.group[i / 2].gb : f.group[i / 2].ga;
+			if (g < 0) continue;
+			for (int q = 0; q < 4; q++)
+			{
+				hw[i].c[q] = P::make(gates[g].c[q].re, gates[g].c[q].im);
+				hw[i].k[q] = P::make(gates[g].k[q].re, gates[g].k[q].im);
+			}
+		}
+		MGCU_TRY(cudaMemcpyAsync(f.d_gates.p, hw.data(), sizeof(FitWhole<T>) * hw.size(), cudaMemcpyHostToDevice, mgcu_stream()));
+		f.qc = 2;
+		f.ok = true;
+		return 0;
+	}
 	std::vector<int> first(nblocks, -1);
 	for (int g = 0; g < ng; g++)
 	{
@@ -365,20 +369,79 @@ static int fit_set_gates(const mgg* gates, int ng, const int* block, int nblocks
 }
 
 template <class P, int NT>
-static void (*fit_kernel_nt(bool qc, bool grad))(FitArgs<P>)
+static void (*fit_kernel_nt(int qc, int mode))(FitArgs<P>)
 {
-	return qc ? (grad ? k_fit<P, true, true, NT> : k_fit<P, true, false, NT>) : (grad ? k_fit<P, false, true, NT> : k_fit<P, false, false, NT>);
+	if constexpr (P::kId == MG_PREC_FP32_ID) return mode == FIT_COLS ? k_fit<P, 2, FIT_COLS, NT> : k_fit<P, 2, FIT_VALUE, NT>;
+	else if (qc)
+		return mode == FIT_COLS ? k_fit<P, 1, FIT_COLS, NT> : mode == FIT_GRAD ? k_fit<P, 1, FIT_GRAD, NT>
+			: mode == FIT_HESS ? k_fit<P, 1, FIT_HESS, NT> : k_fit<P, 1, FIT_VALUE, NT>;
+	else
+		return mode == FIT_COLS ? k_fit<P, 0, FIT_COLS, NT> : mode == FIT_GRAD ? k_fit<P, 0, FIT_GRAD, NT>
+			: mode == FIT_HESS ? k_fit<P, 0, FIT_HESS, NT> : k_fit<P, 0, FIT_VALUE, NT>;
 }
 template <class P>
-static void (*fit_kernel(bool qc, bool grad, int threads))(FitArgs<P>)
+static void (*fit_kernel(int qc, int mode, int threads))(FitArgs<P>)
 {
-	return threads == 512 ? fit_kernel_nt<P, 512>(qc, grad) : threads == 256 ? fit_kernel_nt<P, 256>(qc, grad) : fit_kernel_nt<P, 128>(qc, grad);
+	return threads == 512 ? fit_kernel_nt<P, 512>(qc, mode) : threads == 256 ? fit_kernel_nt<P, 256>(qc, mode) : fit_kernel_nt<P, 128>(qc, mode);
+}
+
+// k_fit's arguments that come from a program
+template <class P>
+static FitArgs<P> fit_args(const FitProg& f, int L)
+{
+	typedef typename P::T T;
+	FitArgs<P> w;
+	memset(&w, 0, sizeof(w));
+	w.L = L; w.nb = L - 1; w.kt = f.kt; w.npass = (int)f.sched.pass.size(); w.ngroups = (int)f.group.size(); w.nc = f.nc;
+	w.S = 1L << (L - 1);
+	w.pass = f.d_pass.as<PassRec>(); w.groups_of = f.d_pgroups.as<FitPass>(); w.groups = f.d_group.as<FitGroup>();
+	w.bases = f.d_bases.as<unsigned>();
+	w.gates = f.d_gates.p; w.tables = f.d_tab.as<T>(); w.final = w.tables + (size_t)2 * w.S * f.nflush;
+	return w;
+}
+
+// The columns of a circuit target by k_fit, for targets that don't conserve particle numbers:
+// factored blocks in complex128 and float-float; in FP32 whole blocks in k_target's order (the
+// same bits), when every block is general there.  f.grid: resident blocks; state 0: not used.
+template <class P>
+static int target_fit(mgcu_target* t, TargetProg& tp, FitProg& f)
+{
+	constexpr int es = sizeof(typename P::T);
+	if (f.built || f.tried) return 0;
+	f.tried = true;
+	const int ng = (int)tp.sched.gate.size();
+	if (ng < 1 || t->L > 18 || t->L < 10) return 0;
+	for (unsigned m : t->smask) if (m) return 0;
+	const bool factored = P::kId != MG_PREC_FP32_ID;
+	std::vector<mgg> g(ng);
+	std::vector<int> w(2 * ng), block(ng);
+	std::map<int, int> id;
+	for (int i = 0; i < ng; i++)
+	{
+		const int q = tp.sched.gate[i].g;
+		g[i] = t->sg[q];
+		w[2 * i] = t->sw[2 * q]; w[2 * i + 1] = t->sw[2 * q + 1];
+		block[i] = id.emplace(tp.first[q], (int)id.size()).first->second;
+		if (!factored && ((tp.kw[q] & 7) != BK_GEN || ((tp.kw[q] >> 3) & 7) != BK_GEN)) return 0;
+	}
+	const int nb = t->L - 1;
+	int e = fit_build(t->L, std::min(nb, es == 16 ? (nb <= 13 ? 13 : 12) : 13), w.data(), ng, block.data(), (int)id.size(), es, !factored, factored, f);
+	if (!e && factored && (size_t)f.nflush * es << (nb + 1) > (256u << 20)) { f.built = false; return 0; }
+	if (!e) e = fit_set_gates<P>(g.data(), ng, block.data(), (int)id.size(), t->L, f.kt, w.data(), f);
+	if (e) { f.built = false; return e; }
+	if (!f.ok) { f.built = false; return 0; }
+	int per = 0;
+	const int lim = (int)std::min<size_t>(mgcu_ctx()->smem_optin, 227 * 1024) - 4096;
+	MGCU_TRY(cudaFuncSetAttribute(fit_kernel<P>(f.qc, FIT_COLS, f.threads), cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+	MGCU_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fit_kernel<P>(f.qc, FIT_COLS, f.threads), f.threads, f.smem));
+	f.grid = mgcu_ctx()->nsm * std::max(per, 1);
+	return 0;
 }
 
 template <class P>
-static void (*fit_hess_kernel(bool qc, int threads))(FitHessArgs<P>, long)
+static void (*fit_hess_kernel(int qc, int threads))(FitHessArgs<P>, long)
 {
-	return threads == 512 ? (qc ? k_fit_hess<P, true, 512> : k_fit_hess<P, false, 512>)
-		: threads == 256 ? (qc ? k_fit_hess<P, true, 256> : k_fit_hess<P, false, 256>)
-		: (qc ? k_fit_hess<P, true, 128> : k_fit_hess<P, false, 128>);
+	return threads == 512 ? (qc ? k_fit_hess<P, 1, 512> : k_fit_hess<P, 0, 512>)
+		: threads == 256 ? (qc ? k_fit_hess<P, 1, 256> : k_fit_hess<P, 0, 256>)
+		: (qc ? k_fit_hess<P, 1, 128> : k_fit_hess<P, 0, 128>);
 }

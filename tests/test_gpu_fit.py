@@ -135,3 +135,36 @@ def test_gate_hessian(mglib, L, ng, prec):
         lib.target_free(t)
     _check([o[:3] for o in out], TOL[prec])
     assert np.max(np.abs(out[0][3] - out[1][3])) <= TOL[prec] * max(np.max(np.abs(out[1][3])), np.max(np.abs(out[1][2])))
+
+
+@pytest.mark.parametrize("prec", [mgcu.PREC_FP64, mgcu.PREC_MIXED, mgcu.PREC_FP32])
+@pytest.mark.parametrize("L,nu,cols", [(10, 1, None), (10, 33, (5, 1020)), (11, 40, None), (13, 25, (300, 420)), (14, 30, (9000, 9040)),
+                                       (15, 30, (9000, 9040)), (16, 40, (65000, 65020))])
+def test_target_columns(mglib, L, nu, cols, prec):
+    """columns of a target without conserved numbers by k_fit (the default from 10 qubits) against
+    the full sweep (MG_OPT_TARGET_DENSE): whole blocks in the same order in FP32, so the same
+    bits; factored otherwise"""
+    lib, rng = mglib, np.random.default_rng(L + nu)
+    u = T.haar_matchgates(nu, rng)
+    uw = np.array([rng.choice(L, 2, replace=False) for _ in range(nu)], np.int32)
+    uw[:: 5, 0], uw[:: 5, 1] = L - 1, rng.integers(0, L - 1, size=len(uw[:: 5]))
+    t = lib.target_circuit(u, uw, L)
+    lib.set_precision(prec)
+    out = []
+    try:
+        for dense in (0, 1):
+            lib.set_option(mgcu.OPT_TARGET_DENSE, dense)
+            if L % 2 == 0:
+                v, perms = T.haar_matchgates(2, np.random.default_rng(1)), T.brickwall_perms(L, 2)
+                out.append(lib.brickwall_columns(lib.mg_target_apply, t, v, perms, L, *(cols or (0, 1 << L))))
+            else:
+                rc, f, dg = lib.circuit_target_and_gradient(lib.mg_target_apply, t, T.haar_matchgates(3, np.random.default_rng(1)),
+                                                            [[0, 1], [L - 1, 2], [3, L - 1]], L)
+                out.append((rc, f, dg))
+    finally:
+        lib.set_option(mgcu.OPT_TARGET_DENSE, 0)
+        lib.set_precision(mgcu.PREC_FP64)
+        lib.target_free(t)
+    if prec == mgcu.PREC_FP32:
+        assert out[0][1] == out[1][1] and np.array_equal(out[0][2], out[1][2])
+    _check(out, TOL[prec])
