@@ -1726,6 +1726,7 @@ __global__ void __launch_bounds__(256, 2) k_hessian(Args<P> a, long nitems)
 }
 
 #include "mgcu_fit.cuh"
+#include "mgcu_wsec.cuh"
 
 // ------------------------------------------------------------------------------------
 // small kernels: staging, reductions, symmetrisation
@@ -1847,6 +1848,20 @@ struct SectorProg
 };
 
 // a fitted circuit's or target's program for k_fit (see mgcu_fit_build.cuh)
+// a particle-conserving fit's levels and sectors for k_ws_grad / k_ws_hess
+struct WsProg
+{
+	bool built = false;            // the target conserves the particle number and the sectors fit
+	bool ok = false;               // the current gates do too
+	int ln = 0, dmax = 0, nlev = 0;
+	size_t smem = 0;
+	std::vector<int> level_of, rstart, pstart, beg;
+	std::vector<std::array<int, 2>> diag;   // per table factor: gate, 0 left / 1 right
+	std::vector<int> pair_of;               // pair table per gate
+	std::vector<unsigned> rows;
+	DevBuf d_levels, d_gates, d_pairs, d_tab, d_rows, d_sec, d_diag, d_beg, d_plevel;
+};
+
 struct FitProg
 {
 	bool factored = true;
@@ -1864,6 +1879,7 @@ struct FitProg
 	int grid_h = 0;                         // k_fit_hess blocks
 	int nflush = 0, grid = 0, nc = 1, threads = 128, kt = 0;
 	size_t smem = 0;
+	WsProg ws;
 	DevBuf d_pass, d_group, d_pgroups, d_gates, d_diag, d_beg, d_gof, d_tab, d_blk, d_bases, d_pgroup, cache;
 };
 
@@ -2574,6 +2590,61 @@ static int launch_target(mgcu_plan* p, long b0, long b1, typename P::T* out)
 	return plan_event(p, 1);
 }
 
+// the same for a particle-conserving Hessian plan in number sectors; done stays false when the
+// plan's caches have no room for the range's column groups
+template <class P>
+static int launch_ws(mgcu_plan* p, long b0, long b1, const typename P::T* dense, long dense_b0, bool& done)
+{
+	typedef typename P::T T;
+	FitProg& f = p->fit;
+	WsProg& w = f.ws;
+	cudaStream_t st = mgcu_stream();
+	std::vector<WsSec> sec;
+	int groups = 0;
+	// the largest sectors first
+	std::vector<int> order;
+	for (int n = 0; n <= p->L; n++) order.push_back(n);
+	std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return w.rstart[x + 1] - w.rstart[x] > w.rstart[y + 1] - w.rstart[y]; });
+	for (int n : order)
+	{
+		const unsigned *r = w.rows.data() + w.rstart[n], *e = w.rows.data() + w.rstart[n + 1];
+		WsSec s;
+		s.first = groups; s.n = n;
+		s.rlo = (int)(std::lower_bound(r, e, (unsigned)b0) - r);
+		s.rhi = (int)(std::lower_bound(r, e, (unsigned)b1) - r);
+		if (s.rhi <= s.rlo) continue;
+		groups += (s.rhi - s.rlo + (1 << w.ln) - 1) >> w.ln;
+		sec.push_back(s);
+	}
+	if ((size_t)groups * w.nlev * ((size_t)w.dmax << w.ln) * sizeof(T) > std::min(p->cache.n, p->dcache.n)) return 0;
+	MGCU_TRY(cudaMemcpyAsync(w.d_sec.p, sec.data(), sizeof(WsSec) * sec.size(), cudaMemcpyHostToDevice, st));
+	WsArgs<P> a;
+	memset(&a, 0, sizeof(a));
+	a.L = p->L; a.nlev = w.nlev; a.ngates = p->d.ngates; a.ln = w.ln; a.dmax = w.dmax; a.nsec = (int)sec.size(); a.ngroups = groups;
+	a.nblocks = p->d.nblocks;
+	for (int n = 0; n <= p->L + 1; n++) a.rstart[n] = w.rstart[n];
+	for (int n = 0; n < p->L; n++) a.pstart[n] = w.pstart[n];
+	a.levels = w.d_levels.as<WsLevel>(); a.gates = w.d_gates.as<WsGate<T>>(); a.pairs = w.d_pairs.as<ushort4>();
+	a.tables = w.d_tab.as<T>(); a.rows = w.d_rows.as<unsigned>(); a.sec = w.d_sec.as<WsSec>();
+	a.dense = dense; a.dense_b0 = dense_b0; a.S = p->S;
+	a.ycache = p->cache.as<T>(); a.ecache = p->dcache.as<T>();
+	a.part = p->part_g.as<double>();
+	a.place = p->d_place.as<int>(); a.place_level = w.d_plevel.as<int>(); a.block = p->d_block.as<int>();
+	a.place_w = p->d_placew.as<double>(); a.nplace = p->d.nplace; a.mdim = 8 * p->d.nblocks; a.hgroup = p->hgroup ? 1 : 0;
+	a.part_h = p->part_h.as<double>();
+	const int slots = 2 * mgcu_ctx()->nsm, ga = std::min({ slots, groups, std::max(p->grid_a, f.grid) });
+	p->rows_a = std::max(p->rows_a, ga);
+	(f.qc ? k_ws_grad<P, true> : k_ws_grad<P, false>)<<<ga, WS_NT, w.smem, st>>>(a);
+	MGCU_LAUNCHED();
+	const long nitems = (long)groups * p->d.nplace * 8;
+	const int gh = (int)std::min<long>({ (long)slots, nitems, (long)std::max(p->grid_b, f.grid_h) });
+	p->rows_h = std::max(p->rows_h, gh);
+	(f.qc ? k_ws_hess<P, true> : k_ws_hess<P, false>)<<<gh, WS_NT, w.smem, st>>>(a, nitems);
+	MGCU_LAUNCHED();
+	done = true;
+	return 0;
+}
+
 // f, gradients (and Hessian items) for columns [b0, b1) whose -conj(U e_b) are in dense
 template <class P>
 static int launch_columns(mgcu_plan* p, long b0, long b1, const typename P::T* dense, long dense_b0)
@@ -2598,6 +2669,13 @@ static int launch_columns(mgcu_plan* p, long b0, long b1, const typename P::T* d
 	if (!a.want_grad) a.cache = nullptr;
 	const long ncols = b1 - b0;
 	const int grid = (int)std::min<long>(p->grid_a, ncols);
+	if constexpr (P::kId != MG_PREC_FP32_ID)
+		if (p->fit.ok && p->fit.ws.ok)
+		{
+			bool done = false;
+			const int e = launch_ws<P>(p, b0, b1, dense, dense_b0, done);
+			if (e || done) return e;
+		}
 	if (p->fit.ok)
 	{
 		const FitProg& f = p->fit;
@@ -3027,6 +3105,16 @@ extern "C" mgcu_plan* mgcu_plan_create(const mgcu_plan_desc* d)
 			}
 			if (opt_cps > 0) ph = (int)std::min<long>(ph, opt_cps);
 			p->fit.grid_h = c->nsm * std::max(ph, 1);
+			// number sectors, where the target conserves the particle number
+			if (p->w_t) e = p->prec == MG_PREC_FP64_ID ? ws_build<PrecD>(p->L, p->wires.data(), d->ngates, p->fit.ws) : ws_build<PrecX>(p->L, p->wires.data(), d->ngates, p->fit.ws);
+			if (!e && p->fit.ws.built)
+			{
+				std::vector<int> pl(std::max(p->d.nplace, 1), 0);
+				for (int q = 0; q < p->d.nplace; q++) pl[q] = p->fit.ws.level_of[p->place[q]];
+				e = p->fit.ws.d_plevel.alloc(sizeof(int) * pl.size());
+				if (!e && cudaMemcpy(p->fit.ws.d_plevel.p, pl.data(), sizeof(int) * pl.size(), cudaMemcpyHostToDevice) != cudaSuccess) e = MG_ERR_DEVICE;
+			}
+			if (e) { delete p; return nullptr; }
 			std::vector<int> pg(std::max(p->d.nplace, 1), 0);
 			for (int q = 0; q < p->d.nplace; q++) pg[q] = p->fit.group_of_gate[p->place[q]];
 			e = p->fit.d_pgroup.alloc(sizeof(int) * pg.size());

@@ -699,6 +699,32 @@ __device__ __forceinline__ Dd dd_neg(Dd a) { a.h = -a.h; a.l = -a.l; return a; }
 // double-double
 struct FitDiag { double v[4][4]; int si, sj; };
 
+// product of the factors beg..end at a full basis index
+template <class P>
+__device__ __forceinline__ typename P::T fit_table_entry(const FitDiag* __restrict__ diag, int beg, int end, unsigned long full)
+{
+	Dd re = { 1, 0 }, im = { 0, 0 };
+	for (int d = beg; d < end; d++)
+	{
+		const FitDiag& D = diag[d];
+		const double* v = D.v[2 * ((full >> D.si) & 1) + ((full >> D.sj) & 1)];
+		if (P::kId == MG_PREC_FP64_ID)
+		{
+			const Dd a = { v[0], v[1] }, b = { v[2], v[3] };
+			const Dd r = dd_add(dd_mul(re, a), dd_neg(dd_mul(im, b)));
+			im = dd_add(dd_mul(re, b), dd_mul(im, a));
+			re = r;
+		}
+		else
+		{
+			const double r = re.h * v[0] - im.h * v[2];
+			im.h = re.h * v[2] + im.h * v[0];
+			re.h = r;
+		}
+	}
+	return P::make(re.h, im.h);
+}
+
 // entry (parity, position) of every flush's table and of the final one (flush == nflush)
 template <class P>
 __global__ void k_fit_tables(const FitDiag* __restrict__ diag, const int* __restrict__ beg, int nflush, const int* __restrict__ group_of,
@@ -724,26 +750,7 @@ __global__ void k_fit_tables(const FitDiag* __restrict__ diag, const int* __rest
 			for (int j = 0; j < nu; j++) c |= ((u >> j) & 1u) << G.cbit[4 + j];
 		}
 		const unsigned long full = ((unsigned long)c << 1) | ((__popc(c) + par) & 1);
-		Dd re = { 1, 0 }, im = { 0, 0 };
-		for (int d = beg[f]; d < beg[f + 1]; d++)
-		{
-			const FitDiag& D = diag[d];
-			const double* v = D.v[2 * ((full >> D.si) & 1) + ((full >> D.sj) & 1)];
-			if (P::kId == MG_PREC_FP64_ID)
-			{
-				const Dd a = { v[0], v[1] }, b = { v[2], v[3] };
-				const Dd r = dd_add(dd_mul(re, a), dd_neg(dd_mul(im, b)));
-				im = dd_add(dd_mul(re, b), dd_mul(im, a));
-				re = r;
-			}
-			else
-			{
-				const double r = re.h * v[0] - im.h * v[2];
-				im.h = re.h * v[2] + im.h * v[0];
-				re.h = r;
-			}
-		}
-		tables[q] = P::make(re.h, im.h);
+		tables[q] = fit_table_entry<P>(diag, beg[f], beg[f + 1], full);
 	}
 }
 

@@ -269,6 +269,143 @@ static bool fit_factor(const mgc* e, FitFactor& F)
 	return std::hypot(dr, di) > 1.0 / 256 && std::hypot(F.q.re, F.q.im) < 256 && F.p < 256;
 }
 
+// Levels, pair tables and row positions for the number sectors (see mgcu_wsec.cuh): w.built when
+// the largest sector leaves two blocks per SM (L <= 14) and the gates fit in shared memory.
+// Columns per block: up to eight, as many as fit.
+template <class P>
+static int ws_build(int L, const int* wires, int ng, WsProg& w)
+{
+	typedef typename P::T T;
+	if (L > 14 || L < 4 || ng > WS_MAXG) return 0;
+	auto bit = [&](int q) { return 1u << (L - 1 - q); };
+	const unsigned N = 1u << L;
+	// rows by (ones, index)
+	w.rstart.assign(L + 2, 0);
+	for (unsigned a = 0; a < N; a++) w.rstart[__builtin_popcount(a) + 1]++;
+	for (int n = 0; n <= L; n++) w.rstart[n + 1] += w.rstart[n];
+	w.rows.assign(N, 0);
+	std::vector<int> row(N), fill(w.rstart);
+	for (unsigned a = 0; a < N; a++)
+	{
+		const int n = __builtin_popcount(a), q = fill[n]++;
+		w.rows[q] = a;
+		row[a] = q - w.rstart[n];
+	}
+	w.dmax = 0;
+	for (int n = 0; n <= L; n++) w.dmax = std::max(w.dmax, w.rstart[n + 1] - w.rstart[n]);
+	const size_t room = 107000;
+	w.ln = 0;
+	while (w.ln < 3 && ((size_t)w.dmax << (w.ln + 1)) * sizeof(T) <= room) w.ln++;
+	w.smem = ((size_t)w.dmax << w.ln) * sizeof(T);
+	if (w.smem > room) return 0;
+	// other wires' values by (ones, value)
+	w.pstart.assign(L, 0);
+	std::vector<unsigned> order(N >> 2);
+	for (unsigned q = 0; q < (N >> 2); q++) order[q] = q;
+	std::stable_sort(order.begin(), order.end(), [](unsigned x, unsigned y) { return __builtin_popcount(x) < __builtin_popcount(y); });
+	for (unsigned q = 0; q < (N >> 2); q++) w.pstart[__builtin_popcount(q) + 1]++;
+	for (int m = 0; m + 1 < L; m++) w.pstart[m + 1] += w.pstart[m];
+	std::map<std::pair<int, int>, int> id;
+	std::vector<ushort4> pairs;
+	w.pair_of.assign(ng, 0);
+	for (int g = 0; g < ng; g++)
+	{
+		const auto ins = id.emplace(std::make_pair(wires[2 * g], wires[2 * g + 1]), (int)id.size());
+		w.pair_of[g] = ins.first->second;
+		if (!ins.second) continue;
+		const unsigned bi = bit(wires[2 * g]), bj = bit(wires[2 * g + 1]), lo = std::min(bi, bj), hi = std::max(bi, bj);
+		for (unsigned q : order)
+		{
+			unsigned a = ((q & ~(lo - 1)) << 1) | (q & (lo - 1));
+			a = ((a & ~(hi - 1)) << 1) | (a & (hi - 1));
+			pairs.push_back(make_ushort4((unsigned short)row[a], (unsigned short)row[a | bj], (unsigned short)row[a | bi], (unsigned short)row[a | bi | bj]));
+		}
+	}
+	// levels: runs of gates on disjoint wires; each level's table holds the left factors of the
+	// level before and its own right factors
+	std::vector<WsLevel> lev;
+	w.level_of.assign(ng, 0);
+	w.diag.clear();
+	w.beg.assign(1, 0);
+	for (int g = 0; g < ng;)
+	{
+		WsLevel V;
+		V.gbeg = g;
+		unsigned used = 0;
+		while (g < ng && !(fit_wires(wires, g) & used)) { used |= fit_wires(wires, g); w.level_of[g++] = (int)lev.size(); }
+		V.gend = g;
+		if (!lev.empty()) for (int s = lev.back().gbeg; s < lev.back().gend; s++) w.diag.push_back({ s, 0 });
+		for (int s = V.gbeg; s < V.gend; s++) w.diag.push_back({ s, 1 });
+		w.beg.push_back((int)w.diag.size());
+		lev.push_back(V);
+	}
+	for (int s = lev.back().gbeg; s < lev.back().gend; s++) w.diag.push_back({ s, 0 });
+	w.beg.push_back((int)w.diag.size());
+	w.nlev = (int)lev.size();
+	int e = w.d_levels.alloc(sizeof(WsLevel) * lev.size());
+	if (!e) e = w.d_gates.alloc(sizeof(WsGate<T>) * ng);
+	if (!e) e = w.d_pairs.alloc(sizeof(ushort4) * pairs.size());
+	if (!e) e = w.d_tab.alloc(sizeof(T) * (size_t)N * (w.nlev + 1));
+	if (!e) e = w.d_rows.alloc(sizeof(unsigned) * N);
+	if (!e) e = w.d_sec.alloc(sizeof(WsSec) * (L + 1));
+	if (!e) e = w.d_diag.alloc(sizeof(FitDiag) * w.diag.size());
+	if (!e) e = w.d_beg.alloc(sizeof(int) * w.beg.size());
+	if (e) return e;
+	cudaStream_t st = mgcu_stream();
+	MGCU_TRY(cudaMemcpyAsync(w.d_levels.p, lev.data(), sizeof(WsLevel) * lev.size(), cudaMemcpyHostToDevice, st));
+	MGCU_TRY(cudaMemcpyAsync(w.d_pairs.p, pairs.data(), sizeof(ushort4) * pairs.size(), cudaMemcpyHostToDevice, st));
+	MGCU_TRY(cudaMemcpyAsync(w.d_rows.p, w.rows.data(), sizeof(unsigned) * N, cudaMemcpyHostToDevice, st));
+	MGCU_TRY(cudaMemcpyAsync(w.d_beg.p, w.beg.data(), sizeof(int) * w.beg.size(), cudaMemcpyHostToDevice, st));
+	MGCU_TRY(cudaStreamSynchronize(st));
+	for (auto k : { k_ws_grad<P, true>, k_ws_grad<P, false> }) MGCU_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
+	for (auto k : { k_ws_hess<P, true>, k_ws_hess<P, false> }) MGCU_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
+	w.built = true;
+	return 0;
+}
+
+// one diagonal factor of a gate for the tables (side 0: left, 1: right)
+static FitDiag fit_diag(const FitFactor& c, const FitFactor& k, int side, int wi, int wj, int L)
+{
+	const Hcx* fc = side ? c.r : c.l;
+	const Hcx* fk = side ? k.r : k.l;
+	const Hcx ent[4] = { fk[0], fc[0], fc[1], fk[1] };   // |00>, |01>, |10>, |11>
+	FitDiag d;
+	for (int q = 0; q < 4; q++)
+	{
+		d.v[q][0] = ent[q].re.h; d.v[q][1] = ent[q].re.l;
+		d.v[q][2] = ent[q].im.h; d.v[q][3] = ent[q].im.l;
+	}
+	d.si = L - 1 - wi; d.sj = L - 1 - wj;
+	return d;
+}
+
+// the number sectors' gates and tables; w.ok when every corner block is exactly diagonal
+template <class P>
+static int ws_set_gates(const mgg* gates, int ng, const int* block, int L, const int* wires, const std::vector<FitFactor>& fac, WsProg& w)
+{
+	typedef typename P::T T;
+	w.ok = false;
+	for (int g = 0; g < ng; g++)
+		if (gates[g].k[1].re != 0 || gates[g].k[1].im != 0 || gates[g].k[2].re != 0 || gates[g].k[2].im != 0) return 0;
+	std::vector<WsGate<T>> hg(ng);
+	for (int g = 0; g < ng; g++)
+	{
+		const FitFactor& c = fac[2 * block[g]];
+		hg[g].p = P::make(c.p, 0); hg[g].q = P::make(c.q.re, c.q.im);
+		hg[g].sw = c.sw; hg[g].pair = w.pair_of[g]; hg[g].blk = block[g]; hg[g].pad = 0;
+	}
+	std::vector<FitDiag> hd;
+	for (const auto& d : w.diag) hd.push_back(fit_diag(fac[2 * block[d[0]]], fac[2 * block[d[0]] + 1], d[1], wires[2 * d[0]], wires[2 * d[0] + 1], L));
+	cudaStream_t st = mgcu_stream();
+	MGCU_TRY(cudaMemcpyAsync(w.d_gates.p, hg.data(), sizeof(WsGate<T>) * ng, cudaMemcpyHostToDevice, st));
+	MGCU_TRY(cudaMemcpyAsync(w.d_diag.p, hd.data(), sizeof(FitDiag) * hd.size(), cudaMemcpyHostToDevice, st));
+	k_ws_tables<P><<<grid_cap((long)(w.nlev + 1) << L, 128), 128, 0, st>>>(w.d_diag.as<FitDiag>(), w.d_beg.as<int>(), w.nlev, L, w.d_rows.as<unsigned>(),
+		w.d_tab.as<T>());
+	MGCU_LAUNCHED();
+	w.ok = true;
+	return 0;
+}
+
 // factors, tables and end transforms of the current gates; f.ok tells whether they factor
 template <class P>
 static int fit_set_gates(const mgg* gates, int ng, const int* block, int nblocks, int L, int kt, const int* wires, FitProg& f)
@@ -345,21 +482,19 @@ static int fit_set_gates(const mgg* gates, int ng, const int* block, int nblocks
 	for (size_t i = 0; i < hd.size(); i++)
 	{
 		const int g = f.diag[i][0];
-		const FitFactor &c = fac[2 * block[g]], &k = fac[2 * block[g] + 1];
-		const Hcx* fc = f.diag[i][1] ? c.r : c.l;
-		const Hcx* fk = f.diag[i][1] ? k.r : k.l;
-		const Hcx ent[4] = { fk[0], fc[0], fc[1], fk[1] };   // |00>, |01>, |10>, |11>
-		for (int q = 0; q < 4; q++)
-		{
-			hd[i].v[q][0] = ent[q].re.h; hd[i].v[q][1] = ent[q].re.l;
-			hd[i].v[q][2] = ent[q].im.h; hd[i].v[q][3] = ent[q].im.l;
-		}
-		hd[i].si = L - 1 - wires[2 * g]; hd[i].sj = L - 1 - wires[2 * g + 1];
+		hd[i] = fit_diag(fac[2 * block[g]], fac[2 * block[g] + 1], f.diag[i][1], wires[2 * g], wires[2 * g + 1], L);
 	}
 	cudaStream_t st = mgcu_stream();
 	MGCU_TRY(cudaMemcpyAsync(f.d_gates.p, hg.data(), sizeof(FitGate<T>) * hg.size(), cudaMemcpyHostToDevice, st));
 	MGCU_TRY(cudaMemcpyAsync(f.d_diag.p, hd.data(), sizeof(FitDiag) * hd.size(), cudaMemcpyHostToDevice, st));
 	MGCU_TRY(cudaMemcpyAsync(f.d_blk.p, fb.data(), sizeof(FitBlock) * nblocks, cudaMemcpyHostToDevice, st));
+	f.ws.ok = false;
+	if constexpr (P::kId != MG_PREC_FP32_ID)
+		if (f.ws.built)
+		{
+			const int e = ws_set_gates<P>(gates, ng, block, L, wires, fac, f.ws);
+			if (e) return e;
+		}
 	const long S = 1L << (L - 1);
 	k_fit_tables<P><<<grid_cap(2 * S * (f.nflush + 1), 128), 128, 0, st>>>(f.d_diag.as<FitDiag>(), f.d_beg.as<int>(), f.nflush, f.d_gof.as<int>(),
 		f.d_group.as<FitGroup>(), f.d_pass.as<PassRec>(), kt, S, f.d_tab.as<T>());

@@ -168,3 +168,39 @@ def test_target_columns(mglib, L, nu, cols, prec):
     if prec == mgcu.PREC_FP32:
         assert out[0][1] == out[1][1] and np.array_equal(out[0][2], out[1][2])
     _check(out, TOL[prec])
+
+
+def _conserving(n, rng):
+    """random gates with diagonal corner blocks"""
+    v = T.haar_matchgates(n, rng)
+    v[:, 4:] = 0
+    v[:, 4], v[:, 7] = np.exp(1j * rng.uniform(0, 6, n)), np.exp(1j * rng.uniform(0, 6, n))
+    v[::3, :4] = np.array([T.hop_gate(1.0, x)[:4] for x in rng.uniform(0, 1.5, len(v[::3]))])
+    return v
+
+
+@pytest.mark.parametrize("prec", [mgcu.PREC_FP64, mgcu.PREC_MIXED])
+@pytest.mark.parametrize("L,n,kind", [(8, 1, "layer"), (8, 4, "layer"), (10, 3, "ti"), (10, 4, "layer"), (12, 2, "ti"), (14, 1, "layer"),
+                                      (7, 1, "gate"), (7, 18, "gate"), (9, 14, "gate"), (11, 7, "gate")])
+def test_conserving_hessian(mglib, L, n, kind, prec):
+    """fits and targets that conserve the particle number: number sectors against k_hessian's items,
+    with and without the conservation broken in one gate (then the parity sectors run)"""
+    lib, rng = mglib, np.random.default_rng(L + n)
+    u = _conserving(24, rng)
+    t = lib.target_circuit(u, np.array([rng.choice(L, 2, replace=False) for _ in range(24)], np.int32), L)
+    w = np.array([rng.choice(L, 2, replace=False) for _ in range(n)], np.int32)
+    lib.set_precision(prec)
+    try:
+        for broken in (False, True):
+            v = _conserving(n, rng)
+            if broken:
+                v[n // 2] = T.haar_matchgates(1, rng)[0]
+            if kind == "gate":
+                out = _both(lib, lambda: lib.circuit_target_gradient_hessian(lib.mg_target_apply, t, v, w, L), 0)
+            else:
+                out = _both(lib, lambda: lib.brickwall_target_gradient_hessian(lib.mg_target_apply, t, v, T.brickwall_perms(L, n), L, ti=kind == "ti"), 0)
+            _check([o[:3] for o in out], TOL[prec])
+            assert np.max(np.abs(out[0][3] - out[1][3])) <= TOL[prec] * max(np.max(np.abs(out[1][3])), np.max(np.abs(out[1][2])))
+    finally:
+        lib.set_precision(mgcu.PREC_FP64)
+        lib.target_free(t)
