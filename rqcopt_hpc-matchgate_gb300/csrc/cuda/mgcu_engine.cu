@@ -1864,7 +1864,7 @@ struct WsProg
 
 struct FitProg
 {
-	bool factored = true;
+	bool factored = true, always_c = false;   // always_c: the complex-q kernels whatever the gates (captured graphs)
 	bool built = false;            // the structure exists (groups, passes, flushes)
 	bool tried = false;            // a target's program: built or found not to apply
 	bool ok = false;               // the current gates factor (else the general kernels run)
@@ -2686,6 +2686,7 @@ static int launch_columns(mgcu_plan* p, long b0, long b1, const typename P::T* d
 		w.cache = p->d.want_hess ? p->cache.as<T>() : f.cache.as<T>();
 		w.dcache = p->d.want_hess ? p->dcache.as<T>() : nullptr;
 		w.part = wg ? p->part_g.as<double>() : p->part_f.as<double>();
+		w.part_f = p->part_f.as<double>();
 		w.nblocks = p->d.nblocks;
 		const int gf = (int)std::min<long>(f.grid, (ncols + f.nc - 1) / f.nc);
 		p->rows_a = std::max(p->rows_a, gf);
@@ -3067,13 +3068,13 @@ extern "C" mgcu_plan* mgcu_plan_create(const mgcu_plan_desc* d)
 	// the factored fitted circuit: gradients from L = 10 (whole evaluation, 5 layers: float-float
 	// 244 against 448 us, complex128 574 against 997 us; at L = 8 138 against 129 us and 263
 	// against 202 us, the tables and the few blocks cost more), f alone from L = 12 (L = 11: 318
-	// against 336 us), while the tables are small.  FP32 gradients keep the general kernels: there
-	// the factors' rounding is as large as the sweep's.  An explicit block size keeps them too
+	// against 336 us), while the tables are small.  In FP32, where the factors' rounding is as large as
+	// the sweep's, the blocks stay whole.  An explicit block size keeps them too
 	e = 0;
 	// (Hessians: one tile, L <= 14)
 	const bool fit_grad = d->want_grad || d->want_hess;
-	// FP32: f alone, with whole blocks
-	if (!p->adj && d->ngates > 0 && opt_thr <= 0 && (p->prec != MG_PREC_FP32_ID || !fit_grad)
+	// FP32: whole blocks, no Hessians
+	if (!p->adj && d->ngates > 0 && opt_thr <= 0 && (p->prec != MG_PREC_FP32_ID || !d->want_hess)
 		&& (d->want_hess ? (d->L >= FIT_HESS_MIN_L && d->L <= 14 && opt_kt <= 0) : (d->L >= (d->want_grad ? 10 : 12) && d->L <= 18)))
 	{
 		p->fit.kt = p->kt;
@@ -3121,7 +3122,7 @@ extern "C" mgcu_plan* mgcu_plan_create(const mgcu_plan_desc* d)
 			if (!e && cudaMemcpy(p->fit.d_pgroup.p, pg.data(), sizeof(int) * pg.size(), cudaMemcpyHostToDevice) != cudaSuccess) e = MG_ERR_DEVICE;
 			if (e) { delete p; return nullptr; }
 		}
-		const size_t slot = (size_t)p->fit.group.size() * p->fit.nc * col_bytes;
+		const size_t slot = (size_t)p->fit.group.size() * (p->fit.factored ? 1 : 2) * p->fit.nc * col_bytes;
 		long gf = std::min((long)c->nsm * std::max(per, 1), (ncols_total + p->fit.nc - 1) / p->fit.nc);
 		if (fit_grad && !d->want_hess) gf = std::max(1L, std::min(gf, (long)((32ull << 30) / slot)));
 		p->fit.grid = (int)gf;
@@ -3195,7 +3196,7 @@ extern "C" int mgcu_plan_begin(mgcu_plan* p)
 	cudaStream_t st = mgcu_stream();
 	p->rows_a = p->rows_h = 0;
 	const bool grad = p->d.want_grad || p->d.want_hess;
-	if (!(p->fit.ok && grad)) MGCU_TRY(cudaMemsetAsync(p->part_f.p, 0, p->part_f.n, st));   // there f is the trace of the gradient sums
+	if (!(p->fit.ok && grad && p->fit.factored)) MGCU_TRY(cudaMemsetAsync(p->part_f.p, 0, p->part_f.n, st));   // there f is the trace of the gradient sums
 	if (grad) MGCU_TRY(cudaMemsetAsync(p->part_g.p, 0, p->part_g.n, st));
 	if (p->d.want_hess) MGCU_TRY(cudaMemsetAsync(p->part_h.p, 0, p->part_h.n, st));
 	return 0;
@@ -3271,6 +3272,11 @@ extern "C" int mgcu_plan_finish(mgcu_plan* p)
 		k_fit_finish<<<p->d.nblocks, FIT_FIN * 16, 0, st>>>(p->part_g.as<double>(), p->rows_a, p->d.nblocks, p->fit.d_blk.as<FitBlock>(),
 			p->out_f.as<double>(), p->out_blk.as<double>());
 		MGCU_LAUNCHED();
+		if (!p->fit.factored)
+		{
+			sum_parts(p->part_f.as<double>(), p->rows_a, 2, p->out_f.as<double>(), st);
+			MGCU_LAUNCHED();
+		}
 		if (!p->d.want_hess) return 0;
 		const long mdim = 8L * p->d.nblocks;
 		double2* A = p->fit.cache.as<double2>();
@@ -3457,12 +3463,12 @@ struct BatchRed
 // parameter block blockIdx.y of instance blockIdx.x (and, with y = 0, f): sixteen sums by
 // sixteen threads each over every sixteenth slot, in a fixed order (one thread per sum over all
 // slots and gates took 2.2 ms for twelve instances)
-__global__ void __launch_bounds__(256) k_batch_reduce(const BatchRed* __restrict__ rd)
+__global__ void __launch_bounds__(256) k_batch_reduce(const BatchRed* __restrict__ rd, const int* __restrict__ skip)
 {
 	__shared__ double sum[16][16];
 	const BatchRed r = rd[blockIdx.x];
 	const int blk = blockIdx.y, e = threadIdx.x & 15, w = threadIdx.x >> 4;
-	if (blk >= r.nblocks) return;
+	if (blk >= r.nblocks || skip[blockIdx.x]) return;   // (instances of k_fit finish by themselves)
 	if (blk == 0)
 	{
 		double s = 0;
@@ -3499,13 +3505,14 @@ struct BatchInst
 	int L, nb, ngates, nblocks, kt_c, kt_t, nslots = 0, npass_t = 0;
 	long S;
 	Sched ws;
-	std::vector<int> block;
+	std::vector<int> block, wires;
 	DevBuf d_pass, d_gate, d_mats, d_block, out_f, out_blk;
 	TargetProg tp;                 // the batch's own copy of the target program
 	mgcu_target* target;
 	size_t smem_t, pm_off, smem_c;
 	double col_cost;               // relative cost of one column
 	bool big = false;              // enough columns to fill the GPU: its own kernels
+	FitProg fit;                   // its fitted circuit for k_fit (big instances)
 	int grid_t = 0, grid_c = 0;    // standalone grids (big instances)
 	long chunk = 0;                // columns per staged chunk (big instances)
 	long part_off;                 // offsets (doubles) of part_f / part_g in the batch's partials
@@ -3519,17 +3526,18 @@ struct mgcu_batch
 	int prec, n, threads = 256;
 	size_t tsize;
 	std::unique_ptr<BatchInst[]> inst;
-	DevBuf args_t, args_c, items, counters, scratch, parts, red;
+	DevBuf args_t, args_c, items, counters, scratch, parts, red, skip;
 	long slot_stride = 0, cache_stride = 0;
 	size_t smem = 0;
 	int grid[3] = { 0, 0, 0 }, nitems = 0;
-	DevBuf stage, bsu, bsw, bcache;   // big instances: staged target columns, k_columns slots and caches
+	DevBuf stage, bsu, bsw, bcache, fparts;   // big instances: staged target columns, k_columns slots and caches
 	std::vector<char> host_args;      // the instances' target and columns Args (kernel parameters of big ones)
 	int class_beg[4] = { 0, 0, 0, 0 };   // items of tile classes 4, 8, any quartets per thread
 	long graph_kernels = 0;        // kernel nodes per replay
 	bool use_graph = true;         // false: plain launches (a batch run once)
 	cudaGraph_t graph = nullptr;
 	cudaGraphExec_t exec = nullptr;
+	std::vector<char> captured;    // per instance: k_fit ran its fitted circuit when the graph was captured
 	DevBuf flush;
 	~mgcu_batch()
 	{
@@ -3663,8 +3671,8 @@ static int batch_build(mgcu_batch* B, const mgcu_batch_inst* d, int tune)
 	// Instances with at least four columns per resident block run the two standalone
 	// kernels (k_target into a staged chunk, then k_columns), which are faster per column
 	// than the fused kernel; the others share the fused persistent launch.
-	size_t stage_bytes = 0, slot_max = 0, cache_max = 0;
-	int grid_c_max = 0;
+	size_t stage_bytes = 0, slot_max = 0, cache_max = 0, fit_cache = 0;
+	int grid_c_max = 0, fit_rows = 0, fit_blocks = 1;
 	for (int i = 0; i < B->n; i++)
 	{
 		BatchInst& I = B->inst[i];
@@ -3677,7 +3685,23 @@ static int batch_build(mgcu_batch* B, const mgcu_batch_inst* d, int tune)
 		I.big = (1L << I.L) >= 4L * std::max(I.grid_t, I.grid_c);
 		if (!I.big) continue;
 		{
-			const int ef = target_fit<P>(I.target, I.tp, I.tp.fit);   // as for plans
+			int ef = target_fit<P>(I.target, I.tp, I.tp.fit);   // as for plans
+			if (!ef && I.L >= 10 && I.L <= 18)
+			{
+				const int kt = P::kId == MG_PREC_FP32_ID ? std::min(I.nb, 13) : I.nb <= 13 ? I.nb : 12;
+				I.fit.always_c = true;
+				ef = fit_build(I.L, kt, d[i].wires, d[i].ngates, d[i].block, d[i].nblocks, (int)sizeof(T), P::kId == MG_PREC_FP32_ID,
+					P::kId != MG_PREC_FP32_ID, I.fit);
+				int per = 0;
+				auto kern = fit_kernel<P>(P::kId == MG_PREC_FP32_ID ? 2 : 1, d[i].want_grad ? FIT_GRAD : FIT_VALUE, I.fit.threads);
+				if (!ef) MGCU_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, I.fit.threads, I.fit.smem));
+				I.fit.grid = (int)std::min<long>((long)c->nsm * std::max(per, 1), ((1L << I.L) + I.fit.nc - 1) / I.fit.nc);
+				const size_t slot = I.fit.group.size() * (I.fit.factored ? 1 : 2) * I.fit.nc * (size_t)I.S;
+				if (d[i].want_grad) fit_cache = std::max(fit_cache, slot * I.fit.grid);
+				fit_rows = std::max(fit_rows, I.fit.grid);
+				fit_blocks = std::max(fit_blocks, I.nblocks);
+				I.wires.assign(d[i].wires, d[i].wires + 2 * d[i].ngates);
+			}
 			if (ef) return ef;
 		}
 		I.chunk = std::max(1L, std::min(1L << I.L, (long)((8ull << 30) / ((size_t)I.S * sizeof(T)))));
@@ -3688,10 +3712,13 @@ static int batch_build(mgcu_batch* B, const mgcu_batch_inst* d, int tune)
 	}
 	if (stage_bytes)
 	{
+		const int rows = std::max(grid_c_max, fit_rows);
 		int e = B->stage.alloc(stage_bytes);
-		if (!e) e = B->bsu.alloc(sizeof(T) * slot_max * grid_c_max);
-		if (!e) e = B->bsw.alloc(sizeof(T) * slot_max * grid_c_max);
-		if (!e && cache_max) e = B->bcache.alloc(sizeof(T) * cache_max * grid_c_max);
+		if (!e) e = B->bsu.alloc(sizeof(T) * slot_max * rows);
+		if (!e) e = B->bsw.alloc(sizeof(T) * slot_max * rows);
+		// (either path of an instance: its gates decide at run time)
+		if (!e && cache_max) e = B->bcache.alloc(sizeof(T) * std::max(cache_max * grid_c_max, fit_cache));
+		if (!e && fit_rows) e = B->fparts.alloc(sizeof(double) * (size_t)fit_rows * (16 * (size_t)fit_blocks + 2));
 		if (e) return e;
 	}
 
@@ -3783,6 +3810,8 @@ static int batch_build(mgcu_batch* B, const mgcu_batch_inst* d, int tune)
 	memcpy(B->host_args.data(), at.data(), sizeof(Args<P>) * B->n);
 	memcpy(B->host_args.data() + sizeof(Args<P>) * B->n, ac.data(), sizeof(Args<P>) * B->n);
 	MGCU_TRY(cudaMemcpy(B->red.p, rd.data(), sizeof(BatchRed) * B->n, cudaMemcpyHostToDevice));
+	if (B->skip.alloc(sizeof(int) * B->n)) return MG_ERR_ALLOC;
+	MGCU_TRY(cudaMemset(B->skip.p, 0, sizeof(int) * B->n));
 	return 0;
 }
 
@@ -3802,6 +3831,8 @@ static int batch_issue(mgcu_batch* B)
 		if (!I.big) continue;
 		void (*kt_)(Args<P>) = target_kernel<P>(I.kt_t, B->threads);
 		const long N = 1L << I.L;
+		double* fpart = B->fparts.as<double>();   // k_fit's rows of this instance: f, then gradients
+		if (I.fit.ok) MGCU_TRY(cudaMemsetAsync(fpart, 0, sizeof(double) * (size_t)I.fit.grid * (16 * (size_t)I.nblocks + 2), st));
 		for (long c0 = 0; c0 < N; c0 += I.chunk)
 		{
 			const long c1 = std::min(N, c0 + I.chunk);
@@ -3818,10 +3849,35 @@ static int batch_issue(mgcu_batch* B)
 				MGCU_LAUNCHED();
 			}
 			Args<P> w = hac[i];
+			if (I.fit.ok)
+			{
+				FitArgs<P> f = fit_args<P>(I.fit, I.L);
+				f.dense = B->stage.as<T>(); f.dense_b0 = c0; f.b0 = c0; f.b1 = c1;
+				f.su = B->bsu.as<T>(); f.sw = B->bsw.as<T>(); f.cache = B->bcache.as<T>();
+				f.part_f = fpart; f.part = w.want_grad ? fpart + 2 * (size_t)I.fit.grid : fpart;
+				f.nblocks = I.nblocks;
+				fit_kernel<P>(I.fit.qc, w.want_grad ? FIT_GRAD : FIT_VALUE, I.fit.threads)
+					<<<(int)std::min<long>(I.fit.grid, (c1 - c0 + I.fit.nc - 1) / I.fit.nc), I.fit.threads, I.fit.smem, st>>>(f);
+				MGCU_LAUNCHED();
+				continue;
+			}
 			w.b0 = c0; w.b1 = c1; w.dense = B->stage.as<T>(); w.dense_b0 = c0;
 			w.su = B->bsu.as<T>(); w.sw = B->bsw.as<T>();
 			w.cache = w.want_grad ? B->bcache.as<T>() : nullptr;
 			k_columns<P, false><<<(int)std::min<long>(I.grid_c, c1 - c0), B->threads, I.smem_c, st>>>(w);
+			MGCU_LAUNCHED();
+		}
+		if (!I.fit.ok) continue;
+		const bool grad = hac[i].want_grad != 0;
+		if (grad)
+		{
+			k_fit_finish<<<I.nblocks, FIT_FIN * 16, 0, st>>>(fpart + 2 * (size_t)I.fit.grid, I.fit.grid, I.nblocks, I.fit.d_blk.as<FitBlock>(),
+				I.out_f.as<double>(), I.out_blk.as<double>());
+			MGCU_LAUNCHED();
+		}
+		if (!grad || !I.fit.factored)
+		{
+			sum_parts(fpart, I.fit.grid, 2, I.out_f.as<double>(), st);
 			MGCU_LAUNCHED();
 		}
 	}
@@ -3836,7 +3892,7 @@ static int batch_issue(mgcu_batch* B)
 	}
 	int nb = 1;
 	for (int i = 0; i < B->n; i++) nb = std::max(nb, B->inst[i].nblocks);
-	k_batch_reduce<<<dim3(B->n, nb), 256, 0, st>>>(B->red.as<BatchRed>());
+	k_batch_reduce<<<dim3(B->n, nb), 256, 0, st>>>(B->red.as<BatchRed>(), B->skip.as<int>());
 	MGCU_LAUNCHED();
 	return 0;
 }
@@ -3846,6 +3902,16 @@ static int batch_issue_graph(mgcu_batch* B)
 {
 	cudaStream_t st = mgcu_stream();
 	if (!B->use_graph) return batch_issue<P>(B);
+	// gates that stopped (or started) factoring change the launches
+	std::vector<char> now;
+	for (int i = 0; i < B->n; i++) now.push_back(B->inst[i].fit.ok);
+	if (B->exec && now != B->captured)
+	{
+		cudaGraphExecDestroy(B->exec);
+		cudaGraphDestroy(B->graph);
+		B->exec = nullptr; B->graph = nullptr;
+	}
+	B->captured = now;
 	if (!B->exec)
 	{
 		MGCU_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -3893,9 +3959,18 @@ extern "C" int mgcu_batch_set_gates(mgcu_batch* B, int i, const mgg* gates)
 {
 	if (i < 0 || i >= B->n) { mg_set_error("batch instance %d out of range", i); return MG_ERR_ARG; }
 	BatchInst& I = B->inst[i];
-	if (B->prec == MG_PREC_FP64_ID) return upload_mats<PrecD>(gates, I.ngates, I.d_mats);
-	if (B->prec == MG_PREC_FP32_ID) return upload_mats<PrecF>(gates, I.ngates, I.d_mats);
-	return upload_mats<PrecX>(gates, I.ngates, I.d_mats);
+	int e;
+	if (B->prec == MG_PREC_FP64_ID) e = upload_mats<PrecD>(gates, I.ngates, I.d_mats);
+	else if (B->prec == MG_PREC_FP32_ID) e = upload_mats<PrecF>(gates, I.ngates, I.d_mats);
+	else e = upload_mats<PrecX>(gates, I.ngates, I.d_mats);
+	if (e || !I.fit.built) return e;
+	const int was = I.fit.ok;
+	if (B->prec == MG_PREC_FP64_ID) e = fit_set_gates<PrecD>(gates, I.ngates, I.block.data(), I.nblocks, I.L, I.fit.kt, I.wires.data(), I.fit);
+	else if (B->prec == MG_PREC_FP32_ID) e = fit_set_gates<PrecF>(gates, I.ngates, I.block.data(), I.nblocks, I.L, I.fit.kt, I.wires.data(), I.fit);
+	else e = fit_set_gates<PrecX>(gates, I.ngates, I.block.data(), I.nblocks, I.L, I.fit.kt, I.wires.data(), I.fit);
+	const int now = I.fit.ok;
+	if (!e && now != was) MGCU_TRY(cudaMemcpyAsync(B->skip.as<int>() + i, &now, sizeof(int), cudaMemcpyHostToDevice, mgcu_stream()));
+	return e;
 }
 
 // one evaluation of every instance (graph replay; the first call captures the graph)

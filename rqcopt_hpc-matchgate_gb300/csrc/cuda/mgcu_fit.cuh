@@ -97,6 +97,7 @@ struct FitArgs
 	T* cache;                   // [slot][group][column of the block][S]; slot: the block, or (FIT_HESS) its columns from b0
 	T* dcache;                  // the derivatives, alike (FIT_HESS)
 	double* part;               // [block][nblocks][16] (gradient) or [block][2]
+	double* part_f;             // [block][2]: f beside a gradient of whole blocks
 	int nblocks;
 };
 
@@ -269,6 +270,57 @@ __device__ __forceinline__ void fit_group(const FitGroup& G, const FitGate<typen
 	}
 }
 
+// The gradient sweeps with whole blocks (FP32), gate by gate in k_columns' arithmetic: forward
+// keeps each gate's input (cache: two slots per group, `slot` apart), backward sums the
+// derivative against it and applies the transpose, one quartet per iteration, the inputs read
+// one quartet ahead.
+template <class P>
+__device__ __forceinline__ void fit_whole_forward(const FitGroup& G, int w, const FitWhole<typename P::T>& g, unsigned tc, unsigned base,
+	typename P::T* __restrict__ out)
+{
+	typedef typename P::T T;
+	char* ob = reinterpret_cast<char*>(out);
+	const T c0 = g.c[0], c1 = g.c[1], c2 = g.c[2], c3 = g.c[3], k0 = g.k[0], k1 = g.k[1], k2 = g.k[2], k3 = g.k[3];
+#pragma unroll 2
+	for (int i = 0; i < 4; i++)
+	{
+		const uint4 o = G.qs[w][i], q = G.qy[w][i];
+		const unsigned ax = tc + (base ^ o.x), ay = tc + (base ^ o.y), az = tc + (base ^ o.z), aw = tc + (base ^ o.w);
+		const T x = lds<T>(ax), y = lds<T>(ay), z = lds<T>(az), v = lds<T>(aw);
+		*reinterpret_cast<T*>(ob + q.x) = x; *reinterpret_cast<T*>(ob + q.y) = y;
+		*reinterpret_cast<T*>(ob + q.z) = z; *reinterpret_cast<T*>(ob + q.w) = v;
+		sts<T>(ax, P::madd2(k0, x, k1, v)); sts<T>(aw, P::madd2(k2, x, k3, v));
+		sts<T>(ay, P::madd2(c0, y, c1, z)); sts<T>(az, P::madd2(c2, y, c3, z));
+	}
+}
+
+template <class P>
+__device__ __forceinline__ void fit_whole_backward(const FitGroup& G, int w, const FitWhole<typename P::T>& g, unsigned tc, unsigned base,
+	const typename P::T* __restrict__ ct, typename P::Acc (&acc)[8])
+{
+	typedef typename P::T T;
+	const char* cb = reinterpret_cast<const char*>(ct);
+	const T c0 = g.c[0], c1 = g.c[1], c2 = g.c[2], c3 = g.c[3], k0 = g.k[0], k1 = g.k[1], k2 = g.k[2], k3 = g.k[3];
+	uint4 q = G.qy[w][0];
+	T nx = *reinterpret_cast<const T*>(cb + q.x), ny = *reinterpret_cast<const T*>(cb + q.y);
+	T nz = *reinterpret_cast<const T*>(cb + q.z), nv = *reinterpret_cast<const T*>(cb + q.w);
+#pragma unroll 2
+	for (int i = 0; i < 4; i++)
+	{
+		const uint4 o = G.qs[w][i];
+		const unsigned ax = tc + (base ^ o.x), ay = tc + (base ^ o.y), az = tc + (base ^ o.z), aw = tc + (base ^ o.w);
+		const T x = nx, y = ny, z = nz, v = nv;
+		q = G.qy[w][min(i + 1, 3)];
+		nx = *reinterpret_cast<const T*>(cb + q.x); ny = *reinterpret_cast<const T*>(cb + q.y);
+		nz = *reinterpret_cast<const T*>(cb + q.z); nv = *reinterpret_cast<const T*>(cb + q.w);
+		const T dx = lds<T>(ax), dy = lds<T>(ay), dz = lds<T>(az), dv = lds<T>(aw);
+		contract_quartet<P>(acc, dx, dv, dy, dz, x, v, y, z);
+		// transpose (no conjugation): reference src/gate.c:725-728
+		sts<T>(ax, P::madd2(k0, dx, k2, dv)); sts<T>(aw, P::madd2(k1, dx, k3, dv));
+		sts<T>(ay, P::madd2(c0, dy, c2, dz)); sts<T>(az, P::madd2(c1, dy, c3, dz));
+	}
+}
+
 // R sums of the gates first..last (1: b, 0: a) of a group over the quartets of a unit: the
 // derivative in the tile and the cached state ct, read one quartet ahead.  One loop for every
 // kind of gate, not unrolled: with each gate's quartets unrolled the kernel's code outgrew the
@@ -336,7 +388,7 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 	const long S = a.S;
 	const unsigned mycol = min(threadIdx.x >> nu, (unsigned)nc - 1), u0 = nc > 1 ? (threadIdx.x & (U - 1)) : threadIdx.x;
 	const unsigned colb = mycol * n * ES;
-	const size_t cstride = (size_t)nc * S;
+	const size_t cstride = (size_t)nc * S * (QC == 2 ? 2 : 1);
 	typename P::Acc acc[8];
 #pragma unroll
 	for (int e = 0; e < 8; e++) acc[e] = P::acc_zero();
@@ -384,7 +436,14 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 						const unsigned u = u0 + i * FIT_NT, base = fit_base(G, a.bases + (size_t)g * U, u, tpar);
 						const T* tab = G.flush >= 0 ? a.tables + ((size_t)(2 * G.flush + par) * S + ((size_t)tau << kt) + u) : nullptr;
 						T* out = GRAD ? cache + (size_t)g * cstride + ((size_t)tau << kt) + u : nullptr;
-						if constexpr (GRAD) fit_group<P, QC, false>(G, stage[g & 1].gate, tb + colb, base, tab, out);
+						if constexpr (GRAD && QC == 2)
+						{
+							const int ngt = (G.ga >= 0 && G.kind_b) ? 2 : 1, w0 = ngt == 2 ? G.order : (G.ga >= 0 ? 0 : 1);
+#pragma unroll 1
+							for (int st = 0; st < ngt; st++)
+								fit_whole_forward<P>(G, w0 ^ st, stage[g & 1].gate[w0 ^ st], tb + colb, base, out + (size_t)(w0 ^ st) * nc * S);
+						}
+						else if constexpr (GRAD) fit_group<P, QC, false>(G, stage[g & 1].gate, tb + colb, base, tab, out);
 						else fit_group16<P, QC>(G, stage[g & 1].gate, tb + colb, base, U, tab);
 					}
 					fit_stage_wait();
@@ -402,7 +461,7 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 						a.ucols[(size_t)(be - a.b0) * S + c] = P::negconj(v);
 					}
 				}
-				if (MODE == FIT_VALUE && last)
+				if ((MODE == FIT_VALUE || (GRAD && QC == 2)) && last)
 				{
 					for (unsigned e = threadIdx.x; e < n * nc; e += FIT_NT)
 					{
@@ -441,14 +500,65 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 					if (last)
 					{
 						const long be = cb + (long)(e >> kt);
-						v = be < a.b1 ? P::mul(a.final[(size_t)(__popcll(be) & 1) * S + c], a.dense[(size_t)(be - a.dense_b0) * S + c])
-							: P::zero();
+						v = be < a.b1 ? a.dense[(size_t)(be - a.dense_b0) * S + c] : P::zero();
+						if (QC != 2 && be < a.b1) v = P::mul(a.final[(size_t)(__popcll(be) & 1) * S + c], v);
 					}
 					else v = a.su[(size_t)blockIdx.x * S + c];
 					sts<T>(tb + ((e & ~(n - 1)) + fsw<ES>(e & (n - 1))) * ES, v);
 				}
 				fit_stage_wait();
 				__syncthreads();
+				if constexpr (QC == 2)
+				{
+					int cblk = -1, merged = 0;   // the parameter block of the sums in acc
+					auto flush = [&]() {
+						if (cblk < 0) return;
+						block_reduce8<P>(acc, s.red, a.part + ((size_t)blockIdx.x * a.nblocks + cblk) * 16, 1.0, nred);
+#pragma unroll
+						for (int e = 0; e < 8; e++) acc[e] = P::acc_zero();
+						cblk = -1;
+						merged = 0;
+					};
+					for (int g = fp.gend - 1; g >= fp.gbeg; g--)
+					{
+						const FitGroup& G = stage[g & 1].g;
+						if (g > fp.gbeg) fit_stage<Gate>(stage[(g - 1) & 1], a.groups + g - 1, static_cast<const Gate*>(a.gates) + 2 * (g - 1));
+						const T* cg = cache + (size_t)g * cstride + ((size_t)tau << kt) + u0;
+						if (g > fp.gbeg)
+						{
+							// the next group's cached inputs to L2, a 128-byte line per thread and slot
+							const T* nx = cg - cstride - (threadIdx.x & 15) + (size_t)(threadIdx.x & 15) * U;
+							for (unsigned i = 0; i < its; i++)
+							{
+								asm volatile("prefetch.global.L2 [%0];" :: "l"(nx + i * FIT_NT));
+								asm volatile("prefetch.global.L2 [%0];" :: "l"(nx + (size_t)nc * S + i * FIT_NT));
+							}
+						}
+						const int ngt = (G.ga >= 0 && G.kind_b) ? 2 : 1, w0 = ngt == 2 ? G.order : (G.ga >= 0 ? 0 : 1);
+#pragma unroll 1
+						for (int st = ngt - 1; st >= 0; st--)
+						{
+							const int w = w0 ^ st, blk = w ? G.blk_b : G.blk_a;
+							if (cblk != blk) flush();
+							cblk = blk;
+							merged += 4 * (int)max(its, 1u);
+							for (unsigned i = 0; i < its; i++)
+								fit_whole_backward<P>(G, w, stage[g & 1].gate[w], tb + colb, fit_base(G, a.bases + (size_t)g * U, u0 + i * FIT_NT, tpar),
+									cg + (size_t)w * nc * S + i * FIT_NT, acc);
+							if (merged >= FIT_RENORM)
+							{
+#pragma unroll
+								for (int e = 0; e < 8; e++) P::acc_norm(acc[e]);
+								merged = 0;
+							}
+						}
+						fit_stage_wait();
+						__syncthreads();
+					}
+					flush();
+				}
+				else
+				{
 				int merged = 0;
 				for (int g = fp.gend - 1; g >= fp.gbeg; g--)
 				{
@@ -511,6 +621,7 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 						__syncthreads();
 					}
 				}
+				}
 				if (p > 0)
 					for (unsigned e = threadIdx.x; e < n; e += FIT_NT) a.su[(size_t)blockIdx.x * S + gidx(s, nlb, e)] = lds<T>(tb + fsw<ES>(e) * ES);
 				__syncthreads();
@@ -519,6 +630,7 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 		}
 	}
 	if (MODE == FIT_VALUE) block_reduce1<P>(facc, s.red, a.part + (size_t)blockIdx.x * 2);
+	if (GRAD && QC == 2) block_reduce1<P>(facc, s.red, a.part_f + (size_t)blockIdx.x * 2);
 }
 
 // ------------------------------------------------------------------------------------
@@ -793,7 +905,7 @@ __global__ void __launch_bounds__(FIT_FIN * 16) k_fit_finish(const double* __res
 		out_blk[blk * 16 + 2 * q] = gr * c[0] - gi * c[1];
 		out_blk[blk * 16 + 2 * q + 1] = gr * c[1] + gi * c[0];
 	}
-	if (blk == 0 && threadIdx.x >= 8 && threadIdx.x < 10)
+	if (blk == 0 && threadIdx.x >= 8 && threadIdx.x < 10 && fb[0].ngates > 0)   // (whole blocks: f has its own sums)
 	{
 		const int c = threadIdx.x - 8;
 		out_f[c] = ((R[0 + c] + R[6 + c]) + (R[8 + c] + R[14 + c])) / fb[0].ngates;

@@ -427,6 +427,11 @@ static int fit_set_gates(const mgg* gates, int ng, const int* block, int nblocks
 			}
 		}
 		MGCU_TRY(cudaMemcpyAsync(f.d_gates.p, hw.data(), sizeof(FitWhole<T>) * hw.size(), cudaMemcpyHostToDevice, mgcu_stream()));
+		std::vector<FitBlock> fb(nblocks);
+		memset(fb.data(), 0, sizeof(FitBlock) * nblocks);   // the sums are the gradients
+		for (FitBlock& b : fb)
+			for (int h = 0; h < 8; h++) { b.scale[h][0] = 1; b.minv[h][0] = (h & 3) == 0 || (h & 3) == 3; }
+		MGCU_TRY(cudaMemcpyAsync(f.d_blk.p, fb.data(), sizeof(FitBlock) * nblocks, cudaMemcpyHostToDevice, mgcu_stream()));
 		f.qc = 2;
 		f.ok = true;
 		return 0;
@@ -466,7 +471,7 @@ static int fit_set_gates(const mgg* gates, int ng, const int* block, int nblocks
 		}
 	}
 	// beyond the rounding of a unitary block q keeps its imaginary part (complex128: always)
-	f.qc = qi > (P::kId == MG_PREC_FP64_ID ? 0.0 : 1e-15);
+	f.qc = f.always_c || qi > (P::kId == MG_PREC_FP64_ID ? 0.0 : 1e-15);
 	std::vector<FitGate<T>> hg(2 * f.group.size());
 	memset(hg.data(), 0, sizeof(FitGate<T>) * hg.size());
 	for (size_t i = 0; i < hg.size(); i++)
@@ -506,7 +511,8 @@ static int fit_set_gates(const mgg* gates, int ng, const int* block, int nblocks
 template <class P, int NT>
 static void (*fit_kernel_nt(int qc, int mode))(FitArgs<P>)
 {
-	if constexpr (P::kId == MG_PREC_FP32_ID) return mode == FIT_COLS ? k_fit<P, 2, FIT_COLS, NT> : k_fit<P, 2, FIT_VALUE, NT>;
+	if constexpr (P::kId == MG_PREC_FP32_ID)
+		return mode == FIT_COLS ? k_fit<P, 2, FIT_COLS, NT> : mode == FIT_GRAD ? k_fit<P, 2, FIT_GRAD, NT> : k_fit<P, 2, FIT_VALUE, NT>;
 	else if (qc)
 		return mode == FIT_COLS ? k_fit<P, 1, FIT_COLS, NT> : mode == FIT_GRAD ? k_fit<P, 1, FIT_GRAD, NT>
 			: mode == FIT_HESS ? k_fit<P, 1, FIT_HESS, NT> : k_fit<P, 1, FIT_VALUE, NT>;

@@ -204,3 +204,30 @@ def test_conserving_hessian(mglib, L, n, kind, prec):
     finally:
         lib.set_precision(mgcu.PREC_FP64)
         lib.target_free(t)
+
+
+@pytest.mark.parametrize("prec", [mgcu.PREC_FP64, mgcu.PREC_MIXED, mgcu.PREC_FP32])
+def test_batch_gates_change_kernels(mglib, prec):
+    """a captured batch whose gates stop factoring and factor again: each run equals the same fits
+    run as plans"""
+    lib, rng = mglib, np.random.default_rng(5)
+    Ls, nls = [10, 12, 12], [3, 2, 4]
+    ts = [lib.target_brickwall(T.haar_matchgates(4, rng), T.brickwall_perms(L, 4), L) for L in Ls]
+    perms = [T.brickwall_perms(L, nl) for L, nl in zip(Ls, nls)]
+    good = [T.haar_matchgates(nl, rng) for nl in nls]
+    bad = [_layers("singular", nl, rng) for nl in nls]
+    lib.set_precision(prec)
+    try:
+        b = lib.batch_create(ts, good, perms, Ls)
+        for vs in (good, bad, good):
+            for i, v in enumerate(vs):
+                assert lib.batch_set_gates(b, i, v) == 0
+            assert lib.batch_run(b) == 0
+            for i, (t, v, L) in enumerate(zip(ts, vs, Ls)):
+                f, dv, _ = lib.batch_results(b, i)
+                _check([(0, f, dv), lib.brickwall_target_and_gradient(lib.mg_target_apply, t, v, perms[i], L)], TOL[prec])
+        lib.batch_free(b)
+    finally:
+        lib.set_precision(mgcu.PREC_FP64)
+        for t in ts:
+            lib.target_free(t)
