@@ -1783,15 +1783,44 @@ void sum_parts(const double* part, int nparts, long len, double* out, cudaStream
 	k_sum_parts<<<(unsigned)((len + SUM_OUT - 1) / SUM_OUT), SUM_OUT * SUM_SPLIT, 0, st>>>(part, nparts, len, out);
 }
 
-// per-gate gradients [ngates][16] -> per-block sums [nblocks][16], gates in order
-__global__ void k_block_sum(const double* __restrict__ g, const int* __restrict__ block, int ngates, int nblocks, double* __restrict__ out)
+// f and per-block gradients of the general kernels from their partial rows in one launch: block
+// blockIdx.x sums its gates' rows, sixteen threads per entry over every sixteenth row, the gates
+// in order; block 0 also sums f (a launch each for f, gates and blocks took 10 us of the smallest
+// evaluations)
+__global__ void __launch_bounds__(256) k_gradient_sum(const double* __restrict__ part_f, const double* __restrict__ part_g, int rows,
+	const int* __restrict__ block, int ngates, double* __restrict__ out_f, double* __restrict__ out_blk)
 {
-	const int t = blockIdx.x * blockDim.x + threadIdx.x;
-	if (t >= nblocks * 16) return;
-	const int blk = t / 16, v = t % 16;
+	__shared__ double sum[16][16];
+	const int blk = blockIdx.x, e = threadIdx.x & 15, w = threadIdx.x >> 4;
+	if (blk == 0)
+	{
+		double s = 0;
+		if (e < 2)
+#pragma unroll 4
+			for (int k = w; k < rows; k += 16) s += part_f[2 * k + e];
+		sum[w][e] = s;
+		__syncthreads();
+		if (threadIdx.x < 2)
+		{
+			s = 0;
+			for (int k = 0; k < 16; k++) s += sum[k][threadIdx.x];
+			out_f[threadIdx.x] = s;
+		}
+		__syncthreads();
+	}
 	double s = 0;
-	for (int q = 0; q < ngates; q++) if (block[q] == blk) s += g[q * 16 + v];
-	out[t] = s;
+	for (int g = 0; g < ngates; g++)
+	{
+		if (block[g] != blk) continue;
+#pragma unroll 4
+		for (int k = w; k < rows; k += 16) s += part_g[((size_t)k * ngates + g) * 16 + e];
+	}
+	sum[w][e] = s;
+	__syncthreads();
+	if (w) return;
+	s = 0;
+	for (int k = 0; k < 16; k++) s += sum[k][e];
+	out_blk[blk * 16 + e] = s;
 }
 
 // diagonal blocks A -> A + A^T, then (second kernel) lower blocks mirrored from upper
@@ -1878,6 +1907,7 @@ struct FitProg
 	std::vector<int> group_of_gate;
 	int grid_h = 0;                         // k_fit_hess blocks
 	int nflush = 0, grid = 0, nc = 1, threads = 128, kt = 0;
+	int split = 1, ncb = 1;        // gradients: threads per unit and columns per block
 	size_t smem = 0;
 	WsProg ws;
 	DevBuf d_pass, d_group, d_pgroups, d_gates, d_diag, d_beg, d_gof, d_tab, d_blk, d_bases, d_pgroup, cache;
@@ -2456,7 +2486,7 @@ struct mgcu_plan
 	bool adj_ok = false;           // the current gates are invertible (else the cached sweep)
 	DevBuf d_mats_inv, ck;
 	DevBuf su, sw, sh, cache, dcache, part_f, part_g, part_h, cols64, cols;
-	DevBuf out_f, out_g, out_blk, out_h, flush;
+	DevBuf out_f, out_blk, out_h, flush;
 	int rows_a = 0, rows_h = 0;    // partial rows (blocks) used in this evaluation
 };
 
@@ -2688,15 +2718,17 @@ static int launch_columns(mgcu_plan* p, long b0, long b1, const typename P::T* d
 		w.part = wg ? p->part_g.as<double>() : p->part_f.as<double>();
 		w.part_f = p->part_f.as<double>();
 		w.nblocks = p->d.nblocks;
-		const int gf = (int)std::min<long>(f.grid, (ncols + f.nc - 1) / f.nc);
+		if (wg) { w.nc = f.ncb; if (!p->d.want_hess) w.ncs = f.ncb; }
+		const int gf = (int)std::min<long>(f.grid, (ncols + w.nc - 1) / w.nc);
 		p->rows_a = std::max(p->rows_a, gf);
-		fit_kernel<P>(f.qc, p->d.want_hess ? FIT_HESS : wg ? FIT_GRAD : FIT_VALUE, f.threads)<<<gf, f.threads, f.smem, mgcu_stream()>>>(w);
+		fit_kernel<P>(f.qc, p->d.want_hess ? FIT_HESS : wg ? FIT_GRAD : FIT_VALUE, f.threads, f.split)<<<gf, f.threads, f.smem, mgcu_stream()>>>(w);
 		MGCU_LAUNCHED();
 		if constexpr (P::kId != MG_PREC_FP32_ID)
 		if (p->d.want_hess)
 		{
 			FitHessArgs<P> h;
 			h.f = w;
+			h.f.nc = f.nc;
 			h.place = p->d_place.as<int>(); h.place_group = f.d_pgroup.as<int>(); h.place_w = p->d_placew.as<double>();
 			h.block = p->d_block.as<int>(); h.nplace = p->d.nplace; h.ngates = p->d.ngates; h.mdim = 8 * p->d.nblocks;
 			h.hgroup = p->hgroup ? 1 : 0; h.part_h = p->part_h.as<double>();
@@ -2762,6 +2794,8 @@ static int set_smem_attr()
 	{
 		const int lim = (int)std::min<size_t>(c->smem_optin, 227 * 1024) - 4096;
 		MGCU_TRY(cudaFuncSetAttribute(fit_kernel<P>(q & 1, (q >> 1) & 3, 128 << (q >> 3)), cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+		if constexpr (P::kId != MG_PREC_FP32_ID)
+			if ((q >> 3) == 0 && (q & 2)) MGCU_TRY(cudaFuncSetAttribute(fit_kernel<P>(q & 1, (q >> 1) & 3, 128, 4), cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
 		if constexpr (P::kId != MG_PREC_FP32_ID)
 			if (!(q & 6)) MGCU_TRY(cudaFuncSetAttribute(fit_hess_kernel<P>(q & 1, 128 << (q >> 3)), cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
 	}
@@ -3089,8 +3123,8 @@ extern "C" mgcu_plan* mgcu_plan_create(const mgcu_plan_desc* d)
 			auto occ = [&](auto k) { return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, p->fit.threads, p->fit.smem) != cudaSuccess; };
 			const bool g = fit_grad;
 			const int mode = d->want_hess ? FIT_HESS : g ? FIT_GRAD : FIT_VALUE;
-			if (p->prec == MG_PREC_FP64_ID ? occ(fit_kernel<PrecD>(1, mode, p->fit.threads)) : p->prec == MG_PREC_FP32_ID
-				? occ(fit_kernel<PrecF>(2, mode, p->fit.threads)) : occ(fit_kernel<PrecX>(1, mode, p->fit.threads))) e = MG_ERR_DEVICE;
+			if (p->prec == MG_PREC_FP64_ID ? occ(fit_kernel<PrecD>(1, mode, p->fit.threads, p->fit.split)) : p->prec == MG_PREC_FP32_ID
+				? occ(fit_kernel<PrecF>(2, mode, p->fit.threads)) : occ(fit_kernel<PrecX>(1, mode, p->fit.threads, p->fit.split))) e = MG_ERR_DEVICE;
 		}
 		if (e) { delete p; return nullptr; }
 		if (opt_cps > 0) per = (int)std::min<long>(per, opt_cps);
@@ -3123,7 +3157,7 @@ extern "C" mgcu_plan* mgcu_plan_create(const mgcu_plan_desc* d)
 			if (e) { delete p; return nullptr; }
 		}
 		const size_t slot = (size_t)p->fit.group.size() * (p->fit.factored ? 1 : 2) * p->fit.nc * col_bytes;
-		long gf = std::min((long)c->nsm * std::max(per, 1), (ncols_total + p->fit.nc - 1) / p->fit.nc);
+		long gf = std::min((long)c->nsm * std::max(per, 1), (ncols_total + (fit_grad ? p->fit.ncb : p->fit.nc) - 1) / (fit_grad ? p->fit.ncb : p->fit.nc));
 		if (fit_grad && !d->want_hess) gf = std::max(1L, std::min(gf, (long)((32ull << 30) / slot)));
 		p->fit.grid = (int)gf;
 		if (fit_grad && !d->want_hess) e = p->fit.cache.alloc(slot * gf);
@@ -3145,7 +3179,6 @@ extern "C" mgcu_plan* mgcu_plan_create(const mgcu_plan_desc* d)
 	if (!e) e = p->part_g.alloc(sizeof(double) * 16 * ng * rows);
 	if (!e && d->want_hess) e = p->part_h.alloc(sizeof(double) * 2 * (size_t)mdim * mdim * std::max(p->grid_b, p->fit.grid_h));
 	if (!e) e = p->out_f.alloc(sizeof(double) * 2);
-	if (!e) e = p->out_g.alloc(sizeof(double) * 16 * ng);
 	if (!e) e = p->out_blk.alloc(sizeof(double) * 16 * std::max(d->nblocks, 1));
 	if (!e && d->want_hess) e = p->out_h.alloc(sizeof(double) * 2 * (size_t)mdim * mdim);
 	if (!e && d->want_hess && p->fit.built) e = p->fit.cache.alloc(sizeof(double) * 2 * (size_t)mdim * mdim);   // the Hessian in moves
@@ -3290,15 +3323,11 @@ extern "C" int mgcu_plan_finish(mgcu_plan* p)
 		MGCU_LAUNCHED();
 		return 0;
 	}
-	sum_parts(p->part_f.as<double>(), p->rows_a, 2, p->out_f.as<double>(), st);
-	MGCU_LAUNCHED();
 	if (p->d.want_grad || p->d.want_hess)
-	{
-		sum_parts(p->part_g.as<double>(), p->rows_a, 16L * ng, p->out_g.as<double>(), st);
-		MGCU_LAUNCHED();
-		k_block_sum<<<(16 * p->d.nblocks + 127) / 128, 128, 0, st>>>(p->out_g.as<double>(), p->d_block.as<int>(), p->d.ngates, p->d.nblocks, p->out_blk.as<double>());
-		MGCU_LAUNCHED();
-	}
+		k_gradient_sum<<<p->d.nblocks, 256, 0, st>>>(p->part_f.as<double>(), p->part_g.as<double>(), p->rows_a, p->d_block.as<int>(), p->d.ngates,
+			p->out_f.as<double>(), p->out_blk.as<double>());
+	else sum_parts(p->part_f.as<double>(), p->rows_a, 2, p->out_f.as<double>(), st);
+	MGCU_LAUNCHED();
 	if (p->d.want_hess)
 	{
 		const long mdim = 8L * p->d.nblocks;
@@ -4065,8 +4094,7 @@ constexpr size_t NA_CACHE = NA_SW + na_al(sizeof(double2) * NA_BLOCKS * NA_S);
 constexpr size_t NA_PART_F = NA_CACHE + na_al(sizeof(double2) * NA_BLOCKS * NA_MAX_FIT_GATES * NA_S);
 constexpr size_t NA_PART_G = NA_PART_F + na_al(sizeof(double) * 2 * NA_BLOCKS);
 constexpr size_t NA_OUT_F = NA_PART_G + na_al(sizeof(double) * 16 * NA_MAX_FIT_GATES * NA_BLOCKS);
-constexpr size_t NA_OUT_G = NA_OUT_F + na_al(sizeof(double) * 2);
-constexpr size_t NA_OUT_BLK = NA_OUT_G + na_al(sizeof(double) * 16 * NA_MAX_FIT_GATES);
+constexpr size_t NA_OUT_BLK = NA_OUT_F + na_al(sizeof(double) * 2);
 constexpr size_t NA_WMAT = NA_OUT_BLK + na_al(sizeof(double) * 16 * NA_MAX_FIT_GATES);
 constexpr size_t NA_UMAT = NA_WMAT + na_al(sizeof(double2) * 8 * NA_MAX_FIT_GATES);
 constexpr size_t NA_PASS = NA_UMAT + na_al(sizeof(double2) * 8 * NA_MAX_TARGET_GATES);
@@ -4221,12 +4249,8 @@ extern "C" int mg_noalloc_brickwall_target_and_gradient(const void* ugates, int 
 		k_columns<PrecD, true><<<grid, threads, smem, st>>>(a);
 		mgcu_count_launch();
 		NA_TRY(cudaGetLastError());
-		sum_parts(a.part_f, grid, 2, reinterpret_cast<double*>(base + NA_OUT_F), st);
-		mgcu_count_launch();
-		sum_parts(a.part_g, grid, 16L * ng, reinterpret_cast<double*>(base + NA_OUT_G), st);
-		mgcu_count_launch();
-		k_block_sum<<<(16 * nlayers + 127) / 128, 128, 0, st>>>(reinterpret_cast<double*>(base + NA_OUT_G), reinterpret_cast<const int*>(base + NA_BLOCK),
-			ng, nlayers, reinterpret_cast<double*>(base + NA_OUT_BLK));
+		k_gradient_sum<<<nlayers, 256, 0, st>>>(a.part_f, a.part_g, grid, reinterpret_cast<const int*>(base + NA_BLOCK), ng,
+			reinterpret_cast<double*>(base + NA_OUT_F), reinterpret_cast<double*>(base + NA_OUT_BLK));
 		mgcu_count_launch();
 		NA_TRY(cudaGetLastError());
 	}

@@ -80,7 +80,7 @@ template <class P>
 struct FitArgs
 {
 	typedef typename P::T T;
-	int L, nb, kt, npass, ngroups, nc;   // nc: columns per block
+	int L, nb, kt, npass, ngroups, nc, ncs;   // nc, ncs: columns per block and per cache slot
 	long S;
 	const PassRec* pass;        // tiles of the passes
 	const FitPass* groups_of;
@@ -230,9 +230,10 @@ __device__ __forceinline__ void fit_group16(const FitGroup& G, const typename Fi
 // both gates of a group on a unit, quartet by quartet in the tile.  Forward: flush (tab or null)
 // with the first gate, the state to the cache (out or null) with the last; transposed (TR):
 // flush with the last
-template <class P, int QC, bool TR>
+// SP: threads per unit, 1 or 4 (one quartet each, part = 0..3)
+template <class P, int QC, bool TR, int SP>
 __device__ __forceinline__ void fit_group(const FitGroup& G, const FitGate<typename P::T>* gates, unsigned tc, unsigned base,
-	const typename P::T* __restrict__ tab, typename P::T* __restrict__ out)
+	const typename P::T* __restrict__ tab, typename P::T* __restrict__ out, int part)
 {
 	typedef typename P::T T;
 	const int w0 = G.ga >= 0 ? 0 : 1, w1 = G.kind_b ? 1 : 0;
@@ -244,8 +245,9 @@ __device__ __forceinline__ void fit_group(const FitGroup& G, const FitGate<typen
 		const bool sk = g.swk, sc = g.swc;
 		const char* tb = (w == (TR ? w1 : w0)) ? reinterpret_cast<const char*>(tab) : nullptr;
 		char* ob = (!TR && w == w1) ? reinterpret_cast<char*>(out) : nullptr;
+		if (SP > 1) __syncwarp();   // the other threads' quartets of the unit
 #pragma unroll 1
-		for (int i = 0; i < 4; i++)
+		for (int i = part; i < 4; i += SP)
 		{
 			const uint4 o = G.qs[w][i], q = G.qy[w][i];
 			const unsigned ax = tc + (base ^ o.x), ay = tc + (base ^ o.y), az = tc + (base ^ o.z), aw = tc + (base ^ o.w);
@@ -327,19 +329,19 @@ __device__ __forceinline__ void fit_whole_backward(const FitGroup& G, int w, con
 // instruction caches (a third of its stalls).
 // EOUT: the derivative also to its cache eout, with the last gate.  SW: the tile holds the
 // state and ct the derivative (Hessian items)
-template <class P, bool SW, bool EOUT>
+template <class P, bool SW, bool EOUT, int SP>
 __device__ __forceinline__ void fit_contract(const FitGroup& G, int first, int last, unsigned tc, unsigned base,
-	const typename P::T* __restrict__ ct, typename P::Acc (&acc)[8], typename P::T* __restrict__ eout = nullptr)
+	const typename P::T* __restrict__ ct, typename P::Acc (&acc)[8], typename P::T* __restrict__ eout, int part)
 {
 	typedef typename P::T T;
 	const char* cb = reinterpret_cast<const char*>(ct);
 	const uint4 *qs = &G.qs[0][0], *qy = &G.qy[0][0];
-	int i = 4 * first;
+	int i = 4 * first + part;
 	uint4 oy = qy[i];
 	T cx = *reinterpret_cast<const T*>(cb + oy.x), cy = *reinterpret_cast<const T*>(cb + oy.y);
 	T cz = *reinterpret_cast<const T*>(cb + oy.z), cw = *reinterpret_cast<const T*>(cb + oy.w);
 #pragma unroll 1
-	for (int k = 4 * (first - last + 1); k > 0; k--)
+	for (int k = 4 * (first - last + 1); k > 0; k -= SP)
 	{
 		const uint4 o = qs[i];
 		const T x = lds<T>(tc + (base ^ o.x)), y = lds<T>(tc + (base ^ o.y)), z = lds<T>(tc + (base ^ o.z)), v = lds<T>(tc + (base ^ o.w));
@@ -351,8 +353,8 @@ __device__ __forceinline__ void fit_contract(const FitGroup& G, int first, int l
 			*reinterpret_cast<T*>(eb + q.x) = x; *reinterpret_cast<T*>(eb + q.y) = y;
 			*reinterpret_cast<T*>(eb + q.z) = z; *reinterpret_cast<T*>(eb + q.w) = v;
 		}
-		i = (i + 1) & 7;   // gate b's quartets 4..7, then gate a's 0..3
-		if (k > 1)
+		i = (i + SP) & 7;   // gate b's quartets 4..7, then gate a's 0..3
+		if (k > SP)
 		{
 			oy = qy[i];
 			cx = *reinterpret_cast<const T*>(cb + oy.x); cy = *reinterpret_cast<const T*>(cb + oy.y);
@@ -364,8 +366,9 @@ __device__ __forceinline__ void fit_contract(const FitGroup& G, int first, int l
 }
 
 // threads per block: 128, or 256 where a tile has that many units; four (two) blocks per SM
-// (registers), three of 128 in complex128, whose pipe is the bound
-template <class P, int QC, int MODE, int FIT_NT>
+// (registers), three of 128 in complex128, whose pipe is the bound.  SP 4 (gradients of few
+// columns, see fit_build): four threads per unit
+template <class P, int QC, int MODE, int FIT_NT, int SP>
 __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 : P::kId == MG_PREC_FP64_ID ? 3 : 4) k_fit(FitArgs<P> a)
 {
 	typedef typename P::T T;
@@ -378,7 +381,7 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 	const unsigned U = 1u << nu, n = 1u << kt;
 	const int nc = a.nc;
 	// units per thread (none for the threads beyond the block's units)
-	const unsigned its = U > FIT_NT ? U / FIT_NT : threadIdx.x < U * nc ? 1 : 0;
+	const unsigned its = U > FIT_NT ? U / FIT_NT : threadIdx.x < U * nc * SP ? 1 : 0;
 	const unsigned tb = smem_u32(smem_raw);
 	Smem s;
 	s.dlo = reinterpret_cast<unsigned*>(smem_raw + (size_t)ES * n * nc);
@@ -386,9 +389,10 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 	s.red = reinterpret_cast<double*>(s.dhi + 128);
 	s.h = kt / 2;
 	const long S = a.S;
-	const unsigned mycol = min(threadIdx.x >> nu, (unsigned)nc - 1), u0 = nc > 1 ? (threadIdx.x & (U - 1)) : threadIdx.x;
+	const unsigned tu = threadIdx.x / SP, mycol = min(tu >> nu, (unsigned)nc - 1), u0 = (nc > 1 || SP > 1) ? (tu & (U - 1)) : tu;
+	const int part = SP > 1 ? (int)(threadIdx.x % SP) : 0;
 	const unsigned colb = mycol * n * ES;
-	const size_t cstride = (size_t)nc * S * (QC == 2 ? 2 : 1);
+	const size_t cstride = (size_t)(MODE == FIT_HESS ? a.ncs : nc) * S * (QC == 2 ? 2 : 1);
 	typename P::Acc acc[8];
 #pragma unroll
 	for (int e = 0; e < 8; e++) acc[e] = P::acc_zero();
@@ -400,7 +404,8 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 		// this thread's column (the last one again past the range: its derivative is zero)
 		const long b = min(cb + (long)mycol, a.b1 - 1);
 		const int par = __popcll(b) & 1;
-		const size_t coff = (size_t)(MODE == FIT_HESS ? (cb - a.b0) / nc : blockIdx.x) * a.ngroups * cstride + (size_t)mycol * S;
+		const size_t coff = MODE == FIT_HESS ? (size_t)((cb - a.b0) / a.ncs) * a.ngroups * cstride + (size_t)((cb - a.b0) % a.ncs + mycol) * S
+			: (size_t)blockIdx.x * a.ngroups * cstride + (size_t)mycol * S;
 		T* cache = GRAD ? a.cache + coff : nullptr;
 		// the state between passes (one column per block then): the output column itself, or a slot
 		auto between = [&]() { return MODE == FIT_COLS ? a.ucols + (size_t)(cb - a.b0) * S : a.sw + (size_t)blockIdx.x * S; };
@@ -443,7 +448,7 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 							for (int st = 0; st < ngt; st++)
 								fit_whole_forward<P>(G, w0 ^ st, stage[g & 1].gate[w0 ^ st], tb + colb, base, out + (size_t)(w0 ^ st) * nc * S);
 						}
-						else if constexpr (GRAD) fit_group<P, QC, false>(G, stage[g & 1].gate, tb + colb, base, tab, out);
+						else if constexpr (GRAD) fit_group<P, QC, false, SP>(G, stage[g & 1].gate, tb + colb, base, tab, out, part);
 						else fit_group16<P, QC>(G, stage[g & 1].gate, tb + colb, base, U, tab);
 					}
 					fit_stage_wait();
@@ -570,7 +575,7 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 					T* eg = MODE == FIT_HESS ? a.dcache + coff + (size_t)g * cstride + ((size_t)tau << kt) + u0 : nullptr;
 					const T* tab = G.flush >= 0 ? a.tables + ((size_t)(2 * G.flush + par) * S + ((size_t)tau << kt) + u0) : nullptr;
 					const int blk = G.ga >= 0 ? G.blk_a : G.blk_b;
-					if (g > fp.gbeg)
+					if (SP == 1 && g > fp.gbeg)
 					{
 						// the next group's cached state to L2: two of the sixteen 128-byte lines that
 						// eight threads' registers take
@@ -583,18 +588,18 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 					if (split)
 					{
 						for (unsigned i = 0; i < its; i++)
-							fit_contract<P, false, false>(G, 1, 1, tb + colb, fit_base(G, a.bases + (size_t)g * U, u0 + i * FIT_NT, tpar), cg + i * FIT_NT, acc);
+							fit_contract<P, false, false, SP>(G, 1, 1, tb + colb, fit_base(G, a.bases + (size_t)g * U, u0 + i * FIT_NT, tpar), cg + i * FIT_NT, acc, nullptr, part);
 						block_reduce8<P>(acc, s.red, a.part + ((size_t)blockIdx.x * a.nblocks + G.blk_b) * 16, 1.0, nred);
 #pragma unroll
 						for (int e = 0; e < 8; e++) acc[e] = P::acc_zero();
 					}
 					for (unsigned i = 0; i < its; i++)
-						fit_contract<P, false, MODE == FIT_HESS>(G, (G.kind_b && !split) ? 1 : 0, G.ga >= 0 ? 0 : 1, tb + colb,
-							fit_base(G, a.bases + (size_t)g * U, u0 + i * FIT_NT, tpar), cg + i * FIT_NT, acc, eg + i * FIT_NT);
+						fit_contract<P, false, MODE == FIT_HESS, SP>(G, (G.kind_b && !split) ? 1 : 0, G.ga >= 0 ? 0 : 1, tb + colb,
+							fit_base(G, a.bases + (size_t)g * U, u0 + i * FIT_NT, tpar), cg + i * FIT_NT, acc, eg + i * FIT_NT, part);
 					if (g > 0)   // nothing uses the derivative before the first group
 						for (unsigned i = 0; i < its; i++)
-							fit_group<P, QC, true>(G, stage[g & 1].gate, tb + colb, fit_base(G, a.bases + (size_t)g * U, u0 + i * FIT_NT, tpar),
-								tab ? tab + i * FIT_NT : nullptr, nullptr);
+							fit_group<P, QC, true, SP>(G, stage[g & 1].gate, tb + colb, fit_base(G, a.bases + (size_t)g * U, u0 + i * FIT_NT, tpar),
+								tab ? tab + i * FIT_NT : nullptr, nullptr, part);
 					merged += 8 * (int)max(its, 1u);
 					fit_stage_wait();
 					// the next group continues this sum when its gates are of the same block
@@ -755,7 +760,7 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 			{
 				const T* tab = G.flush >= 0 ? a.tables + (size_t)(2 * G.flush + par) * a.S + u0 : nullptr;
 				for (unsigned i = 0; i < its; i++)
-					fit_group<P, QC, false>(G, stage[g & 1].gate, tc, fit_base(G, bs, u0 + i * FIT_NT, par), tab ? tab + i * FIT_NT : nullptr, nullptr);
+					fit_group<P, QC, false, 1>(G, stage[g & 1].gate, tc, fit_base(G, bs, u0 + i * FIT_NT, par), tab ? tab + i * FIT_NT : nullptr, nullptr, 0);
 			}
 #pragma unroll 1
 			for (; st < ngt; st++)
@@ -775,7 +780,7 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 				for (unsigned i = 0; i < its; i++)
 				{
 					const unsigned base = fit_base(G, bs, u0 + i * FIT_NT, par);
-					fit_contract<P, true, false>(G, w, w, tc, base, eg + i * FIT_NT, acc);
+					fit_contract<P, true, false, 1>(G, w, w, tc, base, eg + i * FIT_NT, acc, nullptr, 0);
 					if (blk == grp) fit_move<P>(G, w, x, tc, base, cg + i * FIT_NT, false);
 				}
 			}

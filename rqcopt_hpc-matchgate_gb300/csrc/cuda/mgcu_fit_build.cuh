@@ -157,6 +157,10 @@ static int fit_build(int L, int kt, const int* wires, int ng, const int* block, 
 	f.kt = kt;
 	f.factored = factored;
 	f.nc = (U < 128 && nb <= kt) ? 128 / U : 1;   // small sectors share a block
+	// gradients of few columns: four threads per unit and a fourth of the columns per block, while
+	// that leaves blocks unused otherwise
+	f.split = (factored && nb <= kt && U <= 32 && (1L << L) / f.nc < mgcu_ctx()->nsm) ? 4 : 1;
+	f.ncb = f.split > 1 ? f.nc / f.split : f.nc;
 	f.smem = (size_t)f.nc * ((size_t)1 << kt) * es + 2 * 128 * sizeof(unsigned) + red_bytes(f.threads);
 	int e = upload_sched(f.sched, f.d_pass, f.d_gates);
 	if (!e) e = f.d_group.alloc(sizeof(FitGroup) * f.group.size());
@@ -508,22 +512,23 @@ static int fit_set_gates(const mgg* gates, int ng, const int* block, int nblocks
 	return 0;
 }
 
-template <class P, int NT>
+template <class P, int NT, int SP>
 static void (*fit_kernel_nt(int qc, int mode))(FitArgs<P>)
 {
 	if constexpr (P::kId == MG_PREC_FP32_ID)
-		return mode == FIT_COLS ? k_fit<P, 2, FIT_COLS, NT> : mode == FIT_GRAD ? k_fit<P, 2, FIT_GRAD, NT> : k_fit<P, 2, FIT_VALUE, NT>;
+		return mode == FIT_COLS ? k_fit<P, 2, FIT_COLS, NT, 1> : mode == FIT_GRAD ? k_fit<P, 2, FIT_GRAD, NT, 1> : k_fit<P, 2, FIT_VALUE, NT, 1>;
 	else if (qc)
-		return mode == FIT_COLS ? k_fit<P, 1, FIT_COLS, NT> : mode == FIT_GRAD ? k_fit<P, 1, FIT_GRAD, NT>
-			: mode == FIT_HESS ? k_fit<P, 1, FIT_HESS, NT> : k_fit<P, 1, FIT_VALUE, NT>;
+		return mode == FIT_COLS ? k_fit<P, 1, FIT_COLS, NT, 1> : mode == FIT_GRAD ? k_fit<P, 1, FIT_GRAD, NT, SP>
+			: mode == FIT_HESS ? k_fit<P, 1, FIT_HESS, NT, SP> : k_fit<P, 1, FIT_VALUE, NT, 1>;
 	else
-		return mode == FIT_COLS ? k_fit<P, 0, FIT_COLS, NT> : mode == FIT_GRAD ? k_fit<P, 0, FIT_GRAD, NT>
-			: mode == FIT_HESS ? k_fit<P, 0, FIT_HESS, NT> : k_fit<P, 0, FIT_VALUE, NT>;
+		return mode == FIT_COLS ? k_fit<P, 0, FIT_COLS, NT, 1> : mode == FIT_GRAD ? k_fit<P, 0, FIT_GRAD, NT, SP>
+			: mode == FIT_HESS ? k_fit<P, 0, FIT_HESS, NT, SP> : k_fit<P, 0, FIT_VALUE, NT, 1>;
 }
 template <class P>
-static void (*fit_kernel(int qc, int mode, int threads))(FitArgs<P>)
+static void (*fit_kernel(int qc, int mode, int threads, int split = 1))(FitArgs<P>)
 {
-	return threads == 512 ? fit_kernel_nt<P, 512>(qc, mode) : threads == 256 ? fit_kernel_nt<P, 256>(qc, mode) : fit_kernel_nt<P, 128>(qc, mode);
+	return threads == 512 ? fit_kernel_nt<P, 512, 1>(qc, mode) : threads == 256 ? fit_kernel_nt<P, 256, 1>(qc, mode)
+		: split > 1 ? fit_kernel_nt<P, 128, 4>(qc, mode) : fit_kernel_nt<P, 128, 1>(qc, mode);
 }
 
 // k_fit's arguments that come from a program
@@ -533,7 +538,7 @@ static FitArgs<P> fit_args(const FitProg& f, int L)
 	typedef typename P::T T;
 	FitArgs<P> w;
 	memset(&w, 0, sizeof(w));
-	w.L = L; w.nb = L - 1; w.kt = f.kt; w.npass = (int)f.sched.pass.size(); w.ngroups = (int)f.group.size(); w.nc = f.nc;
+	w.L = L; w.nb = L - 1; w.kt = f.kt; w.npass = (int)f.sched.pass.size(); w.ngroups = (int)f.group.size(); w.nc = w.ncs = f.nc;
 	w.S = 1L << (L - 1);
 	w.pass = f.d_pass.as<PassRec>(); w.groups_of = f.d_pgroups.as<FitPass>(); w.groups = f.d_group.as<FitGroup>();
 	w.bases = f.d_bases.as<unsigned>();
