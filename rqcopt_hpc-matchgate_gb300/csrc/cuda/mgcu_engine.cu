@@ -1863,6 +1863,35 @@ int grid_cap(long work, int threads)
 // ======================================================================================
 // targets
 // ======================================================================================
+// Several tables in one device allocation and one upload: add() collects them on the host, up()
+// allocates and copies; a Slice then points at its table.
+struct Slice
+{
+	DevBuf* b = nullptr;
+	size_t off = 0;
+	template <class T> T* as() const { return reinterpret_cast<T*>(static_cast<char*>(b->p) + off); }
+};
+struct Arena
+{
+	std::vector<char> host;
+	DevBuf* b;
+	explicit Arena(DevBuf& buf) : b(&buf) {}
+	void add(Slice& s, const void* src, size_t n)
+	{
+		s.b = b;
+		s.off = host.size();
+		host.resize((host.size() + n + 255) & ~(size_t)255);
+		if (src && n) memcpy(host.data() + s.off, src, n);
+	}
+	int up()
+	{
+		const int e = b->alloc(host.size());
+		if (e) return e;
+		MGCU_TRY(cudaMemcpyAsync(b->p, host.data(), host.size(), cudaMemcpyHostToDevice, mgcu_stream()));
+		return 0;
+	}
+};
+
 // a target's sector sweep (k_sector): the sectors, their row lists and the gate program
 struct SectorProg
 {
@@ -1873,7 +1902,8 @@ struct SectorProg
 	std::vector<Sec> sec;          // largest first
 	std::vector<unsigned> rows;    // full basis index per row, ascending within a sector
 	int nsteps = 0;
-	DevBuf steps, list, offs, drows;
+	Slice steps, list, offs, drows;
+	DevBuf fixed;
 };
 
 // a fitted circuit's or target's program for k_fit (see mgcu_fit_build.cuh)
@@ -1888,7 +1918,8 @@ struct WsProg
 	std::vector<std::array<int, 2>> diag;   // per table factor: gate, 0 left / 1 right
 	std::vector<int> pair_of;               // pair table per gate
 	std::vector<unsigned> rows;
-	DevBuf d_levels, d_gates, d_pairs, d_tab, d_rows, d_sec, d_diag, d_beg, d_plevel;
+	Slice d_levels, d_pairs, d_rows, d_beg, d_plevel, d_gates, d_diag;
+	DevBuf fixed, values, d_tab, d_sec;
 };
 
 struct FitProg
@@ -1910,7 +1941,8 @@ struct FitProg
 	int split = 1, ncb = 1;        // gradients: threads per unit and columns per block
 	size_t smem = 0;
 	WsProg ws;
-	DevBuf d_pass, d_group, d_pgroups, d_gates, d_diag, d_beg, d_gof, d_tab, d_blk, d_bases, d_pgroup, cache;
+	Slice d_pass, d_group, d_pgroups, d_beg, d_gof, d_bases, d_pgroup, d_gates, d_diag, d_blk;
+	DevBuf fixed, values, d_tab, cache;
 };
 
 struct TargetProg
@@ -3116,7 +3148,7 @@ extern "C" mgcu_plan* mgcu_plan_create(const mgcu_plan_desc* d)
 		// against 87 ms in two 64 KB tiles), a larger one tiles of 64 KB (L=16, 5 layers, 6001
 		// columns: 81 ms against 87 ms in tiles of 128 KB, one block per SM)
 		if (opt_kt <= 0 && p->nb <= 13) p->fit.kt = p->nb;
-		e = fit_build(p->L, p->fit.kt, p->wires.data(), d->ngates, p->block.data(), d->nblocks, (int)p->tsize, d->want_hess != 0 || p->prec == MG_PREC_FP32_ID, p->prec != MG_PREC_FP32_ID, p->fit);
+		e = fit_build(p->L, p->fit.kt, p->wires.data(), d->ngates, p->block.data(), d->nblocks, (int)p->tsize, d->want_hess != 0 || p->prec == MG_PREC_FP32_ID, p->prec != MG_PREC_FP32_ID, p->fit, p->place);
 		int per = 0;
 		if (!e)
 		{
@@ -3141,19 +3173,8 @@ extern "C" mgcu_plan* mgcu_plan_create(const mgcu_plan_desc* d)
 			if (opt_cps > 0) ph = (int)std::min<long>(ph, opt_cps);
 			p->fit.grid_h = c->nsm * std::max(ph, 1);
 			// number sectors, where the target conserves the particle number
-			if (p->w_t) e = p->prec == MG_PREC_FP64_ID ? ws_build<PrecD>(p->L, p->wires.data(), d->ngates, p->fit.ws) : ws_build<PrecX>(p->L, p->wires.data(), d->ngates, p->fit.ws);
-			if (!e && p->fit.ws.built)
-			{
-				std::vector<int> pl(std::max(p->d.nplace, 1), 0);
-				for (int q = 0; q < p->d.nplace; q++) pl[q] = p->fit.ws.level_of[p->place[q]];
-				e = p->fit.ws.d_plevel.alloc(sizeof(int) * pl.size());
-				if (!e && cudaMemcpy(p->fit.ws.d_plevel.p, pl.data(), sizeof(int) * pl.size(), cudaMemcpyHostToDevice) != cudaSuccess) e = MG_ERR_DEVICE;
-			}
-			if (e) { delete p; return nullptr; }
-			std::vector<int> pg(std::max(p->d.nplace, 1), 0);
-			for (int q = 0; q < p->d.nplace; q++) pg[q] = p->fit.group_of_gate[p->place[q]];
-			e = p->fit.d_pgroup.alloc(sizeof(int) * pg.size());
-			if (!e && cudaMemcpy(p->fit.d_pgroup.p, pg.data(), sizeof(int) * pg.size(), cudaMemcpyHostToDevice) != cudaSuccess) e = MG_ERR_DEVICE;
+			if (p->w_t) e = p->prec == MG_PREC_FP64_ID ? ws_build<PrecD>(p->L, p->wires.data(), d->ngates, p->place, p->fit.ws)
+				: ws_build<PrecX>(p->L, p->wires.data(), d->ngates, p->place, p->fit.ws);
 			if (e) { delete p; return nullptr; }
 		}
 		const size_t slot = (size_t)p->fit.group.size() * (p->fit.factored ? 1 : 2) * p->fit.nc * col_bytes;

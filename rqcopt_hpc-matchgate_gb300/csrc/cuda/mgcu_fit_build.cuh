@@ -9,7 +9,8 @@ static unsigned fit_wires(const int* w, int g) { return (1u << w[2 * g]) | (1u <
 // table of all pending left factors and of the right factors of every gate that comes next on
 // both of its wires (one flush per brickwall layer when the sector is one tile).  ordered
 // (Hessians, unfactored gates): the groups keep the sequence of the gates; unfactored: no flushes.
-static int fit_build(int L, int kt, const int* wires, int ng, const int* block, int nblocks, int es, bool ordered, bool factored, FitProg& f)
+static int fit_build(int L, int kt, const int* wires, int ng, const int* block, int nblocks, int es, bool ordered, bool factored, FitProg& f,
+	const std::vector<int>& place = {})
 {
 	const int nb = L - 1;
 	schedule(L, kt, wires, ng, !ordered, f.sched, es >= 16 ? 1 : 2);
@@ -162,24 +163,20 @@ static int fit_build(int L, int kt, const int* wires, int ng, const int* block, 
 	f.split = (factored && nb <= kt && U <= 32 && (1L << L) / f.nc < mgcu_ctx()->nsm) ? 4 : 1;
 	f.ncb = f.split > 1 ? f.nc / f.split : f.nc;
 	f.smem = (size_t)f.nc * ((size_t)1 << kt) * es + 2 * 128 * sizeof(unsigned) + red_bytes(f.threads);
-	int e = upload_sched(f.sched, f.d_pass, f.d_gates);
-	if (!e) e = f.d_group.alloc(sizeof(FitGroup) * f.group.size());
-	if (!e) e = f.d_pgroups.alloc(sizeof(FitPass) * f.pass_groups.size());
-	if (!e) e = f.d_gates.alloc(std::max(sizeof(FitGate<double2>), sizeof(FitWhole<double2>)) * 2 * f.group.size());
-	if (!e) e = f.d_diag.alloc(sizeof(FitDiag) * f.diag.size());
-	if (!e) e = f.d_beg.alloc(sizeof(int) * f.beg.size());
-	if (!e) e = f.d_gof.alloc(sizeof(int) * std::max(f.nflush, 1));
+	std::vector<int> pg;
+	for (int q : place) pg.push_back(f.group_of_gate[q]);
+	Arena ar(f.fixed);
+	ar.add(f.d_pass, f.sched.pass.data(), sizeof(PassRec) * f.sched.pass.size());
+	ar.add(f.d_group, f.group.data(), sizeof(FitGroup) * f.group.size());
+	ar.add(f.d_pgroups, f.pass_groups.data(), sizeof(FitPass) * f.pass_groups.size());
+	ar.add(f.d_beg, f.beg.data(), sizeof(int) * f.beg.size());
+	ar.add(f.d_gof, f.group_of.data(), sizeof(int) * f.group_of.size());
+	ar.add(f.d_bases, bases.data(), sizeof(unsigned) * bases.size());
+	ar.add(f.d_pgroup, pg.data(), sizeof(int) * pg.size());
+	int e = ar.up();
 	if (!e) e = f.d_tab.alloc((size_t)es * 2 * ((size_t)1 << nb) * (f.nflush + 1));
-	if (!e) e = f.d_blk.alloc(sizeof(FitBlock) * nblocks);
-	if (!e) e = f.d_bases.alloc(sizeof(unsigned) * bases.size());
 	if (e) return e;
-	cudaStream_t st = mgcu_stream();
-	MGCU_TRY(cudaMemcpyAsync(f.d_group.p, f.group.data(), sizeof(FitGroup) * f.group.size(), cudaMemcpyHostToDevice, st));
-	MGCU_TRY(cudaMemcpyAsync(f.d_pgroups.p, f.pass_groups.data(), sizeof(FitPass) * f.pass_groups.size(), cudaMemcpyHostToDevice, st));
-	MGCU_TRY(cudaMemcpyAsync(f.d_bases.p, bases.data(), sizeof(unsigned) * bases.size(), cudaMemcpyHostToDevice, st));
-	MGCU_TRY(cudaMemcpyAsync(f.d_beg.p, f.beg.data(), sizeof(int) * f.beg.size(), cudaMemcpyHostToDevice, st));
-	if (f.nflush) MGCU_TRY(cudaMemcpyAsync(f.d_gof.p, f.group_of.data(), sizeof(int) * f.nflush, cudaMemcpyHostToDevice, st));
-	MGCU_TRY(cudaStreamSynchronize(st));
+	MGCU_TRY(cudaStreamSynchronize(mgcu_stream()));
 	f.built = true;
 	return 0;
 }
@@ -224,19 +221,25 @@ static Hcx cdiv(Hcx a, Hcx b)
 
 struct FitFactor { double p; mgc q; int sw; Hcx l[2], r[2]; };
 
-// diag(l) M diag(r) of a 2x2 block (entries a, b, c, d), r[0] = 1; false when an entry that M is
-// scaled by is too small (|entry| < 2^-8 of the largest) or M is near singular.  p has 64
+// diag(l) M diag(r) of a 2x2 block (entries a, b, c, d), r[0] = 1; false (general kernels) when an
+// entry is not finite or far from one, when an entry that M is scaled by is small (under a
+// quarter of the largest; at least 0.7 in a unitary block) or M is near singular.  p has 64
 // candidates around |b / a| (|a / b| when swapped): p q = bc / (ad) is fixed, and the candidate
 // whose q rounds best leaves no rounding of the factors common to all amplitudes.
 static bool fit_factor(const mgc* e, FitFactor& F)
 {
 	double ab[4], mx = 0;
-	for (int k = 0; k < 4; k++) { ab[k] = std::hypot(e[k].re, e[k].im); mx = std::max(mx, ab[k]); }
-	if (!(mx > 1e-100 && mx < 1e100)) return false;
+	for (int k = 0; k < 4; k++)
+	{
+		ab[k] = std::hypot(e[k].re, e[k].im);
+		if (!(ab[k] < 1e3)) return false;   // infinities and NaN too
+		mx = std::max(mx, ab[k]);
+	}
+	if (mx < 1e-3) return false;
 	F.sw = ab[1] * ab[2] > ab[0] * ab[3];
 	// pivots (u, v) scaled to 1 and the others: unswapped M = [[1, p], [q, 1]], u = a, v = d
 	const int iu = F.sw ? 1 : 0, iv = F.sw ? 2 : 3, ip = F.sw ? 0 : 1, iq = F.sw ? 3 : 2;
-	if (ab[iu] < mx / 256 || ab[iv] < mx / 256) return false;
+	if (ab[iu] < mx / 4 || ab[iv] < mx / 4) return false;
 	const Hcx u = hcx(e[iu]), v = hcx(e[iv]), ep = hcx(e[ip]), eq = hcx(e[iq]);
 	const Hcx one = { hdd(1), hdd(0) };
 	const Hcx k = cdiv(cmul(ep, eq), cmul(u, v));   // p q
@@ -270,14 +273,14 @@ static bool fit_factor(const mgc* e, FitFactor& F)
 	const Hcx q = cdiv(eq, F.sw ? cmul(F.l[1], F.r[1]) : F.l[1]);
 	F.q = mgc_make(q.re.h, q.im.h);
 	const double dr = 1 - F.p * F.q.re, di = -F.p * F.q.im;
-	return std::hypot(dr, di) > 1.0 / 256 && std::hypot(F.q.re, F.q.im) < 256 && F.p < 256;
+	return std::hypot(dr, di) > 0.125 && std::hypot(F.q.re, F.q.im) < 8 && F.p < 8;
 }
 
 // Levels, pair tables and row positions for the number sectors (see mgcu_wsec.cuh): w.built when
 // the largest sector leaves two blocks per SM (L <= 14) and the gates fit in shared memory.
 // Columns per block: up to eight, as many as fit.
 template <class P>
-static int ws_build(int L, const int* wires, int ng, WsProg& w)
+static int ws_build(int L, const int* wires, int ng, const std::vector<int>& place, WsProg& w)
 {
 	typedef typename P::T T;
 	if (L > 14 || L < 4 || ng > WS_MAXG) return 0;
@@ -346,21 +349,19 @@ static int ws_build(int L, const int* wires, int ng, WsProg& w)
 	for (int s = lev.back().gbeg; s < lev.back().gend; s++) w.diag.push_back({ s, 0 });
 	w.beg.push_back((int)w.diag.size());
 	w.nlev = (int)lev.size();
-	int e = w.d_levels.alloc(sizeof(WsLevel) * lev.size());
-	if (!e) e = w.d_gates.alloc(sizeof(WsGate<T>) * ng);
-	if (!e) e = w.d_pairs.alloc(sizeof(ushort4) * pairs.size());
+	std::vector<int> pl;
+	for (int q : place) pl.push_back(w.level_of[q]);
+	Arena ar(w.fixed);
+	ar.add(w.d_levels, lev.data(), sizeof(WsLevel) * lev.size());
+	ar.add(w.d_pairs, pairs.data(), sizeof(ushort4) * pairs.size());
+	ar.add(w.d_rows, w.rows.data(), sizeof(unsigned) * N);
+	ar.add(w.d_beg, w.beg.data(), sizeof(int) * w.beg.size());
+	ar.add(w.d_plevel, pl.data(), sizeof(int) * pl.size());
+	int e = ar.up();
 	if (!e) e = w.d_tab.alloc(sizeof(T) * (size_t)N * (w.nlev + 1));
-	if (!e) e = w.d_rows.alloc(sizeof(unsigned) * N);
 	if (!e) e = w.d_sec.alloc(sizeof(WsSec) * (L + 1));
-	if (!e) e = w.d_diag.alloc(sizeof(FitDiag) * w.diag.size());
-	if (!e) e = w.d_beg.alloc(sizeof(int) * w.beg.size());
 	if (e) return e;
-	cudaStream_t st = mgcu_stream();
-	MGCU_TRY(cudaMemcpyAsync(w.d_levels.p, lev.data(), sizeof(WsLevel) * lev.size(), cudaMemcpyHostToDevice, st));
-	MGCU_TRY(cudaMemcpyAsync(w.d_pairs.p, pairs.data(), sizeof(ushort4) * pairs.size(), cudaMemcpyHostToDevice, st));
-	MGCU_TRY(cudaMemcpyAsync(w.d_rows.p, w.rows.data(), sizeof(unsigned) * N, cudaMemcpyHostToDevice, st));
-	MGCU_TRY(cudaMemcpyAsync(w.d_beg.p, w.beg.data(), sizeof(int) * w.beg.size(), cudaMemcpyHostToDevice, st));
-	MGCU_TRY(cudaStreamSynchronize(st));
+	MGCU_TRY(cudaStreamSynchronize(mgcu_stream()));
 	for (auto k : { k_ws_grad<P, true>, k_ws_grad<P, false> }) MGCU_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
 	for (auto k : { k_ws_hess<P, true>, k_ws_hess<P, false> }) MGCU_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
 	w.built = true;
@@ -401,8 +402,11 @@ static int ws_set_gates(const mgg* gates, int ng, const int* block, int L, const
 	std::vector<FitDiag> hd;
 	for (const auto& d : w.diag) hd.push_back(fit_diag(fac[2 * block[d[0]]], fac[2 * block[d[0]] + 1], d[1], wires[2 * d[0]], wires[2 * d[0] + 1], L));
 	cudaStream_t st = mgcu_stream();
-	MGCU_TRY(cudaMemcpyAsync(w.d_gates.p, hg.data(), sizeof(WsGate<T>) * ng, cudaMemcpyHostToDevice, st));
-	MGCU_TRY(cudaMemcpyAsync(w.d_diag.p, hd.data(), sizeof(FitDiag) * hd.size(), cudaMemcpyHostToDevice, st));
+	Arena av(w.values);
+	av.add(w.d_gates, hg.data(), sizeof(WsGate<T>) * ng);
+	av.add(w.d_diag, hd.data(), sizeof(FitDiag) * hd.size());
+	const int ev = av.up();
+	if (ev) return ev;
 	k_ws_tables<P><<<grid_cap((long)(w.nlev + 1) << L, 128), 128, 0, st>>>(w.d_diag.as<FitDiag>(), w.d_beg.as<int>(), w.nlev, L, w.d_rows.as<unsigned>(),
 		w.d_tab.as<T>());
 	MGCU_LAUNCHED();
@@ -430,15 +434,17 @@ static int fit_set_gates(const mgg* gates, int ng, const int* block, int nblocks
 				hw[i].k[q] = P::make(gates[g].k[q].re, gates[g].k[q].im);
 			}
 		}
-		MGCU_TRY(cudaMemcpyAsync(f.d_gates.p, hw.data(), sizeof(FitWhole<T>) * hw.size(), cudaMemcpyHostToDevice, mgcu_stream()));
 		std::vector<FitBlock> fb(nblocks);
 		memset(fb.data(), 0, sizeof(FitBlock) * nblocks);   // the sums are the gradients
 		for (FitBlock& b : fb)
 			for (int h = 0; h < 8; h++) { b.scale[h][0] = 1; b.minv[h][0] = (h & 3) == 0 || (h & 3) == 3; }
-		MGCU_TRY(cudaMemcpyAsync(f.d_blk.p, fb.data(), sizeof(FitBlock) * nblocks, cudaMemcpyHostToDevice, mgcu_stream()));
+		Arena av(f.values);
+		av.add(f.d_gates, hw.data(), sizeof(FitWhole<T>) * hw.size());
+		av.add(f.d_blk, fb.data(), sizeof(FitBlock) * nblocks);
+		const int e = av.up();
 		f.qc = 2;
-		f.ok = true;
-		return 0;
+		f.ok = e == 0;
+		return e;
 	}
 	std::vector<int> first(nblocks, -1);
 	for (int g = 0; g < ng; g++)
@@ -494,9 +500,12 @@ static int fit_set_gates(const mgg* gates, int ng, const int* block, int nblocks
 		hd[i] = fit_diag(fac[2 * block[g]], fac[2 * block[g] + 1], f.diag[i][1], wires[2 * g], wires[2 * g + 1], L);
 	}
 	cudaStream_t st = mgcu_stream();
-	MGCU_TRY(cudaMemcpyAsync(f.d_gates.p, hg.data(), sizeof(FitGate<T>) * hg.size(), cudaMemcpyHostToDevice, st));
-	MGCU_TRY(cudaMemcpyAsync(f.d_diag.p, hd.data(), sizeof(FitDiag) * hd.size(), cudaMemcpyHostToDevice, st));
-	MGCU_TRY(cudaMemcpyAsync(f.d_blk.p, fb.data(), sizeof(FitBlock) * nblocks, cudaMemcpyHostToDevice, st));
+	Arena av(f.values);
+	av.add(f.d_gates, hg.data(), sizeof(FitGate<T>) * hg.size());
+	av.add(f.d_diag, hd.data(), sizeof(FitDiag) * hd.size());
+	av.add(f.d_blk, fb.data(), sizeof(FitBlock) * nblocks);
+	const int ev = av.up();
+	if (ev) return ev;
 	f.ws.ok = false;
 	if constexpr (P::kId != MG_PREC_FP32_ID)
 		if (f.ws.built)
@@ -542,7 +551,7 @@ static FitArgs<P> fit_args(const FitProg& f, int L)
 	w.S = 1L << (L - 1);
 	w.pass = f.d_pass.as<PassRec>(); w.groups_of = f.d_pgroups.as<FitPass>(); w.groups = f.d_group.as<FitGroup>();
 	w.bases = f.d_bases.as<unsigned>();
-	w.gates = f.d_gates.p; w.tables = f.d_tab.as<T>(); w.final = w.tables + (size_t)2 * w.S * f.nflush;
+	w.gates = f.d_gates.as<char>(); w.tables = f.d_tab.as<T>(); w.final = w.tables + (size_t)2 * w.S * f.nflush;
 	return w;
 }
 
@@ -581,6 +590,7 @@ static int target_fit(mgcu_target* t, TargetProg& tp, FitProg& f)
 	MGCU_TRY(cudaFuncSetAttribute(fit_kernel<P>(f.qc, FIT_COLS, f.threads), cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
 	MGCU_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fit_kernel<P>(f.qc, FIT_COLS, f.threads), f.threads, f.smem));
 	f.grid = mgcu_ctx()->nsm * std::max(per, 1);
+	MGCU_TRY(cudaStreamSynchronize(mgcu_stream()));   // kept on the target: other threads' streams use it too
 	return 0;
 }
 

@@ -243,17 +243,14 @@ static int build_sector(mgcu_target* t, TargetProg& tp, SectorProg& sp)
 		for (const SectorProg::Sec& s : sp.sec)
 			sector_order(list, offs[s.offs + kv.second], offs[s.offs + kv.second + 1], (ES == 16 ? 8 : 16) >> s.ln, kv.first[0] == 0);
 	sp.nsteps = (int)sg.size();
-	int e = sp.steps.alloc(sizeof(SecStep) * std::max<size_t>(sg.size(), 1));
-	if (!e) e = sp.list.alloc(sizeof(unsigned) * list.size());
-	if (!e) e = sp.offs.alloc(sizeof(int) * offs.size());
-	if (!e) e = sp.drows.alloc(sizeof(unsigned) * N);
+	Arena ar(sp.fixed);
+	ar.add(sp.steps, sg.data(), sizeof(SecStep) * sg.size());
+	ar.add(sp.list, list.data(), sizeof(unsigned) * list.size());
+	ar.add(sp.offs, offs.data(), sizeof(int) * offs.size());
+	ar.add(sp.drows, sp.rows.data(), sizeof(unsigned) * N);
+	const int e = ar.up();
 	if (e) return e;
-	cudaStream_t st = mgcu_stream();
-	MGCU_TRY(cudaMemcpyAsync(sp.steps.p, sg.data(), sizeof(SecStep) * sg.size(), cudaMemcpyHostToDevice, st));
-	MGCU_TRY(cudaMemcpyAsync(sp.list.p, list.data(), sizeof(unsigned) * list.size(), cudaMemcpyHostToDevice, st));
-	MGCU_TRY(cudaMemcpyAsync(sp.offs.p, offs.data(), sizeof(int) * offs.size(), cudaMemcpyHostToDevice, st));
-	MGCU_TRY(cudaMemcpyAsync(sp.drows.p, sp.rows.data(), sizeof(unsigned) * N, cudaMemcpyHostToDevice, st));
-	MGCU_TRY(cudaStreamSynchronize(st));
+	MGCU_TRY(cudaStreamSynchronize(mgcu_stream()));
 	MGCU_TRY(cudaFuncSetAttribute(sector_kernel<P>(sp.threads), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
 	sp.state = 1;
 	return 0;

@@ -231,3 +231,19 @@ def test_batch_gates_change_kernels(mglib, prec):
         lib.set_precision(mgcu.PREC_FP64)
         for t in ts:
             lib.target_free(t)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, 1e-160, 1e5])
+def test_extreme_gate_entries(mglib, bad):
+    """an entry that is not finite, denormal-like or huge gives what the general kernels give"""
+    lib, rng = mglib, np.random.default_rng(3)
+    L = 10
+    v, perms = T.haar_matchgates(3, rng), T.brickwall_perms(L, 3)
+    v[1, 1] = bad
+    t = lib.target_brickwall(T.haar_matchgates(2, rng), T.brickwall_perms(L, 2), L)
+    try:
+        (rc0, f0, dv0), (rc1, f1, dv1) = _both(lib, lambda: lib.brickwall_target_and_gradient(lib.mg_target_apply, t, v, perms, L), 0)
+    finally:
+        lib.target_free(t)
+    assert rc0 == 0 and rc1 == 0
+    np.testing.assert_allclose([f0, *dv0.reshape(-1)], [f1, *dv1.reshape(-1)], rtol=1e-12, atol=1e-12 * np.nanmax(np.abs(dv1)) if np.isfinite(bad) else 0)
