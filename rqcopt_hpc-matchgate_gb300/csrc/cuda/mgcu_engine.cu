@@ -2652,6 +2652,21 @@ static int launch_target(mgcu_plan* p, long b0, long b1, typename P::T* out)
 	return plan_event(p, 1);
 }
 
+// Hessian items go to the blocks in turn (block i takes i, i + grid, ...).  While the cached states
+// and derivatives stay in L2 the items run placement by placement, longest first, so every block
+// gets as many of each; else column group by column group, whose caches are then shared by the
+// blocks at work.  The grid has no common factor with the 8 entries (and the placements), so that
+// no block keeps one entry or placement: with 608 blocks and 19 placements in group order each
+// block had one placement and SMs were idle half the time (L=9 float-float: 2.48 ms).
+static bool items_placewise(size_t cache_bytes) { return 2 * cache_bytes <= (96u << 20); }
+static int item_grid(long most, int nplace, bool placewise)
+{
+	auto gcd = [](long x, long y) { while (y) { const long t = x % y; x = y; y = t; } return x; };
+	for (long g = most; g > most - most / 16 && g > 1; g--)
+		if (gcd(g, placewise ? 8L : 8L * std::max(nplace, 1)) == 1) return (int)g;
+	return (int)most;
+}
+
 // the same for a particle-conserving Hessian plan in number sectors; done stays false when the
 // plan's caches have no room for the range's column groups
 template <class P>
@@ -2699,7 +2714,8 @@ static int launch_ws(mgcu_plan* p, long b0, long b1, const typename P::T* dense,
 	(f.qc ? k_ws_grad<P, true> : k_ws_grad<P, false>)<<<ga, WS_NT, w.smem, st>>>(a);
 	MGCU_LAUNCHED();
 	const long nitems = (long)groups * p->d.nplace * 8;
-	const int gh = (int)std::min<long>({ (long)slots, nitems, (long)std::max(p->grid_b, f.grid_h) });
+	a.placewise = items_placewise((size_t)groups * w.nlev * ((size_t)w.dmax << w.ln) * sizeof(T)) ? groups : 0;
+	const int gh = item_grid(std::min<long>({ (long)slots, nitems, (long)std::max(p->grid_b, f.grid_h) }), p->d.nplace, a.placewise != 0);
 	p->rows_h = std::max(p->rows_h, gh);
 	(f.qc ? k_ws_hess<P, true> : k_ws_hess<P, false>)<<<gh, WS_NT, w.smem, st>>>(a, nitems);
 	MGCU_LAUNCHED();
@@ -2765,7 +2781,9 @@ static int launch_columns(mgcu_plan* p, long b0, long b1, const typename P::T* d
 			h.block = p->d_block.as<int>(); h.nplace = p->d.nplace; h.ngates = p->d.ngates; h.mdim = 8 * p->d.nblocks;
 			h.hgroup = p->hgroup ? 1 : 0; h.part_h = p->part_h.as<double>();
 			const long nitems = (ncols + f.nc - 1) / f.nc * p->d.nplace * 8;
-			const int gh = (int)std::min<long>(f.grid_h, nitems);
+			const long cg = (ncols + f.nc - 1) / f.nc;
+			h.placewise = items_placewise((size_t)cg * f.group.size() * f.nc * p->S * sizeof(T)) ? cg : 0;
+			const int gh = item_grid(std::min<long>(f.grid_h, nitems), p->d.nplace, h.placewise != 0);
 			p->rows_h = std::max(p->rows_h, gh);
 			fit_hess_kernel<P>(f.qc, f.threads)<<<gh, f.threads, f.smem, mgcu_stream()>>>(h, nitems);
 			MGCU_LAUNCHED();
@@ -2803,7 +2821,7 @@ static int launch_columns(mgcu_plan* p, long b0, long b1, const typename P::T* d
 		a.block = p->d_block.as<int>(); a.nplace = p->d.nplace; a.mdim = 8 * p->d.nblocks; a.hgroup = p->hgroup ? 1 : 0;
 		a.part_h = p->part_h.as<double>(); a.sh = p->sh.as<T>();
 		const long nitems = ncols * p->d.nplace * 8;
-		const int gb = (int)std::min<long>(p->grid_b, nitems);
+		const int gb = item_grid(std::min<long>(p->grid_b, nitems), p->d.nplace, false);
 		p->rows_h = std::max(p->rows_h, gb);
 		k_hessian<P><<<gb, p->threads, p->smem, mgcu_stream()>>>(a, nitems);
 		MGCU_LAUNCHED();

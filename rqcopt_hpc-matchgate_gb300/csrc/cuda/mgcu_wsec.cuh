@@ -18,9 +18,9 @@
 // contractions are made without a barrier.
 //
 // Measured against the parity sectors (k_fit with derivative cache, k_fit_hess; the whole items of
-// an evaluation): L=12, 5 layers, complex128 6.8 + 128 -> 1.8 + 29.8 ms; L=12, 9 layers,
-// translation-invariant, float-float 4.1 + 101 -> 1.6 + 41.5 ms; L=10, 5 layers, float-float
-// 0.22 + 1.81 -> 0.12 + 0.86 ms.  Bound: the FP64 pipe in complex128, issue and the L2 reads of
+// an evaluation): L=12, 5 layers, complex128 6.8 + 128 -> 1.8 + 25.6 ms; L=12, 9 layers,
+// translation-invariant, float-float 4.1 + 101 -> 1.6 + 33.4 ms; L=10, 5 layers, float-float
+// 0.22 + 1.81 -> 0.12 + 0.80 ms.  Bound: the FP64 pipe in complex128, issue and the L2 reads of
 // the cached derivatives in float-float.
 
 struct WsLevel { int gbeg, gend; };
@@ -48,6 +48,7 @@ struct WsArgs
 	const int *place, *place_level, *block;
 	const double* place_w;
 	int nplace, mdim, hgroup;
+	long placewise;                 // as in FitHessArgs
 	double* part_h;
 };
 
@@ -95,43 +96,69 @@ __device__ __forceinline__ void ws_contract(const WsArgs<P>& a, int pair, int n,
 	typedef typename P::T T;
 	const ushort4* e = a.pairs + ((size_t)pair << (a.L - 2));
 	const unsigned cm = (1u << a.ln) - 1u, c = threadIdx.x & cm;
-	auto D = [&](unsigned row) { const unsigned i = (row << a.ln) | c; return DT ? lds<T>(tb + i * (unsigned)sizeof(T)) : mem[i]; };
-	auto B = [&](unsigned row) { const unsigned i = (row << a.ln) | c; return DT ? mem[i] : lds<T>(tb + i * (unsigned)sizeof(T)); };
+	auto M = [&](unsigned row) { return mem[(row << a.ln) | c]; };
+	auto S = [&](unsigned row) { return lds<T>(tb + ((row << a.ln) | c) * (unsigned)sizeof(T)); };
 	const unsigned st = WS_NT >> a.ln, t0 = threadIdx.x >> a.ln;
+	// two entries at a time, the reads from memory first: their latency is the bound
+	auto rows = [&](int m, bool w, int k) {
+		unsigned t = a.pstart[m] + t0;
+		const unsigned end = a.pstart[m + 1];
+		for (; t + st < end; t += 2 * st)
+		{
+			const ushort4 e0 = e[t], e1 = e[t + st];
+			const unsigned r0 = w ? e0.w : e0.x, r1 = w ? e1.w : e1.x;
+			const T m0 = M(r0), m1 = M(r1), s0 = S(r0), s1 = S(r1);
+			P::acc_mul_add_short(acc[k], DT ? s0 : m0, DT ? m0 : s0);
+			P::acc_mul_add_short(acc[k], DT ? s1 : m1, DT ? m1 : s1);
+		}
+		if (t < end)
+		{
+			const unsigned r0 = w ? e[t].w : e[t].x;
+			const T m0 = M(r0), s0 = S(r0);
+			P::acc_mul_add_short(acc[k], DT ? s0 : m0, DT ? m0 : s0);
+		}
+	};
+	auto pair4 = [&](const T& my, const T& mz, const T& sy, const T& sz) {
+		const T &dy = DT ? sy : my, &dz = DT ? sz : mz, &y = DT ? my : sy, &z = DT ? mz : sz;
+		P::acc_mul_add_short(acc[0], dy, y); P::acc_mul_add_short(acc[1], dy, z);
+		P::acc_mul_add_short(acc[2], dz, y); P::acc_mul_add_short(acc[3], dz, z);
+	};
 	if (shift == 0)
 	{
 		if (n >= 1 && n < a.L)
-			for (unsigned t = a.pstart[n - 1] + t0; t < (unsigned)a.pstart[n]; t += st)
+		{
+			unsigned t = a.pstart[n - 1] + t0;
+			const unsigned end = a.pstart[n];
+			for (; t + st < end; t += 2 * st)
 			{
-				const ushort4 r = e[t];
-				const T dy = D(r.y), dz = D(r.z), y = B(r.y), z = B(r.z);
-				P::acc_mul_add_short(acc[0], dy, y); P::acc_mul_add_short(acc[1], dy, z);
-				P::acc_mul_add_short(acc[2], dz, y); P::acc_mul_add_short(acc[3], dz, z);
+				const ushort4 e0 = e[t], e1 = e[t + st];
+				const T y0 = M(e0.y), z0 = M(e0.z), y1 = M(e1.y), z1 = M(e1.z);
+				pair4(y0, z0, S(e0.y), S(e0.z));
+				pair4(y1, z1, S(e1.y), S(e1.z));
 			}
-		if (n <= a.L - 2)
-			for (unsigned t = a.pstart[n] + t0; t < (unsigned)a.pstart[n + 1]; t += st)
+			if (t < end)
 			{
-				const unsigned r = e[t].x;
-				P::acc_mul_add_short(acc[4], D(r), B(r));
+				const ushort4 e0 = e[t];
+				const T y0 = M(e0.y), z0 = M(e0.z);
+				pair4(y0, z0, S(e0.y), S(e0.z));
 			}
-		if (n >= 2)
-			for (unsigned t = a.pstart[n - 2] + t0; t < (unsigned)a.pstart[n - 1]; t += st)
-			{
-				const unsigned r = e[t].w;
-				P::acc_mul_add_short(acc[7], D(r), B(r));
-			}
+		}
+		if (n <= a.L - 2) rows(n, false, 4);
+		if (n >= 2) rows(n - 2, true, 7);
 	}
 	else if (shift < 0)
 		for (unsigned t = a.pstart[n - 2] + t0; t < (unsigned)a.pstart[n - 1]; t += st)
 		{
 			const ushort4 r = e[t];
-			P::acc_mul_add_short(acc[6], D(r.w), B(r.x));
+			const T m0 = M(DT ? r.x : r.w), s0 = S(DT ? r.w : r.x);
+			P::acc_mul_add_short(acc[6], DT ? s0 : m0, DT ? m0 : s0);
 		}
 	else
 		for (unsigned t = a.pstart[n] + t0; t < (unsigned)a.pstart[n + 1]; t += st)
 		{
 			const ushort4 r = e[t];
-			P::acc_mul_add_short(acc[5], D(r.x), B(r.w));
+			const T m0 = M(DT ? r.w : r.x), s0 = S(DT ? r.x : r.w);
+			P::acc_mul_add_short(acc[5], DT ? s0 : m0, DT ? m0 : s0);
 		}
 }
 
@@ -249,8 +276,8 @@ __global__ void __launch_bounds__(WS_NT, 2) k_ws_hess(WsArgs<P> a, long nitems)
 	{
 		const int x = (int)(it & 7);
 		const long rest = it >> 3;
-		const int p = (int)(rest % a.nplace);
-		const long grp = rest / a.nplace;
+		const int p = (int)(a.placewise ? rest / a.placewise : rest % a.nplace);
+		const long grp = a.placewise ? rest % a.placewise : rest / a.nplace;
 		const WsSec I = ws_sector(a, grp);
 		const int n = I.n, shift = x == 5 ? -1 : x == 6 ? 1 : 0, m = n + 2 * shift;   // the tangent's sector
 		if (m < 0 || m > a.L) continue;
