@@ -22,8 +22,8 @@
 // summed, and f is the trace of R.
 //
 // Bound: issue (58 %) and the latency of the cached states in float-float, the FP64 pipe in
-// complex128.  Measured against k_columns (which stays for FP32, small sectors, Hessian caches
-// and gates that do not factor): float-float L=12, 7 layers 5.17 -> 2.88 ms; L=14, 9 layers
+// complex128.  Measured against k_columns (which stays for small sectors, FP32 Hessians and
+// gates that do not factor): float-float L=12, 7 layers 5.17 -> 2.88 ms; L=14, 9 layers
 // 122 -> 73 ms; L=16, 5 layers, 6001 columns 119 -> 81 ms; complex128 L=12, 5 layers
 // 12.2 -> 6.4 ms.
 
@@ -366,10 +366,17 @@ __device__ __forceinline__ void fit_contract(const FitGroup& G, int first, int l
 }
 
 // threads per block: 128, or 256 where a tile has that many units; four (two) blocks per SM
-// (registers), three of 128 in complex128, whose pipe is the bound.  SP 4 (gradients of few
-// columns, see fit_build): four threads per unit
+// (registers), three of 128 in complex128, whose pipe is the bound.  In FP32 f and columns keep
+// one state per thread and fit 768 threads on 80 registers: f at L=13, 8192 columns 4.95 ->
+// 4.63 ms (gradients, whose sums spill there, keep 512).  SP 4 (gradients of few columns, see
+// fit_build): four threads per unit
+constexpr int fit_blocks(int prec, int mode, int nt)
+{
+	if (prec == MG_PREC_FP32_ID && mode != FIT_GRAD) return 768 / nt;
+	return nt == 512 ? 1 : nt == 256 ? 2 : prec == MG_PREC_FP64_ID ? 3 : 4;
+}
 template <class P, int QC, int MODE, int FIT_NT, int SP>
-__global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 : P::kId == MG_PREC_FP64_ID ? 3 : 4) k_fit(FitArgs<P> a)
+__global__ void __launch_bounds__(FIT_NT, fit_blocks(P::kId, MODE, FIT_NT)) k_fit(FitArgs<P> a)
 {
 	typedef typename P::T T;
 	constexpr unsigned ES = sizeof(T);
