@@ -481,7 +481,7 @@ static int fit_set_gates(const mgg* gates, int ng, const int* block, int nblocks
 		}
 	}
 	// beyond the rounding of a unitary block q keeps its imaginary part (complex128: always)
-	f.qc = f.always_c || qi > (P::kId == MG_PREC_FP64_ID ? 0.0 : 1e-15);
+	f.qc = qi > (P::kId == MG_PREC_FP64_ID ? 0.0 : 1e-15);
 	std::vector<FitGate<T>> hg(2 * f.group.size());
 	memset(hg.data(), 0, sizeof(FitGate<T>) * hg.size());
 	for (size_t i = 0; i < hg.size(); i++)

@@ -233,6 +233,32 @@ def test_batch_gates_change_kernels(mglib, prec):
             lib.target_free(t)
 
 
+@pytest.mark.parametrize("prec", [mgcu.PREC_FP64, mgcu.PREC_MIXED])
+def test_batch_gates_change_factors(mglib, prec):
+    """a captured batch whose gates go from unitary to scaled (complex q) and back: each run equals
+    the same fits run as plans"""
+    lib, rng = mglib, np.random.default_rng(6)
+    Ls, nls = [12, 12], [3, 2]
+    ts = [lib.target_brickwall(T.haar_matchgates(4, rng), T.brickwall_perms(L, 4), L) for L in Ls]
+    perms = [T.brickwall_perms(L, nl) for L, nl in zip(Ls, nls)]
+    unitary, scaled = [[_layers(kind, nl, rng) for nl in nls] for kind in ("haar", "scaled")]
+    lib.set_precision(prec)
+    try:
+        b = lib.batch_create(ts, unitary, perms, Ls)
+        for vs in (unitary, scaled, [unitary[0], scaled[1]], unitary):
+            for i, v in enumerate(vs):
+                assert lib.batch_set_gates(b, i, v) == 0
+            assert lib.batch_run(b) == 0
+            for i, (t, v, L) in enumerate(zip(ts, vs, Ls)):
+                f, dv, _ = lib.batch_results(b, i)
+                _check([(0, f, dv), lib.brickwall_target_and_gradient(lib.mg_target_apply, t, v, perms[i], L)], TOL[prec])
+        lib.batch_free(b)
+    finally:
+        lib.set_precision(mgcu.PREC_FP64)
+        for t in ts:
+            lib.target_free(t)
+
+
 @pytest.mark.parametrize("bad", [np.nan, np.inf, 1e-160, 1e5])
 def test_extreme_gate_entries(mglib, bad):
     """an entry that is not finite, denormal-like or huge gives what the general kernels give"""
