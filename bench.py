@@ -126,12 +126,11 @@ def headline_config(L, nl, gu, trotter_steps):
             "l2": "per-step working set larger than L2; the GPU arm also writes a 512 MiB buffer between timed steps"}
 
 
-# DRAM bytes (read + write) of the target-sweep kernel per basis column: ncu
-# dram__bytes_read.sum + dram__bytes_write.sum of one k_target_w<PrecX> launch over 912 columns
-# of this workload (L=16, float-float, two columns per resident block).  The kernel's traffic
-# is its output columns plus the tile round trips that miss L2, both proportional to the
-# columns, so per-launch traffic = this x columns per launch.
-TARGET_DRAM_BYTES_PER_COLUMN = {16: (23.944726e9 + 20.012690e9) / 912}
+# DRAM bytes of the target-sweep kernel (k_sector) per basis column of this workload at L=16,
+# float-float: its output column, 2^15 amplitudes of 16 bytes; the column itself stays in shared
+# memory and its row lists in L2 (ncu: 0.7 MB read in a launch over 912 columns, whose 0.48 GB of
+# output partly stay in L2 there).
+TARGET_DRAM_BYTES_PER_COLUMN = {16: 16 << 15}
 
 
 def hbm_view(traffic, launch_s):
@@ -394,15 +393,19 @@ def run_gb300(a):
 
     flops = alg_flops(L, gu, gw, ncols)
     achieved_step = flops / (ms_per_step / 1e3) / 1e12
-    # dominant kernel: the target sweep (k_target), timed by CUDA events around each launch
+    # the target sweep's kernel, timed by CUDA events around each launch (the fitted circuit's, k_fit, is
+    # the rest of the step)
     cols_per_launch = ncols * a.steps / tk_n
     gu_run = lib.lib.mg_target_sweep_gates(mgcu.P(target))   # gates the sweep applies (fermionic swaps relabelled away)
-    # amplitude-columns the sweep visits per launch: the whole parity sector of every column,
-    # or (Hamming-weight-conserving target) the amplitudes of the column's weight only:
-    # sum_b C(L, |b|) = C(2L, L) over all 2^L columns
+    # amplitude-columns the sweep visits per launch: the whole parity sector of every column, or
+    # (particle-conserving target) the amplitudes with the column's numbers only: per spin,
+    # C(L, L/2)^2 over all 2^L columns, where such a sector fits in shared memory, else the
+    # column's Hamming weight, C(2L, L)
     weight = bool(lib.lib.mg_target_conserves_weight(mgcu.P(target)))
     sector_units = float(cols_per_launch) * (1 << (L - 1))
-    live_units = float(math.comb(2 * L, L)) * cols_per_launch / ncols if weight else sector_units
+    per_spin = L <= 18 and math.comb(L // 2, L // 4) ** 2 * (8 if a.precision == "fp32" else 16) <= 230400
+    live_units = (float(math.comb(L, L // 2) ** 2 if per_spin else math.comb(2 * L, L)) * cols_per_launch / ncols
+                  if weight else sector_units)
     tk_avg_s = tk_ms / 1e3 / tk_n
     achieved = live_units * 14 * gu_run / tk_avg_s / 1e12
     bpc = TARGET_DRAM_BYTES_PER_COLUMN.get(L) if a.precision == "mixed" else None
@@ -421,24 +424,25 @@ def run_gb300(a):
                 "timer": "host clock around matchgate_brickwall_unitary_target_and_projected_gradient (synchronous C call)"},
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": fp32_peak / 1e3, "unit": "TFLOP/s",
                      "frac": achieved / (fp32_peak / 1e3), "traffic": traffic,
-                     "kernel": "k_target (target sweep)", "kernel_launches": tk_n,
+                     "kernel": "k_sector (target sweep)" if weight and per_spin else "target sweep", "kernel_launches": tk_n,
                      "kernel_config": lib.plan_target_config(plan),
                      "kernel_ms_per_launch": tk_avg_s * 1e3, "kernel_share_of_step": tk_ms / total_ms,
                      "columns_per_launch": cols_per_launch,
                      "achieved_is": "algorithmic complex-arithmetic flops of the target sweep (14 per visited "
-                                    "amplitude and applied gate) per second of k_target; the target conserves the "
-                                    "Hamming weight, so the sweep visits C(2L, L) amplitude-columns per trace, the "
-                                    "nonzero ones, not the 2^(2L-1) of the parity sectors" if weight else
+                                    "amplitude and applied gate) per second of its kernel; the target conserves "
+                                    "particle numbers, so the sweep visits the amplitudes with the column's numbers "
+                                    "(per spin C(L, L/2)^2 amplitude-columns per trace where such a sector fits in "
+                                    "shared memory, else C(2L, L)), not the 2^(2L-1) of the parity sectors" if weight else
                                     "algorithmic complex-arithmetic flops of the target sweep (14 per parity-sector "
-                                    "amplitude and applied gate) per second of k_target",
+                                    "amplitude and applied gate) per second of its kernel",
                      "visited_amplitudes_per_launch": live_units,
                      "parity_sector_equivalent_tflops": sector_units * 14 * gu_run / tk_avg_s / 1e12,
                      "target_gates_applied": gu_run,
                      "step_achieved": achieved_step,
                      "peak_source": "FP32 FMA microkernel of this library, measured in this run "
                                     "(MEASURED_PEAKS.json holds HBM and bf16 tensor peaks only)",
-                     "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one k_target_w launch over "
-                                       "912 columns of this workload, per column, x columns per launch",
+                     "traffic_source": "the sweep's output columns, its only DRAM traffic (ncu: 0.7 MB read over 912 "
+                                       "columns)",
                      "fp64_peak_tflops": fp64_peak / 1e3,
                      "hbm": hbm_view(traffic, tk_avg_s)},
         "fp64_gpu": fp64,

@@ -27,12 +27,17 @@ int mg_set_precision(int precision);
 int mg_get_precision(void);
 
 /* Tuning options (0 = automatic).  TILE_BITS: log2 of amplitudes per shared-memory
- * tile; THREADS: threads per block; CHUNK_COLUMNS: basis columns per batch when
+ * tile; THREADS: threads per block, which also keeps f, gradients and Hessians on the general
+ * tiled kernels instead of the factored ones (L >= 10, Hessians L >= 7); CHUNK_COLUMNS: basis columns per batch when
  * columns are materialised from a host map or a Hessian is requested;
  * CTAS_PER_SM: resident blocks per SM for the persistent grid; TARGET_TILE_BITS and
  * TARGET_THREADS: the same two for the sweep of a GPU circuit target (default: TILE_BITS
  * and its block size; at most 2^13 amplitudes of 16 B and 512 threads); TARGET_COLUMNS: 2 sweeps
  * two basis columns of equal parity per block (256 threads), sharing the per-gate work.
+ * By default a particle-conserving circuit target is swept with whole columns in shared memory
+ * where they fit and others from L = 10 by the factored kernel; TARGET_THREADS,
+ * TARGET_COLUMNS, TARGET_DENSE and CTAS_PER_SM (for the factored kernel also TILE_BITS and
+ * TARGET_TILE_BITS) keep the tiled sweeps.
  * TRANSLATIONAL_INVARIANCE: 1 makes matchgate_brickwall_unitary_target_gradient_hessian, its
  * parallel_ twin, matchgate_brickwall_unitary_target_gradient_vector_hessian_matrix and
  * mg_optimize_brickwall use the translation-invariant Hessian -- what building the reference
@@ -40,7 +45,7 @@ int mg_get_precision(void);
  * 715, 819); 0 (default) is the reference's plain build.
  * TARGET_DENSE: 1 sweeps every amplitude of a GPU circuit target even when all its gates
  * conserve the Hamming weight (by default such targets are swept on the amplitudes of the
- * basis column's weight only; both give bit-identical results).
+ * basis column's particle numbers only; both give bit-identical results).
  * HOST_THREADS: host threads that call a caller's linear_func (a host map, not a GPU target)
  * concurrently, one basis column per call, as the reference's OpenMP threads do; the map must
  * be re-entrant (it is for the reference's own maps).  0 = the online cores; results do not
@@ -52,7 +57,7 @@ int mg_get_precision(void);
  * per gate, much less device memory and traffic, but a third more arithmetic and about 25 %
  * slower in float-float at L=16-18; gates that are not invertible fall back to the cache).
  * Hessian evaluations always cache.
- * TARGET_TUNE: how the block size of a GPU circuit target's sweep is chosen when
+ * TARGET_TUNE: how the block size of a GPU circuit target's tiled sweep is chosen when
  * TARGET_THREADS is 0.  0 (default): by timing the candidates (128 or 256 threads, and for
  * the full sweep 512) on one resident wave of columns when the trace has at least 2^14
  * columns, once per target, precision and tile size; 1: never (128 threads); 2: always.
