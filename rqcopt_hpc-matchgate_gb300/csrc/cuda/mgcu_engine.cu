@@ -3259,6 +3259,7 @@ extern "C" int mgcu_plan_set_gates(mgcu_plan* p, const mgg* gates)
 		else e = fit_set_gates<PrecX>(gates, d.ngates, d.block, d.nblocks, p->L, p->fit.kt, d.wires, p->fit);
 	}
 	if (e || !p->adj) return e;
+	if (p->prec == MG_PREC_FP64_ID) return upload_inverses<PrecD>(gates, p->d.ngates, p->d_mats_inv, p->adj_ok);
 	if (p->prec == MG_PREC_FP32_ID) return upload_inverses<PrecF>(gates, p->d.ngates, p->d_mats_inv, p->adj_ok);
 	return upload_inverses<PrecX>(gates, p->d.ngates, p->d_mats_inv, p->adj_ok);
 }

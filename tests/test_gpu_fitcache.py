@@ -65,3 +65,26 @@ def test_singular_fitted_gate_uses_the_cache(mglib, oracle):
     f_o, dv_o = oracle.brickwall_target_and_gradient(oracle.Target("brickwall", L, ulist=ul, uperms=up), v, perms, L)
     assert abs(f - f_o) <= 1e-11 * abs(f_o)
     assert np.linalg.norm(dv - dv_o) <= 1e-11 * np.linalg.norm(dv_o)
+
+
+@pytest.mark.parametrize("L,nl", [(6, 3), (10, 3), (12, 5), (14, 2)])
+def test_checkpointed_sweep_complex128(mglib, L, nl):
+    """complex128: the inverses in the sweep's own format; each recovered input carries a few more
+    roundings than a cached one, 1e-12 relative as for complex128 elsewhere in these tests"""
+    lib = mglib
+    rng = np.random.default_rng(500 + L)
+    t = lib.target_brickwall(T.haar_matchgates(6, rng), T.brickwall_perms(L, 6), L)
+    v, perms = T.haar_matchgates(nl, rng), T.brickwall_perms(L, nl)
+    out = []
+    lib.set_precision(mgcu.PREC_FP64)
+    try:
+        for cache in (2, 1):
+            lib.set_option(mgcu.OPT_FIT_CACHE, cache)
+            out.append(lib.brickwall_columns(lib.mg_target_apply, t, v, perms, L, 0, min(1000, 1 << L)))
+    finally:
+        lib.set_option(mgcu.OPT_FIT_CACHE, 0)
+        lib.target_free(t)
+    (rc0, f0, dv0), (rc1, f1, dv1) = out
+    assert rc0 == 0 and rc1 == 0
+    assert abs(f0 - f1) <= 1e-12 * max(abs(f1), np.max(np.abs(dv1)))
+    assert np.max(np.abs(dv0 - dv1)) <= 1e-12 * np.max(np.abs(dv1))
