@@ -2031,7 +2031,7 @@ struct mgcu_target
 	TargetProg progs[3];           // per precision
 	int resident = 0;
 	DevBuf res_cols[3];            // resident -conj(U e_b) per precision
-	int res_kt[3] = { -1, -1, -1 };
+	int res_key[3] = { -1, -1, -1 };   // the sweep that made them: tile bits, 256: factored
 	bool res_valid[3] = { false, false, false };
 	// the gate list the target sweep runs (fermionic swaps relabelled away, see
 	// relabel_fswaps) with per-gate Jordan-Wigner string wires
@@ -3303,14 +3303,17 @@ static int plan_columns_t(mgcu_plan* p, long b0, long b1, const mgc* host_cols)
 		else if (t->resident)
 		{
 			const int id = P::kId;
-			if (!t->res_valid[id] || t->res_kt[id] != p->kt)
+			// the tiled and sector sweeps make the same bits at one tile size (gate order); the
+			// factored sweep rounds differently (in FP32 its blocks are whole: the same bits)
+			const int key = p->kt_t + ((p->tfit && id != MG_PREC_FP32_ID) ? 256 : 0);
+			if (!t->res_valid[id] || t->res_key[id] != key)
 			{
 				const long N = 1L << p->L;
 				int e = t->res_cols[id].alloc((size_t)N * p->S * sizeof(T));
 				if (e) return e;
 				e = launch_target<P>(p, 0, N, t->res_cols[id].as<T>());
 				if (e) return e;
-				t->res_valid[id] = true; t->res_kt[id] = p->kt;
+				t->res_valid[id] = true; t->res_key[id] = key;
 			}
 			dense = t->res_cols[id].as<T>();
 			dense_b0 = 0;

@@ -273,3 +273,35 @@ def test_extreme_gate_entries(mglib, bad):
         lib.target_free(t)
     assert rc0 == 0 and rc1 == 0
     np.testing.assert_allclose([f0, *dv0.reshape(-1)], [f1, *dv1.reshape(-1)], rtol=1e-12, atol=1e-12 * np.nanmax(np.abs(dv1)) if np.isfinite(bad) else 0)
+
+
+@pytest.mark.parametrize("first", [0, 1])
+@pytest.mark.parametrize("prec", [mgcu.PREC_FP64, mgcu.PREC_MIXED])
+def test_resident_columns_follow_the_sweep(mglib, prec, first):
+    """a resident target evaluated with the factored sweep and with the full one
+    (MG_OPT_TARGET_DENSE), in both orders: each result has the bits of the same sweep on a target
+    that is not resident, whatever filled the columns before"""
+    lib, rng = mglib, np.random.default_rng(11)
+    L = 10
+    ul, up = T.haar_matchgates(8, rng), T.brickwall_perms(L, 8)
+    v, perms = T.haar_matchgates(3, rng), T.brickwall_perms(L, 3)
+
+    def run(t, dense):
+        lib.set_option(mgcu.OPT_TARGET_DENSE, dense)
+        rc, f, dv = lib.brickwall_target_and_gradient(lib.mg_target_apply, t, v, perms, L)
+        assert rc == 0, lib.last_error()
+        return f, dv
+    lib.set_precision(prec)
+    ts = [lib.target_brickwall(ul, up, L) for _ in range(2)]
+    try:
+        want = [run(ts[0], dense) for dense in (0, 1)]
+        assert not np.array_equal(want[0][1], want[1][1])   # the two sweeps round differently
+        assert lib.target_set_resident(ts[1], True) == 0
+        for dense in (first, 1 - first, first):
+            f, dv = run(ts[1], dense)
+            assert f == want[dense][0] and np.array_equal(dv, want[dense][1])
+    finally:
+        lib.set_option(mgcu.OPT_TARGET_DENSE, 0)
+        lib.set_precision(mgcu.PREC_FP64)
+        for t in ts:
+            lib.target_free(t)
