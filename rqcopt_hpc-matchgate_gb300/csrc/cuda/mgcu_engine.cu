@@ -3585,6 +3585,7 @@ struct BatchInst
 	double col_cost;               // relative cost of one column
 	bool big = false;              // enough columns to fill the GPU: its own kernels
 	FitProg fit;                   // its fitted circuit for k_fit (big instances)
+	int skip = 0;                  // k_batch_reduce's flag of this instance, as it is on the device
 	int grid_t = 0, grid_c = 0;    // standalone grids (big instances)
 	long chunk = 0;                // columns per staged chunk (big instances)
 	long part_off;                 // offsets (doubles) of part_f / part_g in the batch's partials
@@ -3882,7 +3883,7 @@ static int batch_build(mgcu_batch* B, const mgcu_batch_inst* d, int tune)
 	memcpy(B->host_args.data() + sizeof(Args<P>) * B->n, ac.data(), sizeof(Args<P>) * B->n);
 	MGCU_TRY(cudaMemcpy(B->red.p, rd.data(), sizeof(BatchRed) * B->n, cudaMemcpyHostToDevice));
 	if (B->skip.alloc(sizeof(int) * B->n)) return MG_ERR_ALLOC;
-	MGCU_TRY(cudaMemset(B->skip.p, 0, sizeof(int) * B->n));
+	MGCU_TRY(cudaMemsetAsync(B->skip.p, 0, sizeof(int) * B->n, mgcu_stream()));   // in order with mgcu_batch_set_gates' uploads
 	return 0;
 }
 
@@ -4036,12 +4037,17 @@ extern "C" int mgcu_batch_set_gates(mgcu_batch* B, int i, const mgg* gates)
 	else if (B->prec == MG_PREC_FP32_ID) e = upload_mats<PrecF>(gates, I.ngates, I.d_mats);
 	else e = upload_mats<PrecX>(gates, I.ngates, I.d_mats);
 	if (e || !I.fit.built) return e;
-	const int was = I.fit.ok;
 	if (B->prec == MG_PREC_FP64_ID) e = fit_set_gates<PrecD>(gates, I.ngates, I.block.data(), I.nblocks, I.L, I.fit.kt, I.wires.data(), I.fit);
 	else if (B->prec == MG_PREC_FP32_ID) e = fit_set_gates<PrecF>(gates, I.ngates, I.block.data(), I.nblocks, I.L, I.fit.kt, I.wires.data(), I.fit);
 	else e = fit_set_gates<PrecX>(gates, I.ngates, I.block.data(), I.nblocks, I.L, I.fit.kt, I.wires.data(), I.fit);
+	// (after an error too: the gates do not run on k_fit then, and a flag left set would keep an
+	// earlier run's results)
 	const int now = I.fit.ok;
-	if (!e && now != was) MGCU_TRY(cudaMemcpyAsync(B->skip.as<int>() + i, &now, sizeof(int), cudaMemcpyHostToDevice, mgcu_stream()));
+	if (now != I.skip)
+	{
+		MGCU_TRY(cudaMemcpyAsync(B->skip.as<int>() + i, &now, sizeof(int), cudaMemcpyHostToDevice, mgcu_stream()));
+		I.skip = now;
+	}
 	return e;
 }
 

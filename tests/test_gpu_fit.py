@@ -305,3 +305,30 @@ def test_resident_columns_follow_the_sweep(mglib, prec, first):
         lib.set_precision(mgcu.PREC_FP64)
         for t in ts:
             lib.target_free(t)
+
+
+@pytest.mark.parametrize("prec", [mgcu.PREC_FP64, mgcu.PREC_MIXED])
+def test_batch_created_with_gates_that_do_not_factor(mglib, prec):
+    """the reduction's flags from creation on: gates that do not factor, then some that do, then
+    none again, without a run between two changes of the same instance"""
+    lib, rng = mglib, np.random.default_rng(8)
+    Ls, nls = [12, 12, 10], [2, 3, 2]
+    ts = [lib.target_brickwall(T.haar_matchgates(4, rng), T.brickwall_perms(L, 4), L) for L in Ls]
+    perms = [T.brickwall_perms(L, nl) for L, nl in zip(Ls, nls)]
+    good, bad = [[_layers(kind, nl, rng) for nl in nls] for kind in ("haar", "singular")]
+    lib.set_precision(prec)
+    try:
+        b = lib.batch_create(ts, bad, perms, Ls)
+        for steps in ((bad,), (good, [bad[0], good[1], good[2]]), (bad, good, bad)):
+            for vs in steps:
+                for i, v in enumerate(vs):
+                    assert lib.batch_set_gates(b, i, v) == 0
+            assert lib.batch_run(b) == 0
+            for i, (t, v, L) in enumerate(zip(ts, vs, Ls)):
+                f, dv, _ = lib.batch_results(b, i)
+                _check([(0, f, dv), lib.brickwall_target_and_gradient(lib.mg_target_apply, t, v, perms[i], L)], TOL[prec])
+        lib.batch_free(b)
+    finally:
+        lib.set_precision(mgcu.PREC_FP64)
+        for t in ts:
+            lib.target_free(t)
