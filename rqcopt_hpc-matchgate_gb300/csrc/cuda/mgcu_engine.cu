@@ -1943,6 +1943,14 @@ struct FitProg
 	WsProg ws;
 	Slice d_pass, d_group, d_pgroups, d_beg, d_gof, d_bases, d_pgroup, d_gates, d_diag, d_blk;
 	DevBuf fixed, values, d_tab, cache;
+	// the program of a circuit that the general kernels run: no tables, no records
+	void release()
+	{
+		built = ok = false;
+		sched = Sched();
+		group = {}; pass_groups = {}; diag = {}; beg = {}; group_of = {}; block_gates = {}; group_of_gate = {};
+		fixed.release(); values.release(); d_tab.release();
+	}
 };
 
 struct TargetProg
@@ -3166,7 +3174,7 @@ extern "C" mgcu_plan* mgcu_plan_create(const mgcu_plan_desc* d)
 		// against 87 ms in two 64 KB tiles), a larger one tiles of 64 KB (L=16, 5 layers, 6001
 		// columns: 81 ms against 87 ms in tiles of 128 KB, one block per SM)
 		if (opt_kt <= 0 && p->nb <= 13) p->fit.kt = p->nb;
-		e = fit_build(p->L, p->fit.kt, p->wires.data(), d->ngates, p->block.data(), d->nblocks, (int)p->tsize, d->want_hess != 0 || p->prec == MG_PREC_FP32_ID, p->prec != MG_PREC_FP32_ID, p->fit, p->place);
+		e = fit_build(p->L, p->fit.kt, p->wires.data(), d->ngates, p->block.data(), d->nblocks, (int)p->tsize, d->want_hess != 0 || p->prec == MG_PREC_FP32_ID, p->prec != MG_PREC_FP32_ID, p->fit, SIZE_MAX, p->place);
 		int per = 0;
 		if (!e)
 		{
@@ -3763,7 +3771,7 @@ static int batch_build(mgcu_batch* B, const mgcu_batch_inst* d, int tune)
 			{
 				const int kt = P::kId == MG_PREC_FP32_ID ? std::min(I.nb, 13) : I.nb <= 13 ? I.nb : 12;
 				ef = fit_build(I.L, kt, d[i].wires, d[i].ngates, d[i].block, d[i].nblocks, (int)sizeof(T), P::kId == MG_PREC_FP32_ID,
-					P::kId != MG_PREC_FP32_ID, I.fit);
+					P::kId != MG_PREC_FP32_ID, I.fit, SIZE_MAX);
 				int per = 0;
 				auto kern = fit_kernel<P>(P::kId == MG_PREC_FP32_ID ? 2 : 1, d[i].want_grad ? FIT_GRAD : FIT_VALUE, I.fit.threads);
 				if (!ef) MGCU_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, I.fit.threads, I.fit.smem));

@@ -1,6 +1,9 @@
 // Host side of the factored fitted circuit (mgcu_fit.cuh): groups, flushes, factors.
 // Included by mgcu_engine.cu.
 
+// most bytes of a program's tables before the final one (64 at 18 qubits, where one takes 4 MB)
+constexpr size_t FIT_TABLES = (size_t)256 << 20;
+
 // wires of gate g as a mask
 static unsigned fit_wires(const int* w, int g) { return (1u << w[2 * g]) | (1u << w[2 * g + 1]); }
 
@@ -9,10 +12,13 @@ static unsigned fit_wires(const int* w, int g) { return (1u << w[2 * g]) | (1u <
 // table of all pending left factors and of the right factors of every gate that comes next on
 // both of its wires (one flush per brickwall layer when the sector is one tile).  ordered
 // (Hessians, unfactored gates): the groups keep the sequence of the gates; unfactored: no flushes.
+// Tables of more than `room` bytes are not made: f.built stays false and nothing is kept.
 static int fit_build(int L, int kt, const int* wires, int ng, const int* block, int nblocks, int es, bool ordered, bool factored, FitProg& f,
-	const std::vector<int>& place = {})
+	size_t room, const std::vector<int>& place = {})
 {
 	const int nb = L - 1;
+	const size_t table = (size_t)es * 2 << nb;   // bytes of one table
+	f.built = false;
 	schedule(L, kt, wires, ng, !ordered, f.sched, es >= 16 ? 1 : 2);
 	f.nflush = 0;
 	std::vector<std::vector<int>> onq(L);
@@ -124,6 +130,7 @@ static int fit_build(int L, int kt, const int* wires, int ng, const int* block, 
 			if (need)
 			{
 				G.flush = f.nflush++;
+				if (f.nflush * table > room) { f.release(); return 0; }
 				f.group_of.push_back((int)f.group.size());
 				for (int s : pending) f.diag.push_back({ s, 0 });
 				pending.clear();
@@ -174,7 +181,7 @@ static int fit_build(int L, int kt, const int* wires, int ng, const int* block, 
 	ar.add(f.d_bases, bases.data(), sizeof(unsigned) * bases.size());
 	ar.add(f.d_pgroup, pg.data(), sizeof(int) * pg.size());
 	int e = ar.up();
-	if (!e) e = f.d_tab.alloc((size_t)es * 2 * ((size_t)1 << nb) * (f.nflush + 1));
+	if (!e) e = f.d_tab.alloc(table * (f.nflush + 1));
 	if (e) return e;
 	MGCU_TRY(cudaStreamSynchronize(mgcu_stream()));
 	f.built = true;
@@ -557,7 +564,9 @@ static FitArgs<P> fit_args(const FitProg& f, int L)
 
 // The columns of a circuit target by k_fit, for targets that don't conserve particle numbers:
 // factored blocks in complex128 and float-float; in FP32 whole blocks in k_target's order (the
-// same bits), when every block is general there.  f.grid: resident blocks; state 0: not used.
+// same bits), when every block is general there.  f.grid: resident blocks.  Where it does not
+// apply (f.built stays false: gates that do not factor, tables past FIT_TABLES or with no memory
+// left for them) the tiled sweep runs, which needs none of it, and nothing is kept here.
 template <class P>
 static int target_fit(mgcu_target* t, TargetProg& tp, FitProg& f)
 {
@@ -580,11 +589,15 @@ static int target_fit(mgcu_target* t, TargetProg& tp, FitProg& f)
 		if (!factored && ((tp.kw[q] & 7) != BK_GEN || ((tp.kw[q] >> 3) & 7) != BK_GEN)) return 0;
 	}
 	const int nb = t->L - 1;
-	int e = fit_build(t->L, std::min(nb, es == 16 ? (nb <= 13 ? 13 : 12) : 13), w.data(), ng, block.data(), (int)id.size(), es, !factored, factored, f);
-	if (!e && factored && (size_t)f.nflush * es << (nb + 1) > (256u << 20)) { f.built = false; return 0; }
+	int e = fit_build(t->L, std::min(nb, es == 16 ? (nb <= 13 ? 13 : 12) : 13), w.data(), ng, block.data(), (int)id.size(), es, !factored, factored, f, FIT_TABLES);
+	if (!e && !f.built) return 0;
 	if (!e) e = fit_set_gates<P>(g.data(), ng, block.data(), (int)id.size(), t->L, f.kt, w.data(), f);
-	if (e) { f.built = false; return e; }
-	if (!f.ok) { f.built = false; return 0; }
+	if (e || !f.ok)
+	{
+		f.release();
+		if (e == MG_ERR_ALLOC) { cudaGetLastError(); e = 0; }
+		return e;
+	}
 	int per = 0;
 	const int lim = (int)std::min<size_t>(mgcu_ctx()->smem_optin, 227 * 1024) - 4096;
 	MGCU_TRY(cudaFuncSetAttribute(fit_kernel<P>(f.qc, FIT_COLS, f.threads), cudaFuncAttributeMaxDynamicSharedMemorySize, lim));

@@ -332,3 +332,35 @@ def test_batch_created_with_gates_that_do_not_factor(mglib, prec):
         lib.set_precision(mgcu.PREC_FP64)
         for t in ts:
             lib.target_free(t)
+
+
+def _free_bytes(lib):
+    import ctypes
+    lib.lib.mgcu_device_free_bytes.restype = ctypes.c_double
+    return lib.lib.mgcu_device_free_bytes()
+
+
+@pytest.mark.parametrize("prec", [mgcu.PREC_FP64, mgcu.PREC_MIXED])
+def test_deep_target_keeps_no_tables(mglib, prec):
+    """a target whose factored tables would pass their limit (70 layers of 4 MB): the tiled sweep
+    runs, and what the target keeps once the plan is gone is its gate program, not the tables"""
+    lib, rng = mglib, np.random.default_rng(3)
+    L, ul = 18, 70
+    v, perms = T.haar_matchgates(1, rng), T.brickwall_perms(L, 1)
+    t = lib.target_brickwall(T.haar_matchgates(ul, rng), T.brickwall_perms(L, ul), L)
+    lib.set_precision(prec)
+    out = []
+    try:
+        before = _free_bytes(lib)
+        plan = lib.plan_brickwall(lib.mg_target_apply, t, v, perms, L, mgcu.EVAL_TARGET)
+        lib.lib.mg_plan_free(mgcu.P(plan))
+        assert before - _free_bytes(lib) < 64 << 20
+        for dense in (0, 1):
+            lib.set_option(mgcu.OPT_TARGET_DENSE, dense)
+            out.append(lib.brickwall_columns(lib.mg_target_apply, t, v, perms, L, 1000, 1003))
+        assert out[0][0] == 0 and out[1][0] == 0
+        assert out[0][1] == out[1][1] and np.array_equal(out[0][2], out[1][2])
+    finally:
+        lib.set_option(mgcu.OPT_TARGET_DENSE, 0)
+        lib.set_precision(mgcu.PREC_FP64)
+        lib.target_free(t)
