@@ -3160,7 +3160,7 @@ extern "C" mgcu_plan* mgcu_plan_create(const mgcu_plan_desc* d)
 	// the factored fitted circuit: gradients from L = 10 (whole evaluation, 5 layers: float-float
 	// 244 against 448 us, complex128 574 against 997 us; at L = 8 138 against 129 us and 263
 	// against 202 us, the tables and the few blocks cost more), f alone from L = 12 (L = 11: 318
-	// against 336 us), while the tables are small.  In FP32, where the factors' rounding is as large as
+	// against 336 us), while the tables stay within FIT_PLAN_TABLES.  In FP32, where the factors' rounding is as large as
 	// the sweep's, the blocks stay whole.  An explicit block size keeps them too
 	e = 0;
 	// (Hessians: one tile, L <= 14)
@@ -3174,16 +3174,16 @@ extern "C" mgcu_plan* mgcu_plan_create(const mgcu_plan_desc* d)
 		// against 87 ms in two 64 KB tiles), a larger one tiles of 64 KB (L=16, 5 layers, 6001
 		// columns: 81 ms against 87 ms in tiles of 128 KB, one block per SM)
 		if (opt_kt <= 0 && p->nb <= 13) p->fit.kt = p->nb;
-		e = fit_build(p->L, p->fit.kt, p->wires.data(), d->ngates, p->block.data(), d->nblocks, (int)p->tsize, d->want_hess != 0 || p->prec == MG_PREC_FP32_ID, p->prec != MG_PREC_FP32_ID, p->fit, SIZE_MAX, p->place);
+		e = fit_build(p->L, p->fit.kt, p->wires.data(), d->ngates, p->block.data(), d->nblocks, (int)p->tsize, d->want_hess != 0 || p->prec == MG_PREC_FP32_ID, p->prec != MG_PREC_FP32_ID, p->fit, FIT_PLAN_TABLES, p->place);
+		if (e) { delete p; return nullptr; }
+	}
+	if (p->fit.built)
+	{
 		int per = 0;
-		if (!e)
-		{
-			auto occ = [&](auto k) { return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, p->fit.threads, p->fit.smem) != cudaSuccess; };
-			const bool g = fit_grad;
-			const int mode = d->want_hess ? FIT_HESS : g ? FIT_GRAD : FIT_VALUE;
-			if (p->prec == MG_PREC_FP64_ID ? occ(fit_kernel<PrecD>(1, mode, p->fit.threads, p->fit.split)) : p->prec == MG_PREC_FP32_ID
-				? occ(fit_kernel<PrecF>(2, mode, p->fit.threads)) : occ(fit_kernel<PrecX>(1, mode, p->fit.threads, p->fit.split))) e = MG_ERR_DEVICE;
-		}
+		auto occ = [&](auto k) { return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, p->fit.threads, p->fit.smem) != cudaSuccess; };
+		const int mode = d->want_hess ? FIT_HESS : fit_grad ? FIT_GRAD : FIT_VALUE;
+		if (p->prec == MG_PREC_FP64_ID ? occ(fit_kernel<PrecD>(1, mode, p->fit.threads, p->fit.split)) : p->prec == MG_PREC_FP32_ID
+			? occ(fit_kernel<PrecF>(2, mode, p->fit.threads)) : occ(fit_kernel<PrecX>(1, mode, p->fit.threads, p->fit.split))) e = MG_ERR_DEVICE;
 		if (e) { delete p; return nullptr; }
 		if (opt_cps > 0) per = (int)std::min<long>(per, opt_cps);
 		if (d->want_hess)
@@ -3771,10 +3771,14 @@ static int batch_build(mgcu_batch* B, const mgcu_batch_inst* d, int tune)
 			{
 				const int kt = P::kId == MG_PREC_FP32_ID ? std::min(I.nb, 13) : I.nb <= 13 ? I.nb : 12;
 				ef = fit_build(I.L, kt, d[i].wires, d[i].ngates, d[i].block, d[i].nblocks, (int)sizeof(T), P::kId == MG_PREC_FP32_ID,
-					P::kId != MG_PREC_FP32_ID, I.fit, SIZE_MAX);
+					P::kId != MG_PREC_FP32_ID, I.fit, FIT_PLAN_TABLES);
+			}
+			if (ef) return ef;
+			if (I.fit.built)
+			{
 				int per = 0;
 				auto kern = fit_kernel<P>(P::kId == MG_PREC_FP32_ID ? 2 : 1, d[i].want_grad ? FIT_GRAD : FIT_VALUE, I.fit.threads);
-				if (!ef) MGCU_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, I.fit.threads, I.fit.smem));
+				MGCU_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, I.fit.threads, I.fit.smem));
 				I.fit.grid = (int)std::min<long>((long)c->nsm * std::max(per, 1), ((1L << I.L) + I.fit.nc - 1) / I.fit.nc);
 				const size_t slot = I.fit.group.size() * (I.fit.factored ? 1 : 2) * I.fit.nc * (size_t)I.S;
 				if (d[i].want_grad) fit_cache = std::max(fit_cache, slot * I.fit.grid);
@@ -3782,7 +3786,6 @@ static int batch_build(mgcu_batch* B, const mgcu_batch_inst* d, int tune)
 				fit_blocks = std::max(fit_blocks, I.nblocks);
 				I.wires.assign(d[i].wires, d[i].wires + 2 * d[i].ngates);
 			}
-			if (ef) return ef;
 		}
 		I.chunk = std::max(1L, std::min(1L << I.L, (long)((8ull << 30) / ((size_t)I.S * sizeof(T)))));
 		stage_bytes = std::max(stage_bytes, sizeof(T) * (size_t)I.S * (size_t)I.chunk);

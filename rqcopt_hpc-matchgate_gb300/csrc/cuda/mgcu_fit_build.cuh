@@ -1,8 +1,10 @@
 // Host side of the factored fitted circuit (mgcu_fit.cuh): groups, flushes, factors.
 // Included by mgcu_engine.cu.
 
-// most bytes of a program's tables before the final one (64 at 18 qubits, where one takes 4 MB)
-constexpr size_t FIT_TABLES = (size_t)256 << 20;
+// most bytes of a program's tables before the final one: of a target's, which live as long as the
+// target (64 tables at 18 qubits, where one takes 4 MB), and of a plan's or batch's, a quarter of
+// the room in which those stage target columns (512 at 18 qubits)
+constexpr size_t FIT_TABLES = (size_t)256 << 20, FIT_PLAN_TABLES = (size_t)2 << 30;
 
 // wires of gate g as a mask
 static unsigned fit_wires(const int* w, int g) { return (1u << w[2 * g]) | (1u << w[2 * g + 1]); }

@@ -364,3 +364,30 @@ def test_deep_target_keeps_no_tables(mglib, prec):
         lib.set_option(mgcu.OPT_TARGET_DENSE, 0)
         lib.set_precision(mgcu.PREC_FP64)
         lib.target_free(t)
+
+
+@pytest.mark.parametrize("prec", [mgcu.PREC_FP64, mgcu.PREC_MIXED])
+def test_deep_fit_plans_stay_small(mglib, prec):
+    """a fitted circuit whose factored tables would pass a plan's limit (600 layers of 4 MB): the
+    general kernels run, in about the memory that they take by themselves (MG_OPT_THREADS)"""
+    lib, rng = mglib, np.random.default_rng(4)
+    L, nl = 18, 600
+    v, perms = T.haar_matchgates(nl, rng), T.brickwall_perms(L, nl)
+    t = lib.target_brickwall(T.haar_matchgates(2, rng), T.brickwall_perms(L, 2), L)
+    lib.set_precision(prec)
+    used = []
+    try:
+        for threads in (256, 0, 256):   # (the first also makes what the target keeps)
+            lib.set_option(mgcu.OPT_THREADS, threads)
+            before = _free_bytes(lib)
+            plan = lib.plan_brickwall(lib.mg_target_apply, t, v, perms, L, mgcu.EVAL_TARGET)
+            used.append(before - _free_bytes(lib))
+            lib.lib.mg_plan_free(mgcu.P(plan))
+        assert abs(used[1] - used[2]) < 512 << 20
+        lib.set_option(mgcu.OPT_THREADS, 0)
+        _check([(rc, f, np.ones(1)) for rc, f, _ in _both(lib, lambda: lib.brickwall_columns(lib.mg_target_apply, t, v, perms, L, 7, 9, gradient=False), 0)],
+               TOL[prec])
+    finally:
+        lib.set_option(mgcu.OPT_THREADS, 0)
+        lib.set_precision(mgcu.PREC_FP64)
+        lib.target_free(t)
