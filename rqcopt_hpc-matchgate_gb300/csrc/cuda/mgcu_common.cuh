@@ -22,6 +22,7 @@ struct MgcuContext
 
 MgcuContext* mgcu_ctx();                 // initialises on first use; NULL on failure
 cudaStream_t mgcu_stream();              // the calling host thread's stream (default: the library's)
+int mgcu_upload(void* dst, const void* src, size_t n);   // src may be reused when it returns
 void mgcu_count_launch(long n = 1);
 int mgcu_check(cudaError_t e, const char* what, const char* file, int line);
 

@@ -1887,8 +1887,7 @@ struct Arena
 	{
 		const int e = b->alloc(host.size());
 		if (e) return e;
-		MGCU_TRY(cudaMemcpyAsync(b->p, host.data(), host.size(), cudaMemcpyHostToDevice, mgcu_stream()));
-		return 0;
+		return mgcu_upload(b->p, host.data(), host.size());
 	}
 };
 
@@ -2141,10 +2140,7 @@ static int upload_mats(const mgg* gates, int ng, DevBuf& buf)
 			h[(size_t)g * 8 + 4 + q] = P::make(gates[g].k[q].re, gates[g].k[q].im);
 		}
 	int e = buf.alloc(sizeof(T) * h.size());
-	if (e) return e;
-	// (from pageable memory: the copy has left h when the call returns)
-	MGCU_TRY(cudaMemcpyAsync(buf.p, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice, mgcu_stream()));
-	return 0;
+	return e ? e : mgcu_upload(buf.p, h.data(), sizeof(T) * h.size());
 }
 
 // the 2x2 block inverses of the gates (k_columns_adj); 1 when every block is invertible with
@@ -2578,8 +2574,8 @@ static int launch_sector(mgcu_plan* p, TargetProg& tp, long b0, long b1, typenam
 		}
 		p->sec_b0 = -1;
 		int e = p->sec_items.alloc(sizeof(SecItem) * std::max<size_t>(sp.sec.size(), 1));
+		if (!e) e = mgcu_upload(p->sec_items.p, items.data(), sizeof(SecItem) * items.size());
 		if (e) return e;
-		MGCU_TRY(cudaMemcpyAsync(p->sec_items.p, items.data(), sizeof(SecItem) * items.size(), cudaMemcpyHostToDevice, st));
 		p->sec_nitems = (int)items.size(); p->sec_grid = grid;
 		p->sec_b0 = b0; p->sec_b1 = b1;
 	}
@@ -2702,7 +2698,8 @@ static int launch_ws(mgcu_plan* p, long b0, long b1, const typename P::T* dense,
 		sec.push_back(s);
 	}
 	if ((size_t)groups * w.nlev * ((size_t)w.dmax << w.ln) * sizeof(T) > std::min(p->cache.n, p->dcache.n)) return 0;
-	MGCU_TRY(cudaMemcpyAsync(w.d_sec.p, sec.data(), sizeof(WsSec) * sec.size(), cudaMemcpyHostToDevice, st));
+	const int eu = mgcu_upload(w.d_sec.p, sec.data(), sizeof(WsSec) * sec.size());
+	if (eu) return eu;
 	WsArgs<P> a;
 	memset(&a, 0, sizeof(a));
 	a.L = p->L; a.nlev = w.nlev; a.ngates = p->d.ngates; a.ln = w.ln; a.dmax = w.dmax; a.nsec = (int)sec.size(); a.ngroups = groups;
@@ -3298,6 +3295,7 @@ static int plan_columns_t(mgcu_plan* p, long b0, long b1, const mgc* host_cols)
 		if (!t)
 		{
 			MGCU_TRY(cudaMemcpyAsync(p->cols64.p, host_cols + (size_t)(c0 - b0) * p->S, sizeof(double2) * n, cudaMemcpyHostToDevice, mgcu_stream()));
+			MGCU_TRY(cudaStreamSynchronize(mgcu_stream()));   // the caller fills host_cols again while the kernels below run
 			k_convert<P><<<grid_cap(n, 256), 256, 0, mgcu_stream()>>>(p->cols64.as<double2>(), n, p->cols.as<T>());
 			MGCU_LAUNCHED();
 			dense = p->cols.as<T>();
@@ -4056,7 +4054,8 @@ extern "C" int mgcu_batch_set_gates(mgcu_batch* B, int i, const mgg* gates)
 	const int now = I.fit.ok;
 	if (now != I.skip)
 	{
-		MGCU_TRY(cudaMemcpyAsync(B->skip.as<int>() + i, &now, sizeof(int), cudaMemcpyHostToDevice, mgcu_stream()));
+		const int eu = mgcu_upload(B->skip.as<int>() + i, &now, sizeof(int));
+		if (eu) return eu;
 		I.skip = now;
 	}
 	return e;

@@ -3,7 +3,10 @@
 #include "mgcu_common.cuh"
 
 #include <atomic>
+#include <map>
+#include <memory>
 #include <stdlib.h>
+#include <string.h>
 
 static MgcuContext g_ctx;
 static int g_ctx_state = 0;   // 0 uninitialised, 1 ready, -1 failed
@@ -81,9 +84,62 @@ extern "C" int mgcu_stream_sync(void)
 	return 0;
 }
 
+// Uploads on the calling thread's stream from host memory that its owner frees or rewrites as
+// soon as the call returns (gates, tables).  An asynchronous copy from pageable memory may read
+// it later -- a GPU that reaches pageable memory need not stage the copy -- so the bytes are
+// kept in the stream's ring until its half is used again, after the event recorded when the
+// half was full.  One event per half: one after every copy held the next kernel up by 3 us (L=4
+// gradient 117 us, 114 us without).  Larger arrays wait for their copy.  Callers hold the library lock.
+namespace {
+struct UploadRing
+{
+	static constexpr size_t HALF = 512 << 10;
+	std::unique_ptr<char[]> p;
+	cudaEvent_t ev[2] = {};
+	int half = 0;
+	size_t used = 0;
+	~UploadRing() { for (cudaEvent_t e : ev) if (e) cudaEventDestroy(e); }
+};
+std::map<cudaStream_t, UploadRing> g_up;
+}  // namespace
+
+int mgcu_upload(void* dst, const void* src, size_t n)
+{
+	cudaStream_t st = mgcu_stream();
+	if (n > UploadRing::HALF)
+	{
+		MGCU_TRY(cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, st));
+		MGCU_TRY(cudaStreamSynchronize(st));
+		return 0;
+	}
+	UploadRing& r = g_up[st];
+	if (!r.p)
+	{
+		for (cudaEvent_t& e : r.ev) if (!e) MGCU_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+		r.p.reset(new char[2 * UploadRing::HALF]);
+	}
+	if (r.used + n > UploadRing::HALF)
+	{
+		MGCU_TRY(cudaEventRecord(r.ev[r.half], st));
+		MGCU_TRY(cudaEventSynchronize(r.ev[r.half ^ 1]));
+		r.half ^= 1;
+		r.used = 0;
+	}
+	char* s = r.p.get() + UploadRing::HALF * r.half + r.used;
+	memcpy(s, src, n);
+	r.used += (n + 63) & ~(size_t)63;
+	MGCU_TRY(cudaMemcpyAsync(dst, s, n, cudaMemcpyHostToDevice, st));
+	return 0;
+}
+
 extern "C" void mgcu_stream_destroy(void* s)
 {
-	if (s) cudaStreamDestroy((cudaStream_t)s);
+	if (!s) return;
+	mgcu_lock();
+	cudaStreamSynchronize((cudaStream_t)s);
+	g_up.erase((cudaStream_t)s);
+	cudaStreamDestroy((cudaStream_t)s);
+	mgcu_unlock();
 }
 
 void mgcu_count_launch(long n) { g_launches += n; }

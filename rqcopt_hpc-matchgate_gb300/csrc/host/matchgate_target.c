@@ -412,8 +412,8 @@ static int run_eval(linear_func ufunc, void* udata, const eval_req* q)
 		else
 		{
 			/* chunks of at most 1/8 of the range (at least 1024 columns): the caller's map fills
-			 * chunk k + 1 on the host threads while the GPU works on chunk k (the copy of a
-			 * chunk from this pageable buffer completes before its call returns) */
+			 * chunk k + 1 on the host threads while the GPU works on chunk k (mgcu_plan_columns
+			 * waits for its copy from this buffer, not for the kernels) */
 			long chunk = mgcu_plan_chunk_columns(p);
 			const long part = (b1 - b0 + 7) / 8 > 1024 ? (b1 - b0 + 7) / 8 : 1024;
 			if (chunk > part) chunk = part;

@@ -391,3 +391,31 @@ def test_deep_fit_plans_stay_small(mglib, prec):
         lib.set_option(mgcu.OPT_THREADS, 0)
         lib.set_precision(mgcu.PREC_FP64)
         lib.target_free(t)
+
+
+@pytest.mark.parametrize("prec", [mgcu.PREC_FP64, mgcu.PREC_MIXED, mgcu.PREC_FP32])
+@pytest.mark.parametrize("nl,updates", [(3, 400), (140, 12)])
+def test_updates_queued_without_waiting(mglib, prec, nl, updates):
+    """gates set and runs queued one after the other, with no result read in between (many small
+    uploads, and uploads of 700 gates, past 64 KB): the results are the last gates', bit for bit
+    those of a plan that had them from the start"""
+    lib, rng = mglib, np.random.default_rng(6)
+    L = 10
+    perms = T.brickwall_perms(L, nl)
+    t = lib.target_brickwall(T.haar_matchgates(4, rng), T.brickwall_perms(L, 4), L)
+    vs = [np.ascontiguousarray(T.haar_matchgates(nl, rng)) for _ in range(updates)]
+    lib.set_precision(prec)
+    out = []
+    try:
+        for first, rest in ((vs[-1], []), (vs[0], vs[1:])):
+            plan = lib.plan_brickwall(lib.mg_target_apply, t, first, perms, L, mgcu.EVAL_GRADIENT)
+            assert lib.lib.mg_plan_run(mgcu.P(plan)) == 0
+            for v in rest:
+                assert lib.lib.mg_plan_set_gates(mgcu.P(plan), v.ctypes.data_as(mgcu.P)) == 0
+                assert lib.lib.mg_plan_run(mgcu.P(plan)) == 0
+            out.append(lib.plan_results(plan, nl, grad=True))
+            lib.lib.mg_plan_free(mgcu.P(plan))
+    finally:
+        lib.set_precision(mgcu.PREC_FP64)
+        lib.target_free(t)
+    assert out[0][0] == out[1][0] and np.array_equal(out[0][1], out[1][1])
