@@ -2220,6 +2220,8 @@ static int build_target_prog(mgcu_target* t, int kt, int threads, TargetProg& tp
 	{
 		typedef typename P::T T;
 		prepare_sweep(t);
+		// another thread's stream may still be sweeping with the program that this one replaces
+		if (tp.mats.p) MGCU_TRY(cudaDeviceSynchronize());
 		const std::vector<mgg>& gates = t->sg;
 		schedule(t->L, kt, t->sw.data(), (int)gates.size(), true, tp.sched, sizeof(T) >= 16 ? 1 : 2, t->smask.data());
 		// distinct matrices, then passes split so that each stages at most MAXPM of them
@@ -2357,8 +2359,8 @@ static int build_target_prog(mgcu_target* t, int kt, int threads, TargetProg& tp
 			tp.wcons = tp.wcons && (kk == BK_ID || kk == BK_D1 || kk == BK_NEG1 || kk == BK_DIAG);
 		}
 		e = tp.tg.alloc(sizeof(TGate) * tg.size());
+		if (!e) e = mgcu_upload(tp.tg.p, tg.data(), sizeof(TGate) * tg.size());
 		if (e) return e;
-		MGCU_TRY(cudaMemcpy(tp.tg.p, tg.data(), sizeof(TGate) * tg.size(), cudaMemcpyHostToDevice));
 		// staged matrices: the classified entries of each slot's first gate
 		std::vector<T> hm(std::max<size_t>(pm_first.size(), 1) * 8);
 		for (size_t i = 0; i < pm_first.size(); i++)
@@ -2375,9 +2377,10 @@ static int build_target_prog(mgcu_target* t, int kt, int threads, TargetProg& tp
 		}
 		e = tp.pmats.alloc(sizeof(T) * hm.size());
 		if (!e) e = tp.pm.alloc(sizeof(int2) * std::max<size_t>(pmh.size(), 1));
+		if (!e) e = mgcu_upload(tp.pmats.p, hm.data(), sizeof(T) * hm.size());
+		if (!e) e = mgcu_upload(tp.pm.p, pmh.data(), sizeof(int2) * pmh.size());
 		if (e) return e;
-		MGCU_TRY(cudaMemcpy(tp.pmats.p, hm.data(), sizeof(T) * hm.size(), cudaMemcpyHostToDevice));
-		MGCU_TRY(cudaMemcpy(tp.pm.p, pmh.data(), sizeof(int2) * pmh.size(), cudaMemcpyHostToDevice));
+		MGCU_TRY(cudaStreamSynchronize(mgcu_stream()));   // kept on the target: other threads' streams use them too
 		tp.kw = kw;
 		tp.sector.state = -1;
 		tp.fit.built = tp.fit.tried = false;
@@ -2429,7 +2432,8 @@ extern "C" mgcu_target* mgcu_target_dense(const mgc* U, int L)
 	t->L = L; t->kind = 1;
 	const size_t n = (size_t)1 << L;
 	if (t->dense.alloc(sizeof(double2) * n * n)) { delete t; return nullptr; }
-	if (cudaMemcpy(t->dense.p, U, sizeof(double2) * n * n, cudaMemcpyHostToDevice) != cudaSuccess)
+	if (cudaMemcpyAsync(t->dense.p, U, sizeof(double2) * n * n, cudaMemcpyHostToDevice, mgcu_stream()) != cudaSuccess
+		|| cudaStreamSynchronize(mgcu_stream()) != cudaSuccess)
 	{
 		mg_set_error("copying a dense target to the GPU failed");
 		delete t;
@@ -3724,8 +3728,8 @@ static int batch_build(mgcu_batch* B, const mgcu_batch_inst* d, int tune)
 		if (!e) e = I.d_block.alloc(sizeof(int) * std::max(D.ngates, 1));
 		if (!e) e = I.out_f.alloc(sizeof(double) * 2);
 		if (!e) e = I.out_blk.alloc(sizeof(double) * 16 * std::max(D.nblocks, 1));
+		if (!e) e = mgcu_upload(I.d_block.p, D.block, sizeof(int) * D.ngates);
 		if (e) return e;
-		MGCU_TRY(cudaMemcpy(I.d_block.p, D.block, sizeof(int) * D.ngates, cudaMemcpyHostToDevice));
 		I.col_cost = (double)I.S * ((double)mgcu_target_sweep_gates(D.target) + 3.0 * D.ngates);
 		B->smem = std::max(B->smem, std::max(I.smem_t, I.smem_c));
 		B->slot_stride = std::max(B->slot_stride, I.S);
@@ -3861,8 +3865,8 @@ static int batch_build(mgcu_batch* B, const mgcu_batch_inst* d, int tune)
 	if (!e) e = B->args_t.alloc(sizeof(Args<P>) * B->n);
 	if (!e) e = B->args_c.alloc(sizeof(Args<P>) * B->n);
 	if (!e) e = B->red.alloc(sizeof(BatchRed) * B->n);
+	if (!e) e = mgcu_upload(B->items.p, items.data(), sizeof(BatchItem) * items.size());
 	if (e) return e;
-	MGCU_TRY(cudaMemcpy(B->items.p, items.data(), sizeof(BatchItem) * items.size(), cudaMemcpyHostToDevice));
 	std::vector<Args<P>> at(B->n), ac(B->n);
 	std::vector<BatchRed> rd(B->n);
 	double* parts = B->parts.as<double>();
@@ -3885,12 +3889,13 @@ static int batch_build(mgcu_batch* B, const mgcu_batch_inst* d, int tune)
 		r.out_f = I.out_f.as<double>(); r.out_blk = I.out_blk.as<double>();
 		r.nslots = I.nslots; r.ngates = I.ngates; r.nblocks = I.nblocks;
 	}
-	MGCU_TRY(cudaMemcpy(B->args_t.p, at.data(), sizeof(Args<P>) * B->n, cudaMemcpyHostToDevice));
-	MGCU_TRY(cudaMemcpy(B->args_c.p, ac.data(), sizeof(Args<P>) * B->n, cudaMemcpyHostToDevice));
+	if (!e) e = mgcu_upload(B->args_t.p, at.data(), sizeof(Args<P>) * B->n);
+	if (!e) e = mgcu_upload(B->args_c.p, ac.data(), sizeof(Args<P>) * B->n);
+	if (!e) e = mgcu_upload(B->red.p, rd.data(), sizeof(BatchRed) * B->n);
+	if (e) return e;
 	B->host_args.resize(sizeof(Args<P>) * 2 * B->n);
 	memcpy(B->host_args.data(), at.data(), sizeof(Args<P>) * B->n);
 	memcpy(B->host_args.data() + sizeof(Args<P>) * B->n, ac.data(), sizeof(Args<P>) * B->n);
-	MGCU_TRY(cudaMemcpy(B->red.p, rd.data(), sizeof(BatchRed) * B->n, cudaMemcpyHostToDevice));
 	if (B->skip.alloc(sizeof(int) * B->n)) return MG_ERR_ALLOC;
 	MGCU_TRY(cudaMemsetAsync(B->skip.p, 0, sizeof(int) * B->n, mgcu_stream()));   // in order with mgcu_batch_set_gates' uploads
 	return 0;

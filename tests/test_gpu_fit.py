@@ -419,3 +419,73 @@ def test_updates_queued_without_waiting(mglib, prec, nl, updates):
         lib.set_precision(mgcu.PREC_FP64)
         lib.target_free(t)
     assert out[0][0] == out[1][0] and np.array_equal(out[0][1], out[1][1])
+
+
+def _on_own_stream(lib, work):
+    """work() on a host thread with a stream of its own, as the request server's plan lane has"""
+    import ctypes
+    import threading
+    L = lib.lib
+    L.mgcu_stream_create.restype = ctypes.c_void_p
+    err = []
+
+    def body():
+        s = L.mgcu_stream_create()
+        L.mgcu_stream_set(ctypes.c_void_p(s))
+        try:
+            work()
+            assert L.mgcu_stream_sync() == 0
+        except BaseException as x:   # handed to the caller's thread
+            err.append(x)
+        finally:
+            L.mgcu_stream_set(None)
+            L.mgcu_stream_destroy(ctypes.c_void_p(s))
+    th = threading.Thread(target=body)
+    th.start()
+    return th, err
+
+
+def _two_streams(lib, prec, L, conserving, resident, rounds=12):
+    """two plans of one target whose sweeps differ in tile size, so that each replaces the other's
+    gate program, run by two threads on two streams without waiting for results in between"""
+    rng = np.random.default_rng(L)
+    ul = T.brickwall_perms(L, 6)
+    u = T.haar_matchgates(6, rng)
+    if conserving:
+        u[:, 4:] = [1, 0, 0, np.exp(0.3j)]
+    v, perms = T.haar_matchgates(3, rng), T.brickwall_perms(L, 3)
+    t = lib.target_brickwall(u, ul, L)
+    lib.set_precision(prec)
+    plans, want, got = [], [], [[], []]
+    try:
+        assert lib.target_set_resident(t, resident) == 0
+        for bits in (0, 7):
+            lib.set_option(mgcu.OPT_TARGET_TILE_BITS, bits)
+            plans.append(lib.plan_brickwall(lib.mg_target_apply, t, v, perms, L, mgcu.EVAL_GRADIENT))
+            assert lib.lib.mg_plan_run(mgcu.P(plans[-1])) == 0
+            want.append(lib.plan_results(plans[-1], 3, grad=True))
+
+        def runs(i):
+            for _ in range(rounds):
+                for _ in range(3):
+                    assert lib.lib.mg_plan_run(mgcu.P(plans[i])) == 0
+                got[i].append(lib.plan_results(plans[i], 3, grad=True))
+        th, err = _on_own_stream(lib, lambda: runs(1))
+        runs(0)
+        th.join()
+        assert not err, err
+    finally:
+        lib.set_option(mgcu.OPT_TARGET_TILE_BITS, 0)
+        lib.set_precision(mgcu.PREC_FP64)
+        for plan in plans:
+            lib.lib.mg_plan_free(mgcu.P(plan))
+        lib.target_free(t)
+    for i in range(2):
+        for f, dv, *_ in got[i]:
+            assert f == want[i][0] and np.array_equal(dv, want[i][1])
+
+
+@pytest.mark.parametrize("prec", [mgcu.PREC_FP64, mgcu.PREC_MIXED, mgcu.PREC_FP32])
+@pytest.mark.parametrize("conserving", [False, True])
+def test_two_streams_share_a_target(mglib, prec, conserving):
+    _two_streams(mglib, prec, 12, conserving, False)
