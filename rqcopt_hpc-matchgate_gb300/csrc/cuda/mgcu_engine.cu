@@ -3319,10 +3319,14 @@ static int plan_columns_t(mgcu_plan* p, long b0, long b1, const mgc* host_cols)
 			if (!t->res_valid[id] || t->res_key[id] != key)
 			{
 				const long N = 1L << p->L;
+				// the columns are every stream's: the ones that still read the old ones end first,
+				// and no other starts on the new ones before they are made
+				if (t->res_valid[id]) MGCU_TRY(cudaDeviceSynchronize());
+				t->res_valid[id] = false;
 				int e = t->res_cols[id].alloc((size_t)N * p->S * sizeof(T));
+				if (!e) e = launch_target<P>(p, 0, N, t->res_cols[id].as<T>());
 				if (e) return e;
-				e = launch_target<P>(p, 0, N, t->res_cols[id].as<T>());
-				if (e) return e;
+				MGCU_TRY(cudaStreamSynchronize(mgcu_stream()));
 				t->res_valid[id] = true; t->res_key[id] = key;
 			}
 			dense = t->res_cols[id].as<T>();

@@ -489,3 +489,9 @@ def _two_streams(lib, prec, L, conserving, resident, rounds=12):
 @pytest.mark.parametrize("conserving", [False, True])
 def test_two_streams_share_a_target(mglib, prec, conserving):
     _two_streams(mglib, prec, 12, conserving, False)
+
+
+@pytest.mark.parametrize("prec", [mgcu.PREC_FP64, mgcu.PREC_MIXED])
+def test_two_streams_share_resident_columns(mglib, prec):
+    """the same with the target's columns resident: each plan's sweep replaces the other's columns"""
+    _two_streams(mglib, prec, 12, False, True)
