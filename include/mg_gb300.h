@@ -291,6 +291,9 @@ int mg_plan_target_kernel_ms(mg_plan* plan, double* ms, long* launches);
  * MG_OPT_TARGET_TUNE chose them); cfg[3] live quartets per thread and iteration
  * (weight-restricted) or basis columns per block (every amplitude). */
 int mg_plan_target_config(const mg_plan* plan, int cfg[4]);
+/* The kernel of that sweep: "k_sector" (whole columns in shared memory), "k_fit" (factored),
+ * "k_target_w" or "k_target" (tiled, weight-restricted or not); "" without a GPU sweep. */
+const char* mg_plan_target_kernel(const mg_plan* plan);
 /* Number of kernels this library has launched since it was loaded. */
 long mg_launch_count(void);
 /* Peak FP32 FMA rate of this GPU, measured by a dependent-FMA kernel of this library

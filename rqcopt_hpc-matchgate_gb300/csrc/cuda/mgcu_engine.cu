@@ -3513,7 +3513,13 @@ extern "C" void mgcu_plan_target_config(const mgcu_plan* p, int* cfg)
 	}
 }
 
-// k_target launches of the last mgcu_plan_time_ms: their number and summed duration
+extern "C" const char* mgcu_plan_target_kernel(const mgcu_plan* p)
+{
+	if (!p->d.target || p->d.target->kind != 0) return "";
+	return p->sec ? "k_sector" : p->tfit ? "k_fit" : p->w_t ? "k_target_w" : "k_target";
+}
+
+// target sweep launches of the last mgcu_plan_time_ms: their number and summed duration
 extern "C" int mgcu_plan_target_kernel_ms(mgcu_plan* p, double* ms, long* launches)
 {
 	double t = 0;

@@ -774,6 +774,11 @@ int mg_plan_target_config(const mg_plan* pl, int cfg[4])
 	return 0;
 }
 
+const char* mg_plan_target_kernel(const mg_plan* pl)
+{
+	return pl ? mgcu_plan_target_kernel(pl->p) : "";
+}
+
 /* ======================================================================================
  * batches
  * ====================================================================================== */

@@ -145,6 +145,7 @@ int mgcu_batch_info(const mgcu_batch* b, int i, int* target_tile_bits, int* targ
 double mgcu_batch_time_ms(mgcu_batch* b, int steps, int flush_l2);
 int mgcu_plan_target_kernel_ms(mgcu_plan* p, double* ms, long* launches);
 void mgcu_plan_target_config(const mgcu_plan* p, int* cfg);
+const char* mgcu_plan_target_kernel(const mgcu_plan* p);
 
 /* ---- FP64 algebra on the GPU ---- */
 int mgcu_retract(const mgg* u, const double* eta, int n, mgg* v);

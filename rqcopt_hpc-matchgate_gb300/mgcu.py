@@ -161,6 +161,8 @@ class MatchgateLib:
             L.mg_plan_time_ms.restype = C.c_double
             L.mg_plan_target_kernel_ms.argtypes = [P, P, P]
             L.mg_plan_target_config.argtypes = [P, P]
+            L.mg_plan_target_kernel.argtypes = [P]
+            L.mg_plan_target_kernel.restype = C.c_char_p
             L.mg_launch_count.restype = C.c_long
             L.mg_get_option.restype = C.c_long
             L.mg_set_option.argtypes = [C.c_int, C.c_long]
@@ -192,6 +194,10 @@ class MatchgateLib:
         if rc != 0:
             raise RuntimeError(self.last_error())
         return {"kind": cfg[0], "tile_bits": cfg[1], "threads": cfg[2], "per_thread": cfg[3]}
+
+    def plan_target_kernel(self, plan):
+        """the kernel of the plan's target sweep ("" without one on the GPU)"""
+        return self.lib.mg_plan_target_kernel(P(plan)).decode()
 
     def plan_target_kernel_ms(self, plan):
         """(summed ms, launches) of the target-sweep kernel in the last plan timing"""
