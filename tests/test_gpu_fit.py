@@ -495,3 +495,51 @@ def test_two_streams_share_a_target(mglib, prec, conserving):
 def test_two_streams_share_resident_columns(mglib, prec):
     """the same with the target's columns resident: each plan's sweep replaces the other's columns"""
     _two_streams(mglib, prec, 12, False, True)
+
+
+@pytest.mark.parametrize("prec", [mgcu.PREC_FP64, mgcu.PREC_MIXED, mgcu.PREC_FP32])
+def test_largest_brickwall(mglib, oracle, prec):
+    """18 qubits, the largest size of the factored kernels: columns of the target and gradient of the
+    fit by k_fit in several passes, against the oracle and the general kernels on a few columns"""
+    lib, rng = mglib, np.random.default_rng(18)
+    L, nl, ul = 18, 3, 4
+    u, up = T.haar_matchgates(ul, rng), T.brickwall_perms(L, ul)
+    v, perms = _layers("scaled", nl, rng), T.brickwall_perms(L, nl)
+    t = lib.target_brickwall(u, up, L)
+    lib.set_precision(prec)
+    try:
+        plan = lib.plan_brickwall(lib.mg_target_apply, t, v, perms, L, mgcu.EVAL_TARGET)
+        assert lib.plan_target_kernel(plan) == "k_fit"
+        lib.lib.mg_plan_free(mgcu.P(plan))
+        for cols in ((0, 3), (200001, 200004)):
+            out = _both(lib, lambda: lib.brickwall_columns(lib.mg_target_apply, t, v, perms, L, *cols), 0)
+            _check(out, TOL[prec])
+            f_o, dv_o = oracle.brickwall_target_and_gradient(oracle.Target("brickwall", L, ulist=u, uperms=up), v, perms, L, col_range=cols)
+            _check([out[0], (0, f_o, dv_o)], TOL[prec])
+    finally:
+        lib.set_precision(mgcu.PREC_FP64)
+        lib.target_free(t)
+
+
+@pytest.mark.parametrize("prec", [mgcu.PREC_FP64, mgcu.PREC_MIXED, mgcu.PREC_FP32])
+def test_largest_odd_circuit(mglib, prec):
+    """17 qubits, whole trace: k_fit's columns and gradient against the full sweep and the general kernels"""
+    lib, rng = mglib, np.random.default_rng(17)
+    L, ng = 17, 5
+    pairs = lambda n: np.array([rng.choice(L, 2, replace=False) for _ in range(n)], np.int32)   # noqa: E731
+    w = pairs(ng)
+    w[0] = (L - 1, 3)
+    g, t = T.haar_matchgates(ng, rng), lib.target_circuit(T.haar_matchgates(4, rng), pairs(4), L)
+    lib.set_precision(prec)
+    out = []
+    try:
+        for dense, threads in ((0, 0), (1, 256)):
+            lib.set_option(mgcu.OPT_TARGET_DENSE, dense)
+            lib.set_option(mgcu.OPT_THREADS, threads)
+            out.append(lib.circuit_target_and_gradient(lib.mg_target_apply, t, g, w, L))
+        _check(out, TOL[prec])
+    finally:
+        lib.set_option(mgcu.OPT_TARGET_DENSE, 0)
+        lib.set_option(mgcu.OPT_THREADS, 0)
+        lib.set_precision(mgcu.PREC_FP64)
+        lib.target_free(t)
