@@ -63,9 +63,9 @@ __global__ void k_mirror_real(int m, double* __restrict__ H)
 	}
 }
 
-// ---- retraction (reference src/matchgate.c:548-562) ----
-// two threads per gate, one per 2x2 block: mgg_retract with its Newton iteration's inverses and
-// divisions, a serial chain of FP64 latencies (150 us with one thread per gate), side by side;
+// ---- retraction: v = polar(u (I + A(eta))) (reference src/matchgate.c:548-562) ----
+// two threads per gate, one per 2x2 block: mgg_polar's Newton iteration, whose inverses and
+// divisions are a serial chain of FP64 latencies (150 us with one thread per gate), side by side;
 // both blocks stop together, as there
 __global__ void k_retract(const mgg* __restrict__ u, const double* __restrict__ eta, int n, mgg* __restrict__ v)
 {

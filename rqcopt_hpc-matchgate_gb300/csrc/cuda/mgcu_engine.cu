@@ -1905,7 +1905,6 @@ struct SectorProg
 	DevBuf fixed;
 };
 
-// a fitted circuit's or target's program for k_fit (see mgcu_fit_build.cuh)
 // a particle-conserving fit's levels and sectors for k_ws_grad / k_ws_hess
 struct WsProg
 {
@@ -1921,6 +1920,7 @@ struct WsProg
 	DevBuf fixed, values, d_tab, d_sec;
 };
 
+// a fitted circuit's or target's program for k_fit (see mgcu_fit_build.cuh)
 struct FitProg
 {
 	bool factored = true;
@@ -3354,9 +3354,7 @@ extern "C" int mgcu_plan_columns(mgcu_plan* p, long b0, long b1, const mgc* host
 
 extern "C" int mgcu_plan_finish(mgcu_plan* p)
 {
-	MgcuContext* c = mgcu_ctx();
 	cudaStream_t st = mgcu_stream();
-	const int ng = std::max(p->d.ngates, 1);
 	if (p->fit.ok && (p->d.want_grad || p->d.want_hess))
 	{
 		k_fit_finish<<<p->d.nblocks, FIT_FIN * 16, 0, st>>>(p->part_g.as<double>(), p->rows_a, p->d.nblocks, p->fit.d_blk.as<FitBlock>(),
@@ -3395,18 +3393,6 @@ extern "C" int mgcu_plan_finish(mgcu_plan* p)
 		k_mirror<<<grid_cap(mdim * mdim, 256), 256, 0, st>>>(p->d.nblocks, p->out_h.as<double2>());
 		MGCU_LAUNCHED();
 	}
-	return 0;
-}
-
-extern "C" int mgcu_plan_fetch(mgcu_plan* p, mgc* f, mgg* dblocks, mgc* hess)
-{
-	cudaStream_t st = mgcu_stream();
-	if (f) MGCU_TRY(cudaMemcpyAsync(f, p->out_f.p, sizeof(double) * 2, cudaMemcpyDeviceToHost, st));
-	if (dblocks && (p->d.want_grad || p->d.want_hess))
-		MGCU_TRY(cudaMemcpyAsync(dblocks, p->out_blk.p, sizeof(double) * 16 * p->d.nblocks, cudaMemcpyDeviceToHost, st));
-	if (hess && p->d.want_hess)
-		MGCU_TRY(cudaMemcpyAsync(hess, p->out_h.p, sizeof(double) * 2 * 64 * (size_t)p->d.nblocks * p->d.nblocks, cudaMemcpyDeviceToHost, st));
-	MGCU_TRY(cudaStreamSynchronize(st));
 	return 0;
 }
 

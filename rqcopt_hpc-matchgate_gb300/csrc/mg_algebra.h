@@ -246,16 +246,6 @@ MG_HD void mgg_polar(const mgg* a, mgg* u)
 	*u = cur;
 }
 
-/* v = polar(u (I + A(eta))) (src/matchgate.c:548-562) */
-MG_HD void mgg_retract(const mgg* u, const double* eta, mgg* v)
-{
-	mgg z, w;
-	mgg_real_to_antisymm(eta, &z);
-	z.k[0].re += 1; z.c[0].re += 1; z.c[3].re += 1; z.k[3].re += 1;
-	mgg_mul(u, &z, &w);
-	mgg_polar(&w, v);
-}
-
 /* One 8-column block of the real Riemannian Hessian (src/matchgate_target.c:910-961):
  * for layer pair (i, j) and unit tangent direction k at gate j, given the complex
  * Hessian blocks hij (8x8 row-major, rows x of layer i, columns y of layer j),

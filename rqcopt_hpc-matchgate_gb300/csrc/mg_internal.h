@@ -115,9 +115,8 @@ int mgcu_plan_begin(mgcu_plan* p);                              /* zero accumula
 int mgcu_plan_columns(mgcu_plan* p, long b0, long b1, const mgc* host_cols);
 /* final reductions on the GPU; outputs stay on the device */
 int mgcu_plan_finish(mgcu_plan* p);
-/* copy results: f, per-block gradients [nblocks], complex Hessian [(8 nblocks)^2] */
-int mgcu_plan_fetch(mgcu_plan* p, mgc* f, mgg* dblocks, mgc* hess);
-/* both at once: the copies of mgcu_plan_fetch and, with grad_vec or H, of the projection */
+/* copy results: f, per-block gradients [nblocks], complex Hessian [(8 nblocks)^2] and, with
+ * grad_vec [8 nblocks] or H [(8 nblocks)^2], their projection */
 int mgcu_plan_results(mgcu_plan* p, mgc* f, mgg* dblocks, mgc* hess, const mgg* vblocks, double* grad_vec, double* H);
 long mgcu_plan_chunk_columns(const mgcu_plan* p);
 double mgcu_plan_time_ms(mgcu_plan* p, long b0, long b1, int steps, int flush_l2);
