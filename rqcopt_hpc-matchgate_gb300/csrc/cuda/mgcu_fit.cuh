@@ -799,10 +799,11 @@ __global__ void __launch_bounds__(FIT_NT, FIT_NT == 512 ? 1 : FIT_NT == 256 ? 2 
 	}
 }
 
-// complex products in double-double, for the tables of complex128 (every entry correctly rounded
-// to a few 2^-100, so that the tables carry no common rounding error into all columns)
+// complex products in double-double, for the factors (on the host) and the tables of complex128
+// (every entry correctly rounded to a few 2^-100, so that the tables carry no common rounding
+// error into all columns)
 struct Dd { double h, l; };
-__device__ __forceinline__ Dd dd_add(Dd a, Dd b)
+__host__ __device__ __forceinline__ Dd dd_add(Dd a, Dd b)
 {
 	const double s = a.h + b.h, bb = s - a.h, e = (a.h - (s - bb)) + (b.h - bb) + (a.l + b.l);
 	Dd r;
@@ -810,7 +811,7 @@ __device__ __forceinline__ Dd dd_add(Dd a, Dd b)
 	r.l = e - (r.h - s);
 	return r;
 }
-__device__ __forceinline__ Dd dd_mul(Dd a, Dd b)
+__host__ __device__ __forceinline__ Dd dd_mul(Dd a, Dd b)
 {
 	const double p = a.h * b.h, e = fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h);
 	Dd r;
@@ -818,7 +819,7 @@ __device__ __forceinline__ Dd dd_mul(Dd a, Dd b)
 	r.l = e - (r.h - p);
 	return r;
 }
-__device__ __forceinline__ Dd dd_neg(Dd a) { a.h = -a.h; a.l = -a.l; return a; }
+__host__ __device__ __forceinline__ Dd dd_neg(Dd a) { a.h = -a.h; a.l = -a.l; return a; }
 
 // one diagonal factor: entry 2 bit_i + bit_j (bits si, sj of the full index), (re, im) as
 // double-double

@@ -190,41 +190,27 @@ static int fit_build(int L, int kt, const int* wires, int ng, const int* block, 
 	return 0;
 }
 
-// host double-double complex arithmetic for the factors
-struct Hdd { double h, l; };
-static Hdd hdd(double x) { return { x, 0 }; }
-static Hdd hadd(Hdd a, Hdd b)
-{
-	const double s = a.h + b.h, bb = s - a.h, e = (a.h - (s - bb)) + (b.h - bb) + (a.l + b.l);
-	const double r = s + e;
-	return { r, e - (r - s) };
-}
-static Hdd hneg(Hdd a) { return { -a.h, -a.l }; }
-static Hdd hmul(Hdd a, Hdd b)
-{
-	const double p = a.h * b.h, e = std::fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h);
-	const double r = p + e;
-	return { r, e - (r - p) };
-}
-static Hdd hdiv(Hdd a, Hdd b)
+// complex arithmetic in double-double for the factors
+static Dd hdd(double x) { return { x, 0 }; }
+static Dd hdiv(Dd a, Dd b)
 {
 	const double q = a.h / b.h;
-	const Hdd r = hadd(a, hneg(hmul(hdd(q), b)));
+	const Dd r = dd_add(a, dd_neg(dd_mul(hdd(q), b)));
 	const double q2 = r.h / b.h;
 	const double s = q + q2;
 	return { s, q2 - (s - q) };
 }
-struct Hcx { Hdd re, im; };
+struct Hcx { Dd re, im; };
 static Hcx hcx(mgc z) { return { hdd(z.re), hdd(z.im) }; }
 static Hcx cmul(Hcx a, Hcx b)
 {
-	return { hadd(hmul(a.re, b.re), hneg(hmul(a.im, b.im))), hadd(hmul(a.re, b.im), hmul(a.im, b.re)) };
+	return { dd_add(dd_mul(a.re, b.re), dd_neg(dd_mul(a.im, b.im))), dd_add(dd_mul(a.re, b.im), dd_mul(a.im, b.re)) };
 }
-static Hcx cscale(Hcx a, double s) { return { hmul(a.re, hdd(s)), hmul(a.im, hdd(s)) }; }
+static Hcx cscale(Hcx a, double s) { return { dd_mul(a.re, hdd(s)), dd_mul(a.im, hdd(s)) }; }
 static Hcx cdiv(Hcx a, Hcx b)
 {
-	const Hdd d = hadd(hmul(b.re, b.re), hmul(b.im, b.im));
-	const Hcx n = cmul(a, { b.re, hneg(b.im) });
+	const Dd d = dd_add(dd_mul(b.re, b.re), dd_mul(b.im, b.im));
+	const Hcx n = cmul(a, { b.re, dd_neg(b.im) });
 	return { hdiv(n.re, d), hdiv(n.im, d) };
 }
 
