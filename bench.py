@@ -393,23 +393,25 @@ def run_gb300(a):
 
     flops = alg_flops(L, gu, gw, ncols)
     achieved_step = flops / (ms_per_step / 1e3) / 1e12
-    # the target sweep's kernel, timed by CUDA events around each launch (the fitted circuit's, k_fit, is
-    # the rest of the step)
+    # the target sweep's kernel, timed by CUDA events around each launch; the rest of the step is the fitted
+    # circuit's kernel (and launches of microseconds)
     cols_per_launch = ncols * a.steps / tk_n
     gu_run = lib.lib.mg_target_sweep_gates(mgcu.P(target))   # gates the sweep applies (fermionic swaps relabelled away)
     # amplitude-columns the sweep visits per launch: the whole parity sector of every column, or
     # (particle-conserving target) the amplitudes with the column's numbers only: per spin,
-    # C(L, L/2)^2 over all 2^L columns, where such a sector fits in shared memory, else the
-    # column's Hamming weight, C(2L, L)
+    # C(L, L/2)^2 over all 2^L columns, where k_sector sweeps, else the column's Hamming weight, C(2L, L)
     weight = bool(lib.lib.mg_target_conserves_weight(mgcu.P(target)))
     sector_units = float(cols_per_launch) * (1 << (L - 1))
-    per_spin = L <= 18 and math.comb(L // 2, L // 4) ** 2 * (8 if a.precision == "fp32" else 16) <= 230400
+    kernel = lib.plan_target_kernel(plan)
+    per_spin = kernel == "k_sector"
     live_units = (float(math.comb(L, L // 2) ** 2 if per_spin else math.comb(2 * L, L)) * cols_per_launch / ncols
                   if weight else sector_units)
     tk_avg_s = tk_ms / 1e3 / tk_n
     achieved = live_units * 14 * gu_run / tk_avg_s / 1e12
     bpc = TARGET_DRAM_BYTES_PER_COLUMN.get(L) if a.precision == "mixed" else None
-    traffic = bpc * cols_per_launch if bpc else None
+    traffic = bpc * cols_per_launch if bpc and per_spin else None
+    fit_s = (total_ms - tk_ms) / 1e3 / a.steps
+    fit_tflops = float(ncols) * (1 << (L - 1)) * (44 * gw + 8) / fit_s / 1e12
     out = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": a.steps, "warmup": a.warmup,
         "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
@@ -424,15 +426,14 @@ def run_gb300(a):
                 "timer": "host clock around matchgate_brickwall_unitary_target_and_projected_gradient (synchronous C call)"},
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": fp32_peak / 1e3, "unit": "TFLOP/s",
                      "frac": achieved / (fp32_peak / 1e3), "traffic": traffic,
-                     "kernel": "k_sector (target sweep)" if weight and per_spin else "target sweep", "kernel_launches": tk_n,
+                     "kernel": f"{kernel} (target sweep)", "kernel_launches": tk_n,
                      "kernel_config": lib.plan_target_config(plan),
                      "kernel_ms_per_launch": tk_avg_s * 1e3, "kernel_share_of_step": tk_ms / total_ms,
                      "columns_per_launch": cols_per_launch,
                      "achieved_is": "algorithmic complex-arithmetic flops of the target sweep (14 per visited "
                                     "amplitude and applied gate) per second of its kernel; the target conserves "
                                     "particle numbers, so the sweep visits the amplitudes with the column's numbers "
-                                    "(per spin C(L, L/2)^2 amplitude-columns per trace where such a sector fits in "
-                                    "shared memory, else C(2L, L)), not the 2^(2L-1) of the parity sectors" if weight else
+                                    "(per spin C(L, L/2)^2 amplitude-columns per trace by k_sector, else C(2L, L)), not the 2^(2L-1) of the parity sectors" if weight else
                                     "algorithmic complex-arithmetic flops of the target sweep (14 per parity-sector "
                                     "amplitude and applied gate) per second of its kernel",
                      "visited_amplitudes_per_launch": live_units,
@@ -441,10 +442,16 @@ def run_gb300(a):
                      "step_achieved": achieved_step,
                      "peak_source": "FP32 FMA microkernel of this library, measured in this run "
                                     "(MEASURED_PEAKS.json holds HBM and bf16 tensor peaks only)",
-                     "traffic_source": "the sweep's output columns, its only DRAM traffic (ncu: 0.7 MB read over 912 "
-                                       "columns)",
+                     "traffic_source": "computed: the bytes of the launch's output columns (not counted in this run; "
+                                       "ncu found 0.7 MB read in a launch over 912 columns)",
                      "fp64_peak_tflops": fp64_peak / 1e3,
                      "hbm": hbm_view(traffic, tk_avg_s)},
+        "roofline_fit": {"bound": "fp32", "achieved": fit_tflops, "peak": fp32_peak / 1e3, "unit": "TFLOP/s",
+                         "frac": fit_tflops / (fp32_peak / 1e3), "kernel": "k_fit (fitted circuit)",
+                         "ms_per_step": fit_s * 1e3, "share_of_step": 1 - tk_ms / total_ms,
+                         "achieved_is": "algorithmic complex-arithmetic flops of the fitted circuit (44 per parity-sector "
+                                        "amplitude and gate, 8 for the overlap) per second of the step less the target "
+                                        "sweep's launches; in factored form most of them are not executed"},
         "fp64_gpu": fp64,
         "accuracy": accuracy,
         "serving": serving,
