@@ -90,3 +90,30 @@ def test_sector_sweep_equals_full_sweep(mglib, case, prec):
     (rc0, f0, dv0), (rc1, f1, dv1) = out
     assert rc0 == 0 and rc1 == 0, lib.last_error()
     assert f0 == f1 and np.array_equal(dv0, dv1)
+
+
+@pytest.mark.parametrize("parts,prec", [(3, mgcu.PREC_FP64), (3, mgcu.PREC_MIXED), (3, mgcu.PREC_FP32), (2, mgcu.PREC_FP32)])
+def test_sector_sweep_at_18_qubits(mglib, parts, prec):
+    """the largest size of the sector sweep, with conserved numbers enough for its sectors to fit (8000
+    rows with three, 15 876 with two): the sector kernel runs and has the full sweep's bits"""
+    lib, rng = mglib, np.random.default_rng(parts)
+    L = 18
+    g, w = _circuit(L, 14, rng, [list(range(i, L, parts)) for i in range(parts)])
+    v, perms = T.haar_matchgates(2, rng), T.brickwall_perms(L, 2)
+    t = lib.target_circuit(g, w, L)
+    lib.set_precision(prec)
+    out = []
+    try:
+        plan = lib.plan_brickwall(lib.mg_target_apply, t, v, perms, L, mgcu.EVAL_TARGET)
+        assert lib.plan_target_kernel(plan) == "k_sector"
+        lib.lib.mg_plan_free(mgcu.P(plan))
+        for dense in (0, 1):
+            lib.set_option(mgcu.OPT_TARGET_DENSE, dense)
+            out.append(lib.brickwall_columns(lib.mg_target_apply, t, v, perms, L, 87000, 87013))
+    finally:
+        lib.set_option(mgcu.OPT_TARGET_DENSE, 0)
+        lib.set_precision(mgcu.PREC_FP64)
+        lib.target_free(t)
+    (rc0, f0, dv0), (rc1, f1, dv1) = out
+    assert rc0 == 0 and rc1 == 0, lib.last_error()
+    assert f0 == f1 and np.array_equal(dv0, dv1)
