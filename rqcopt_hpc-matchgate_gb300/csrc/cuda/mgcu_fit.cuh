@@ -655,8 +655,8 @@ __global__ void __launch_bounds__(FIT_NT, fit_blocks(P::kId, MODE, FIT_NT)) k_fi
 // 124 FP32 operations in float-float (176 unfactored) or 10.7 FP64 operations (16).  Measured
 // against k_hessian (which stays for FP32, several tiles and gates that do not factor):
 // translation-invariant L=12, 9 layers, float-float 152 -> 101 ms; per-layer L=12, 5 layers,
-// complex128 169 -> 128 ms (81 % of the FP64 rate); per-gate L=9, 19 gates, float-float
-// 3.97 -> 2.45 ms, 1.30 ms with the items in balanced order (item_grid).
+// complex128 169 -> 128 ms; per-gate L=9, 19 gates, float-float 3.97 -> 2.45 ms.  With the items
+// in balanced order (item_grid) the last two take 113 ms (FP64 pipe 95 % busy) and 1.30 ms.
 // ------------------------------------------------------------------------------------
 template <class P>
 struct FitHessArgs

@@ -28,7 +28,7 @@
 // complex128.  Measured against the tiled sweep that it replaces (k_target_w, which stays for
 // sectors too large for shared memory): L=16 spinful, 6001 columns, float-float 267 -> 27.6 ms;
 // L=14 spinful, whole trace, float-float 147 -> 16.6 ms; L=12 spinless (3606 gates), complex128
-// 101 -> 75 ms (64 % of the FP64 rate); L=12 spinful, complex128 18.2 -> 5.3 ms.  Reading each
+// 101 -> 75 ms (FP64 pipe 87 % busy); L=12 spinful, complex128 18.2 -> 5.3 ms.  Reading each
 // thread's first entries before the barrier, or one task list for pairs and rows, measured
 // slower (33.4 and 22.4 ms for the first two): the sweep is not bound by the entries' latency.
 
